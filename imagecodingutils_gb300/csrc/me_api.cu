@@ -246,8 +246,11 @@ int run(vppgpu_me* me, const short* d_src16, const short* d_ref16, const unsigne
         // GetBestVector's lambda: 0.9 (MultiresCrossVer2.cpp:1050), 1.1 (Multires.cpp:958)
         const bool v2 = me->kind == VPPGPU_ME_MULTIRES_CROSS_V2;
         VPP_CUDA(cudaMemsetAsync(me->changed, 0, sizeof(int) * (size_t)me->sweep_limit, ctx->stream));
-        if (v2 && v2_lambda)  // Estimate(long*, void* lambda) (MultiresCrossVer2.cpp:1162-1742)
-            return vppgpu::mrc2_launch(ctx, 4, me->mode, me->d_mrc, full_args(me, lambda), d_src16, d_ref16);
+        if (v2 && v2_lambda) {  // Estimate(long*, void* lambda) (MultiresCrossVer2.cpp:1162-1742)
+            vppgpu::FullArgs a = full_args(me, lambda);
+            a.grid_sweeps = a.relax_sweeps;  // an evaluation is a search: every sweep over the whole GPU
+            return vppgpu::mrc2_launch(ctx, 4, me->mode, me->d_mrc, a, d_src16, d_ref16);
+        }
         return vppgpu::mrc2_launch(ctx, v2 ? 1 : 2, me->mode, me->d_mrc, full_args(me, v2 ? 0.9 : 1.1), d_src16,
                                    d_ref16);
     }
@@ -428,13 +431,13 @@ int vppgpu_me_create(vppgpu_ctx* ctx, int kind, int width, int height, int motio
     me->sweep_limit = vppgpu::RELAX_SWEEPS + 2 + (me->nmb + 31) / 32;  // sweep counters, then the dirty bitmap
     if (searches_from_prediction(kind) && me->sweep_limit < 2 * vppgpu::UMHS_EVALS)  // change and search counts
         me->sweep_limit = 2 * vppgpu::UMHS_EVALS;
-    // Sweep policy by how the estimator's predictions settle on moving content
-    // (measured over 1080p pans): the full-search estimator mostly settles
-    // within 8 sweeps over every MB, a few more over the dirty sets; Multires
-    // keeps settling with more sweeps, cheaply over the dirty sets; Ver2
-    // rarely settles, so its wavefront starts early.
+    // One sweep over every MB on the whole GPU, then the cluster's rounds, which
+    // visit only what moves (1080p pans: 0, 1, 2 and 4 such sweeps give 442,
+    // 434, 433 and 434 us a Full estimate).  relax_sweeps bounds the sweeps of
+    // Ver2's Lagrangian overload and, for the others, tells only which rounds
+    // last_stats counts as relaxation.
     me->relax_sweeps = kind == VPPGPU_ME_MULTIRES_CROSS_V2 ? 4 : (searches_from_prediction(kind) ? 20 : vppgpu::RELAX_SWEEPS);
-    me->grid_sweeps = kind == VPPGPU_ME_MULTIRES ? 4 : (kind == VPPGPU_ME_MULTIRES_CROSS_V2 ? 4 : 8);
+    me->grid_sweeps = 1;
     me->relax_blocks_per_sm = 4;
     me->mrc_warps = 8;
     size_t npix = (size_t)width * height;
@@ -468,9 +471,7 @@ int vppgpu_me_create(vppgpu_ctx* ctx, int kind, int width, int height, int motio
             (rc = dalloc(&me->tie_list, me->nmb)) ||
             (rc = dalloc(&me->d_job, 1)) || (rc = dalloc(&me->spec, 5 * (size_t)me->nmb)) ||
             (rc = dalloc(&me->state, 3 * (size_t)me->nmb)) ||
-            (rc = dalloc(&me->cache, (size_t)me->nmb * vppgpu::KCACHE)) || (rc = dalloc(&me->dict, vppgpu::NDICT)) ||
-            (rc = dalloc(&me->d_wave_rec, vppgpu::wave_rec_count(me->cols, me->rows))) ||
-            (rc = dalloc(&me->d_wave_choice, me->nmb)) || (rc = dalloc(&me->changed, (size_t)me->sweep_limit)) ||
+            (rc = dalloc(&me->changed, (size_t)me->sweep_limit)) ||
             (rc = dalloc(&me->d_out_mv, me->nmb)) || (rc = dalloc(&me->d_out_dist, me->nmb)) ||
             (rc = dalloc(&me->d_out_avg, 1)) || (rc = dalloc(&me->d_incl, me->nmb)) ||
             (rc = dalloc(&me->d_slice, me->nmb)) || (rc = dalloc(&me->ctrl, 1))) {
@@ -567,9 +568,11 @@ int vppgpu_me_create(vppgpu_ctx* ctx, int kind, int width, int height, int motio
             (rc = dalloc(&me->tie_list, me->nmb)) ||
             (rc = dalloc(&me->d_job, 1)) || (rc = dalloc(&me->spec, 5 * (size_t)me->nmb)) ||
             (rc = dalloc(&me->state, 3 * (size_t)me->nmb)) ||
-            (rc = dalloc(&me->cache, (size_t)me->nmb * vppgpu::KCACHE)) || (rc = dalloc(&me->dict, vppgpu::NDICT)) ||
-            (rc = dalloc(&me->d_wave_rec, vppgpu::wave_rec_count(me->cols, me->rows))) ||
-            (rc = dalloc(&me->d_wave_choice, me->nmb)) || (rc = dalloc(&me->changed, (size_t)me->sweep_limit)) ||
+            (kind == VPPGPU_ME_MULTIRES_CROSS_V2 &&  // the Lagrangian overload's records
+             ((rc = dalloc(&me->cache, (size_t)me->nmb * vppgpu::KCACHE)) || (rc = dalloc(&me->dict, vppgpu::NDICT)) ||
+              (rc = dalloc(&me->d_wave_rec, vppgpu::wave_rec_count(me->cols, me->rows))) ||
+              (rc = dalloc(&me->d_wave_choice, me->nmb)))) ||
+            (rc = dalloc(&me->changed, (size_t)me->sweep_limit)) ||
             (rc = dalloc(&me->d_out_mv, me->nmb)) || (rc = dalloc(&me->d_out_dist, me->nmb)) ||
             (rc = dalloc(&me->d_out_avg, 1)) || (rc = dalloc(&me->d_incl, me->nmb)) ||
             (rc = dalloc(&me->d_slice, me->nmb)) || (rc = dalloc(&me->ctrl, 1))) {
@@ -589,10 +592,9 @@ int vppgpu_me_create(vppgpu_ctx* ctx, int kind, int width, int height, int motio
     }
     if ((rc = dalloc(&me->d_src16, npix)) || (rc = dalloc(&me->d_ref16, npix)) || (rc = dalloc(&me->d_src8, npix)) ||
         (rc = dalloc(&me->d_refp, npad)) || (rc = dalloc(&me->d_hpel, 3 * npad)) ||
-        (rc = dalloc(&me->d_wave_rec, vppgpu::wave_rec_count(me->cols, me->rows))) || (rc = dalloc(&me->d_wave_choice, me->nmb)) || (rc = dalloc(&me->spec, 5 * (size_t)me->nmb)) ||
+        (rc = dalloc(&me->spec, 5 * (size_t)me->nmb)) ||
         (rc = dalloc(&me->tables, (size_t)me->nmb * 64 * 64)) ||
         (kind == VPPGPU_ME_FULL && (rc = dalloc(&me->energy, npad))) || (rc = dalloc(&me->d_job, 1)) || (rc = dalloc(&me->tie_list, me->nmb)) || (rc = dalloc(&me->state, 3 * (size_t)me->nmb)) ||
-        (rc = dalloc(&me->cache, (size_t)me->nmb * vppgpu::KCACHE)) || (rc = dalloc(&me->dict, vppgpu::NDICT)) ||
         (rc = dalloc(&me->d_out_mv, me->nmb)) || (rc = dalloc(&me->d_out_dist, me->nmb)) ||
         (rc = dalloc(&me->d_out_avg, 1)) || (rc = dalloc(&me->d_incl, me->nmb)) ||
         (rc = dalloc(&me->d_slice, me->nmb)) || (rc = dalloc(&me->ctrl, 1)) ||

@@ -151,6 +151,15 @@ static __device__ __noinline__ int best_of3(int bx, int by, int bd, int px, int 
     return pos;
 }
 
+// sqrt within 2^-23 relative (the PTX instruction's stated bound), for costs
+// whose comparison has a guard band.
+__device__ __forceinline__ float sqrt_approx(float x)
+{
+    float r;
+    asm("sqrt.approx.f32 %0, %1;" : "=f"(r) : "f"(x));
+    return r;
+}
+
 // Same decision without FP64 in the common cases (norm a power of two: 256,
 // or 64 for the Cross estimator).  Two costs with the same sqrt argument
 // differ only in D/norm, and D/norm is exact; with |lambda| <
@@ -168,9 +177,9 @@ __device__ __forceinline__ int best_of3_fast(int bx, int by, int bd, int px, int
     const int m1 = (px - xref) * (px - xref) + (py - yref) * (py - yref);
     const int m2 = xref * xref + yref * yref;
     const float lf = (float)lambda, inv = 1.0f / (float)norm;
-    const float c0 = (float)bd * inv + lf * sqrtf((float)m0);
-    const float c1 = (float)pd * inv + lf * sqrtf((float)m1);
-    const float c2 = (float)zd * inv + lf * sqrtf((float)m2);
+    const float c0 = (float)bd * inv + lf * sqrt_approx((float)m0);
+    const float c1 = (float)pd * inv + lf * sqrt_approx((float)m1);
+    const float c2 = (float)zd * inv + lf * sqrt_approx((float)m2);
     bool slow = false;
     const bool small_lambda = fabs(lambda) < 1048576.0;
     // strict "cost a < cost b" in the double arithmetic of best_of3

@@ -7,30 +7,30 @@
 // prediction depends on the left / above / above-right (else above-left)
 // neighbours' final vectors: a DAG in raster order.
 //
-// Every evaluation of a macroblock at a prediction is kept as a record
-// {prediction, distortion at it, final vector, final distortion} in a small
-// per-MB cache, so a later visit with the same prediction is a lookup.  The
-// distortion at a prediction reads the frame's precomputed half-pel planes
-// (two byte loads per sample at most).
+// The estimators whose evaluation is short (all but Ver2's Lagrangian
+// overload) relax from the searched vectors to the fixed point, which is the
+// sequential result: k_resolve_first, k_resolve_sweep, k_resolve_finish below.
+//
+// The Lagrangian overload, whose evaluation is a whole search, keeps every
+// evaluation as a record {prediction, distortion at it, final vector, final
+// distortion} in a small per-MB cache, so that a later visit with the same
+// prediction is a lookup:
 //
 //   k_full_sweep0      every MB at once, prediction from the current vectors
 //                      (initially the searched ones).
 //   k_full_relax_sweep up to FullArgs::relax_sweeps launches, each re-evaluating the
 //                      MBs whose prediction moved.  A sweep without change
-//                      is the unique fixed point of the DAG, i.e. the
-//                      sequential result; most frames stop here
-//                      (k_full_relax_outcome writes their outputs).
-//                      Otherwise (long copy chains: the prediction wins and
-//                      is copied along rows and columns) k_full_relax_outcome
-//                      builds a dictionary of the frame's dominant vectors.
-//   k_full_precompute  records of every MB at every dictionary vector.
+//                      is the fixed point (k_full_relax_outcome writes the
+//                      outputs).  Otherwise (long copy chains: the prediction
+//                      wins and is copied along rows and columns)
+//                      k_full_relax_outcome builds a dictionary of the frame's
+//                      dominant vectors.
+//   k_full_precompute, k_full_closure  records of every MB at every dictionary
+//                      vector and at medians of its neighbours' possible vectors.
 //   k_full_wave        one CTA replays the exact sequential order, pipelined
-//                      by rows: warp w owns rows w, w+32, ...; a row advances
-//                      one MB per step once the row above has finished the
-//                      MB above-right, signalled through shared-memory
-//                      progress counters.  A step is a median, a key match
-//                      against the MB's records (prefetched with cp.async)
-//                      and, on a miss only, a full evaluation by the warp.
+//                      by rows (below).
+#include <cooperative_groups.h>
+
 #include "me_cross_search.cuh"
 #include "me_full_common.cuh"
 #include "me_mrc_search.cuh"
@@ -1034,6 +1034,434 @@ __global__ void k_full_average(FullArgs a)
     if (a.job->out_avg) *a.job->out_avg = c ? t / c : 0;
 }
 
+// ---------------------------------------------------------------------------
+// The resolve of every estimator but Ver2's Lagrangian overload: an evaluation
+// there is one round trip to L2 (the distortion at the prediction from the
+// half-pel planes), so nothing is precomputed or kept; what counts is how many
+// evaluations follow one another.
+//
+//   k_resolve_first   every MB at the median of the searched vectors
+//   k_resolve_sweep   every MB whose prediction moved, over the whole GPU
+//   k_resolve_finish  the rest, by one CTA
+//
+// k_resolve_finish keeps the frame's vectors in the shared memory of a cluster,
+// a band of rows per CTA with the last row of the band above beside it, and
+// works in rounds: every marked macroblock takes the median of its neighbours'
+// vectors; those whose prediction moved are listed and evaluated, half a warp
+// each, and where the vector changed it is replaced and its four dependents
+// are marked.  After up to kFinishSub such rounds, fewer when nothing of the
+// band moves, the cluster meets: the copies of the band's last row and the
+// marks that the CTA above sent (distributed shared memory) count from then
+// on.  The state always satisfies vector = f(prediction used), and a vector
+// that changes marks all that read it, so a meeting after which nobody had
+// work is the fixed point, which is the sequential result.  A median reads
+// only earlier anti-diagonals c + 2r, so a meeting settles at least the first
+// one that still moves: a frame takes at most cols + 2 rows meetings.
+//
+// What bounds a round is a chain: the L2 latency of an evaluation's samples
+// (~800 cycles) and its instructions one after the other; a meeting costs
+// ~1300 cycles more (1080p, 8 pairs of a pan with moving objects: 440 us a
+// frame with a meeting after each round, 416, 403 and 397 with 2, 4 and 8).  No
+// round writes global memory: the barrier would wait for it.  Against this
+// resolve's predecessor (up to 14 sweeps, records at dictionary vectors and
+// neighbours' medians, a one-CTA wavefront over them): 613 -> 397 us a frame.
+
+// Sixteen consecutive bytes from any address, by two 16-byte loads: a warp's
+// rows lie in 32 different lines, and the load unit takes a cycle or more for
+// each line of an instruction (five word loads: 10 x 32 of them for the two
+// samples of a quarter position, 0.35 us of a round).
+__device__ __forceinline__ void load_row16(const unsigned char* p, unsigned* w)
+{
+    const uint4* q = reinterpret_cast<const uint4*>(reinterpret_cast<uintptr_t>(p) & ~(uintptr_t)15);
+    const uint4 lo = __ldg(q), hi = __ldg(q + 1);
+    const unsigned o = (unsigned)(reinterpret_cast<uintptr_t>(p) & 15), sh = 8 * (o & 3);
+    const bool s2 = o & 8, s1 = o & 4;
+    const unsigned a0 = s2 ? lo.z : lo.x, a1 = s2 ? lo.w : lo.y, a2 = s2 ? hi.x : lo.z, a3 = s2 ? hi.y : lo.w;
+    const unsigned a4 = s2 ? hi.z : hi.x, a5 = s2 ? hi.w : hi.y;
+    const unsigned v0 = s1 ? a1 : a0, v1 = s1 ? a2 : a1, v2 = s1 ? a3 : a2, v3 = s1 ? a4 : a3, v4 = s1 ? a5 : a4;
+    w[0] = __funnelshift_r(v0, v1, sh);
+    w[1] = __funnelshift_r(v1, v2, sh);
+    w[2] = __funnelshift_r(v2, v3, sh);
+    w[3] = __funnelshift_r(v3, v4, sh);
+}
+
+// One MB per half warp (16 lanes, a row of 16 samples each): the final vector
+// and distortion of MB k (origin n, m) at prediction `key`, from its searched
+// result `sp` and this lane's row of the input.  Lanes of a half without work
+// (act false) pass any valid MB.
+template <int kEst>
+__device__ __forceinline__ int2 evaluate_half(const FullArgs& a, bool act, int k, int n, int m, int key, int4 sp,
+                                              uint4 cur, int lane, mrc::Lattice* lt)
+{
+    const int px = mv_x(key), py = mv_y(key);
+    if constexpr (kEst == cross::EST_CROSS) {  // its path distortion is a whole warp's
+        int2 out = make_int2(0, 0);
+#pragma unroll 1
+        for (int h = 0; h < 2; h++) {
+            if (!__shfl_sync(0xffffffffu, (int)act, 16 * h)) continue;
+            const int4 rec = evaluate<kEst>(a, __shfl_sync(0xffffffffu, k, 16 * h), __shfl_sync(0xffffffffu, px, 16 * h),
+                                            __shfl_sync(0xffffffffu, py, 16 * h), lane, lt);
+            if ((lane >> 4) == h) out = make_int2(rec.z, rec.w);
+        }
+        return out;
+    }
+    const PredGeom g = pred_geom(n, m, a.W, a.H, px, py);
+    // qpel_block8's sixteen cases by bit fields: the plane (0 full pel, 1 b, 2 h, 3 j) and the column and
+    // row offset of both averaged samples; the cases of one sample average it with itself
+    const int s = g.fx | (g.fy << 2);
+    constexpr unsigned kP1 = 0u | 0u << 2 | 1u << 4 | 0u << 6 | 0u << 8 | 1u << 10 | 3u << 12 | 1u << 14 | 2u << 16 |
+                             3u << 18 | 3u << 20 | 3u << 22 | 0u << 24 | 2u << 26 | 3u << 28 | 2u << 30;
+    constexpr unsigned kP2 = 0u | 1u << 2 | 1u << 4 | 1u << 6 | 2u << 8 | 2u << 10 | 1u << 12 | 2u << 14 | 2u << 16 |
+                             2u << 18 | 3u << 20 | 2u << 22 | 2u << 24 | 1u << 26 | 1u << 28 | 1u << 30;
+    constexpr unsigned kX1 = 1u << 3 | 1u << 15, kX2 = 1u << 7 | 1u << 11;
+    constexpr unsigned kY1 = 1u << 12, kY2 = 1u << 13 | 1u << 14 | 1u << 15;
+    const int p1 = (kP1 >> (2 * s)) & 3, p2 = (kP2 >> (2 * s)) & 3;
+    const int at = (g.oy + (lane & 15) + PAD) * a.rstride + g.ox + PAD;
+    const unsigned char* b1 = p1 ? a.hpel + (size_t)(p1 - 1) * a.plane_size : a.refp;
+    const unsigned char* b2 = p2 ? a.hpel + (size_t)(p2 - 1) * a.plane_size : a.refp;
+    b1 += at + (int)((kX1 >> s) & 1) + ((kY1 >> s) & 1 ? a.rstride : 0);
+    b2 += at + (int)((kX2 >> s) & 1) + ((kY2 >> s) & 1 ? a.rstride : 0);
+    unsigned w1[4], w2[4];
+    load_row16(b1, w1);
+    load_row16(b2, w2);
+    const unsigned c4[4] = {cur.x, cur.y, cur.z, cur.w};
+    unsigned acc = 0;
+#pragma unroll
+    for (int i = 0; i < 4; i++) {
+        const unsigned d = __vabsdiffu4(c4[i], __vavgu4(w1[i], w2[i]));
+        acc = __dp4a(d, d, acc);
+    }
+    const unsigned lo = __reduce_add_sync(0xffffffffu, lane < 16 ? acc : 0u);
+    const unsigned hi = __reduce_add_sync(0xffffffffu, lane < 16 ? 0u : acc);
+    const int pd = (int)(lane < 16 ? lo : hi);
+    int mvx = mv_x(sp.x), mvy = mv_y(sp.x), minD = sp.y;
+    const bool tie = act && (sp.w & FLAG_TIE) && (kEst != 0 || round_pred(px) != 0 || round_pred(py) != 0);
+    const unsigned ties = __ballot_sync(0xffffffffu, tie);
+    if (ties) {  // rare: the searched vector depends on the prediction; a whole warp's work
+#pragma unroll 1
+        for (int h = 0; h < 2; h++) {
+            if (!((ties >> (16 * h)) & 1u)) continue;
+            const int hk = __shfl_sync(0xffffffffu, k, 16 * h), hx = __shfl_sync(0xffffffffu, px, 16 * h);
+            const int hy = __shfl_sync(0xffffffffu, py, 16 * h), hf = __shfl_sync(0xffffffffu, sp.w, 16 * h);
+            int tx = __shfl_sync(0xffffffffu, mvx, 16 * h), ty = __shfl_sync(0xffffffffu, mvy, 16 * h);
+            int td = __shfl_sync(0xffffffffu, minD, 16 * h);
+            if constexpr (kEst == 0) tie_path(a, hk, hx, hy, hf, lane, &tx, &ty, &td);
+            else pred_search_at<kEst>(a, hk, hx, hy, lane, &tx, &ty, &td, lt);
+            if ((lane >> 4) == h) {
+                mvx = tx;
+                mvy = ty;
+                minD = td;
+            }
+        }
+    }
+    const int pos = best_of3_fast(mvx, mvy, minD, g.pcx, g.pcy, pd, sp.z, a.lambda, g.pcx, g.pcy);
+    return pos == 0 ? make_int2(pack_mv(mvx, mvy), minD) : pos == 1 ? make_int2(pack_mv(g.pcx, g.pcy), pd)
+                                                                    : make_int2(0, sp.z);
+}
+
+// This lane's row of MB (n, m)'s input.
+__device__ __forceinline__ uint4 load_cur16(const FullArgs& a, int n, int m, int lane)
+{
+    return __ldg(reinterpret_cast<const uint4*>(a.src8 + (size_t)(m + (lane & 15)) * a.W + n));
+}
+
+// The median prediction from the vectors in global memory; the neighbours are
+// read by position, beside the record that says which of them count.
+__device__ __forceinline__ int median_global(const FullArgs& a, int k, int r, int c, int4* sp)
+{
+    const int cols = a.cols;
+    *sp = __ldcg(a.spec4 + k);
+    const int A = c > 0 ? __ldcg(a.final_mv + k - 1) : 0;
+    const int B = r > 0 ? __ldcg(a.final_mv + k - cols) : 0;
+    const int C = r > 0 && c + 1 < cols ? __ldcg(a.final_mv + k - cols + 1) : 0;
+    const int D = r > 0 && c > 0 ? __ldcg(a.final_mv + k - cols - 1) : 0;
+    return median_packed(sp->w, A, B, C, D);
+}
+
+template <int kEst>
+__global__ void __launch_bounds__(256) k_resolve_first(const __grid_constant__ FullArgs a)
+{
+    const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
+    const int item = (blockIdx.x * 8 + wib) * 2 + (lane >> 4);
+    const bool act = item < a.nmb;
+    if (!__any_sync(0xffffffffu, act)) return;
+    const int k = act ? item : 0, r = k / a.cols, c = k - r * a.cols;
+    const uint4 cur = load_cur16(a, 16 * c, 16 * r, lane);
+    int4 sp;
+    const int key = median_global(a, k, r, c, &sp);
+    const int2 out = evaluate_half<kEst>(a, act, k, 16 * c, 16 * r, key, sp, cur, lane, LatticeSlots<kEst>::get(wib));
+    if (act && (lane & 15) == 0) {
+        __stcg(a.pred_used + k, key);
+        __stcg(a.final_dist + k, out.y);
+        __stcg(a.final_mv + k, out.x);
+    }
+}
+
+// One sweep over every MB: lane per MB (MBs gwarp + lane*nwarps ...) to find
+// those whose prediction moved, then a half warp on each.  Skipped once an
+// earlier sweep changed no vector.
+template <int kEst>
+__global__ void __launch_bounds__(256) k_resolve_sweep(const __grid_constant__ FullArgs a, int sweep)
+{
+    if (sweep > 1 && *((volatile int*)&a.changed[sweep - 1]) == 0) return;
+    const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
+    const int gwarp = blockIdx.x * 8 + wib, nwarps = gridDim.x * 8;
+    int changed = 0, evals = 0;
+    for (int base = gwarp; base < a.nmb; base += 32 * nwarps) {
+        const int k = base + lane * nwarps;
+        int key = 0;
+        int4 sp;
+        bool moved = false;
+        if (k < a.nmb) {
+            const int r = k / a.cols;
+            key = median_global(a, k, r, k - r * a.cols, &sp);
+            moved = __ldcg(a.pred_used + k) != key;
+        }
+        unsigned todo = __ballot_sync(0xffffffffu, moved);
+        while (todo) {
+            const int f0 = __ffs(todo) - 1;
+            todo &= todo - 1;
+            const int f1 = todo ? __ffs(todo) - 1 : f0;
+            const bool two = todo != 0;
+            todo &= todo - 1;
+            const int f = lane < 16 ? f0 : f1;
+            const bool act = lane < 16 || two;
+            const int kk = base + f * nwarps, r = kk / a.cols, c = kk - r * a.cols;
+            const int fkey = __shfl_sync(0xffffffffu, key, f);
+            int4 fsp;
+            fsp.x = __shfl_sync(0xffffffffu, sp.x, f);
+            fsp.y = __shfl_sync(0xffffffffu, sp.y, f);
+            fsp.z = __shfl_sync(0xffffffffu, sp.z, f);
+            fsp.w = __shfl_sync(0xffffffffu, sp.w, f);
+            const uint4 cur = load_cur16(a, 16 * c, 16 * r, lane);
+            const int old = __ldcg(a.final_mv + kk);
+            const int2 out = evaluate_half<kEst>(a, act, kk, 16 * c, 16 * r, fkey, fsp, cur, lane,
+                                                 LatticeSlots<kEst>::get(wib));
+            if (act && (lane & 15) == 0) {
+                __stcg(a.pred_used + kk, fkey);
+                __stcg(a.final_dist + kk, out.y);
+                if (old != out.x) __stcg(a.final_mv + kk, out.x);
+                evals++;
+                changed += old != out.x;
+            }
+            __syncwarp();
+        }
+    }
+    evals = __reduce_add_sync(0xffffffffu, evals);
+    changed = __reduce_add_sync(0xffffffffu, changed);
+    if (lane == 0 && evals) {
+        atomicAdd(&a.ctrl->relax_evals, evals);
+        atomicAdd(&a.ctrl->relax_miss, evals);
+        if (changed) atomicAdd(&a.changed[sweep], changed);
+    }
+}
+
+constexpr int kFinishThreads = 512;
+constexpr int kFinishHalves = kFinishThreads / 16;  // evaluations in flight per CTA
+constexpr int kFinishSub = 8;                       // most rounds between two meetings of the cluster
+constexpr int kFinishSmem = 220 * 1024;             // most dynamic shared memory of a CTA
+
+// A CTA of the cluster holds `band` rows: per macroblock its vector, the
+// prediction it was evaluated at, its distortion (`dist`; else that stays in
+// global memory), a work entry, its neighbour mask and its mark; the row
+// above the band, and the marks that arrive from there (two buffers).
+struct FinishShape {
+    int ctas, band, dist;
+    size_t smem;
+};
+FinishShape finish_shape(int cols, int rows)
+{
+    FinishShape f;
+    f.ctas = cols * rows <= kFinishThreads ? 1 : cols * rows <= 4 * kFinishThreads ? 4 : 8;
+    for (;;) {
+        f.band = (rows + f.ctas - 1) / f.ctas;
+        const size_t n = (size_t)f.band * cols;
+        f.dist = 1;
+        f.smem = 4 * (3 * n + cols) + 4 * ((n + 3) / 4 * 4) + (size_t)(2 * cols + 3) / 4 * 4;
+        if (f.smem <= (size_t)kFinishSmem) return f;
+        if (f.ctas == 16) break;
+        f.ctas = 16;  // beyond ~110000 macroblocks: the non-portable size
+    }
+    f.dist = 0;  // 8192 x 8192: 200 KB
+    f.smem -= 4 * (size_t)f.band * cols;
+    return f;
+}
+
+template <int kEst>
+__global__ void __launch_bounds__(kFinishThreads, 1)
+    k_resolve_finish(const __grid_constant__ FullArgs a, int first, int band, int keep_dist)
+{
+    extern __shared__ __align__(16) int fin_smem[];
+    __shared__ int s_n[2], s_any[3], s_evals[2], s_changed[RELAX_SWEEPS + 1];
+    namespace cg = cooperative_groups;
+    const cg::cluster_group cluster = cg::this_cluster();
+    const int rank = (int)cluster.block_rank(), ctas = (int)cluster.num_blocks();
+    const int cols = a.cols, rows = a.nmb / cols;
+    const int r0 = rank * band, nrow = max(0, min(rows - r0, band)), nloc = nrow * cols, k0 = r0 * cols;
+    const int tid = threadIdx.x, lane = tid & 31, wib = tid >> 5, half = lane >> 4;
+    const int most_loc = band * cols, quads = (most_loc + 3) >> 2;
+    volatile int* s_fin = fin_smem;            // the row above the band, then the band
+    int* s_pu = fin_smem + cols + most_loc;    // prediction used
+    // marks, a byte each: macroblock i at byte 4 * (i % quads) + i / quads, so that neighbours lie in
+    // different words
+    unsigned* s_mark = reinterpret_cast<unsigned*>(s_pu + most_loc);
+    unsigned char* s_av = reinterpret_cast<unsigned char*>(s_mark + quads);
+    unsigned short* s_work = reinterpret_cast<unsigned short*>(s_av + 4 * quads);  // macroblocks whose prediction moved
+    unsigned char* s_in = reinterpret_cast<unsigned char*>(s_work + 4 * quads);  // arriving marks of the first row, [2][cols]
+    int* s_dist = reinterpret_cast<int*>(s_in + (2 * cols + 3) / 4 * 4);
+    const bool has_below = rank + 1 < ctas;
+    int* below = has_below ? cluster.map_shared_rank(fin_smem, rank + 1) : fin_smem;  // its row above the band
+    unsigned char* below_in = has_below ? cluster.map_shared_rank(s_in, rank + 1) : s_in;
+    const float per_col = 1.0f / (float)cols;
+
+    auto mark = [&](int i) {  // i < 4 * quads
+        const int q = i >= 2 * quads ? (i >= 3 * quads ? 3 : 2) : (i >= quads ? 1 : 0);
+        reinterpret_cast<volatile unsigned char*>(s_mark)[4 * (i - q * quads) + q] = 1;
+    };
+    auto median_at = [&](int i) {  // local index; the row above is at i
+        const int av = s_av[i], at = i + cols;
+        const int A = (av & AV_A) ? s_fin[at - 1] : 0;
+        const int B = (av & AV_B) ? s_fin[at - cols] : 0;
+        const int C = (av & AV_C) ? s_fin[at - cols + 1] : 0;
+        const int D = (!(av & AV_C) && (av & AV_D)) ? s_fin[at - cols - 1] : 0;
+        return median_packed(av, A, B, C, D);
+    };
+    if (r0 > 0 && nrow > 0)
+        for (int c = tid; c < cols; c += kFinishThreads) s_fin[c] = __ldcg(a.final_mv + k0 - cols + c);
+#pragma unroll 2
+    for (int i = tid; i < nloc; i += kFinishThreads) {
+        s_fin[cols + i] = __ldcg(a.final_mv + k0 + i);
+        s_pu[i] = __ldcg(a.pred_used + k0 + i);
+        s_av[i] = (unsigned char)__ldcg(&a.spec4[k0 + i].w);
+        if (keep_dist) s_dist[i] = __ldcg(a.final_dist + k0 + i);
+    }
+    for (int i = tid; i < quads; i += kFinishThreads) s_mark[i] = 0x01010101u;
+    for (int i = tid; i < 2 * cols; i += kFinishThreads) s_in[i] = 0;
+    if (tid < 3) s_any[tid] = 0;
+    if (tid < 2) s_n[tid] = s_evals[tid] = 0;
+    if (tid <= RELAX_SWEEPS) s_changed[tid] = 0;
+    cluster.sync();
+
+    const int most = 64 * (cols + 2 * rows) + 65536;  // far above what the argument at the top allows
+    int round = first;
+    for (;; round++) {
+        for (int sub = 0; sub < kFinishSub; sub++) {
+            // list the marked macroblocks whose prediction moved
+            int* n = &s_n[sub & 1];
+            for (int q = tid; q < quads; q += kFinishThreads) {
+                const unsigned m = s_mark[q];
+                if (!m) continue;
+                s_mark[q] = 0u;
+#pragma unroll
+                for (int b = 0; b < 4; b++) {
+                    const int i = q + b * quads;
+                    if (((m >> (8 * b)) & 0xffu) && i < nloc && median_at(i) != s_pu[i])
+                        s_work[atomicAdd(n, 1)] = (unsigned short)i;
+                }
+            }
+            __syncthreads();
+            const int nw = *n;
+            if (nw == 0) break;
+            if (tid == 0) {
+                s_n[(sub + 1) & 1] = 0;
+                s_evals[round > a.relax_sweeps] += nw;
+            }
+            if (tid < ctas) *cluster.map_shared_rank(&s_any[round % 3], tid) = 1;
+            for (int w = 2 * wib; w < nw; w += kFinishHalves) {
+                const bool act = w + half < nw;
+                const int i = s_work[act ? w + half : w];
+                const int lr = (int)(((float)i + 0.5f) * per_col);  // i / cols: never near a whole number
+                const int r = r0 + lr, c = i - lr * cols, k = k0 + i;
+                const int4 sp = __ldg(a.spec4 + k);
+                const uint4 in = load_cur16(a, 16 * c, 16 * r, lane);
+                // one reading of the neighbours for the half warp: others change meanwhile
+                const int key = __shfl_sync(0xffffffffu, median_at(i), lane & 16);
+                const int old = s_fin[cols + i];
+                const int2 out = evaluate_half<kEst>(a, act, k, 16 * c, 16 * r, key, sp, in, lane, nullptr);
+                const bool changed = act && old != out.x;
+                const int d = lane & 15;
+                if (act && d == 0) {
+                    s_pu[i] = key;
+                    if (keep_dist) s_dist[i] = out.y;
+                    else __stcg(a.final_dist + k, out.y);
+                    if (changed) {
+                        s_fin[cols + i] = out.x;
+                        if (lr == band - 1 && has_below) below[c] = out.x;
+                        if (round <= a.relax_sweeps) atomicAdd(&s_changed[round], 1);
+                    }
+                }
+                // its dependents, a lane each: right, below, below left, below right
+                const int c2 = c + (d == 0 ? 1 : (d == 1 ? 0 : (d == 2 ? -1 : 1)));
+                if (changed && d < 4 && c2 >= 0 && c2 < cols) {
+                    if (d == 0) mark(i + 1);
+                    else if (lr < band - 1) mark(i + cols + c2 - c);
+                    else if (has_below) below_in[(round & 1) * cols + c2] = 1;
+                }
+                __syncwarp();
+            }
+            __syncthreads();
+        }
+        if (tid == 0) {
+            s_n[0] = s_n[1] = 0;
+            s_any[(round + 1) % 3] = 0;
+        }
+        cluster.sync();
+        // what arrived before the meeting; the other buffer takes what follows it
+        for (int c = tid; c < cols; c += kFinishThreads)
+            if (s_in[(round & 1) * cols + c]) {
+                s_in[(round & 1) * cols + c] = 0;
+                mark(c);
+            }
+        __syncthreads();
+        if (!*((volatile int*)&s_any[round % 3])) break;
+        if (round - first > most) {
+            if (tid == 0) atomicOr(&a.ctrl->status, ST_TIMEOUT);
+            break;
+        }
+    }
+    // outputs and the included-distortion average (Full.cpp:581-611)
+    const JobDesc job = *a.job;
+    long long tot = 0;
+    int cnt = 0;
+#pragma unroll 2
+    for (int i = tid; i < nloc; i += kFinishThreads) {
+        const int k = k0 + i, fmv = s_fin[cols + i], d = keep_dist ? s_dist[i] : __ldcg(a.final_dist + k);
+        const int inc = job.incl ? job.incl[k] : 0;
+        job.out_mv[k] = fmv;
+        if (job.out_dist) job.out_dist[k] = d;
+        if (inc) {
+            tot += d;
+            cnt++;
+        }
+    }
+    for (int o = 16; o > 0; o >>= 1) {
+        tot += __shfl_xor_sync(0xffffffffu, tot, o);
+        cnt += __shfl_xor_sync(0xffffffffu, cnt, o);
+    }
+    if (lane == 0 && cnt) {
+        atomicAdd(reinterpret_cast<unsigned long long*>(&a.ctrl->total), (unsigned long long)tot);
+        atomicAdd(&a.ctrl->count, cnt);
+    }
+    if (tid == 0) {
+        if (s_evals[0]) {
+            atomicAdd(&a.ctrl->relax_evals, s_evals[0]);
+            atomicAdd(&a.ctrl->relax_miss, s_evals[0]);
+        }
+        if (s_evals[1]) atomicAdd(&a.ctrl->wave_miss, s_evals[1]);
+    }
+    if (tid <= RELAX_SWEEPS && s_changed[tid]) atomicAdd(&a.changed[tid], s_changed[tid]);
+    cluster.sync();
+    if (rank == 0 && tid == 0) {
+        const int settled = round - 1;  // the last round (or sweep) with work
+        const bool relaxed = a.relax_sweeps > 0 && settled <= a.relax_sweeps;
+        a.ctrl->sweeps = relaxed ? (settled > 0 ? settled : 1) : a.relax_sweeps + 1000;
+        a.ctrl->converged = relaxed;
+        const long long t = (long long)__ldcg(reinterpret_cast<const unsigned long long*>(&a.ctrl->total));
+        const int n = __ldcg(&a.ctrl->count);
+        if (job.out_avg) *job.out_avg = n ? t / n : 0;
+    }
+}
+
 // The integer-pel SAD stage's tail.  The prediction enters only the exact-tie
 // decisions of the scan (MotionEstimatorH264ImplFull.cpp:424-441), so every
 // macroblock without a tie already holds its final vector.  One CTA walks the
@@ -1191,38 +1619,26 @@ constexpr int kWaveMaxCols = 512;  // 8192 / 16
 
 }  // namespace
 
+namespace {
+template <int kEst>
+int finish_prepare();
+}
+
 int full_resolve_prepare(vppgpu_ctx* ctx, int* resolve_cap)
 {
     *resolve_cap = ctx->sm_count * 8;
     // dirty bitmaps of the largest picture (8192 x 8192)
     const int tail_smem = 2 * (512 * 512 / 32) * (int)sizeof(unsigned);
-    VPP_CUDA(cudaFuncSetAttribute(k_full_relax_tail<0>, cudaFuncAttributeMaxDynamicSharedMemorySize, tail_smem));
-    VPP_CUDA(cudaFuncSetAttribute(k_full_relax_tail<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, tail_smem));
-    VPP_CUDA(cudaFuncSetAttribute(k_full_relax_tail<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, tail_smem));
     VPP_CUDA(cudaFuncSetAttribute(k_full_relax_tail<mrc::EST_V2_LAMBDA>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                   tail_smem));
-    VPP_CUDA(cudaFuncSetAttribute(k_full_relax_tail<cross::EST_CROSS>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                  tail_smem));
-    VPP_CUDA(cudaFuncSetAttribute(k_full_wave<4, 0>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                  (int)wave_smem_bytes(3, kWaveMaxCols, 4)));
-    VPP_CUDA(cudaFuncSetAttribute(k_full_wave<2, 0>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                  (int)wave_smem_bytes(kWaveMaxWarps, kWaveMaxCols, 2)));
-    VPP_CUDA(cudaFuncSetAttribute(k_full_wave<4, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                  (int)wave_smem_bytes(3, kWaveMaxCols, 4)));
-    VPP_CUDA(cudaFuncSetAttribute(k_full_wave<2, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                  (int)wave_smem_bytes(kWaveMaxWarps, kWaveMaxCols, 2)));
-    VPP_CUDA(cudaFuncSetAttribute(k_full_wave<4, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                  (int)wave_smem_bytes(3, kWaveMaxCols, 4)));
-    VPP_CUDA(cudaFuncSetAttribute(k_full_wave<2, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                  (int)wave_smem_bytes(kWaveMaxWarps, kWaveMaxCols, 2)));
     VPP_CUDA(cudaFuncSetAttribute(k_full_wave<4, mrc::EST_V2_LAMBDA>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                   (int)wave_smem_bytes(3, kWaveMaxCols, 4)));
     VPP_CUDA(cudaFuncSetAttribute(k_full_wave<2, mrc::EST_V2_LAMBDA>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                   (int)wave_smem_bytes(kWaveMaxWarps, kWaveMaxCols, 2)));
-    VPP_CUDA(cudaFuncSetAttribute(k_full_wave<4, cross::EST_CROSS>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                  (int)wave_smem_bytes(3, kWaveMaxCols, 4)));
-    VPP_CUDA(cudaFuncSetAttribute(k_full_wave<2, cross::EST_CROSS>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                  (int)wave_smem_bytes(kWaveMaxWarps, kWaveMaxCols, 2)));
+    int rc;
+    if ((rc = finish_prepare<0>()) || (rc = finish_prepare<1>()) || (rc = finish_prepare<2>()) ||
+        (rc = finish_prepare<cross::EST_CROSS>()))
+        return rc;
     // the SAD resolve's largest dynamic shared memory: the local final vectors
     // end at kSadSmemMbs macroblocks (larger pictures keep only the tie bits)
     VPP_CUDA(cudaFuncSetAttribute(k_sad_resolve, cudaFuncAttributeMaxDynamicSharedMemorySize,
@@ -1232,8 +1648,9 @@ int full_resolve_prepare(vppgpu_ctx* ctx, int* resolve_cap)
 
 namespace {
 
+// Ver2's Lagrangian overload: an evaluation is a whole search, so records, dictionary and closure pay.
 template <int kEst>
-int resolve_launch(vppgpu_ctx* ctx, const FullArgs& args)
+int resolve_launch_records(vppgpu_ctx* ctx, const FullArgs& args)
 {
     const int rows = args.nmb / args.cols, nbands = (rows + 31) / 32;
     if (args.cols > kWaveMaxCols) return VPPGPU_ERR_UNSUPPORTED;
@@ -1285,6 +1702,43 @@ int resolve_launch(vppgpu_ctx* ctx, const FullArgs& args)
     return VPPGPU_OK;
 }
 
+template <int kEst>
+int resolve_launch(vppgpu_ctx* ctx, const FullArgs& args)
+{
+    k_resolve_first<kEst><<<(args.nmb + 15) / 16, 256, 0, ctx->stream>>>(args);
+    VPP_CHECK_LAUNCH(ctx);
+    const int want = (args.nmb + 7) / 8, cap = ctx->sm_count * args.relax_blocks_per_sm;
+    const int blocks = want < cap ? want : cap;
+    const int sweeps = args.relax_sweeps < args.grid_sweeps ? args.relax_sweeps : args.grid_sweeps;
+    for (int sweep = 1; sweep <= sweeps; sweep++) {
+        k_resolve_sweep<kEst><<<blocks, 256, 0, ctx->stream>>>(args, sweep);
+        VPP_CHECK_LAUNCH(ctx);
+    }
+    const FinishShape f = finish_shape(args.cols, args.nmb / args.cols);
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(f.ctas);
+    cfg.blockDim = dim3(kFinishThreads);
+    cfg.dynamicSmemBytes = f.smem;
+    cfg.stream = ctx->stream;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = f.ctas;
+    attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    VPP_CUDA(cudaLaunchKernelEx(&cfg, k_resolve_finish<kEst>, args, sweeps + 1, f.band, f.dist));
+    VPP_CHECK_LAUNCH(ctx);
+    return VPPGPU_OK;
+}
+
+template <int kEst>
+int finish_prepare()
+{
+    VPP_CUDA(cudaFuncSetAttribute(k_resolve_finish<kEst>, cudaFuncAttributeMaxDynamicSharedMemorySize, kFinishSmem));
+    VPP_CUDA(cudaFuncSetAttribute(k_resolve_finish<kEst>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
+    return VPPGPU_OK;
+}
+
 }  // namespace
 
 int full_resolve_launch(vppgpu_ctx* ctx, const FullArgs& args, int resolve_grid, int est)
@@ -1295,7 +1749,7 @@ int full_resolve_launch(vppgpu_ctx* ctx, const FullArgs& args, int resolve_grid,
     case 1: return resolve_launch<1>(ctx, args);
     case 2: return resolve_launch<2>(ctx, args);
     case cross::EST_CROSS: return resolve_launch<cross::EST_CROSS>(ctx, args);
-    case mrc::EST_V2_LAMBDA: return resolve_launch<mrc::EST_V2_LAMBDA>(ctx, args);
+    case mrc::EST_V2_LAMBDA: return resolve_launch_records<mrc::EST_V2_LAMBDA>(ctx, args);
     default: return VPPGPU_ERR_INVALID_ARG;
     }
 }

@@ -42,14 +42,7 @@ constexpr size_t kSpecBytes = 8192;                        // 5 ints per macrobl
 constexpr size_t kStateBytes = 4864;                       // 3 ints per macroblock
 constexpr size_t kCtrlBytes = 256;                         // vppgpu::MeCtrl
 constexpr size_t kChangedBytes = 1792;                     // sweep counters + dirty bitmap
-constexpr size_t kCacheBytes = 202752;                     // KCACHE 16-byte records per macroblock
-constexpr size_t kDictBytes = 256;                         // NDICT vectors
 constexpr size_t kHpelBytes = 3 * kRefBytes;               // b, h, j planes of the padded reference
-// Wavefront records, wave_rec_count(cols, rows): at most 2*(12+62)*32 = 4736
-// for 396 macroblocks no wider or taller than 64 (rows 33..64 leave at most
-// 12 columns; 32 rows or fewer at most 64 columns, 4032).
-constexpr size_t kWaveRecBytes = 4736 * sizeof(vppgpu::WaveRec);
-constexpr size_t kChoiceBytes = 1600;                      // one int per macroblock
 constexpr size_t kTieListBytes = 1600;                     // one int per macroblock
 constexpr size_t kJobBytes = 64;                           // vppgpu::JobDesc
 constexpr size_t kTableBytes = (size_t)VPPGPU_NOALLOC_MAX_MBS * 64 * 64 * 4;
@@ -60,23 +53,13 @@ constexpr size_t kOffSpec = kOffRef + kRefBytes;
 constexpr size_t kOffState = kOffSpec + kSpecBytes;
 constexpr size_t kOffCtrl = kOffState + kStateBytes;
 constexpr size_t kOffChanged = kOffCtrl + kCtrlBytes;
-constexpr size_t kOffCache = kOffChanged + kChangedBytes;
-constexpr size_t kOffDict = kOffCache + kCacheBytes;
-constexpr size_t kOffHpel = kOffDict + kDictBytes;
-constexpr size_t kOffWaveRec = kOffHpel + kHpelBytes;
-constexpr size_t kOffChoice = kOffWaveRec + kWaveRecBytes;
-constexpr size_t kOffTieList = kOffChoice + kChoiceBytes;
+constexpr size_t kOffHpel = kOffChanged + kChangedBytes;
+constexpr size_t kOffTieList = kOffHpel + kHpelBytes;
 constexpr size_t kOffJob = kOffTieList + kTieListBytes;
 constexpr size_t kOffTables = kOffJob + kJobBytes;
 constexpr size_t kOffEnergy = kOffTables + kTableBytes;
 static_assert(sizeof(vppgpu::JobDesc) <= kJobBytes && kOffJob % 16 == 0, "job descriptor does not fit");
-static_assert(16 * vppgpu::KCACHE * VPPGPU_NOALLOC_MAX_MBS <= kCacheBytes && 4 * vppgpu::NDICT <= kDictBytes,
-              "resolve caches do not fit");
-static_assert(sizeof(vppgpu::WaveRec) * VPPGPU_NOALLOC_MAX_MBS <= kWaveRecBytes &&
-                  4 * VPPGPU_NOALLOC_MAX_MBS <= kChoiceBytes,
-              "wavefront records do not fit");
-static_assert(kOffSpec % 16 == 0 && kOffCache % 16 == 0 && kOffHpel % 16 == 0 &&
-                  kOffWaveRec % 16 == 0 && kOffTables % 16 == 0 && kOffEnergy % 16 == 0,
+static_assert(kOffSpec % 16 == 0 && kOffHpel % 16 == 0 && kOffTables % 16 == 0 && kOffEnergy % 16 == 0,
               "vector records and planes need 16-byte alignment");
 constexpr size_t kScratchBytes = 12u << 20;
 static_assert(kOffEnergy + kEnergyBytes <= kScratchBytes, "scratch layout exceeds the array");
@@ -141,8 +124,7 @@ extern "C" int vppgpu_me_full_estimate_noalloc(const short* d_src, const short* 
     const int cols = width / 16, nmb = cols * (height / 16);
     if (width > VPPGPU_NOALLOC_MAX_DIM || height > VPPGPU_NOALLOC_MAX_DIM || nmb > VPPGPU_NOALLOC_MAX_MBS ||
         motion_range > 128 || (size_t)width * height > kSrcBytes ||
-        (size_t)(width + 2 * vppgpu::PAD) * (height + 2 * vppgpu::PAD) > kRefBytes ||
-        vppgpu::wave_rec_count(cols, height / 16) * sizeof(vppgpu::WaveRec) > kWaveRecBytes)
+        (size_t)(width + 2 * vppgpu::PAD) * (height + 2 * vppgpu::PAD) > kRefBytes )
         return VPPGPU_ERR_UNSUPPORTED;
 
     int dev = 0;
@@ -169,16 +151,12 @@ extern "C" int vppgpu_me_full_estimate_noalloc(const short* d_src, const short* 
     a.refp = base + kOffRef;
     a.hpel = base + kOffHpel;
     a.plane_size = (size_t)a.rstride * (height + 2 * vppgpu::PAD);
-    a.wave_rec = (vppgpu::WaveRec*)(base + kOffWaveRec);
-    a.wave_choice = (int*)(base + kOffChoice);
     a.tie_list = (int*)(base + kOffTieList);
     int* spec = (int*)(base + kOffSpec);
     a.spec4 = reinterpret_cast<int4*>(spec);
     a.spec_imv = spec + 4 * nmb;
     a.tables = (int*)(base + kOffTables);
     a.energy = (const int*)(base + kOffEnergy);
-    a.cache = (int4*)(base + kOffCache);
-    a.dict = (int*)(base + kOffDict);
     int* state = (int*)(base + kOffState);
     a.final_mv = state;
     a.final_dist = state + nmb;
@@ -190,7 +168,7 @@ extern "C" int vppgpu_me_full_estimate_noalloc(const short* d_src, const short* 
     a.sweep_limit = vppgpu::RELAX_SWEEPS + 2 + (nmb + 31) / 32;  // sweep counters, then the dirty bitmap
     a.dirty = reinterpret_cast<unsigned*>(a.changed + vppgpu::RELAX_SWEEPS + 2);
     a.relax_sweeps = 8;
-    a.grid_sweeps = 8;
+    a.grid_sweeps = 1;
     a.relax_blocks_per_sm = 4;
     a.mrc = nullptr;
     a.lattice = nullptr;
