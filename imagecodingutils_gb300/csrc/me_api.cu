@@ -30,7 +30,8 @@ struct vppgpu_me {
     int graph_state;  // 0 not tried, 1 captured, -1 unavailable (direct launches)
     int* spec;  // 5 * nmb: {vector, distortion, zero distortion, flags} per MB, then full-pel winners
     int* tables;
-    int* energy;  // block energies of the padded reference (full search by SSD)
+    float* energy;  // block energies of the padded reference (full search by SSD)
+    float* rowmin;  // minima of the SSD search
     vppgpu::SearchMaps* maps;  // the search kernel's tensor maps over this handle's buffers
     int* tie_list;
     int4* cache;
@@ -44,7 +45,6 @@ struct vppgpu_me {
     vppgpu::MeCtrl* ctrl;
     int* changed;
     int sweep_limit;
-    int resolve_grid;
     int relax_sweeps;  // relaxation sweeps before the wavefront (0..RELAX_SWEEPS)
     int grid_sweeps;   // ... of which over every MB
     int relax_blocks_per_sm;  // grid of a sweep over every MB
@@ -134,6 +134,7 @@ void me_free(vppgpu_me* me)
     cudaFree(me->spec);
     cudaFree(me->tables);
     cudaFree(me->energy);
+    cudaFree(me->rowmin);
     delete me->maps;
     cudaFree(me->tie_list);
     cudaFree(me->cache);
@@ -179,6 +180,7 @@ vppgpu::FullArgs full_args(vppgpu_me* me, double lambda)
     a.dict = me->dict;
     a.tables = me->tables;
     a.energy = me->energy;
+    a.rowmin = me->rowmin;
     a.tie_list = me->tie_list;
     a.final_mv = me->state;
     a.final_dist = me->state + me->nmb;
@@ -278,7 +280,7 @@ int run(vppgpu_me* me, const short* d_src16, const short* d_ref16, const unsigne
             int crc = VPPGPU_OK;
             if (cudaMemsetAsync(me->changed, 0, sizeof(int) * (size_t)me->sweep_limit, ctx->stream) != cudaSuccess)
                 crc = VPPGPU_ERR_CUDA;
-            if (!crc) crc = vppgpu::full_launch(ctx, a, *me->maps, me->nmb, me->resolve_grid, nullptr);
+            if (!crc) crc = vppgpu::full_launch(ctx, a, me->nmb, nullptr);
             const cudaError_t e = cudaStreamEndCapture(ctx->stream, &g);
             if (!crc && e == cudaSuccess && g && cudaGraphInstantiate(&me->graph, g, 0) == cudaSuccess) {
                 me->graph_state = 1;
@@ -295,7 +297,7 @@ int run(vppgpu_me* me, const short* d_src16, const short* d_ref16, const unsigne
         return VPPGPU_OK;
     }
     VPP_CUDA(cudaMemsetAsync(me->changed, 0, sizeof(int) * (size_t)me->sweep_limit, ctx->stream));
-    return vppgpu::full_launch(ctx, a, *me->maps, me->nmb, me->resolve_grid, ev);
+    return vppgpu::full_launch(ctx, a, me->nmb, ev);
 }
 
 int status_from_ctrl(const vppgpu::MeCtrl& c) { return vppgpu::status_from_bits(c.status); }
@@ -482,7 +484,7 @@ int vppgpu_me_create(vppgpu_ctx* ctx, int kind, int width, int height, int motio
             me_free(me);
             return VPPGPU_ERR_OUT_OF_MEMORY;
         }
-        if ((rc = vppgpu::full_prepare(ctx, me->nmb, &me->resolve_grid))) {
+        if ((rc = vppgpu::full_prepare(ctx))) {
             me_free(me);
             return rc;
         }
@@ -583,7 +585,7 @@ int vppgpu_me_create(vppgpu_ctx* ctx, int kind, int width, int height, int motio
             me_free(me);
             return VPPGPU_ERR_OUT_OF_MEMORY;
         }
-        if ((rc = vppgpu::full_prepare(ctx, me->nmb, &me->resolve_grid))) {
+        if ((rc = vppgpu::full_prepare(ctx))) {
             me_free(me);
             return rc;
         }
@@ -594,7 +596,7 @@ int vppgpu_me_create(vppgpu_ctx* ctx, int kind, int width, int height, int motio
         (rc = dalloc(&me->d_refp, npad)) || (rc = dalloc(&me->d_hpel, 3 * npad)) ||
         (rc = dalloc(&me->spec, 5 * (size_t)me->nmb)) ||
         (rc = dalloc(&me->tables, (size_t)me->nmb * 64 * 64)) ||
-        (kind == VPPGPU_ME_FULL && (rc = dalloc(&me->energy, npad))) || (rc = dalloc(&me->d_job, 1)) || (rc = dalloc(&me->tie_list, me->nmb)) || (rc = dalloc(&me->state, 3 * (size_t)me->nmb)) ||
+        (kind == VPPGPU_ME_FULL && ((rc = dalloc(&me->energy, npad)) || (rc = dalloc(&me->rowmin, 512 * (size_t)me->nmb)))) || (rc = dalloc(&me->d_job, 1)) || (rc = dalloc(&me->tie_list, me->nmb)) || (rc = dalloc(&me->state, 3 * (size_t)me->nmb)) ||
         (rc = dalloc(&me->d_out_mv, me->nmb)) || (rc = dalloc(&me->d_out_dist, me->nmb)) ||
         (rc = dalloc(&me->d_out_avg, 1)) || (rc = dalloc(&me->d_incl, me->nmb)) ||
         (rc = dalloc(&me->d_slice, me->nmb)) || (rc = dalloc(&me->ctrl, 1)) ||
@@ -606,11 +608,11 @@ int vppgpu_me_create(vppgpu_ctx* ctx, int kind, int width, int height, int motio
         me_free(me);
         return VPPGPU_ERR_OUT_OF_MEMORY;
     }
-    if ((rc = vppgpu::full_prepare(ctx, me->nmb, &me->resolve_grid))) {
+    if ((rc = vppgpu::full_prepare(ctx))) {
         me_free(me);
         return rc;
     }
-    if (kind == VPPGPU_ME_FULL || kind == VPPGPU_ME_FULL_SAD) {
+    if (kind == VPPGPU_ME_FULL_SAD) {
         me->maps = new (std::nothrow) vppgpu::SearchMaps();
         if (!me->maps) {
             me_free(me);

@@ -37,12 +37,7 @@ __device__ __forceinline__ int tap6(int a, int b, int c, int d, int e, int f)
 }
 
 // Sum over the warp (every lane gets it).
-__device__ __forceinline__ int warp_sum(int v)
-{
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-    return v;
-}
+__device__ __forceinline__ int warp_sum(int v) { return __reduce_add_sync(0xffffffffu, v); }
 
 // ---------------------------------------------------------------------------
 // Median prediction (MacroBlockH264::GetMbMotionMedianPred,

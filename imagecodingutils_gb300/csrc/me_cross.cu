@@ -62,7 +62,7 @@ int cross_launch(vppgpu_ctx* ctx, const FullArgs& args)
     VPP_CHECK_LAUNCH(ctx);
     k_cross_tietree<<<ctx->sm_count * 2, mrc::V2_TIE_RUNS * 32, 0, ctx->stream>>>(args);
     VPP_CHECK_LAUNCH(ctx);
-    return full_resolve_launch(ctx, args, 0, cross::EST_CROSS);
+    return full_resolve_launch(ctx, args, cross::EST_CROSS);
 }
 
 }  // namespace vppgpu

@@ -14,17 +14,20 @@
 //                   predicted vector) and the 16x16 block energies (the B^2 of
 //                   every candidate's SSD = A^2 + B^2 - 2 sum(ab)); the input's
 //                   byte packing rides along.
-//   k_full_search   persistent, warp-specialised: compute warps build each
-//                   macroblock's (2R+1)^2 SSD table in shared memory (cross
-//                   terms with dp4a, tiles staged by TMA tensor copies), a scan
-//                   warp replays the reference's sequential raster scan over
-//                   it (rows whose minimum or range cannot win are skipped).
-//                   Only the tables of macroblocks whose scan met an exact tie
-//                   leave the SM (for their tie tree).
-//   k_full_subpel   half-pel then quarter-pel refinement, a warp per MB.
-//   k_full_tietree  for the tie MBs, the scan outcome of every tie decision
-//                   pattern (the tie tree), read by the prediction-dependent
-//                   stage.
+//   k_ssd_rowmin    (me_full_tc.cu) the minimum SSD of every 8 neighbouring
+//                   candidates of every macroblock, by the tensor cores.
+//   k_full_scan     a warp per MB: replays the reference's sequential raster
+//                   scan, forming the SSDs of the few groups of candidates
+//                   whose minimum and range can win, then the half-pel and
+//                   quarter-pel refinement.
+//   k_full_tietree  for the MBs whose scan met an exact tie, the whole table
+//                   and the scan outcome of every tie decision pattern (the
+//                   tie tree), read by the prediction-dependent stage.
+//   k_sad_search    the SAD search's table: persistent, warp-specialised:
+//                   compute warps build each macroblock's (2R+1)^2 table in
+//                   shared memory (vabsdiff4, tiles staged by TMA tensor
+//                   copies), a scan warp replays the scan over it.  Only the
+//                   tables of tie macroblocks leave the SM.
 //   resolve         (me_full_resolve.cu) the prediction-dependent tail:
 //                   median prediction, tie rescans, prediction distortion
 //                   and the Lagrangian pick, in the reference's raster order.
@@ -39,11 +42,6 @@ namespace vppgpu {
 namespace {
 using namespace full;
 
-struct TieSmem {
-    alignas(16) int tab[TAB][TAB];
-    int run[TIE_RUNS][sizeof(TieRun) / sizeof(int)];
-};
-
 // ---------------------------------------------------------------------------
 // The frame's planes in one pass, a CTA per PL_TX x PL_TY tile of the padded
 // reference (PAD samples of edge replication each side, OverlayExtMem2Dv2's
@@ -55,8 +53,9 @@ struct TieSmem {
 //           clipped to 0..255 -- the samples QuarterRead combines
 //           (OverlayMem2Dv2.cpp:704-1052)
 //   energy  (SSD search only) E(Y, X) = sum of squares of the 16x16 block at
-//           (Y, X), for Y <= PH-16, X <= PW-16: the B^2 term of every
-//           candidate's SSD = A^2 + B^2 - 2 sum(ab)
+//           (Y, X), its samples less 128, for Y <= PH-16, X <= PW-16: the B^2
+//           term of every candidate's SSD = A^2 + B^2 - 2 sum(ab); below 2^23,
+//           stored as the floats the row minima are formed with
 // plus a share of the input's byte packing (src8, 0..255 checked).  The tile
 // and its halo (2 before, 15 after in each direction) are staged once as
 // bytes; taps read clamped coordinates, which differs from a clamped padded
@@ -73,7 +72,7 @@ __device__ __forceinline__ unsigned char clip_tap(int v, int round, int shift)
 __global__ void __launch_bounds__(256) k_full_planes(const JobDesc* __restrict__ job, int W, int H, int rstride,
                                                      unsigned char* __restrict__ src8, unsigned char* __restrict__ refp,
                                                      unsigned char* __restrict__ hpel, size_t plane_size,
-                                                     int* __restrict__ energy, int* status)
+                                                     float* __restrict__ energy, int* status)
 {
     __shared__ __align__(16) unsigned char px[PL_SY][PL_SX];
     __shared__ short vt[PL_TY][PL_TX + 5];            // unrounded vertical taps, columns X0-2 .. X0+66
@@ -119,11 +118,11 @@ __global__ void __launch_bounds__(256) k_full_planes(const JobDesc* __restrict__
             const unsigned char* p = &px[r + 2][c0 + 2];
             int acc = 0;
 #pragma unroll
-            for (int d = 0; d < 16; d++) acc += p[d] * p[d];
+            for (int d = 0; d < 16; d++) acc += (p[d] - 128) * (p[d] - 128);
             hs[r][c0] = acc;
 #pragma unroll
-            for (int c = 1; c < 16; c++) {
-                acc += p[c + 15] * p[c + 15] - p[c - 1] * p[c - 1];
+            for (int c = 1; c < 16; c++) {  // (u - 128)^2 - (v - 128)^2
+                acc += (p[c + 15] - p[c - 1]) * (p[c + 15] + p[c - 1] - 256);
                 hs[r][c0 + c] = acc;
             }
         }
@@ -162,7 +161,7 @@ __global__ void __launch_bounds__(256) k_full_planes(const JobDesc* __restrict__
             for (int r = r0; r < r0 + 16; r++) {
                 if (r > r0) acc += hs[r + 15][c] - hs[r - 1][c];
                 const int Y = Y0 + r;
-                if (X <= PW - 16 && Y <= PH - 16) energy[(size_t)Y * rstride + X] = acc;
+                if (X <= PW - 16 && Y <= PH - 16) energy[(size_t)Y * rstride + X] = (float)acc;
             }
         }
     }
@@ -182,7 +181,7 @@ __device__ __forceinline__ unsigned sad4_add(unsigned a, unsigned b, unsigned c)
 // Search stage: one persistent CTA per slot (SEARCH_CTAS_PER_SM per SM),
 // macroblocks blockIdx.x, blockIdx.x + gridDim.x, ...; warp-specialised.
 //
-//   compute warps      the SSD (kSad: the SAD, OverlayMem2Dv2::Tad16x16,
+//   compute warps      the SAD (OverlayMem2Dv2::Tad16x16,
 //                      OverlayMem2Dv2.cpp:2655-2730) of all (2R+1)^2 full-pel
 //                      candidates of a macroblock into a shared-memory table,
 //                      with its row minima; warp 0 also stages the next
@@ -190,44 +189,35 @@ __device__ __forceinline__ unsigned sad4_add(unsigned a, unsigned b, unsigned c)
 //   scan warp (1)      the reference's sequential raster scan over each
 //                      table (prediction (0, 0) for ties, Full.cpp:394-446);
 //                      tables of macroblocks whose scan met an exact tie go to
-//                      global memory for their tie tree; then, in the buffer
-//                      it released, it stages the energies of the candidates
-//                      two macroblocks on (a TMA copy; the SSDs overwrite them
-//                      in place), so the compute warps never wait for a scan
-//                      unless it falls two tables behind.  The sub-pel stages
-//                      follow in k_full_subpel, whose global-memory round trips
-//                      would otherwise lengthen the scan warp's chain.
+//                      global memory for their tie tree; then it releases the
+//                      buffer, so the compute warps wait for a scan only when
+//                      it falls two tables behind
 //
 // Two window buffers and two table buffers; the hand-offs are shared-memory
 // barriers (mbarrier) whose waits are bounded: a wait that runs out sets
 // ST_TIMEOUT and every role leaves, after the copies it issued landed.
 // Launch shape, measured on 1080p frames: 8 candidate rows per thread with the
 // template rows in two passes of the ring's period (a loop body small enough
-// for the instruction cache; the full 16-step unroll stalled on instruction
-// fetch, 0.179 against 0.167 ms), at 3 CTAs per SM, where the loop needs no
-// spills (4 CTAs with a 96-register cap: the same time; 4 candidate rows per
-// thread, i.e. 8 compute warps, took 0.182 ms at 3 CTAs and 0.190 ms at 2).
+// for the instruction cache), at 3 CTAs per SM, where the loop needs no spills.
 constexpr int SEARCH_ROWS = 8;    // candidate rows per thread (the window-row ring's period)
 constexpr int SEARCH_UNROLL = 8;  // template rows per unrolled loop body (a multiple of SEARCH_ROWS)
 constexpr int SEARCH_WARPS = 64 / (2 * SEARCH_ROWS);  // compute warps: 2 row groups of a warp each
 constexpr int SEARCH_THREADS = 32 * (SEARCH_WARPS + 1);
 constexpr int SEARCH_CTAS_PER_SM = 3;
 constexpr unsigned WIN_BYTES = WROWS * WSTRIDE + 256;     // window rows + template
-constexpr unsigned E_BYTES = (2 * RMAX + 1) * TAB * 4;    // candidate rows of energies
 // one window, 128-byte aligned, with room for a row 78 that the TMA box does
 // not fill (only the unused candidate row 63 reads it)
 constexpr int WIN_BUF = (WROWS * WSTRIDE + WSTRIDE + 127) / 128 * 128;
 static_assert(SEARCH_UNROLL % SEARCH_ROWS == 0 && 16 % SEARCH_UNROLL == 0, "unroll must cover ring periods");
 
 struct SearchSmem {
-    alignas(128) int tab[2][TAB][TAB];  // rows 0 .. 2R: SSDs (column 0: row minima)
+    alignas(128) int tab[2][TAB][TAB];  // rows 0 .. 2R: SADs (column 0: row minima)
     alignas(128) unsigned char win[2][WIN_BUF];  // WROWS rows of WSTRIDE bytes
     alignas(128) unsigned char cur[2][256];
     unsigned long long wfull[2];   // window b staged
     unsigned long long wfree[2];   // window b read by every compute thread
-    unsigned long long efull[2];   // SSD: energies staged in table b (the scan released it)
     unsigned long long tfull[2];   // table b written by every compute thread
-    unsigned long long tempty[2];  // SAD: table b released by the scan warp
+    unsigned long long tempty[2];  // table b released by the scan warp
     int abort;
 };
 
@@ -258,9 +248,8 @@ __device__ __forceinline__ void search_drain(unsigned long long* bars, int from,
     }
 }
 
-template <bool kSad>
 __global__ void __launch_bounds__(SEARCH_THREADS, SEARCH_CTAS_PER_SM)
-    k_full_search(FullArgs a, const __grid_constant__ SearchMaps maps)
+    k_sad_search(FullArgs a, const __grid_constant__ SearchMaps maps)
 {
     extern __shared__ __align__(128) unsigned char smem_raw[];
     SearchSmem& S = *reinterpret_cast<SearchSmem*>(smem_raw);
@@ -271,7 +260,6 @@ __global__ void __launch_bounds__(SEARCH_THREADS, SEARCH_CTAS_PER_SM)
         for (int b = 0; b < 2; b++) {
             mbar_init(&S.wfull[b], 1);
             mbar_init(&S.wfree[b], 32 * SEARCH_WARPS);
-            mbar_init(&S.efull[b], 1);
             mbar_init(&S.tfull[b], 32 * SEARCH_WARPS);
             mbar_init(&S.tempty[b], 32);
         }
@@ -312,11 +300,11 @@ __global__ void __launch_bounds__(SEARCH_THREADS, SEARCH_CTAS_PER_SM)
             }
             if (!search_wait(&S.wfull[b], use, a, abort)) break;
 
-            // cross terms with dp4a (kSad: vabsdiff4 with accumulate); each thread:
+            // vabsdiff4 with accumulate; each thread:
             // SEARCH_ROWS candidate rows x 4 word offsets, one byte shift s.  Each window
             // row is byte-aligned once for the thread's shift (funnel shifts: word i holds
             // bytes 4i+s .. 4i+s+3 of the thread's 32-byte slice) and kept in a ring of
-            // SEARCH_ROWS rows; every 16-pixel row product is then 4 dp4a against the
+            // SEARCH_ROWS rows; every 16-pixel row is then 4 of them against the
             // template row.
             unsigned acc[SEARCH_ROWS][4];
             {
@@ -348,8 +336,7 @@ __global__ void __launch_bounds__(SEARCH_THREADS, SEARCH_CTAS_PER_SM)
                             for (int q = 0; q < 4; q++) {
                                 unsigned c = acc[r][q];
 #pragma unroll
-                                for (int w = 0; w < 4; w++)
-                                    c = kSad ? sad4_add(A[w], B[q + w], c) : __dp4a(A[w], B[q + w], c);
+                                for (int w = 0; w < 4; w++) c = sad4_add(A[w], B[q + w], c);
                                 acc[r][q] = c;
                             }
                         }
@@ -357,21 +344,9 @@ __global__ void __launch_bounds__(SEARCH_THREADS, SEARCH_CTAS_PER_SM)
                     }
                 }
             }
-            // template energy
-            int a2 = 0;
-            if (!kSad) {
-#pragma unroll
-                for (int t = 0; t < 8; t++) {
-                    const int v = S.cur[b][lane + 32 * t];
-                    a2 += v * v;
-                }
-                a2 = warp_sum(a2);
-            }
             mbar_arrive(&S.wfree[b]);  // this thread is done with window b and its template
 
-            // the table buffer: its energies staged (the scan warp stages them once it released
-            // the buffer), or, for the SAD, released
-            if (!search_wait(kSad ? &S.tempty[b] : &S.efull[b], kSad ? use ^ 1u : use, a, abort)) break;
+            if (!search_wait(&S.tempty[b], use ^ 1u, a, abort)) break;  // the scan warp released the table
             const int k = mb_of(it);
             const int n = (k % a.cols) * 16, m = (k / a.cols) * 16;
             int xl, xr, yu, yd;
@@ -383,7 +358,7 @@ __global__ void __launch_bounds__(SEARCH_THREADS, SEARCH_CTAS_PER_SM)
 #pragma unroll
                 for (int q = 0; q < 4; q++) {
                     const int jj = 16 * qg + 4 * q + s;
-                    v[q] = kSad ? (int)acc[r][q] : a2 + (ii < 2 * RMAX + 1 ? S.tab[b][ii][jj] : 0) - 2 * (int)acc[r][q];
+                    v[q] = (int)acc[r][q];
                     const int j = jj - RMAX - 1;
                     if (j >= xl && j <= xr) mn = min(mn, v[q]);
                 }
@@ -402,20 +377,6 @@ __global__ void __launch_bounds__(SEARCH_THREADS, SEARCH_CTAS_PER_SM)
         if (warp == 0) search_drain(S.wfull, it, wissued, a.spin_limit);
     } else {
         // ---------------- scan warp ----------------
-        // energies of iteration `it`'s candidates into table buffer it & 1 (SSD)
-        auto stage_energy = [&](int it) {
-            if (lane == 0) {
-                const int b = it & 1, k = mb_of(it);
-                const int n = (k % a.cols) * 16, m = (k / a.cols) * 16;
-                mbar_expect_tx(&S.efull[b], E_BYTES);
-                tma_load_2d(&S.tab[b][0][0], &maps.energy, n - 32 + PAD, m - 31 + PAD, &S.efull[b]);
-            }
-        };
-        int eissued = 0;  // energies staged for iterations 0 .. eissued-1
-        if (!kSad) {      // both table buffers start free
-            eissued = min(nit, 2);
-            for (int i = 0; i < eissued; i++) stage_energy(i);
-        }
         int it = 0;
         for (; it < nit; it++) {
             const int b = it & 1;
@@ -432,13 +393,8 @@ __global__ void __launch_bounds__(SEARCH_THREADS, SEARCH_CTAS_PER_SM)
                 for (int i = lane; i < (2 * RMAX + 1) * TAB / 4; i += 32) __stcg(dst + i, src[i]);
             }
             __syncwarp();
-            if (kSad) {
-                mbar_arrive(&S.tempty[b]);
-            } else if (it + 2 < nit) {
-                stage_energy(it + 2);  // the buffer is released: the table two iterations on
-                eissued = it + 3;
-            }
-            if (lane == 0) {  // the full-pel result; k_full_subpel refines it (SSD search)
+            mbar_arrive(&S.tempty[b]);
+            if (lane == 0) {  // the full-pel result
                 const int qmv = pack_mv(4 * mx, 4 * my);
                 const int av = neighbour_mask(a.job->slice, k, a.cols, a.nmb / a.cols);
                 a.spec4[k] = make_int4(qmv, minD, zero_d, (tie ? FLAG_TIE : 0) | av);
@@ -447,51 +403,218 @@ __global__ void __launch_bounds__(SEARCH_THREADS, SEARCH_CTAS_PER_SM)
                 if (tie) a.tie_list[atomicAdd(&a.ctrl->ntie, 1)] = k;
             }
         }
-        if (!kSad) search_drain(S.efull, it, eissued, a.spin_limit);
     }
 }
 
-// Half-pel then quarter-pel refinement around each macroblock's full-pel
-// winner (Full.cpp:452-517), one warp per macroblock, many per SM: the
-// prediction-independent result the resolve starts from.
-__global__ void __launch_bounds__(256) k_full_subpel(FullArgs a)
+// The window of macroblock (n, m)'s candidates in shared memory: WROWS rows
+// from m - 31, columns n - 32 .. n + 47.  At this pitch (22 words) 16 rows at
+// one column, and the word beside it, lie in 32 different banks.
+constexpr int SCAN_PITCH = 88;
+constexpr int SCAN_WIN = WROWS * SCAN_PITCH;
+
+__device__ __forceinline__ void stage_window(const FullArgs& a, int n, int m, unsigned char* win, int tid, int nthreads)
 {
-    const int lane = threadIdx.x & 31, k = blockIdx.x * 8 + (threadIdx.x >> 5);
+    const unsigned char* src = a.refp + (size_t)(m - RMAX + PAD) * a.rstride + n - RMAX - 1 + PAD;
+    // five 16-byte pieces a row, six rows a warp and step (lanes 30 and 31 idle)
+    const int lane = tid & 31, step = 6 * (nthreads >> 5), q = lane % 5, r0 = 6 * (tid >> 5) + lane / 5;
+    if (lane >= 30) return;
+    const unsigned char* p = src + (size_t)r0 * a.rstride + 16 * q;
+    unsigned char* d = win + r0 * SCAN_PITCH + 16 * q;
+#pragma unroll 13
+    for (int r = r0; r < WROWS; r += step) {
+        const uint4 v = __ldg(reinterpret_cast<const uint4*>(p));
+        reinterpret_cast<uint2*>(d)[0] = make_uint2(v.x, v.y);
+        reinterpret_cast<uint2*>(d)[1] = make_uint2(v.z, v.w);
+        p += (size_t)step * a.rstride;
+        d += step * SCAN_PITCH;
+    }
+}
+
+// This lane's row of the template (row lane / 2).
+__device__ __forceinline__ uint4 template_row(const FullArgs& a, int n, int m, int lane)
+{
+    return __ldg(reinterpret_cast<const uint4*>(a.src8 + (size_t)(m + (lane >> 1)) * a.W + n));
+}
+
+// The SSDs of the 8 candidates in table columns 8g .. 8g+7 of candidate row ii
+// (i + RMAX): lane c < 8 gets column 8g + c.  One warp, a lane four candidates
+// on one template row, which read five words of one window row.
+__device__ __forceinline__ int group_ssd(const unsigned char* win, uint4 t, int ii, int g, int lane)
+{
+    const unsigned* q = reinterpret_cast<const unsigned*>(win + (ii + (lane >> 1)) * SCAN_PITCH + 8 * g + 4 * (lane & 1));
+    const unsigned w[5] = {q[0], q[1], q[2], q[3], q[4]}, tw[4] = {t.x, t.y, t.z, t.w};
+    unsigned acc[4] = {0u, 0u, 0u, 0u};
+#pragma unroll
+    for (int s = 0; s < 4; s++)
+#pragma unroll
+        for (int i = 0; i < 4; i++) {
+            const unsigned d = __vabsdiffu4(tw[i], s ? __funnelshift_r(w[i], w[i + 1], 8 * s) : w[i]);
+            acc[s] = __dp4a(d, d, acc[s]);
+        }
+    // over the 16 template rows; a lane keeps two, then one of its candidates: 4 (lane & 1) + 2 (bit 4) + bit 3
+    const bool b4 = lane & 16, b3 = lane & 8;
+    const unsigned u0 = (b4 ? acc[2] : acc[0]) + __shfl_xor_sync(0xffffffffu, b4 ? acc[0] : acc[2], 16);
+    const unsigned u1 = (b4 ? acc[3] : acc[1]) + __shfl_xor_sync(0xffffffffu, b4 ? acc[1] : acc[3], 16);
+    unsigned v = (b3 ? u1 : u0) + __shfl_xor_sync(0xffffffffu, b3 ? u0 : u1, 8);
+    v += __shfl_xor_sync(0xffffffffu, v, 4);
+    v += __shfl_xor_sync(0xffffffffu, v, 2);
+    return (int)__shfl_sync(0xffffffffu, v, ((lane >> 2) & 1) | ((lane & 2) << 3) | ((lane & 1) << 3));
+}
+
+// The reference's integer scan of each macroblock (prediction (0, 0) for ties,
+// Full.cpp:394-446, see scan_table_t) and the half-pel then quarter-pel
+// refinement around its winner (Full.cpp:452-517), one warp per macroblock:
+// the prediction-independent result the resolve starts from.
+//
+// A group of 8 candidates (a.rowmin) can accept one only if its minimum is at
+// or below the running minimum and some of its columns are in range of the
+// running best (the skip rule adds the best's vector to the candidate's).  A
+// lane holds the minima of two candidate rows; the first row that has such a
+// minimum is visited next, and only such groups' SSDs are formed: on a 1080p
+// pan 6 rows and 7.5 groups a macroblock.
+constexpr int SCAN_WARPS = 4;
+__global__ void __launch_bounds__(32 * SCAN_WARPS) k_full_scan(const __grid_constant__ FullArgs a)
+{
+    __shared__ __align__(16) unsigned char s_win[SCAN_WARPS][SCAN_WIN];
+    __shared__ __align__(16) int s_min[SCAN_WARPS][64][8];  // the groups' minima, rows yu ..
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, k = blockIdx.x * SCAN_WARPS + w;
     if (k >= a.nmb) return;
     const int n = (k % a.cols) * 16, m = (k / a.cols) * 16;
-    const int imv = __ldcg(a.spec_imv + k);
-    const int mx = mv_x(imv), my = mv_y(imv);
-    int minD = __ldcg(&a.spec4[k].y), qmx = 0, qmy = 0;
-    subpel_refine_planes(a, n + mx, m + my, load_cur8(a, n, m, lane), lane, &minD, &qmx, &qmy);
+    const unsigned char* win = s_win[w];
+    const uint2 cur = load_cur8(a, n, m, lane);
+    const uint2 at0 = *reinterpret_cast<const uint2*>(even_block(a, n, m, 0, 0, lane));
+    const uint4 t = template_row(a, n, m, lane);
+    constexpr int kNone = 0x7fffffff;
+    int xl, xr, yu, yd;
+    full_range(n, m, a.W, a.H, a.motion_range, xl, xr, yu, yd);
+    float4 p[2][2];
+#pragma unroll
+    for (int h = 0; h < 2; h++) {
+        const float4* q = reinterpret_cast<const float4*>(a.rowmin + ((size_t)k * 64 + min(yu + lane + 32 * h, yd) + RMAX) * 8);
+        p[h][0] = __ldcg(q);
+        p[h][1] = __ldcg(q + 1);
+    }
+    stage_window(a, n, m, s_win[w], lane, 32);
+    // A^2 of the samples less 128, which the minima are without
+    const int c0 = (int)(cur.x ^ 0x80808080u), c1 = (int)(cur.y ^ 0x80808080u);
+    const int energy = warp_sum(__dp4a(c0, c0, __dp4a(c1, c1, 0)));
+    const int ga = (xl + 32) >> 3, gb = (xr + 32) >> 3;  // groups that hold candidates
+    int rm[2];
+#pragma unroll
+    for (int h = 0; h < 2; h++) {
+        const float f[8] = {p[h][0].x, p[h][0].y, p[h][0].z, p[h][0].w, p[h][1].x, p[h][1].y, p[h][1].z, p[h][1].w};
+        int v[8];
+        rm[h] = kNone;
+#pragma unroll
+        for (int g = 0; g < 8; g++) {
+            v[g] = g >= ga && g <= gb ? energy + (int)f[g] : kNone;
+            rm[h] = min(rm[h], v[g]);
+        }
+        int4* d = reinterpret_cast<int4*>(s_min[w][lane + 32 * h]);
+        d[0] = make_int4(v[0], v[1], v[2], v[3]);
+        d[1] = make_int4(v[4], v[5], v[6], v[7]);
+    }
+    __syncwarp();
+    const int zero_d = warp_sum(ssd8(cur, at0));
+
+    int minD = zero_d, mx = 0, my = 0, tie = 0;
+    int done = 0;  // rows yu .. yu+done-1 are behind the scan
+    while (true) {
+        const int r0 = yu + lane + my, r1 = r0 + 32;
+        const unsigned m0 = __ballot_sync(0xffffffffu, rm[0] <= minD && lane >= done && r0 >= yu && r0 <= yd &&
+                                                           yu + lane <= yd);
+        const unsigned m1 = __ballot_sync(0xffffffffu, rm[1] <= minD && lane + 32 >= done && r1 >= yu && r1 <= yd &&
+                                                           yu + lane + 32 <= yd);
+        if (!m0 && !m1) break;
+        const int off = m0 ? __ffs(m0) - 1 : 31 + __ffs(m1), i = yu + off;
+        done = off + 1;
+        const int gmin = s_min[w][off][lane & 7], jl = 8 * (lane & 7) - 32;  // lane g: the row's group g
+        unsigned left = 0xffu;  // groups not yet behind the scan
+        while (i + my >= yu && i + my <= yd) {
+            // the next group of the row that can accept, at the best as it is
+            const unsigned can = __ballot_sync(0xffffffffu, gmin <= minD && jl + 7 + mx >= xl && jl + mx <= xr) & left;
+            if (!can) break;
+            const int g = __ffs(can) - 1;
+            left &= ~((2u << g) - 1u);
+            const int d = group_ssd(win, t, i + RMAX, g, lane);
+            const int base = 8 * g - 32, j = base + lane;
+            const bool valid = lane < 8 && j >= xl && j <= xr && !(i == 0 && j == 0);
+            unsigned pending = 0xffu;
+            while (true) {
+                const bool ok = valid && d <= minD && i + my >= yu && i + my <= yd && j + mx >= xl && j + mx <= xr;
+                const unsigned b = __ballot_sync(0xffffffffu, ok) & pending;
+                if (!b) break;
+                const int f = __ffs(b) - 1, df = __shfl_sync(0xffffffffu, d, f), jf = base + f;
+                bool accept = true;
+                if (df == minD) {
+                    tie = 1;
+                    accept = (my * my + mx * mx) - (i * i + jf * jf) >= 0;
+                }
+                if (accept) {
+                    minD = df;
+                    mx = jf;
+                    my = i;
+                }
+                pending &= ~((2u << f) - 1u);
+            }
+        }
+    }
+    int qmx, qmy;
+    subpel_refine_planes(a, n + mx, m + my, cur, lane, &minD, &qmx, &qmy);
     if (lane == 0) {
         const int qmv = pack_mv(4 * mx + qmx, 4 * my + qmy);
-        a.spec4[k].x = qmv;
-        a.spec4[k].y = minD;
+        const int av = neighbour_mask(a.job->slice, k, a.cols, a.nmb / a.cols);
+        a.spec4[k] = make_int4(qmv, minD, zero_d, (tie ? FLAG_TIE : 0) | av);
+        a.spec_imv[k] = pack_mv(mx, my);
         __stcg(a.final_mv + k, qmv);
+        if (tie) a.tie_list[atomicAdd(&a.ctrl->ntie, 1)] = k;
     }
 }
 
 // ---------------------------------------------------------------------------
 // Tie trees of the listed macroblocks (see TieRun), one CTA per MB: the table
-// in shared memory, warp p computes run p (forced scan, then the sub-pel
-// stage of its winner when that is not the searched one).  FLAG_DEEP when a
-// run reachable by some prediction met more ties than the tree holds (the
-// prediction-dependent stage then rescans).
-__global__ void __launch_bounds__(TIE_RUNS * 32) k_full_tietree(FullArgs a)
+// in shared memory (kSad: the search kept it; else formed here, warp p the rows
+// p, p + 8, ..), warp p computes run p (forced scan, then the sub-pel stage of
+// its winner when that is not the searched one).  FLAG_DEEP when a run
+// reachable by some prediction met more ties than the tree holds (the
+// prediction-dependent stage then rescans the kept table).
+struct TieSmem {
+    alignas(16) int tab[TAB][TAB];
+    int run[TIE_RUNS][sizeof(TieRun) / sizeof(int)];
+    int deep;
+    alignas(16) unsigned char win[SCAN_WIN];
+};
+
+template <bool kSad>
+__global__ void __launch_bounds__(TIE_RUNS * 32) k_full_tietree(const __grid_constant__ FullArgs a)
 {
     extern __shared__ __align__(16) unsigned char tie_smem[];
     TieSmem& S = *reinterpret_cast<TieSmem*>(tie_smem);
     const int tid = threadIdx.x, lane = tid & 31, p = tid >> 5;
     const int ntie = *((volatile int*)&a.ctrl->ntie);
+    constexpr int kWords = (2 * RMAX + 1) * TAB / 4;
     for (int t = blockIdx.x; t < ntie; t += gridDim.x) {
         const int k = a.tie_list[t];
         const int n = (k % a.cols) * 16, m = (k / a.cols) * 16;
         int* gt = a.tables + (size_t)k * TAB * TAB;
-        for (int i = tid; i < (2 * RMAX + 1) * TAB / 4; i += blockDim.x)
-            reinterpret_cast<int4*>(&S.tab[0][0])[i] = __ldcg(reinterpret_cast<const int4*>(gt) + i);
-        __syncthreads();
         int xl, xr, yu, yd;
         full_range(n, m, a.W, a.H, a.motion_range, xl, xr, yu, yd);
+        if constexpr (kSad) {
+            for (int i = tid; i < kWords; i += blockDim.x)
+                reinterpret_cast<int4*>(&S.tab[0][0])[i] = __ldcg(reinterpret_cast<const int4*>(gt) + i);
+        } else {
+            const uint4 tm = template_row(a, n, m, lane);
+            stage_window(a, n, m, S.win, tid, blockDim.x);
+            __syncthreads();
+            for (int ii = p; ii < 2 * RMAX + 1; ii += TIE_RUNS)
+                for (int g = 0; g < TAB / 8; g++) {
+                    const int v = group_ssd(S.win, tm, ii, g, lane);
+                    if (lane < 8) S.tab[ii][8 * g + lane] = v;
+                }
+            __syncthreads();
+            table_row_minima(S.tab, xl, xr, yu, yd, p, TIE_RUNS, lane);
+        }
+        __syncthreads();
         const int4 sp = a.spec4[k];
         const int imv = a.spec_imv[k];
         int rmx, rmy, rmin, rt, nev, ev[TIE_DEPTH] = {0, 0, 0};
@@ -499,7 +622,7 @@ __global__ void __launch_bounds__(TIE_RUNS * 32) k_full_tietree(FullArgs a)
         int rq = sp.x, rqmin = sp.y;
         if (rmx != mv_x(imv) || rmy != mv_y(imv)) {
             int sx = 0, sy = 0;
-            if (!a.intpel) subpel_refine_planes(a, n + rmx, m + rmy, load_cur8(a, n, m, lane), lane, &rmin, &sx, &sy);
+            if (!kSad) subpel_refine_planes(a, n + rmx, m + rmy, load_cur8(a, n, m, lane), lane, &rmin, &sx, &sy);
             rq = pack_mv(4 * rmx + sx, 4 * rmy + sy);
             rqmin = rmin;
         }
@@ -526,7 +649,12 @@ __global__ void __launch_bounds__(TIE_RUNS * 32) k_full_tietree(FullArgs a)
                 deep |= reach[q] && S.run[q][3] < 0;
             }
             if (deep) a.spec4[k].w = sp.w | FLAG_DEEP;
+            S.deep = deep;
         }
+        __syncthreads();
+        if (!kSad && S.deep)
+            for (int i = tid; i < kWords; i += blockDim.x)
+                __stcg(reinterpret_cast<int4*>(gt) + i, reinterpret_cast<const int4*>(&S.tab[0][0])[i]);
         __syncthreads();
     }
 }
@@ -548,7 +676,7 @@ int full_planes_launch(vppgpu_ctx* ctx, const FullArgs& args)
     dim3 grid((PW + PL_TX - 1) / PL_TX, (PH + PL_TY - 1) / PL_TY);
     k_full_planes<<<grid, 256, 0, ctx->stream>>>(args.job, args.W, args.H, args.rstride, (unsigned char*)args.src8,
                                                  (unsigned char*)args.refp, (unsigned char*)args.hpel, args.plane_size,
-                                                 const_cast<int*>(args.energy), &args.ctrl->status);
+                                                 const_cast<float*>(args.energy), &args.ctrl->status);
     VPP_CHECK_LAUNCH(ctx);
     return VPPGPU_OK;
 }
@@ -599,29 +727,23 @@ int search_maps_encode(const FullArgs& a, SearchMaps* maps)
     const int PW = a.W + 2 * PAD, PH = a.H + 2 * PAD;
     int rc = encode_2d(&maps->win, a.refp, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, PW, PH, (size_t)a.rstride, WSTRIDE, WROWS);
     if (!rc) rc = encode_2d(&maps->cur, a.src8, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, a.W, a.H, (size_t)a.W, 16, 16);
-    if (!rc && a.energy)
-        rc = encode_2d(&maps->energy, a.energy, CU_TENSOR_MAP_DATA_TYPE_INT32, 4, PW, PH, (size_t)a.rstride * 4, TAB,
-                       2 * RMAX + 1);
     return rc;
 }
 
-int full_launch(vppgpu_ctx* ctx, const FullArgs& args, const SearchMaps& maps, int nmb, int resolve_grid,
-                cudaEvent_t* ev)
+int full_launch(vppgpu_ctx* ctx, const FullArgs& args, int nmb, cudaEvent_t* ev)
 {
     if (ev) VPP_CUDA(cudaEventRecord(ev[0], ctx->stream));
     int rc = full_planes_launch(ctx, args);  // with the block energies (args.energy)
     if (rc) return rc;
     if (ev) VPP_CUDA(cudaEventRecord(ev[1], ctx->stream));
-    k_full_search<false><<<search_grid(ctx, nmb), SEARCH_THREADS, sizeof(SearchSmem), ctx->stream>>>(args, maps);
-    VPP_CHECK_LAUNCH(ctx);
+    if ((rc = rowmin_launch(ctx, args))) return rc;
     if (ev) VPP_CUDA(cudaEventRecord(ev[2], ctx->stream));
-    k_full_subpel<<<(nmb + 7) / 8, 256, 0, ctx->stream>>>(args);
+    k_full_scan<<<(nmb + SCAN_WARPS - 1) / SCAN_WARPS, 32 * SCAN_WARPS, 0, ctx->stream>>>(args);
     VPP_CHECK_LAUNCH(ctx);
-    k_full_tietree<<<ctx->sm_count, TIE_RUNS * 32, sizeof(TieSmem), ctx->stream>>>(args);
+    k_full_tietree<false><<<ctx->sm_count, TIE_RUNS * 32, sizeof(TieSmem), ctx->stream>>>(args);
     VPP_CHECK_LAUNCH(ctx);
     if (ev) VPP_CUDA(cudaEventRecord(ev[3], ctx->stream));
-    rc = full_resolve_launch(ctx, args, resolve_grid, 0);
-    if (rc) return rc;
+    if ((rc = full_resolve_launch(ctx, args, 0))) return rc;
     if (ev) VPP_CUDA(cudaEventRecord(ev[4], ctx->stream));
     return VPPGPU_OK;
 }
@@ -632,27 +754,22 @@ int sad_launch(vppgpu_ctx* ctx, const FullArgs& args, const SearchMaps& maps, in
 {
     int rc = full_planes_launch(ctx, args);
     if (rc) return rc;
-    k_full_search<true><<<search_grid(ctx, nmb), SEARCH_THREADS, sizeof(SearchSmem), ctx->stream>>>(args, maps);
+    k_sad_search<<<search_grid(ctx, nmb), SEARCH_THREADS, sizeof(SearchSmem), ctx->stream>>>(args, maps);
     VPP_CHECK_LAUNCH(ctx);
-    k_full_tietree<<<ctx->sm_count, TIE_RUNS * 32, sizeof(TieSmem), ctx->stream>>>(args);
+    k_full_tietree<true><<<ctx->sm_count, TIE_RUNS * 32, sizeof(TieSmem), ctx->stream>>>(args);
     VPP_CHECK_LAUNCH(ctx);
     return sad_resolve_launch(ctx, args);
 }
 
-int full_prepare(vppgpu_ctx* ctx, int nmb, int* resolve_grid)
+int full_prepare(vppgpu_ctx* ctx)
 {
-    VPP_CUDA(cudaFuncSetAttribute(k_full_search<false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                  (int)sizeof(SearchSmem)));
-    VPP_CUDA(cudaFuncSetAttribute(k_full_search<true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                  (int)sizeof(SearchSmem)));
-    VPP_CUDA(cudaFuncSetAttribute(k_full_tietree, cudaFuncAttributeMaxDynamicSharedMemorySize,
+    VPP_CUDA(cudaFuncSetAttribute(k_sad_search, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(SearchSmem)));
+    VPP_CUDA(cudaFuncSetAttribute(k_full_tietree<false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                   (int)sizeof(TieSmem)));
-    int cap = 0;
-    int rc = full_resolve_prepare(ctx, &cap);
-    if (rc) return rc;
-    int want = (nmb + 7) / 8;
-    *resolve_grid = want < cap ? want : cap;
-    return VPPGPU_OK;
+    VPP_CUDA(cudaFuncSetAttribute(k_full_tietree<true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                  (int)sizeof(TieSmem)));
+    int rc = rowmin_prepare();
+    return rc ? rc : full_resolve_prepare(ctx);
 }
 
 }  // namespace vppgpu

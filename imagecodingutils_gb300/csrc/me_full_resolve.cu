@@ -1624,9 +1624,8 @@ template <int kEst>
 int finish_prepare();
 }
 
-int full_resolve_prepare(vppgpu_ctx* ctx, int* resolve_cap)
+int full_resolve_prepare(vppgpu_ctx*)
 {
-    *resolve_cap = ctx->sm_count * 8;
     // dirty bitmaps of the largest picture (8192 x 8192)
     const int tail_smem = 2 * (512 * 512 / 32) * (int)sizeof(unsigned);
     VPP_CUDA(cudaFuncSetAttribute(k_full_relax_tail<mrc::EST_V2_LAMBDA>, cudaFuncAttributeMaxDynamicSharedMemorySize,
@@ -1741,9 +1740,8 @@ int finish_prepare()
 
 }  // namespace
 
-int full_resolve_launch(vppgpu_ctx* ctx, const FullArgs& args, int resolve_grid, int est)
+int full_resolve_launch(vppgpu_ctx* ctx, const FullArgs& args, int est)
 {
-    (void)resolve_grid;
     switch (est) {
     case 0: return resolve_launch<0>(ctx, args);
     case 1: return resolve_launch<1>(ctx, args);

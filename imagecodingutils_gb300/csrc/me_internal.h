@@ -76,7 +76,12 @@ struct FullArgs {
     int* spec_imv;   // packed full-pel winner
     int* tables;     // 64x64 SSD table per macroblock, kept for the tie macroblocks only (row
                      // minima in column 0, tie tree in row 63)
-    const int* energy;  // 16x16 block energies of the padded reference (int, rstride per row)
+    // SSD search: sums of squares of the samples less 128 of the 16x16 blocks of the padded reference
+    // (whole numbers, rstride per row)
+    const float* energy;
+    // SSD search: per MB and candidate row (64 of them) 8 minima of the energy less twice the cross term
+    // over table columns 8g .. 8g+7, whole numbers
+    float* rowmin;
     int* tie_list;   // macroblocks whose scan met an exact tie (MeCtrl::ntie of them)
     // resolve state
     int* final_mv;
@@ -214,31 +219,34 @@ int set_job(vppgpu_ctx* ctx, JobDesc* d_job, const JobDesc& v);
 // Motion-compensated luma residual of the last estimate's planes at vectors d_mv.
 int full_residual_launch(vppgpu_ctx* ctx, const FullArgs& args, const int* d_mv, short* d_res);
 
-// 2-D tensor maps the search kernel stages its tiles with (one TMA copy each
-// per macroblock): the padded reference (80 x 78 window box), the packed
-// input (16 x 16 template box) and the block energies (64 x 63 box).  They
-// describe buffers, not a frame: encode once per buffer set.
+// 2-D tensor maps the SAD search stages its tiles with (one TMA copy each per
+// macroblock): the padded reference (80 x 78 window box) and the packed input
+// (16 x 16 template box).  They describe buffers, not a frame: encode once per
+// buffer set.
 struct SearchMaps {
-    CUtensorMap win, cur, energy;
+    CUtensorMap win, cur;
 };
 int search_maps_encode(const FullArgs& args, SearchMaps* maps);
 // Byte-packed input (args.src8), padded reference and its half-pel planes
 // from the int16 planes of args.job, and the block energies when args.energy
 // is set (the SSD full search), in one kernel.
 int full_planes_launch(vppgpu_ctx* ctx, const FullArgs& args);
+// Minima of the SSD search (args.rowmin) from the planes and energies, on the tensor cores
+// (me_full_tc.cu); prepare once per device.
+int rowmin_launch(vppgpu_ctx* ctx, const FullArgs& args);
+int rowmin_prepare();
 // Launch the prediction-dependent tail (sweep 0, relaxation, dictionary
 // precompute, exact wavefront) of an estimate whose search has run.
 // est: 0 MotionEstimatorH264ImplFull, 1 MotionEstimatorH264ImplMultiresCrossVer2,
 // 2 MotionEstimatorH264ImplMultires, 3 MotionEstimatorH264ImplCross, 4 Ver2's
 // Lagrangian overload.
-int full_resolve_launch(vppgpu_ctx* ctx, const FullArgs& args, int resolve_grid, int est);
-int full_resolve_prepare(vppgpu_ctx* ctx, int* resolve_cap);
-int full_prepare(vppgpu_ctx* ctx, int nmb, int* resolve_grid);
-// ev: nullptr, or 5 events recorded before the pack kernel, before the
-// search kernel, after it (before the sub-pel stage and the tie trees),
+int full_resolve_launch(vppgpu_ctx* ctx, const FullArgs& args, int est);
+int full_resolve_prepare(vppgpu_ctx* ctx);
+int full_prepare(vppgpu_ctx* ctx);  // once per device: shared-memory limits
+// ev: nullptr, or 5 events recorded before the planes kernel, before the row
+// minima, after them (before the scan, the sub-pel stage and the tie trees),
 // before the resolve and after it.
-int full_launch(vppgpu_ctx* ctx, const FullArgs& args, const SearchMaps& maps, int nmb, int resolve_grid,
-                cudaEvent_t* ev);
+int full_launch(vppgpu_ctx* ctx, const FullArgs& args, int nmb, cudaEvent_t* ev);
 // Integer-pel SAD full search: the MotionEstimatorH264ImplFull integer stage
 // (MotionEstimatorH264ImplFull.cpp:341-446) with the MEH264IF_ABS_DIFF distortion.
 int sad_launch(vppgpu_ctx* ctx, const FullArgs& args, const SearchMaps& maps, int nmb);

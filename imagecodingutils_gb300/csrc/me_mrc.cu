@@ -875,7 +875,7 @@ int mrc2_launch(vppgpu_ctx* ctx, int est, int mode, unsigned char* scratch, cons
         k_pred_tietree<EST_VER2><<<ctx->sm_count * 2, V2_TIE_RUNS * 32, 0, ctx->stream>>>(m, args);
     }
     VPP_CHECK_LAUNCH(ctx);
-    return full_resolve_launch(ctx, args, 0, est);
+    return full_resolve_launch(ctx, args, est);
 }
 
 int h263v2_prepare()

@@ -46,7 +46,8 @@ constexpr size_t kHpelBytes = 3 * kRefBytes;               // b, h, j planes of 
 constexpr size_t kTieListBytes = 1600;                     // one int per macroblock
 constexpr size_t kJobBytes = 64;                           // vppgpu::JobDesc
 constexpr size_t kTableBytes = (size_t)VPPGPU_NOALLOC_MAX_MBS * 64 * 64 * 4;
-constexpr size_t kEnergyBytes = 4 * kRefBytes;               // one int per padded reference sample
+constexpr size_t kEnergyBytes = 4 * kRefBytes;               // one float per padded reference sample
+constexpr size_t kRowMinBytes = 2048 * (size_t)VPPGPU_NOALLOC_MAX_MBS;  // minima, 512 floats per macroblock
 constexpr size_t kOffSrc = 0;
 constexpr size_t kOffRef = kOffSrc + kSrcBytes;
 constexpr size_t kOffSpec = kOffRef + kRefBytes;
@@ -58,11 +59,12 @@ constexpr size_t kOffTieList = kOffHpel + kHpelBytes;
 constexpr size_t kOffJob = kOffTieList + kTieListBytes;
 constexpr size_t kOffTables = kOffJob + kJobBytes;
 constexpr size_t kOffEnergy = kOffTables + kTableBytes;
+constexpr size_t kOffRowMin = kOffEnergy + kEnergyBytes;
 static_assert(sizeof(vppgpu::JobDesc) <= kJobBytes && kOffJob % 16 == 0, "job descriptor does not fit");
 static_assert(kOffSpec % 16 == 0 && kOffHpel % 16 == 0 && kOffTables % 16 == 0 && kOffEnergy % 16 == 0,
               "vector records and planes need 16-byte alignment");
 constexpr size_t kScratchBytes = 12u << 20;
-static_assert(kOffEnergy + kEnergyBytes <= kScratchBytes, "scratch layout exceeds the array");
+static_assert(kOffRowMin + kRowMinBytes <= kScratchBytes, "scratch layout exceeds the array");
 static_assert(sizeof(vppgpu::MeCtrl) <= kCtrlBytes, "control block does not fit");
 static_assert(5 * 4 * VPPGPU_NOALLOC_MAX_MBS <= kSpecBytes && 3 * 4 * VPPGPU_NOALLOC_MAX_MBS <= kStateBytes &&
                   4 * (vppgpu::RELAX_SWEEPS + 2 + (VPPGPU_NOALLOC_MAX_MBS + 31) / 32) <= kChangedBytes,
@@ -75,7 +77,6 @@ struct DeviceSetup {
     bool ready;
     unsigned char* scratch;  // device address of g_noalloc_scratch on this device
     int sm_count;
-    int resolve_cap;         // co-resident blocks of the cooperative resolve kernel
 };
 
 constexpr int kMaxDevices = 64;
@@ -99,12 +100,10 @@ int setup_device(int dev, DeviceSetup** out)
         vppgpu_ctx probe = {};
         probe.device = dev;
         probe.sm_count = sms;
-        int cap = 0;
-        int rc = vppgpu::full_prepare(&probe, 1 << 28, &cap);
+        int rc = vppgpu::full_prepare(&probe);
         if (rc) return rc;
         s.scratch = (unsigned char*)p;
         s.sm_count = sms;
-        s.resolve_cap = cap;
         s.ready = true;
     }
     *out = &s;
@@ -156,7 +155,8 @@ extern "C" int vppgpu_me_full_estimate_noalloc(const short* d_src, const short* 
     a.spec4 = reinterpret_cast<int4*>(spec);
     a.spec_imv = spec + 4 * nmb;
     a.tables = (int*)(base + kOffTables);
-    a.energy = (const int*)(base + kOffEnergy);
+    a.energy = (const float*)(base + kOffEnergy);
+    a.rowmin = (float*)(base + kOffRowMin);
     int* state = (int*)(base + kOffState);
     a.final_mv = state;
     a.final_dist = state + nmb;
@@ -179,14 +179,10 @@ extern "C" int vppgpu_me_full_estimate_noalloc(const short* d_src, const short* 
     // the words that must start at zero on every call
     VPP_CUDA(cudaMemsetAsync(a.ctrl, 0, sizeof(vppgpu::MeCtrl), ctx.stream));
     VPP_CUDA(cudaMemsetAsync(a.changed, 0, sizeof(int) * (size_t)a.sweep_limit, ctx.stream));
-    int grid = (nmb + 7) / 8;
-    if (grid > s->resolve_cap) grid = s->resolve_cap;
     rc = vppgpu::set_job(&ctx, (vppgpu::JobDesc*)(base + kOffJob),
                          vppgpu::JobDesc{d_src, d_ref, d_dist_included, d_mb_slice, (int*)d_mv_out, d_mb_dist_out, nullptr});
     if (rc) return rc;
-    vppgpu::SearchMaps maps;  // host-side descriptors of the array's planes, passed by value
-    if ((rc = vppgpu::search_maps_encode(a, &maps))) return rc;
-    rc = vppgpu::full_launch(&ctx, a, maps, nmb, grid, nullptr);
+    rc = vppgpu::full_launch(&ctx, a, nmb, nullptr);
     if (rc) return rc;
 
     vppgpu::MeCtrl h = {};
