@@ -117,6 +117,31 @@ __device__ __forceinline__ Terms block_terms(int su, int sv, const YuvParams& p)
     return t;
 }
 
+// The bound of a whole-number g term (about one (u, v) pair in a thousand): out of line, FP64.
+__device__ __noinline__ int below_limit_g(int u, int v, int m)
+{
+    return below_limit(__dadd_rn(__dadd_rn(__dmul_rn(-0.394, (double)u), __dmul_rn(-0.581, (double)v)), 0.5), m);
+}
+
+// block_terms for chroma u, v in -128 .. 127: |terms| < 270000 thousandths, so a
+// smaller bias keeps the numerators positive, and both tables hold.
+__device__ __forceinline__ Terms block_terms_byte(int u, int v, const YuvParams& p)
+{
+    constexpr int kBias = 512;  // of thousands
+    const unsigned nb = (unsigned)(p.a0 * u + 500 + 1000 * kBias), nr = (unsigned)(1140 * v + 500 + 1000 * kBias);
+    const unsigned ng = (unsigned)(-394 * u - 581 * v + 500 + 1000 * kBias);
+    const unsigned qb = nb / 1000u, qg = ng / 1000u, qr = nr / 1000u;
+    Terms t;
+    t.qb = (int)qb - kBias;
+    t.qg = (int)qg - kBias;
+    t.qr = (int)qr - kBias;
+    t.lb = t.lg = t.lr = 0;
+    if (qb * 1000u == nb) t.lb = p.lim_b[u + 128];
+    if (qr * 1000u == nr) t.lr = p.lim_r[v + 128];
+    if (qg * 1000u == ng) t.lg = below_limit_g(u, v, t.qg);
+    return t;
+}
+
 __device__ __forceinline__ int luma(int s, const YuvParams& p)
 {
     return p.byte_casts ? (int)(unsigned char)s : (p.six_bit ? 4 * s : s - p.luma_off);
@@ -128,23 +153,73 @@ __device__ __forceinline__ int chan(int l, int q, int lim)
     return clip255(k - ((unsigned)(k - 1) < (unsigned)lim ? 1 : 0));  // 1 <= k <= lim
 }
 
-// b, g, r of one pixel packed in the low 24 bits; kExact: some term of the
-// block needs below_limit's correction
-template <bool kExact = true>
+// b, g, r of one pixel packed in the low 24 bits
 __device__ __forceinline__ unsigned pixel(int s, const Terms& t, const YuvParams& p)
 {
     const int l = luma(s, p);
-    if constexpr (!kExact)
-        return (unsigned)clip255(l + t.qb) | ((unsigned)clip255(l + t.qg) << 8) | ((unsigned)clip255(l + t.qr) << 16);
     return (unsigned)chan(l, t.qb, t.lb) | ((unsigned)chan(l, t.qg, t.lg) << 8) | ((unsigned)chan(l, t.qr, t.lr) << 16);
+}
+
+// clip255(y + q) of both 16-bit halves: y 0 .. 255, |q| < 2^15 - 256
+__device__ __forceinline__ unsigned add_clip2(unsigned y, unsigned q) { return __viaddmin_s16x2_relu(y, q, 0x00ff00ffu); }
+
+// One taken from the halves of a packed channel whose sum k (the sample of y
+// plus q) is one that the reference's sum falls below: 1 <= k <= lim.  Above
+// 255 the clip hides it.
+__device__ __forceinline__ unsigned fall_below2(unsigned c, unsigned y, int q, int lim)
+{
+    const unsigned m = (unsigned)min(lim, 255);
+    const int k0 = (int)(y & 0xffffu) + q - 1, k1 = (int)(y >> 16) + q - 1;
+    return c - ((unsigned)k0 < m ? 1u : 0u) - ((unsigned)k1 < m ? 0x10000u : 0u);
+}
+
+// Four 2x2 blocks of any samples, packed; out of line, so that its code does
+// not lie between the instructions of the usual path.
+__device__ __noinline__ void general_group(uint4 ya, uint4 yb, uint2 uu, uint2 vv, const YuvParams& p, unsigned* wa,
+                                           unsigned* wb)
+{
+    const short* su = reinterpret_cast<const short*>(&uu);
+    const short* sv = reinterpret_cast<const short*>(&vv);
+    const short* sa = reinterpret_cast<const short*>(&ya);
+    const short* sb = reinterpret_cast<const short*>(&yb);
+    auto pack = [](const unsigned* q, unsigned* w) {
+        w[0] = q[0] | (q[1] << 24);
+        w[1] = (q[1] >> 8) | (q[2] << 16);
+        w[2] = (q[2] >> 16) | (q[3] << 8);
+    };
+#pragma unroll
+    for (int k = 0; k < 4; k += 2) {
+        unsigned ra[4], rb[4];
+#pragma unroll
+        for (int i = 0; i < 2; i++) {
+            const Terms t = block_terms(su[k + i], sv[k + i], p);
+#pragma unroll
+            for (int e = 0; e < 2; e++) {
+                ra[2 * i + e] = pixel(sa[2 * (k + i) + e], t, p);
+                rb[2 * i + e] = pixel(sb[2 * (k + i) + e], t, p);
+            }
+        }
+        pack(ra, wa + 3 * (k >> 1));
+        pack(rb, wb + 3 * (k >> 1));
+    }
 }
 
 // Rows layout (NonRotate, or bottom-up with kFlip), four 2x2 blocks per
 // thread: two 16-byte luma loads, 8-byte chroma loads, three 8-byte stores
 // per output row.  Needs width % 8 == 0 and aligned planes.
+//
+// Samples within 0 .. 255 (every real picture; a thread with others takes the
+// general pixel) go two at a time: a channel of two pixels is one add, clamp
+// and floor in 16-bit halves, and the bytes are packed by permutations from
+// the channel pairs.  The blocks with a term that is a whole number (one in
+// fifty of natural chroma, so a few in most warps) have the pixels below
+// their bound corrected afterwards.  Issue-bound (permutations, packed adds and
+// products issue every other cycle): 16 1080p frames in 52.5 us with every
+// pixel alone, 38.9 now (the copy rate's floor is 29; b and r terms from
+// shared-memory tables in a persistent grid took 42, 5 or 8 CTAs per SM 41, 42).
 template <bool kFlip>
-__global__ void __launch_bounds__(256) k_yuv_rgb_x8(const short* __restrict__ Y, const short* __restrict__ U,
-                                                    const short* __restrict__ V, YuvParams p,
+__global__ void __launch_bounds__(256, 6) k_yuv_rgb_x8(const short* __restrict__ Y, const short* __restrict__ U,
+                                                    const short* __restrict__ V, const __grid_constant__ YuvParams p,
                                                     unsigned char* __restrict__ rgb)
 {
     const int f = blockIdx.y;
@@ -159,48 +234,56 @@ __global__ void __launch_bounds__(256) k_yuv_rgb_x8(const short* __restrict__ Y,
         const uint4 yb = __ldg(reinterpret_cast<const uint4*>(y0 + (size_t)(y + 1) * p.w + x));
         const uint2 uu = __ldg(reinterpret_cast<const uint2*>(u0 + (size_t)qy * (p.w >> 1) + 4 * gx));
         const uint2 vv = __ldg(reinterpret_cast<const uint2*>(v0 + (size_t)qy * (p.w >> 1) + 4 * gx));
-        const short* sa = reinterpret_cast<const short*>(&ya);
-        const short* sb = reinterpret_cast<const short*>(&yb);
         const short* su = reinterpret_cast<const short*>(&uu);
         const short* sv = reinterpret_cast<const short*>(&vv);
-        unsigned ra[8], rb[8];
-        Terms tk[4];
-        int lims = 0;
-#pragma unroll
-        for (int k = 0; k < 4; k++) {
-            tk[k] = block_terms(su[k], sv[k], p);
-            lims |= tk[k].lb | tk[k].lg | tk[k].lr;
-        }
-        if (__any_sync(__activemask(), lims != 0)) {  // a block of the warp needs the correction
+        const unsigned la[4] = {ya.x, ya.y, ya.z, ya.w}, lb[4] = {yb.x, yb.y, yb.z, yb.w};
+        unsigned wa[6], wb[6];  // 8 pixels x 3 bytes = six little-endian words per row
+        const unsigned any = la[0] | la[1] | la[2] | la[3] | lb[0] | lb[1] | lb[2] | lb[3] | uu.x | uu.y | vv.x | vv.y;
+        if ((any & 0xff00ff00u) == 0u) {
+            unsigned ca[2][3], cb[2][3];  // channels b, g, r of a block's two pixels, rows a and b
 #pragma unroll
             for (int k = 0; k < 4; k++) {
-                ra[2 * k] = pixel<true>(sa[2 * k], tk[k], p);
-                ra[2 * k + 1] = pixel<true>(sa[2 * k + 1], tk[k], p);
-                rb[2 * k] = pixel<true>(sb[2 * k], tk[k], p);
-                rb[2 * k + 1] = pixel<true>(sb[2 * k + 1], tk[k], p);
+                const int u = p.byte_casts ? (int)(signed char)(su[k] + p.chr_off) : su[k] - 128;
+                const int v = p.byte_casts ? (int)(signed char)(sv[k] + p.chr_off) : sv[k] - 128;
+                const Terms t = block_terms_byte(u, v, p);
+                // the luma offset of CCIR601 goes into the terms
+                const int q[3] = {t.qb - p.luma_off, t.qg - p.luma_off, t.qr - p.luma_off};
+                const int l[3] = {t.lb, t.lg, t.lr};
+#pragma unroll
+                for (int c = 0; c < 3; c++) {
+                    const unsigned qq = __byte_perm((unsigned)q[c], 0u, 0x1010);
+                    ca[k & 1][c] = add_clip2(la[k], qq);
+                    cb[k & 1][c] = add_clip2(lb[k], qq);
+                }
+                if (l[0] | l[1] | l[2]) {
+#pragma unroll
+                    for (int c = 0; c < 3; c++)
+                        if (l[c]) {
+                            ca[k & 1][c] = fall_below2(ca[k & 1][c], la[k], q[c], l[c]);
+                            cb[k & 1][c] = fall_below2(cb[k & 1][c], lb[k], q[c], l[c]);
+                        }
+                }
+                if (k & 1) {  // four pixels: b0 g0 r0 b1 | g1 r1 b2 g2 | r2 b3 g3 r3
+                    auto pack = [&](const unsigned (&c)[2][3], unsigned* w) {
+                        const unsigned t0 = __byte_perm(c[0][0], c[0][1], 0x6240);  // b0 g0 b1 g1
+                        const unsigned t1 = __byte_perm(c[1][0], c[1][1], 0x6240);
+                        w[0] = __byte_perm(t0, c[0][2], 0x2410);
+                        w[1] = __byte_perm(__byte_perm(t0, c[0][2], 0x0063), t1, 0x5410);
+                        w[2] = __byte_perm(t1, c[1][2], 0x6324);
+                    };
+                    pack(ca, wa + 3 * (k >> 1));
+                    pack(cb, wb + 3 * (k >> 1));
+                }
             }
         } else {
+            unsigned ga[6], gb[6];  // (so that wa and wb stay in registers)
+            general_group(ya, yb, uu, vv, p, ga, gb);
 #pragma unroll
-            for (int k = 0; k < 4; k++) {
-                ra[2 * k] = pixel<false>(sa[2 * k], tk[k], p);
-                ra[2 * k + 1] = pixel<false>(sa[2 * k + 1], tk[k], p);
-                rb[2 * k] = pixel<false>(sb[2 * k], tk[k], p);
-                rb[2 * k + 1] = pixel<false>(sb[2 * k + 1], tk[k], p);
+            for (int i = 0; i < 6; i++) {
+                wa[i] = ga[i];
+                wb[i] = gb[i];
             }
         }
-        // 8 pixels x 3 bytes = six little-endian words per row
-        auto pack = [](const unsigned* q, unsigned* w) {
-#pragma unroll
-            for (int i = 0; i < 2; i++) {
-                const unsigned a = q[4 * i], b = q[4 * i + 1], c = q[4 * i + 2], d = q[4 * i + 3];
-                w[3 * i] = a | (b << 24);
-                w[3 * i + 1] = (b >> 8) | (c << 16);
-                w[3 * i + 2] = (c >> 16) | (d << 8);
-            }
-        };
-        unsigned wa[6], wb[6];
-        pack(ra, wa);
-        pack(rb, wb);
         const int ya_out = kFlip ? p.h - 1 - y : y, yb_out = kFlip ? p.h - 2 - y : y + 1;
         uint2* da = reinterpret_cast<uint2*>(o0 + ((size_t)ya_out * p.w + x) * 3);
         uint2* db = reinterpret_cast<uint2*>(o0 + ((size_t)yb_out * p.w + x) * 3);

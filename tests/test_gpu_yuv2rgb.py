@@ -173,3 +173,31 @@ def test_zoom_against_golden_and_oracle(vpp, ctx, golden, orc):
     out = np.zeros(1440 * 810 * 3, np.uint8)
     c.Convert(y, u, v, out)
     np.testing.assert_array_equal(out.reshape(810, 1440, 3), orc.yuv_to_rgb_zoom(y, u, v, 1440, 810))
+
+
+@pytest.mark.parametrize("okind", [0, 1, 2])
+@pytest.mark.parametrize("flip", [0, 1])
+def test_packed_path_every_luma_at_whole_terms(vpp, ctx, orc, okind, flip):
+    """The kernel's path for samples in 0..255: every luma at every chroma pair with a whole-number term (its sums are
+    corrected below a bound), and rows where single samples outside the range send a thread to the general path."""
+    import torch
+    # whole thousandths of the g term (and of the r and b terms where they have any)
+    pairs = [(a, b) for a in range(256) for b in range(256)
+             if (-394 * (a - 128) - 581 * (b - 128) + 500) % 1000 == 0 or (b - 128) % 50 == 25 and a % 32 == 0]
+    w, h = 512, 2 * len(pairs)  # a chroma row per pair, the 512 lumas of its first row run through 0..255 twice
+    u = np.repeat(np.array([a for a, _ in pairs], np.int16)[:, None], w // 2, axis=1)
+    v = np.repeat(np.array([b for _, b in pairs], np.int16)[:, None], w // 2, axis=1)
+    y = np.tile((np.arange(w) // 2 % 256).astype(np.int16), (h, 1))
+    y[1::2] = 255 - y[1::2]
+    rng = np.random.default_rng(60 + okind)
+    for plane, n in ((y, 300), (u, 100), (v, 100)):  # out of range here and there
+        i = rng.integers(0, plane.size, n)
+        plane.reshape(-1)[i] = rng.integers(-3000, 3000, n)
+    L = vpp.load()
+    dy, du, dv = _dev(torch, y), _dev(torch, u), _dev(torch, v)
+    out = torch.zeros(w * h * 3, dtype=torch.uint8, device="cuda")
+    assert L.vppgpu_yuv420_to_rgb24_device(ctx.handle, okind, C.c_void_p(dy.data_ptr()), C.c_void_p(du.data_ptr()),
+                                           C.c_void_p(dv.data_ptr()), w, h, -128, 0, flip, C.c_void_p(out.data_ptr())) == 0
+    torch.cuda.synchronize()
+    want = orc.yuv_to_rgb(okind, y, u, v, -128, 0, flip)
+    np.testing.assert_array_equal(out.cpu().numpy().reshape(want.shape), want)
