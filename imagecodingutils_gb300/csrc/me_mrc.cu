@@ -35,6 +35,8 @@
 // (0, 0) with their tie trees (MultiresCrossVer2, Multires; their resolve is me_full_resolve.cu),
 // and MotionEstimatorH263ImplMultiresCrossVer2 whole (k_v263_*: search, tie trees, relaxation
 // sweeps over work lists, the one-CTA exact pass, outputs).
+#include <type_traits>
+
 #include "me_full_common.cuh"
 #include "me_mrc_search.cuh"
 
@@ -122,7 +124,9 @@ __global__ void __launch_bounds__(256) k_mrc_level2(const unsigned char* __restr
 template <bool kH263>
 __global__ void __launch_bounds__(256) k_mrc_search(MrcArgs a)
 {
-    extern __shared__ Lattice lattice[];  // one per warp
+    using Store = std::conditional_t<kH263, Window, Lattice>;  // one per warp
+    extern __shared__ uint4 mrc_store[];
+    Store* lattice = reinterpret_cast<Store*>(mrc_store);
     const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
     const int k = blockIdx.x * (blockDim.x >> 5) + wib;
     if (k >= a.cols * a.rows_all) return;
@@ -275,7 +279,7 @@ __device__ __forceinline__ void h263_levels(int px, int py, int* pl)
 // The search with the estimator's tie rule (…:714-721, 787-794, 844-851, 912-919): the current best
 // is kept when the candidate is farther from the level's prediction, the candidate's y distance being
 // taken as my + i + predY (the prediction added where the current best's subtracts it).
-__device__ __forceinline__ MbSearch h263v2_search(const MrcArgs& a, Lattice& lt, int mbr, int mbc, const int* pl,
+__device__ __forceinline__ MbSearch h263v2_search(const MrcArgs& a, Window& lt, int mbr, int mbc, const int* pl,
                                                   int lane, bool& bad)
 {
     auto skip = [pl](int lvl, int mx, int my, int rmx, int rmy, int j, int i) {
@@ -366,7 +370,7 @@ __device__ __forceinline__ int2 h263v2_choose(const MbSearch& s, int pv, int pre
 // Tie tree of a macroblock (V2TieRun, as the H.264 Ver2 trees): run `run` of eight decides its t-th tie
 // (t < 3) by bit t of run (1 takes the candidate) and records the tie's level and the two vectors
 // compared, current (cx, cy) and candidate (nx, ny) in level units.
-__device__ void h263v2_run(const MrcArgs& a, Lattice& lt, int mbr, int mbc, int run, V2TieRun* rec, int lane,
+__device__ void h263v2_run(const MrcArgs& a, Window& lt, int mbr, int mbc, int run, V2TieRun* rec, int lane,
                            bool& bad)
 {
     int t = 0, lvls = 0, geo[V2_TIE_BITS] = {0, 0, 0};
@@ -429,7 +433,7 @@ __device__ __forceinline__ unsigned rec_slot(int p) { return ((unsigned)p * 2654
 // (0, 0), s0: that search where its ties do not involve the prediction, else the tie tree's answer,
 // else a search at p; then the choice, recorded.  One warp.  ghost: a macroblock of a partial bottom
 // row (not recorded).
-__device__ int2 h263v2_compute(const V263& v, Lattice& lt, int k, int mbr, int mbc, int p, int4 s0, bool ghost,
+__device__ int2 h263v2_compute(const V263& v, Window& lt, int k, int mbr, int mbc, int p, int4 s0, bool ghost,
                                int lane, bool& bad, int& misses, int& searches)
 {
     const int px = mv_x(p), py = mv_y(p);
@@ -465,7 +469,7 @@ __device__ int2 h263v2_compute(const V263& v, Lattice& lt, int k, int mbr, int m
 
 // The same from the macroblock's record when it holds prediction p (its records and its search at
 // (0, 0) are loaded together).
-__device__ int2 h263v2_eval(const V263& v, Lattice& lt, int k, int mbr, int mbc, int p, bool ghost, int lane,
+__device__ int2 h263v2_eval(const V263& v, Window& lt, int k, int mbr, int mbc, int p, bool ghost, int lane,
                             bool& bad, int& misses, int& searches)
 {
     const int4 s0 = __ldcg(v.s0 + k);
@@ -494,7 +498,8 @@ __device__ __forceinline__ int h263v2_pred(int k, int cols, Ld&& ld)
 // there: the first state.
 __global__ void __launch_bounds__(256) k_v263_search(V263 v)
 {
-    __shared__ Lattice lt;  // never touched by the H.263 search (no sub-pel lattice)
+    __shared__ Window lts[8];
+    Window& lt = lts[threadIdx.x >> 5];
     const int lane = threadIdx.x & 31, k = blockIdx.x * 8 + (threadIdx.x >> 5);
     if (k >= v.m.cols * v.m.rows_all) return;
     bool bad = false;
@@ -517,8 +522,9 @@ __global__ void __launch_bounds__(256) k_v263_search(V263 v)
 // The tie trees of the macroblocks whose search met a tie: warp r of a block makes run r.
 __global__ void __launch_bounds__(V2_TIE_RUNS * 32) k_v263_tietree(V263 v)
 {
-    __shared__ Lattice lt;
+    __shared__ Window lts[V2_TIE_RUNS];
     const int lane = threadIdx.x & 31, run = threadIdx.x >> 5;
+    Window& lt = lts[run];
     const int n = __ldcg(&v.m.ctrl->tie_mbs);
     bool bad = false;
     for (int i = blockIdx.x; i < n; i += gridDim.x) {
@@ -538,7 +544,8 @@ static_assert(H263V2_SWEEPS <= kListLen, "change counts and list lengths must no
 // prediction: the fixed point.  A sweep after one that changed nothing returns at once.
 __global__ void __launch_bounds__(256) k_v263_sweep(V263 v, int sweep)
 {
-    __shared__ Lattice lt;
+    __shared__ Window lts[8];
+    Window& lt = lts[threadIdx.x >> 5];
     if (sweep > 0 && __ldcg(v.changed + sweep - 1) == 0) return;
     const int lane = threadIdx.x & 31, cols = v.m.cols, rows = v.m.nmb / cols;
     const int n = sweep == 0 ? v.m.nmb : __ldcg(v.changed + kListLen + sweep - 1);
@@ -608,7 +615,8 @@ __host__ __device__ constexpr size_t diag_smem(int rows)
 __global__ void __launch_bounds__(kDiagThreads, 1) k_v263_diag(V263 v)
 {
     extern __shared__ __align__(16) int4 dsm4[];  // prefetch slots, search-at-(0, 0) list, then the int arrays
-    __shared__ Lattice lt;
+    __shared__ Window lts[kDiagThreads / 32];
+    Window& lt = lts[threadIdx.x >> 5];
     __shared__ int s_nmiss[2];
     if (v263_relaxed(v)) return;
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, nw = blockDim.x >> 5;
@@ -708,7 +716,8 @@ __global__ void __launch_bounds__(kDiagThreads, 1) k_v263_diag(V263 v)
 // pDistortionIncluded is NULL, …:1095-1101).
 __global__ void __launch_bounds__(256) k_v263_outputs(V263 v)
 {
-    __shared__ Lattice lt;
+    __shared__ Window lts[8];
+    Window& lt = lts[threadIdx.x >> 5];
     if (*((volatile int*)&v.m.ctrl->status) & ST_TIMEOUT) return;
     const int* fin = v263_relaxed(v) ? v.state : v.wave;
     const int lane = threadIdx.x & 31, cols = v.m.cols, nmb = v.m.nmb;
@@ -838,7 +847,7 @@ int mrc_launch(vppgpu_ctx* ctx, int W, int H, int motion_range, int mode, const 
     if (rc) return rc;
     const int mbs = a.cols * a.rows_all, wpb = (warps == 2 || warps == 4) ? warps : 8;
     if (h263)
-        k_mrc_search<true><<<(mbs + wpb - 1) / wpb, 32 * wpb, wpb * sizeof(Lattice), ctx->stream>>>(a);
+        k_mrc_search<true><<<(mbs + wpb - 1) / wpb, 32 * wpb, wpb * sizeof(Window), ctx->stream>>>(a);
     else
         k_mrc_search<false><<<(mbs + wpb - 1) / wpb, 32 * wpb, wpb * sizeof(Lattice), ctx->stream>>>(a);
     VPP_CHECK_LAUNCH(ctx);

@@ -10,6 +10,15 @@
 // (a column beyond the row continues on the next row).  The device copies
 // keep exactly that flat geometry, so the same addresses hold the same
 // samples; a read outside a copy sets an error instead of reading.
+//
+// One warp searches one macroblock, and what bounds it is instructions issued.  Scored a candidate at a
+// time over the warp, with a shuffle chain and a ballot for each partial distortion and the sub-pel window
+// in shorts, a MultiresCross macroblock took 11.7 thousand (a 1280x720 frame 62 us; the Multires search of a
+// 1920x1080 frame 174 us, its tie trees 60).  But a candidate's decision needs only two numbers of its own,
+// its distortion and the smallest minimum that no phase of it rejects (phase_limit), so the candidates of
+// an integer stage are scored independently, a lane each with packed bytes, and then settled in their order
+// against the running minimum (settle); the sub-pel stages give a candidate four lanes, and their window
+// is made two samples at a time: 3.5 thousand instructions, 20 us; 37 and 20 us.
 #pragma once
 
 #include "me_common.cuh"
@@ -20,10 +29,6 @@ namespace mrc {
 namespace {
 
 constexpr int MRC_NOISE_FLOOR = 512;
-
-// Phase order of the partial distortion (OverlayMem2Dv2.cpp:79-80), p = 1..16.
-__constant__ int kPhaseRow[17] = {0, 0, 2, 0, 2, 1, 3, 1, 3, 0, 2, 1, 3, 0, 2, 1, 3};
-__constant__ int kPhaseCol[17] = {0, 0, 2, 2, 0, 1, 3, 3, 1, 1, 3, 0, 2, 3, 1, 2, 0};
 
 struct Buf {
     const unsigned char* p;
@@ -68,10 +73,6 @@ __device__ __forceinline__ int rd(const Buf& b, int r, int c, bool& bad)
     return __ldg(b.p + f);
 }
 
-// A read inside a block that origin() placed in its buffer (every row and column of the block lies
-// within the copy, as the clamp guarantees): no check needed.
-__device__ __forceinline__ int rdb(const Buf& b, int r, int c) { return __ldg(b.p + (size_t)r * b.w + c); }
-
 // GetMotionRange of the multi-resolution estimators (…MultiresCross.cpp:1195-1262).
 struct Level {
     int boundary, width, height, vec_range;
@@ -91,137 +92,457 @@ __device__ __forceinline__ void mr_range(const Level& L, int xpos, int ypos, int
 }
 
 // ---------------------------------------------------------------------------
-// Partial distortion of an n x n block (n = 8 or 16): lane pair 2(p-1),
-// 2(p-1)+1 holds phase p; `part` is this lane's share of that phase.  Returns
-// PartialLessThan's value against `min`: 16*D_p at the first phase p with
-// 16*D_p > p*min (shifts wrap as the reference's int arithmetic), else D.
-__device__ __forceinline__ int partial_value(int part, int min, int lane)
+// Phase order of the partial distortion (OverlayMem2Dv2.cpp:79-80), p = 1..16: phase p sums the squared
+// differences at rows phase_row + 4i, columns phase_col + 4j of the block, so the sixteen phases are the
+// sixteen classes (row mod 4, column mod 4).  PartialLessThan rejects a candidate at the first phase with
+// 16 * D_p > p * min (D_p: the sum of phases 1..p), with a value above min, and otherwise returns D_16.
+// Whether any phase rejects is thus decided by one number of the candidate, the largest ceil(16 * D_p / p):
+// it is accepted exactly when that is at most min.  s: the class sums, [4 * row + column].  (16 * D_16 of
+// a 16x16 block of bytes is below 2^29.)
+__device__ __forceinline__ void phase_limit(const unsigned (&s)[16], int& d, int& t)
 {
-    int v = part + __shfl_xor_sync(0xffffffffu, part, 1);  // the phase sum
+    constexpr int kRow[16] = {0, 2, 0, 2, 1, 3, 1, 3, 0, 2, 1, 3, 0, 2, 1, 3};
+    constexpr int kCol[16] = {0, 2, 2, 0, 1, 3, 3, 1, 1, 3, 0, 2, 3, 1, 2, 0};
+    unsigned run = 0, top = 0;
 #pragma unroll
-    for (int o = 2; o < 32; o <<= 1) {
-        const int t = __shfl_up_sync(0xffffffffu, v, o);
-        if (lane >= o) v += t;
+    for (int p = 1; p <= 16; p++) {
+        run += s[4 * kRow[p - 1] + kCol[p - 1]];
+        top = max(top, (16u * run + (unsigned)(p - 1)) / (unsigned)p);
     }
-    const int p = (lane >> 1) + 1;
-    const int s = (int)((unsigned)v << 4);
-    const unsigned rej = __ballot_sync(0xffffffffu, (lane & 1) == 0 && s > p * min);
-    if (rej) return __shfl_sync(0xffffffffu, s, __ffs(rej) - 1);
-    return __shfl_sync(0xffffffffu, v, 31);
+    d = (int)run;
+    t = (int)top;
 }
 
-// This lane's samples of phase p (lane pair), half h = lane & 1: rows
-// phase_row + 4*(2h + i), i < n/8; columns phase_col + 4*j, j < n/4.
+// N words of a row of samples from any byte address: the aligned words around them.  Reads up to four
+// bytes past them and three before, which stay inside the levels' scratch.
 template <int N>
-__device__ __forceinline__ void phase_coords(int lane, int& r0, int& c0)
+__device__ __forceinline__ void row_words(const unsigned char* p, unsigned (&w)[N])
 {
-    const int p = (lane >> 1) + 1;
-    r0 = kPhaseRow[p] + 4 * (N / 8) * (lane & 1);
-    c0 = kPhaseCol[p];
-}
-
-// Full n x n SSD of two overlays placed by origin(), one warp (lane per column/row chunk).
-__device__ __forceinline__ int full_ssd(const Buf& a, Org oa, const Buf& b, Org ob, int n, int lane, bool& bad)
-{
-    (void)bad;  // both blocks lie inside their copies
-    int acc = 0;
-    for (int i = lane; i < n * n; i += 32) {
-        const int r = i / n, c = i - r * n;
-        const int d = rdb(a, oa.y + r, oa.x + c) - rdb(b, ob.y + r, ob.x + c);
-        acc += d * d;
+    const unsigned* q = reinterpret_cast<const unsigned*>(reinterpret_cast<uintptr_t>(p) & ~(uintptr_t)3);
+    const unsigned sh = (unsigned)(reinterpret_cast<uintptr_t>(p) & 3) * 8;
+    unsigned lo = __ldg(q);
+#pragma unroll
+    for (int i = 0; i < N; i++) {
+        const unsigned hi = __ldg(q + i + 1);
+        w[i] = __funnelshift_r(lo, hi, sh);
+        lo = hi;
     }
-    return warp_sum(acc);
 }
 
-// ---------------------------------------------------------------------------
-// The sub-pel window as a lattice of 22 x 22 full-pel points (fr, fc), each
-// with the four even quarter samples G (0,0), h (2,0), b (0,2), j (2,2)
-// (LoadHalfQuartPelWindow, …MultiresCross.cpp:1281-1349): raw h for rows 2..18
-// over all columns, raw b for all rows over columns 2..18, j from the raw h,
-// then h, b scaled and G copied for rows and columns 2..18 only; every other
-// sample is never written (0).
-struct Lattice {
-    short g[22][22], h[22][22], b[22][22], j[22][22];
+// Squares of the bytes of four words of absolute differences, summed by byte position.
+__device__ __forceinline__ void add_classes(unsigned d0, unsigned d1, unsigned d2, unsigned d3, unsigned* s)
+{
+    const unsigned a = __byte_perm(d0, d1, 0x5140), b = __byte_perm(d2, d3, 0x5140);
+    const unsigned c = __byte_perm(d0, d1, 0x7362), e = __byte_perm(d2, d3, 0x7362);
+    const unsigned k0 = __byte_perm(a, b, 0x5410), k1 = __byte_perm(a, b, 0x7632);
+    const unsigned k2 = __byte_perm(c, e, 0x5410), k3 = __byte_perm(c, e, 0x7632);
+    s[0] = __dp4a(k0, k0, s[0]);
+    s[1] = __dp4a(k1, k1, s[1]);
+    s[2] = __dp4a(k2, k2, s[2]);
+    s[3] = __dp4a(k3, k3, s[3]);
+}
+
+// What a warp's search keeps in shared memory: the input blocks of levels 1 and 0, and the level-0
+// reference around the centre of the last integer stage, rows and columns -5..+20 (22 with the word
+// padding) of its block: all that the +-2 refinement and the sub-pel window of any of its winners read.
+// Samples outside the copy are 0.
+constexpr int WPITCH = 7;                   // words per row
+constexpr int WROWS = 26;
+struct Window {
+    uint4 cur[16];
+    uint2 cur1[8];
+    unsigned win[WROWS * WPITCH + 2];  // (+2: the whole is a multiple of 16 bytes)
+};
+static_assert(sizeof(Window) % 16 == 0, "what a Lattice adds follows it at once");
+// The sub-pel window (LoadHalfQuartPelWindow, …MultiresCross.cpp:1281-1349) as a lattice of 22 x 22 points
+// (fr, fc), each with the four even quarter samples G (0,0), h (2,0), b (0,2), j (2,2); the block's sample
+// (r, c) is point (3 + r, 3 + c).  h, b and j are byte planes of rows 2..19 in the window's columns; G is the
+// window itself.  The reference scales h and b and copies G for rows and columns 2..18 only, which leaves
+// (MultiresCross, Multires) the raw b in row 19, the raw h in column 19 and zeros for G there: raw holds h
+// (rows 2..18) and row19 b, both + 2560.  Ver2 completes that row and column.
+constexpr int SUB_PLANE = 18 * WPITCH;
+constexpr int RAW_BIAS = 2560;              // a multiple of 32 above the most negative 6-tap sum, 2550
+struct Lattice : Window {
+    unsigned sub[3 * SUB_PLANE];            // h, b, j: row fr - 2
+    unsigned raw[17 * 2 * WPITCH];          // pairs of shorts
+    unsigned row19[2 * WPITCH];
 };
 
-__device__ __forceinline__ int lat(const Lattice& L, int qr, int qc)
+// Words of 16 samples from byte column `col` of a row of the window or of a plane.
+__device__ __forceinline__ void window_row(const unsigned* row, int col, unsigned (&w)[4])
 {
-    const int fr = qr >> 2, fc = qc >> 2;
-    if ((qr & 3) == 0) return (qc & 3) == 0 ? L.g[fr][fc] : L.b[fr][fc];
-    return (qc & 3) == 0 ? L.h[fr][fc] : L.j[fr][fc];
+    const unsigned* q = row + (col >> 2);
+    const unsigned sh = (unsigned)(col & 3) * 8;
+    unsigned lo = q[0];
+#pragma unroll
+    for (int i = 0; i < 4; i++) {
+        const unsigned hi = q[i + 1];
+        w[i] = __funnelshift_r(lo, hi, sh);
+        lo = hi;
+    }
 }
 
-template <bool kVer2>
-__device__ void build_lattice(Lattice& L, const Buf& e0, Org o, int lane, bool& bad)
+// Distortion of the zero vector, the input block kept in L.cur on the way: lane = half a row.
+__device__ __forceinline__ int zero_distortion(const MrcArgs& a, Window& L, Org oi, int n, int m, int lane)
 {
-    for (int i = lane; i < 22 * 22; i += 32) {
-        const int fr = i / 22, fc = i - fr * 22;
-        L.g[fr][fc] = 0;
-        L.h[fr][fc] = 0;
-        L.b[fr][fc] = 0;
-        L.j[fr][fc] = 0;
-    }
-    __syncwarp();
-    for (int i = lane; i < 17 * 22; i += 32) {  // raw h: rows 2..18, all columns
-        const int fr = 2 + i / 22, fc = i % 22;
-        const int rr = o.y + fr - 3, cc = o.x + fc - 3;
-        L.h[fr][fc] = (short)tap6(rd(e0, rr - 2, cc, bad), rd(e0, rr - 1, cc, bad), rd(e0, rr, cc, bad),
-                                  rd(e0, rr + 1, cc, bad), rd(e0, rr + 2, cc, bad), rd(e0, rr + 3, cc, bad));
-    }
-    for (int i = lane; i < 22 * 17; i += 32) {  // raw b: all rows, columns 2..18
-        const int fr = i / 17, fc = 2 + i % 17;
-        const int rr = o.y + fr - 3, cc = o.x + fc - 3;
-        L.b[fr][fc] = (short)tap6(rd(e0, rr, cc - 2, bad), rd(e0, rr, cc - 1, bad), rd(e0, rr, cc, bad),
-                                  rd(e0, rr, cc + 1, bad), rd(e0, rr, cc + 2, bad), rd(e0, rr, cc + 3, bad));
-    }
-    __syncwarp();
-    for (int i = lane; i < 17 * 17; i += 32) {  // j from the raw h (columns fc-2 .. fc+3)
-        const int fr = 2 + i / 17, fc = 2 + i % 17;
-        const short* hr = L.h[fr];
-        const int v = ((int)hr[fc - 2] - 5 * hr[fc - 1] + 20 * hr[fc] + 20 * hr[fc + 1] - 5 * hr[fc + 2] + hr[fc + 3] +
-                       512) >> 10;
-        L.j[fr][fc] = (short)clip255(v);
-    }
-    __syncwarp();
-    for (int i = lane; i < 17 * 17; i += 32) {  // scale h and b, copy G: rows and columns 2..18
-        const int fr = 2 + i / 17, fc = 2 + i % 17;
-        L.h[fr][fc] = (short)clip255((L.h[fr][fc] + 16) >> 5);
-        L.b[fr][fc] = (short)clip255((L.b[fr][fc] + 16) >> 5);
-        L.g[fr][fc] = (short)rd(e0, o.y + fr - 3, o.x + fc - 3, bad);
-    }
-    if (kVer2 && lane < 18) {
-        // Ver2 completes column and row 19 (…MultiresCrossVer2.cpp:2075-2093):
-        // scaled h and G at column 19 of rows 2..18, scaled b and G at row 19
-        // of columns 2..18, G at (19, 19)
-        if (lane < 17) {
-            const int f = 2 + lane;
-            L.h[f][19] = (short)clip255((L.h[f][19] + 16) >> 5);
-            L.g[f][19] = (short)rd(e0, o.y + f - 3, o.x + 16, bad);
-            L.b[19][f] = (short)clip255((L.b[19][f] + 16) >> 5);
-            L.g[19][f] = (short)rd(e0, o.y + 16, o.x + f - 3, bad);
-        } else {
-            L.g[19][19] = (short)rd(e0, o.y + 16, o.x + 16, bad);
+    const int r = lane >> 1, c = 8 * (lane & 1);
+    const Org o = origin(a.e0, 16, 16, 19, n, m);
+    unsigned x[2], y[2];
+    row_words(a.in0.p + (size_t)(oi.y + r) * a.in0.w + oi.x + c, x);
+    row_words(a.e0.p + (size_t)(o.y + r) * a.e0.w + o.x + c, y);
+    reinterpret_cast<uint2*>(L.cur)[lane] = make_uint2(x[0], x[1]);
+    const unsigned d0 = __vabsdiffu4(x[0], y[0]), d1 = __vabsdiffu4(x[1], y[1]);
+    return warp_sum((int)__dp4a(d1, d1, __dp4a(d0, d0, 0u)));
+}
+
+// Stage the window around block o of the level-0 copy: eight lanes a row, an aligned word each, joined
+// with the next lane's.
+__device__ __forceinline__ void stage_level0(const Buf& e0, Window& L, Org o, int lane)
+{
+    const int first = (o.y - 5) * e0.w + o.x - 5, size = e0.w * e0.h;
+    if (first >= 0 && first + (WROWS - 1) * e0.w + 4 * WPITCH <= size) {
+        const int wd = lane & 7;
+#pragma unroll
+        for (int i = 0; i < (WROWS + 3) / 4; i++) {
+            const int r = min(4 * i + (lane >> 3), WROWS - 1);
+            const uintptr_t u = reinterpret_cast<uintptr_t>(e0.p + first + r * e0.w);
+            const unsigned v = __ldg(reinterpret_cast<const unsigned*>(u & ~(uintptr_t)3) + wd);
+            const unsigned w = __funnelshift_r(v, __shfl_down_sync(0xffffffffu, v, 1), (unsigned)(u & 3) * 8);
+            if (wd < WPITCH) L.win[r * WPITCH + wd] = w;
+        }
+    } else {
+        for (int i = lane; i < WROWS * WPITCH; i += 32) {
+            const int r = i / WPITCH, f = first + r * e0.w + 4 * (i - r * WPITCH);
+            unsigned w = 0;
+#pragma unroll
+            for (int k = 0; k < 4; k++)
+                if ((unsigned)(f + k) < (unsigned)size) w |= (unsigned)__ldg(e0.p + f + k) << (8 * k);
+            L.win[i] = w;
         }
     }
     __syncwarp();
 }
 
-// Quarter sample at offset (sy, sx) around the even point (qr, qc), the
-// assignments of LoadQuartPelWindow (…MultiresCross.cpp:1365-1389).
-__device__ __forceinline__ int quarter(const Lattice& L, int qr, int qc, int sy, int sx)
+// One lane's candidate: its distortion d and limit t (kPartial: phase_limit; else t = d).
+__device__ __forceinline__ int score4(const unsigned (&cur)[4], const Buf& e, Org o)
 {
-    int a, b;
-    if (sy < 0) {
-        a = lat(L, qr - 2, sx < 0 ? qc - 2 : qc);
-        b = sx > 0 ? lat(L, qr, qc + 2) : lat(L, qr, qc);
-    } else if (sy == 0) {
-        a = lat(L, qr, qc + (sx < 0 ? -2 : 2));
-        b = lat(L, qr, qc);
-    } else {
-        a = sx < 0 ? lat(L, qr, qc - 2) : lat(L, qr + 2, qc);
-        b = sx > 0 ? lat(L, qr, qc + 2) : (sx < 0 ? lat(L, qr + 2, qc) : lat(L, qr, qc));
+    unsigned d = 0;
+#pragma unroll
+    for (int r = 0; r < 4; r++) {
+        unsigned w[1];
+        row_words(e.p + (size_t)(o.y + r) * e.w + o.x, w);
+        const unsigned x = __vabsdiffu4(cur[r], w[0]);
+        d = __dp4a(x, x, d);
     }
-    return (a + b + 1) >> 1;
+    return (int)d;
+}
+
+template <bool kPartial>
+__device__ __forceinline__ void score8(const Window& L, const Buf& e, Org o, int& d, int& t)
+{
+    const unsigned char* p = e.p + (size_t)o.y * e.w + o.x;
+    unsigned s[16] = {0u};
+#pragma unroll
+    for (int r = 0; r < 4; r++) {
+        unsigned w[2], x[2];
+        row_words(p + (size_t)r * e.w, w);
+        row_words(p + (size_t)(r + 4) * e.w, x);
+        const uint2 c = L.cur1[r], f = L.cur1[r + 4];
+        const unsigned d0 = __vabsdiffu4(c.x, w[0]), d1 = __vabsdiffu4(c.y, w[1]);
+        const unsigned d2 = __vabsdiffu4(f.x, x[0]), d3 = __vabsdiffu4(f.y, x[1]);
+        if (kPartial) add_classes(d0, d1, d2, d3, s + 4 * r);
+        else s[0] = __dp4a(d3, d3, __dp4a(d2, d2, __dp4a(d1, d1, __dp4a(d0, d0, s[0]))));
+    }
+    if (kPartial) phase_limit(s, d, t);
+    else t = d = (int)s[0];
+}
+
+template <bool kPartial>
+__device__ __forceinline__ void score16(const Window& L, int row, int col, int& d, int& t)
+{
+    unsigned s[16] = {0u};
+#pragma unroll 1
+    for (int i = 0; i < 16; i += 4)
+#pragma unroll
+        for (int r = 0; r < 4; r++) {
+            const uint4 c = L.cur[i + r];
+            unsigned w[4];
+            window_row(L.win + (row + i + r) * WPITCH, col, w);
+            const unsigned d0 = __vabsdiffu4(c.x, w[0]), d1 = __vabsdiffu4(c.y, w[1]);
+            const unsigned d2 = __vabsdiffu4(c.z, w[2]), d3 = __vabsdiffu4(c.w, w[3]);
+            if (kPartial) add_classes(d0, d1, d2, d3, s + 4 * r);
+            else s[0] = __dp4a(d3, d3, __dp4a(d2, d2, __dp4a(d1, d1, __dp4a(d0, d0, s[0]))));
+        }
+    if (kPartial) phase_limit(s, d, t);
+    else t = d = (int)s[0];
+}
+
+// Decide the warp's candidates in lane order against the running minimum: a lane's candidate v (a packed
+// offset) replaces it when its limit t is at most min, an equal distortion only if tie(x, y) returns
+// false.  tie and take are called with the same arguments in every lane.
+template <typename Tie, typename Take>
+__device__ __forceinline__ void settle(bool valid, int d, int t, int v, int& min, Tie&& tie, Take&& take)
+{
+    unsigned todo = __ballot_sync(0xffffffffu, valid && t <= min);
+    while (todo) {
+        const int l = __ffs(todo) - 1;
+        todo &= todo - 1;
+        const int dl = __shfl_sync(0xffffffffu, d, l), vl = __shfl_sync(0xffffffffu, v, l);
+        if (dl == min) {
+            if (tie(mv_x(vl), mv_y(vl))) continue;
+        } else {
+            min = dl;
+            todo &= __ballot_sync(0xffffffffu, t <= dl);
+        }
+        take(mv_x(vl), mv_y(vl), dl);
+    }
+}
+
+// A full search of the offsets [xl, xr] x [yu, yd] in raster order, the centre's distortion first, which
+// starts the minimum.  score(x, y, d, t): a lane's candidate.
+template <typename Score, typename Tie, typename Take>
+__device__ __forceinline__ void raster(int xl, int xr, int yu, int yd, int& min, int lane, Score&& score, Tie&& tie,
+                                       Take&& take)
+{
+    const int nx = xr - xl + 1, ny = yd - yu + 1, n = nx > 0 && ny > 0 ? nx * ny : 0;
+    for (int e0 = 0; e0 <= n; e0 += 32) {
+        const int e = e0 + lane - 1;  // -1: the centre
+        const bool in = e >= 0 && e < n;
+        const int r = in ? (int)((unsigned)e / (unsigned)nx) : 0;
+        const int j = in ? xl + e - r * nx : 0, i = in ? yu + r : 0;
+        int d, t;
+        score(j, i, d, t);
+        if (e0 == 0) min = __shfl_sync(0xffffffffu, d, 0);
+        settle(in && (i || j), d, t, pack_mv(j, i), min, tie, take);
+    }
+}
+
+// The four offsets of a cross step in the estimators' order: left, right, up, down.
+__device__ __forceinline__ void cross_offset(int lane, int s, int& j, int& i)
+{
+    const int v = (lane & 1) ? s : -s;
+    j = (lane & 2) ? 0 : v;
+    i = (lane & 2) ? v : 0;
+}
+
+// Two 16-bit 6-tap sums + RAW_BIAS (never negative, below 2^14), and their rounded, clipped samples.
+__device__ __forceinline__ unsigned tap_pair(unsigned a, unsigned b, unsigned c, unsigned d, unsigned e, unsigned f)
+{
+    return (a + f + RAW_BIAS * 0x10001u) + 20u * (c + d) - 5u * (b + e);
+}
+__device__ __forceinline__ unsigned scale_pair(unsigned t)
+{
+    constexpr unsigned off = 0x10000u - RAW_BIAS / 32;  // -(RAW_BIAS / 32) in each half
+    return __viaddmin_s16x2_relu(((t + 0x00100010u) >> 5) & 0x07ff07ffu, off << 16 | off, 0x00ff00ffu);
+}
+
+// The lattice whose row 0 is the window's row wy; its column 0 may be any of the window's columns 0..4.
+template <bool kVer2>
+__device__ __forceinline__ void build_lattice(Lattice& L, int wy, int lane)
+{
+    constexpr unsigned m = 0x00ff00ffu;
+    unsigned *h = L.sub, *b = L.sub + SUB_PLANE, *jp = L.sub + 2 * SUB_PLANE;
+    if (lane < 4 * WPITCH) {  // h, rows 2..18: a word column and five rows per lane
+        const int g = lane / WPITCH, wd = lane - g * WPITCH;
+        unsigned ev[10], od[10];
+#pragma unroll
+        for (int i = 0; i < 10; i++) {
+            const unsigned w = L.win[(wy + 4 * g + i) * WPITCH + wd];
+            ev[i] = w & m;
+            od[i] = (w >> 8) & m;
+        }
+#pragma unroll
+        for (int i = 0; i < 5; i++) {
+            const unsigned te = tap_pair(ev[i], ev[i + 1], ev[i + 2], ev[i + 3], ev[i + 4], ev[i + 5]);
+            const unsigned to = tap_pair(od[i], od[i + 1], od[i + 2], od[i + 3], od[i + 4], od[i + 5]);
+            const int at = (4 * g + i) * WPITCH + wd;
+            L.raw[2 * at] = __byte_perm(te, to, 0x5410);
+            L.raw[2 * at + 1] = __byte_perm(te, to, 0x7632);
+            h[at] = scale_pair(te) | scale_pair(to) << 8;
+        }
+    }
+    for (int i = lane; i < 18 * 6; i += 32) {  // b, rows 2..19: words 0..5 hold its columns 2..18
+        const int r = i / 6, wd = i - 6 * r;
+        const unsigned* q = L.win + (wy + 2 + r) * WPITCH + wd;
+        const unsigned p = wd ? q[-1] : 0u;
+        const unsigned e0 = p & m, o0 = (p >> 8) & m, e1 = q[0] & m, o1 = (q[0] >> 8) & m, e2 = q[1] & m,
+                       o2 = (q[1] >> 8) & m;
+        const unsigned em = __funnelshift_r(e0, e1, 16), om = __funnelshift_r(o0, o1, 16);
+        const unsigned ep = __funnelshift_r(e1, e2, 16), op = __funnelshift_r(o1, o2, 16);
+        const unsigned te = tap_pair(em, om, e1, o1, ep, op), to = tap_pair(om, e1, o1, ep, op, e2);
+        b[r * WPITCH + wd] = scale_pair(te) | scale_pair(to) << 8;
+        if (!kVer2 && r == 17) {
+            L.row19[2 * wd] = __byte_perm(te, to, 0x5410);
+            L.row19[2 * wd + 1] = __byte_perm(te, to, 0x7632);
+        }
+    }
+    __syncwarp();
+    for (int i = lane; i < 17 * 6; i += 32) {  // j, rows 2..18, from the raw h; the taps sum to 32
+        const int r = i / 6, wd = i - 6 * r;
+        const unsigned* q = L.raw + 2 * (r * WPITCH + wd);
+        const int p0 = wd ? (int)q[-1] : 0, p1 = (int)q[0], p2 = (int)q[1], p3 = (int)q[2], p4 = (int)q[3];
+        constexpr int c0 = 512 - 32 * RAW_BIAS;
+        // pairs of taps as bytes: (1, -5), (20, 20), (-5, 1) from an even sample, (0, 1), (-5, 20), (20, -5),
+        // (1, 0) from an odd one
+        constexpr int ka = 0x1414fb01, kb = 0x000001fb, kc = 0x14fb0100, kd = 0x0001fb14;
+        const int v0 = __dp2a_lo(p2, kb, __dp2a_hi(p1, ka, __dp2a_lo(p0, ka, c0)));
+        const int v1 = __dp2a_hi(p3, kd, __dp2a_lo(p2, kd, __dp2a_hi(p1, kc, __dp2a_lo(p0, kc, c0))));
+        const int v2 = __dp2a_lo(p3, kb, __dp2a_hi(p2, ka, __dp2a_lo(p1, ka, c0)));
+        const int v3 = __dp2a_hi(p4, kd, __dp2a_lo(p3, kd, __dp2a_hi(p2, kc, __dp2a_lo(p1, kc, c0))));
+        const unsigned ve = __byte_perm((unsigned)(v0 >> 10), (unsigned)(v2 >> 10), 0x5410);
+        const unsigned vo = __byte_perm((unsigned)(v1 >> 10), (unsigned)(v3 >> 10), 0x5410);
+        jp[r * WPITCH + wd] = __viaddmin_s16x2_relu(ve, 0u, 0x00ff00ffu) | __viaddmin_s16x2_relu(vo, 0u, 0x00ff00ffu) << 8;
+    }
+    __syncwarp();
+}
+
+// Where the samples of even quarter point (qr, qc) lie for block sample (0, 0): the word of the lattice
+// their row starts at, and the byte column.
+struct Point {
+    int word, col;
+};
+__device__ __forceinline__ Point lattice_point(int wy, int wx, int qr, int qc)
+{
+    constexpr int win = 16 * 4 + 8 * 2, sub = (int)sizeof(Window) / 4;
+    const int plane = ((qr >> 1) & 1) | (qc & 2);  // G, h, b, j
+    const int fr = qr >> 2;
+    return Point{plane ? sub + (plane - 1) * SUB_PLANE + (fr - 2) * WPITCH : win + (wy + fr) * WPITCH, wx + (qc >> 2)};
+}
+
+// Of the four lanes of a candidate, each with the class sums of one row class: settle the eight
+// candidates (v, the lane's), strict improvements.
+template <bool kPartial, typename Take>
+__device__ __forceinline__ void settle_quads(const unsigned (&s)[4], int v, int& min, int lane, Take&& take)
+{
+    int d = (int)(s[0] + s[1] + s[2] + s[3]);
+    d += __shfl_xor_sync(0xffffffffu, d, 1);
+    d += __shfl_xor_sync(0xffffffffu, d, 2);
+    if (!__any_sync(0xffffffffu, d < min)) return;
+    int t = d;
+    if (kPartial) {
+        unsigned all[16];
+#pragma unroll
+        for (int r = 0; r < 4; r++)
+#pragma unroll
+            for (int c = 0; c < 4; c++) all[4 * r + c] = __shfl_sync(0xffffffffu, s[c], (lane & 28) | r);
+        phase_limit(all, d, t);
+    }
+    settle((lane & 3) == 0 && d < min, d, t, v, min, [](int, int) { return true; }, take);
+}
+
+__device__ __forceinline__ int byte_of(unsigned w, int k) { return (int)((w >> (8 * k)) & 0xffu); }
+__device__ __forceinline__ int raw_of(const unsigned* w, int i)
+{
+    return (int)reinterpret_cast<const unsigned short*>(w)[i] - RAW_BIAS;
+}
+
+// Half then quarter pel in the estimator's window around block o (…MultiresCross.cpp:875-941), strict
+// improvements: eight candidates of a pass at once, four lanes each (a row class per lane).  The quarter
+// samples are the averages of two even ones that LoadQuartPelWindow (…MultiresCross.cpp:1365-1389) pairs.
+// take(qx, qy, d): an accepted quarter-pel offset.
+template <bool kVer2, bool kPartial, typename Take>
+__device__ __forceinline__ void subpel(Lattice& L, const Buf& e0, Org oc, Org o, int& min_d, int& qmx, int& qmy,
+                                       int lane, bool& bad, Take&& take)
+{
+    const int wy = o.y - oc.y + 2, wx = o.x - oc.x + 2;
+    // the reference reads the samples of all 22 x 22 points
+    bad |= (o.y - 3) * e0.w + o.x - 3 < 0 || (o.y + 18) * e0.w + o.x + 18 >= e0.w * e0.h;
+    build_lattice<kVer2>(L, wy, lane);
+    const unsigned* words = reinterpret_cast<const unsigned*>(&L);
+    const int rho = lane & 3, c9 = (lane >> 2) + (lane >= 16), sy = c9 / 3 - 1, sx = c9 - 3 * (c9 / 3) - 1;
+    {
+        const Point a = lattice_point(wy, wx, 12 + 2 * sy, 12 + 2 * sx);
+        unsigned s[4] = {0u, 0u, 0u, 0u};
+#pragma unroll
+        for (int i = 0; i < 4; i++) {
+            const int r = rho + 4 * i;
+            const uint4 c = L.cur[r];
+            unsigned w[4];
+            window_row(words + a.word + r * WPITCH, a.col, w);
+            add_classes(__vabsdiffu4(c.x, w[0]), __vabsdiffu4(c.y, w[1]), __vabsdiffu4(c.z, w[2]),
+                        __vabsdiffu4(c.w, w[3]), s);
+        }
+        settle_quads<kPartial>(s, pack_mv(2 * sx, 2 * sy), min_d, lane, [&](int x, int y, int d) {
+            qmx = x;
+            qmy = y;
+            take(x, y, d);
+        });
+    }
+    const int hmx = qmx, hmy = qmy, qr = 12 + hmy, qc = 12 + hmx;
+    Point a, b;
+    if (sy == 0) {
+        a = lattice_point(wy, wx, qr, qc + 2 * sx);
+        b = lattice_point(wy, wx, qr, qc);
+    } else {
+        const Point up = lattice_point(wy, wx, qr + 2 * sy, qc);
+        a = sy < 0 ? lattice_point(wy, wx, qr - 2, sx < 0 ? qc - 2 : qc) : (sx < 0 ? lattice_point(wy, wx, qr, qc - 2) : up);
+        b = sx > 0 ? lattice_point(wy, wx, qr, qc + 2) : (sy > 0 && sx < 0 ? up : lattice_point(wy, wx, qr, qc));
+    }
+    // the incomplete row and column 19, met in block row 15 and column 15
+    const bool row_edge = !kVer2 && hmy == 2 && sy > 0, col_edge = !kVer2 && hmx == 2 && sx > 0;
+    unsigned s[4] = {0u, 0u, 0u, 0u};
+#pragma unroll
+    for (int i = 0; i < 4; i++) {
+        const int r = rho + 4 * i;
+        const uint4 c = L.cur[r];
+        unsigned wa[4], wb[4];
+        window_row(words + a.word + r * WPITCH, a.col, wa);
+        window_row(words + b.word + r * WPITCH, b.col, wb);
+        const unsigned cw[4] = {c.x, c.y, c.z, c.w};
+        int edge = 0;  // column 19's sample
+        if (col_edge && hmy) edge = raw_of(L.raw + 2 * WPITCH * ((qr >> 2) - 2 + r), wx + 19);
+        if (i == 3 && row_edge && rho == 3) {
+            const int at = wx + (qc >> 2);
+#pragma unroll
+            for (int k = 0; k < 16; k++) {
+                const int x = hmx ? raw_of(L.row19, at + k) : 0;
+                const int y = k == 15 && col_edge ? edge : byte_of(sx < 0 ? wa[k >> 2] : wb[k >> 2], k & 3);
+                const int e = byte_of(cw[k >> 2], k & 3) - ((x + y + 1) >> 1);
+                s[k & 3] += (unsigned)(e * e);
+            }
+        } else {
+            unsigned d[4];
+#pragma unroll
+            for (int k = 0; k < 4; k++) d[k] = __vabsdiffu4(cw[k], __vavgu4(wa[k], wb[k]));
+            if (col_edge) {
+                const int y = byte_of(sy == 0 ? wb[3] : wa[3], 3);
+                const int e = byte_of(cw[3], 3) - ((edge + y + 1) >> 1);
+                d[3] &= 0x00ffffffu;
+                s[3] += (unsigned)(e * e);
+            }
+            add_classes(d[0], d[1], d[2], d[3], s);
+        }
+    }
+    settle_quads<kPartial>(s, pack_mv(hmx + sx, hmy + sy), min_d, lane, [&](int x, int y, int d) {
+        qmx = x;
+        qmy = y;
+        take(x, y, d);
+    });
+    __syncwarp();  // the lattice is reused by this warp's next search
+}
+
+// The input block of level 1 into L.cur1.
+__device__ __forceinline__ void stage_level1(const MrcArgs& a, Window& L, int q, int p, int lane)
+{
+    const Org o = origin(a.in1, 8, 8, 0, q, p);
+    if (lane < 16) {
+        unsigned w[1];
+        row_words(a.in1.p + (size_t)(o.y + (lane >> 1)) * a.in1.w + o.x + 4 * (lane & 1), w);
+        reinterpret_cast<unsigned*>(L.cur1)[lane] = w[0];
+    }
+    __syncwarp();
+}
+
+// The input block of level 2, in every lane.
+__device__ __forceinline__ void load_level2(const MrcArgs& a, int ll, int kk, unsigned (&cur)[4])
+{
+    const Org o = origin(a.in2, 4, 4, 0, ll, kk);
+#pragma unroll
+    for (int r = 0; r < 4; r++) {
+        unsigned w[1];
+        row_words(a.in2.p + (size_t)(o.y + r) * a.in2.w + o.x, w);
+        cur[r] = w[0];
+    }
 }
 
 // ---------------------------------------------------------------------------
@@ -264,43 +585,44 @@ __device__ __forceinline__ bool farther(int mx, int my, int rmx, int rmy, int j,
 // decides an exact tie at an integer level: true keeps the current best
 // (offset (rmx, rmy) from the centre (mx, my)), false takes the candidate at
 // offset (j, i).  It is called with the same arguments in every lane.
-template <bool kVer2, typename Skip, bool kH263 = false>
-__device__ MbSearch search_mb_with(const MrcArgs& a, Lattice& LT, int mbr, int mbc, Skip&& skip, int lane, bool& bad)
+template <bool kVer2, typename Skip, bool kH263 = false, typename Store>
+__device__ MbSearch search_mb_with(const MrcArgs& a, Store& LT, int mbr, int mbc, Skip&& skip, int lane, bool& bad)
 {
     const int m = 16 * mbr, n = 16 * mbc, p = 8 * mbr, q = 8 * mbc, kk = 4 * mbr, ll = 4 * mbc;
     const int w1 = a.W / 2, h1 = a.H / 2, w2 = w1 / 2, h2 = h1 / 2;
     const int l1_range = a.motion_range / 8, l2_range = l1_range / 2;
     const int lcl_l1_range = a.mode == 2 ? 2 : l1_range;
     const Level L0{16, a.W, a.H, a.motion_range / 4}, L1{8, w1, h1, l1_range}, L2{4, w2, h2, l2_range};
-    constexpr int CRX[4] = {-1, 1, 0, 0}, CRY[4] = {0, 0, -1, 1};
-    constexpr int SX[8] = {-1, 0, 1, -1, 1, -1, 0, 1}, SY[8] = {-1, -1, -1, 0, 0, 1, 1, 1};
     MbSearch out;
     out.tie = 0;
 
-    const Org oin0 = origin(a.in0, 16, 16, 0, n, m);
-    out.zero_d = full_ssd(a.in0, oin0, a.e0, origin(a.e0, 16, 16, 19, n, m), 16, lane, bad);
+    __syncwarp();
+    out.zero_d = zero_distortion(a, LT, origin(a.in0, 16, 16, 0, n, m), n, m, lane);
+    stage_level1(a, LT, q, p, lane);
     int mx = 0, my = 0, rmx = 0, rmy = 0, xl, xr, yu, yd;
+    int min, lvl = 2;
+    auto tie = [&](int j, int i) {
+        out.tie |= TIE_L0 >> lvl;
+        return skip(lvl, mx, my, rmx, rmy, j, i);
+    };
+    auto take = [&](int j, int i, int) {
+        rmx = j;
+        rmy = i;
+    };
 
     if (a.mode == 2) {  // level 2 cross search (…MultiresCross.cpp:639-697)
-        const Org oin2 = origin(a.in2, 4, 4, 0, ll, kk);
-        int min2 = full_ssd(a.in2, oin2, a.e2, origin(a.e2, 4, 4, 5, ll, kk), 4, lane, bad);
+        // Tsd4x4LessThan stops early only on a sum already above min: a full SSD decides the same
+        unsigned cur2[4];
+        load_level2(a, ll, kk, cur2);
+        min = score4(cur2, a.e2, origin(a.e2, 4, 4, 5, ll, kk));
         mr_range(L2, ll, kk, 0, 0, l2_range - 1, xl, xr, yu, yd);
         for (int s = l2_range / 2; s > 0; s /= 2) {
             rmx = rmy = 0;
-            for (int c = 0; c < 4; c++) {
-                const int i = s * CRY[c], j = s * CRX[c];
-                if (i + my < yu || i + my > yd || j + mx < xl || j + mx > xr) continue;
-                // Tsd4x4LessThan stops early only on a sum already above min: a full SSD decides the same
-                const int d = full_ssd(a.in2, oin2, a.e2, origin(a.e2, 4, 4, 5, j + ll + mx, i + kk + my), 4, lane, bad);
-                if (d > min2) continue;
-                if (d == min2) {
-                    out.tie |= TIE_L2;
-                    if (skip(2, mx, my, rmx, rmy, j, i)) continue;
-                }
-                min2 = d;
-                rmx = j;
-                rmy = i;
-            }
+            int j, i;
+            cross_offset(lane, s, j, i);
+            const int d = score4(cur2, a.e2, origin(a.e2, 4, 4, 5, j + ll + mx, i + kk + my));
+            settle(lane < 4 && i + my >= yu && i + my <= yd && j + mx >= xl && j + mx <= xr, d, d, pack_mv(j, i), min, tie,
+                   take);
             mx += rmx;
             my += rmy;
         }
@@ -308,49 +630,26 @@ __device__ MbSearch search_mb_with(const MrcArgs& a, Lattice& LT, int mbr, int m
         my <<= 1;
     }
 
-    // level 1 (…MultiresCross.cpp:699-816): input samples of this lane's phase share, kept
-    const Org oin1 = origin(a.in1, 8, 8, 0, q, p);
-    int r1, c1;
-    phase_coords<8>(lane, r1, c1);
-    int cur1[2];
-#pragma unroll
-    for (int j = 0; j < 2; j++) cur1[j] = rdb(a.in1, oin1.y + r1, oin1.x + c1 + 4 * j);
-    auto part8 = [&](Org o) {
-        int acc = 0;
-#pragma unroll
-        for (int j = 0; j < 2; j++) {
-            const int d = cur1[j] - rdb(a.e1, o.y + r1, o.x + c1 + 4 * j);
-            acc += d * d;
-        }
-        return acc;
-    };
-    int min1 = full_ssd(a.in1, oin1, a.e1, origin(a.e1, 8, 8, 9, mx + q, my + p), 8, lane, bad);
+    // level 1 (…MultiresCross.cpp:699-816)
+    lvl = 1;
     rmx = rmy = 0;
-    auto consider1 = [&](int i, int j) {
-        const int d = partial_value(part8(origin(a.e1, 8, 8, 9, j + mx + q, i + my + p)), min1, lane);
-        if (d > min1) return;
-        if (d == min1) {
-            out.tie |= TIE_L1;
-            if (skip(1, mx, my, rmx, rmy, j, i)) return;
-        }
-        min1 = d;
-        rmx = j;
-        rmy = i;
+    auto score1 = [&](int j, int i, int& d, int& t) {
+        score8<true>(LT, a.e1, origin(a.e1, 8, 8, 9, j + mx + q, i + my + p), d, t);
     };
     if (a.mode == 2) {
         mr_range(L1, q, p, mx, my, lcl_l1_range, xl, xr, yu, yd);
-        for (int i = yu; i <= yd; i++)
-            for (int j = xl; j <= xr; j++)
-                if (i || j) consider1(i, j);
+        raster(xl, xr, yu, yd, min, lane, score1, tie, take);
     } else {
+        int t;
+        score1(0, 0, min, t);
         for (int s = l1_range / 2; s > 0; s /= 2) {
             mr_range(L1, q, p, mx, my, lcl_l1_range - 1, xl, xr, yu, yd);
             rmx = rmy = 0;
-            for (int c = 0; c < 4; c++) {
-                const int i = s * CRY[c], j = s * CRX[c];
-                if (i + my < yu || i + my > yd || j + mx < xl || j + mx > xr) continue;
-                consider1(i, j);
-            }
+            int j, i, d;
+            cross_offset(lane, s, j, i);
+            score1(j, i, d, t);
+            settle(lane < 4 && i + my >= yu && i + my <= yd && j + mx >= xl && j + mx <= xr, d, t, pack_mv(j, i), min, tie,
+                   take);
             mx += rmx;
             my += rmy;
         }
@@ -360,151 +659,75 @@ __device__ MbSearch search_mb_with(const MrcArgs& a, Lattice& LT, int mbr, int m
     my = (my + rmy) * 2;
 
     // level 0 +-2 refinement (…MultiresCross.cpp:819-873)
-    int r0, c0;
-    phase_coords<16>(lane, r0, c0);
-    int cur0[8];
-#pragma unroll
-    for (int i = 0; i < 2; i++)
-#pragma unroll
-        for (int j = 0; j < 4; j++) cur0[4 * i + j] = rdb(a.in0, oin0.y + r0 + 4 * i, oin0.x + c0 + 4 * j);
-    auto part16 = [&](Org o) {
-        int acc = 0;
-#pragma unroll
-        for (int i = 0; i < 2; i++)
-#pragma unroll
-            for (int j = 0; j < 4; j++) {
-                const int d = cur0[4 * i + j] - rdb(a.e0, o.y + r0 + 4 * i, o.x + c0 + 4 * j);
-                acc += d * d;
-            }
-        return acc;
-    };
-    int min_d = full_ssd(a.in0, oin0, a.e0, origin(a.e0, 16, 16, 19, n + mx, m + my), 16, lane, bad);
+    lvl = 0;
     rmx = rmy = 0;
+    const Org oc = origin(a.e0, 16, 16, 19, n + mx, m + my);
+    stage_level0(a.e0, LT, oc, lane);
     mr_range(L0, n, m, mx, my, 2, xl, xr, yu, yd);
-    for (int i = yu; i <= yd; i++)
-        for (int j = xl; j <= xr; j++) {
-            if (!(i || j)) continue;
-            const int d = partial_value(part16(origin(a.e0, 16, 16, 19, n + mx + j, m + my + i)), min_d, lane);
-            if (d > min_d) continue;
-            if (d == min_d) {
-                out.tie |= TIE_L0;
-                if (skip(0, mx, my, rmx, rmy, j, i)) continue;
-            }
-            min_d = d;
-            rmx = j;
-            rmy = i;
-        }
+    raster(xl, xr, yu, yd, min, lane,
+           [&](int j, int i, int& d, int& t) {
+               const Org c = origin(a.e0, 16, 16, 19, n + mx + j, m + my + i);
+               score16<true>(LT, c.y - oc.y + 5, c.x - oc.x + 5, d, t);
+           },
+           tie, take);
     mx += rmx;
     my += rmy;
+    const Org o = origin(a.e0, 16, 16, 19, n + mx, m + my);
     if constexpr (kH263) {
         // MotionEstimatorH263ImplMultiresCross (…H263ImplMultiresCross.cpp:885-940): the best of the
         // four diagonal half-pel corners, then the two points beside the winning corner (the full cross
         // if no corner won), each an OverlayMem2Dv2::HalfRead block (bilinear, +2 >> 2 diagonal, +1 >> 1
         // linear; the left neighbour for -1) of the level-0 reference, strict improvements; half pels.
         // Every sample read lies within 17 of the picture, where the border-19 copy holds the same edge
-        // replication as the reference's border-17 one.
-        constexpr int CX4[4] = {-1, 1, -1, 1}, CY4[4] = {-1, -1, 1, 1};
-        constexpr int RX[4][2] = {{0, -1}, {0, 1}, {0, -1}, {0, 1}}, RY[4][2] = {{-1, 0}, {-1, 0}, {1, 0}, {1, 0}};
-        const Org o = origin(a.e0, 16, 16, 19, n + mx, m + my);
-        auto half_part = [&](int hx, int hy) {
-            int acc = 0;
+        // replication as the reference's border-17 one.  Four lanes a candidate, a row class each.
+        bad |= (o.y - 1) * a.e0.w + o.x - 1 < 0 || (o.y + 16) * a.e0.w + o.x + 16 >= a.e0.w * a.e0.h;
+        const int row = o.y - oc.y + 5, col = o.x - oc.x + 5, rho = lane & 3, k = lane >> 2;
+        int hmx = 0, hmy = 0;
+        auto half_stage = [&](int hx, int hy, bool valid) {
+            unsigned s[4] = {0u, 0u, 0u, 0u};
 #pragma unroll
-            for (int i = 0; i < 2; i++)
+            for (int i = 0; i < 4; i++) {
+                const uint4 c = LT.cur[rho + 4 * i];
+                const unsigned cw[4] = {c.x, c.y, c.z, c.w};
+                const unsigned* w = LT.win + (row + rho + 4 * i) * WPITCH;
+                unsigned w00[4], w01[4], w10[4], w11[4], d[4];
+                window_row(w, col, w00);
+                window_row(w, col + hx, w01);
+                window_row(w + hy * WPITCH, col, w10);
+                window_row(w + hy * WPITCH, col + hx, w11);
 #pragma unroll
-                for (int j = 0; j < 4; j++) {
-                    const int r = o.y + r0 + 4 * i, c = o.x + c0 + 4 * j + (hx < 0 ? -1 : 0);
-                    int v;
-                    if (hx && hy)
-                        v = (rd(a.e0, r, c, bad) + rd(a.e0, r + hy, c, bad) + rd(a.e0, r, c + 1, bad) +
-                             rd(a.e0, r + hy, c + 1, bad) + 2) >> 2;
-                    else if (hx)
-                        v = (rd(a.e0, r, c, bad) + rd(a.e0, r, c + 1, bad) + 1) >> 1;
-                    else
-                        v = (rd(a.e0, r, c, bad) + rd(a.e0, r + hy, c, bad) + 1) >> 1;
-                    const int d = cur0[4 * i + j] - v;
-                    acc += d * d;
-                }
-            return acc;
+                for (int e = 0; e < 4; e++) d[e] = __vabsdiffu4(cw[e], half4(w00[e], w01[e], w10[e], w11[e], hx, hy));
+                add_classes(d[0], d[1], d[2], d[3], s);
+            }
+            if (!valid) s[0] = 0x10000000u;  // above any block's distortion
+            settle_quads<true>(s, pack_mv(hx, hy), min, lane, [&](int x, int y, int) {
+                hmx = x;
+                hmy = y;
+            });
         };
-        int hmx = 0, hmy = 0, best_corner = 0;
-        for (int k = 0; k < 4; k++) {
-            const int d = partial_value(half_part(CX4[k], CY4[k]), min_d, lane);
-            if (d < min_d) {
-                best_corner = k;
-                min_d = d;
-                hmx = CX4[k];
-                hmy = CY4[k];
-            }
-        }
-        const bool won = hmx || hmy;
-        for (int k = 0; k < (won ? 2 : 4); k++) {
-            const int hx = won ? RX[best_corner][k] : CRX[k], hy = won ? RY[best_corner][k] : CRY[k];
-            const int d = partial_value(half_part(hx, hy), min_d, lane);
-            if (d < min_d) {
-                min_d = d;
-                hmx = hx;
-                hmy = hy;
-            }
-        }
-        out.min_d = min_d;
+        half_stage((k & 1) ? 1 : -1, (k & 2) ? 1 : -1, k < 4);
+        const int vx = hmx, vy = hmy;  // the winning corner
+        if (vx || vy) half_stage((k & 1) ? vx : 0, (k & 1) ? 0 : vy, k < 2);
+        else half_stage((k & 2) ? 0 : ((k & 1) ? 1 : -1), (k & 2) ? ((k & 1) ? 1 : -1) : 0, k < 4);
+        __syncwarp();
+        out.min_d = min;
         out.mvx = 2 * mx + hmx;
         out.mvy = 2 * my + hmy;
         return out;
+    } else {
+        int qmx = 0, qmy = 0;
+        subpel<kVer2, true>(LT, a.e0, oc, o, min, qmx, qmy, lane, bad, [](int, int, int) {});
+        out.min_d = min;
+        out.mvx = mx * 4 + qmx;
+        out.mvy = my * 4 + qmy;
+        return out;
     }
-    int mvx = mx * 4, mvy = my * 4;
-
-    // half then quarter pel in the estimator's window (…MultiresCross.cpp:875-941), strict improvements
-    build_lattice<kVer2>(LT, a.e0, origin(a.e0, 16, 16, 19, n + mx, m + my), lane, bad);
-    int hmx = 0, hmy = 0;
-    for (int c = 0; c < 8; c++) {
-        const int qx = 2 * SX[c], qy = 2 * SY[c];
-        int acc = 0;
-#pragma unroll
-        for (int i = 0; i < 2; i++)
-#pragma unroll
-            for (int j = 0; j < 4; j++) {
-                const int d = cur0[4 * i + j] - lat(LT, 12 + qy + 4 * (r0 + 4 * i), 12 + qx + 4 * (c0 + 4 * j));
-                acc += d * d;
-            }
-        const int d = partial_value(acc, min_d, lane);
-        if (d < min_d) {
-            min_d = d;
-            hmx = qx;
-            hmy = qy;
-        }
-    }
-    int qmx = hmx, qmy = hmy;
-    for (int c = 0; c < 8; c++) {
-        int acc = 0;
-#pragma unroll
-        for (int i = 0; i < 2; i++)
-#pragma unroll
-            for (int j = 0; j < 4; j++) {
-                const int d = cur0[4 * i + j] -
-                              quarter(LT, 12 + hmy + 4 * (r0 + 4 * i), 12 + hmx + 4 * (c0 + 4 * j), SY[c], SX[c]);
-                acc += d * d;
-            }
-        const int d = partial_value(acc, min_d, lane);
-        if (d < min_d) {
-            min_d = d;
-            qmx = hmx + SX[c];
-            qmy = hmy + SY[c];
-        }
-    }
-    __syncwarp();  // the lattice is reused by this warp's next search
-    out.min_d = min_d;
-    out.mvx = mvx + qmx;
-    out.mvy = mvy + qmy;
-    return out;
 }
 
 // The search of MotionEstimatorH264ImplMultires (…Multires.cpp:644-906): full
 // searches at level 2 (+-(range/16 - 1)) and level 1 (+-2 after level 2, else
 // +-range/8), +-2 at level 0, half and quarter pel in the MultiresCross-style
-// window; LessThan distortions, which decide exactly as full SSDs do.  The
-// warp scores candidates in raster order: level 0 and 1 one candidate at a
-// time, each lane holding a fixed share of the input block; level 2 (4x4)
-// two at a time, one per half-warp.
+// window; LessThan distortions, which decide exactly as full SSDs do.
 template <typename Skip>
 __device__ MbSearch search_mr_with(const MrcArgs& a, Lattice& LT, int mbr, int mbc, Skip&& skip, int lane, bool& bad)
 {
@@ -513,166 +736,66 @@ __device__ MbSearch search_mr_with(const MrcArgs& a, Lattice& LT, int mbr, int m
     const int l1_range = a.motion_range / 8, l2_range = l1_range / 2;
     const int lcl_l1_range = a.mode == 2 ? 2 : l1_range;
     const Level L0{16, a.W, a.H, a.motion_range / 4}, L1{8, w1, h1, l1_range}, L2{4, w2, h2, l2_range};
-    constexpr int SX[8] = {-1, 0, 1, -1, 1, -1, 0, 1}, SY[8] = {-1, -1, -1, 0, 0, 1, 1, 1};
     MbSearch out;
     out.tie = 0;
-    const Org oin0 = origin(a.in0, 16, 16, 0, n, m);
-    out.zero_d = full_ssd(a.in0, oin0, a.e0, origin(a.e0, 16, 16, 19, n, m), 16, lane, bad);
-    int mx = 0, my = 0, xl, xr, yu, yd;
+    __syncwarp();
+    out.zero_d = zero_distortion(a, LT, origin(a.in0, 16, 16, 0, n, m), n, m, lane);
+    stage_level1(a, LT, q, p, lane);
+    int mx = 0, my = 0, rmx = 0, rmy = 0, xl, xr, yu, yd, min, lvl = 2;
+    auto tie = [&](int j, int i) {
+        out.tie |= TIE_L0 >> lvl;
+        return skip(lvl, mx, my, rmx, rmy, j, i);
+    };
+    auto take = [&](int j, int i, int) {
+        rmx = j;
+        rmy = i;
+    };
 
     if (a.mode == 2) {  // level 2 full search around (0, 0) (…Multires.cpp:667-731)
-        // 8 candidates of a row at a time, 4 lanes each (one block row per lane)
-        const Org oin2 = origin(a.in2, 4, 4, 0, ll, kk);
-        const int sub = lane >> 2, br = lane & 3;
-        int cur2[4];
-#pragma unroll
-        for (int c = 0; c < 4; c++) cur2[c] = rdb(a.in2, oin2.y + br, oin2.x + c);
-        int min2 = full_ssd(a.in2, oin2, a.e2, origin(a.e2, 4, 4, 5, ll, kk), 4, lane, bad);
+        unsigned cur2[4];
+        load_level2(a, ll, kk, cur2);
         mr_range(L2, ll, kk, 0, 0, l2_range - 1, xl, xr, yu, yd);
-        for (int i = yu; i <= yd; i++)
-            for (int j0 = xl; j0 <= xr; j0 += 8) {
-                int d = 0;
-                if (j0 + sub <= xr) {
-                    const Org o = origin(a.e2, 4, 4, 5, ll + j0 + sub, kk + i);
-#pragma unroll
-                    for (int c = 0; c < 4; c++) {
-                        const int e = cur2[c] - rdb(a.e2, o.y + br, o.x + c);
-                        d += e * e;
-                    }
-                }
-                d += __shfl_xor_sync(0xffffffffu, d, 1);
-                d += __shfl_xor_sync(0xffffffffu, d, 2);
-                const int nj = xr - j0 + 1 < 8 ? xr - j0 + 1 : 8;
-                for (int t = 0; t < nj; t++) {
-                    const int j = j0 + t, dt = __shfl_sync(0xffffffffu, d, 4 * t);
-                    if (!(i || j) || dt > min2) continue;
-                    if (dt == min2) {
-                        out.tie |= TIE_L2;
-                        if (skip(2, 0, 0, mx, my, j, i)) continue;
-                    }
-                    min2 = dt;
-                    mx = j;
-                    my = i;
-                }
-            }
-        mx <<= 1;
-        my <<= 1;
+        raster(xl, xr, yu, yd, min, lane,
+               [&](int j, int i, int& d, int& t) { t = d = score4(cur2, a.e2, origin(a.e2, 4, 4, 5, ll + j, kk + i)); },
+               tie, take);
+        mx = rmx << 1;
+        my = rmy << 1;
     }
 
-    // level 1 around (mx, my) (…Multires.cpp:735-790): this lane's 2 samples of the 8x8 block
-    const Org oin1 = origin(a.in1, 8, 8, 0, q, p);
-    int r1, c1;
-    phase_coords<8>(lane, r1, c1);
-    int cur1[2];
-#pragma unroll
-    for (int j = 0; j < 2; j++) cur1[j] = rdb(a.in1, oin1.y + r1, oin1.x + c1 + 4 * j);
-    int min1 = full_ssd(a.in1, oin1, a.e1, origin(a.e1, 8, 8, 9, mx + q, my + p), 8, lane, bad);
-    int rmx = 0, rmy = 0;
+    // level 1 around (mx, my) (…Multires.cpp:735-790)
+    lvl = 1;
+    rmx = rmy = 0;
     mr_range(L1, q, p, mx, my, lcl_l1_range, xl, xr, yu, yd);
-    for (int i = yu; i <= yd; i++)
-        for (int j = xl; j <= xr; j++) {
-            if (!(i || j)) continue;
-            const Org o = origin(a.e1, 8, 8, 9, j + mx + q, i + my + p);
-            int acc = 0;
-#pragma unroll
-            for (int t = 0; t < 2; t++) {
-                const int e = cur1[t] - rdb(a.e1, o.y + r1, o.x + c1 + 4 * t);
-                acc += e * e;
-            }
-            const int d = warp_sum(acc);
-            if (d > min1) continue;
-            if (d == min1) {
-                out.tie |= TIE_L1;
-                if (skip(1, mx, my, rmx, rmy, j, i)) continue;
-            }
-            min1 = d;
-            rmx = j;
-            rmy = i;
-        }
+    raster(xl, xr, yu, yd, min, lane,
+           [&](int j, int i, int& d, int& t) {
+               score8<false>(LT, a.e1, origin(a.e1, 8, 8, 9, j + mx + q, i + my + p), d, t);
+           },
+           tie, take);
     mx = (mx + rmx) * 2;
     my = (my + rmy) * 2;
 
-    // level 0 +-2 (…Multires.cpp:792-849): this lane's 8 samples of the 16x16 block
-    int r0, c0;
-    phase_coords<16>(lane, r0, c0);
-    int cur0[8];
-#pragma unroll
-    for (int i = 0; i < 2; i++)
-#pragma unroll
-        for (int j = 0; j < 4; j++) cur0[4 * i + j] = rdb(a.in0, oin0.y + r0 + 4 * i, oin0.x + c0 + 4 * j);
-    auto ssd16 = [&](Org o) {
-        int acc = 0;
-#pragma unroll
-        for (int i = 0; i < 2; i++)
-#pragma unroll
-            for (int j = 0; j < 4; j++) {
-                const int e = cur0[4 * i + j] - rdb(a.e0, o.y + r0 + 4 * i, o.x + c0 + 4 * j);
-                acc += e * e;
-            }
-        return warp_sum(acc);
-    };
-    int min_d = ssd16(origin(a.e0, 16, 16, 19, n + mx, m + my));
+    // level 0 +-2 (…Multires.cpp:792-849)
+    lvl = 0;
     rmx = rmy = 0;
+    const Org oc = origin(a.e0, 16, 16, 19, n + mx, m + my);
+    stage_level0(a.e0, LT, oc, lane);
     mr_range(L0, n, m, mx, my, 2, xl, xr, yu, yd);
-    for (int i = yu; i <= yd; i++)
-        for (int j = xl; j <= xr; j++) {
-            if (!(i || j)) continue;
-            const int d = ssd16(origin(a.e0, 16, 16, 19, n + mx + j, m + my + i));
-            if (d > min_d) continue;
-            if (d == min_d) {
-                out.tie |= TIE_L0;
-                if (skip(0, mx, my, rmx, rmy, j, i)) continue;
-            }
-            min_d = d;
-            rmx = j;
-            rmy = i;
-        }
+    raster(xl, xr, yu, yd, min, lane,
+           [&](int j, int i, int& d, int& t) {
+               const Org c = origin(a.e0, 16, 16, 19, n + mx + j, m + my + i);
+               score16<false>(LT, c.y - oc.y + 5, c.x - oc.x + 5, d, t);
+           },
+           tie, take);
     mx += rmx;
     my += rmy;
-    int mvx = mx * 4, mvy = my * 4;
 
     // half then quarter pel (…Multires.cpp:851-917), strict improvements, full distortions
-    build_lattice<false>(LT, a.e0, origin(a.e0, 16, 16, 19, n + mx, m + my), lane, bad);
-    int hmx = 0, hmy = 0;
-    for (int c = 0; c < 8; c++) {
-        const int qx = 2 * SX[c], qy = 2 * SY[c];
-        int acc = 0;
-#pragma unroll
-        for (int i = 0; i < 2; i++)
-#pragma unroll
-            for (int j = 0; j < 4; j++) {
-                const int d = cur0[4 * i + j] - lat(LT, 12 + qy + 4 * (r0 + 4 * i), 12 + qx + 4 * (c0 + 4 * j));
-                acc += d * d;
-            }
-        const int d = warp_sum(acc);
-        if (d < min_d) {
-            min_d = d;
-            hmx = qx;
-            hmy = qy;
-        }
-    }
-    int qmx = hmx, qmy = hmy;
-    for (int c = 0; c < 8; c++) {
-        int acc = 0;
-#pragma unroll
-        for (int i = 0; i < 2; i++)
-#pragma unroll
-            for (int j = 0; j < 4; j++) {
-                const int d = cur0[4 * i + j] -
-                              quarter(LT, 12 + hmy + 4 * (r0 + 4 * i), 12 + hmx + 4 * (c0 + 4 * j), SY[c], SX[c]);
-                acc += d * d;
-            }
-        const int d = warp_sum(acc);
-        if (d < min_d) {
-            min_d = d;
-            qmx = hmx + SX[c];
-            qmy = hmy + SY[c];
-        }
-    }
-    __syncwarp();
-    out.min_d = min_d;
-    out.mvx = mvx + qmx;
-    out.mvy = mvy + qmy;
+    int qmx = 0, qmy = 0;
+    subpel<false, false>(LT, a.e0, oc, origin(a.e0, 16, 16, 19, n + mx, m + my), min, qmx, qmy, lane, bad,
+                         [](int, int, int) {});
+    out.min_d = min;
+    out.mvx = mx * 4 + qmx;
+    out.mvy = my * 4 + qmy;
     return out;
 }
 
@@ -751,36 +874,36 @@ __device__ MbSearch search_lambda(const MrcArgs& a, Lattice& LT, int mbr, int mb
     const int l1_range = a.motion_range / 8, l2_range = l1_range / 2;
     const int lcl_l1_range = a.mode == 2 ? 2 : l1_range;
     const Level L0{16, a.W, a.H, a.motion_range / 4}, L1{8, w1, h1, l1_range}, L2{4, w2, h2, l2_range};
-    constexpr int CRX[4] = {-1, 1, 0, 0}, CRY[4] = {0, 0, -1, 1};
-    constexpr int SX[8] = {-1, 0, 1, -1, 1, -1, 0, 1}, SY[8] = {-1, -1, -1, 0, 0, 1, 1, 1};
     const double lam = a.lambda;
     MbSearch out;
     out.tie = TIE_ALL;
     Fifo5 f;
 
-    const Org oin0 = origin(a.in0, 16, 16, 0, n, m);
-    out.zero_d = full_ssd(a.in0, oin0, a.e0, origin(a.e0, 16, 16, 19, n, m), 16, lane, bad);
-    int mx = 0, my = 0, rmx = 0, rmy = 0, xl, xr, yu, yd;
+    __syncwarp();
+    out.zero_d = zero_distortion(a, LT, origin(a.in0, 16, 16, 0, n, m), n, m, lane);
+    stage_level1(a, LT, q, p, lane);
+    int mx = 0, my = 0, rmx = 0, rmy = 0, xl, xr, yu, yd, min, lvl = 2;
+    auto tie = [&](int j, int i) { return farther(mx, my, rmx, rmy, j, i, pl[2 * lvl], pl[2 * lvl + 1]); };
+    auto take = [&](int j, int i, int d) {
+        rmx = j;
+        rmy = i;
+        f.push(j + mx, i + my, d, lane);
+    };
 
     if (a.mode == 2) {  // level 2 cross search (…:1287-1370)
-        const Org oin2 = origin(a.in2, 4, 4, 0, ll, kk);
-        int min2 = full_ssd(a.in2, oin2, a.e2, origin(a.e2, 4, 4, 5, ll, kk), 4, lane, bad);
-        f.reset(0, 0, min2);
+        // Tsd4x4LessThan stops early only on a sum already above min: a full SSD decides the same
+        unsigned cur2[4];
+        load_level2(a, ll, kk, cur2);
+        min = score4(cur2, a.e2, origin(a.e2, 4, 4, 5, ll, kk));
+        f.reset(0, 0, min);
         mr_range(L2, ll, kk, 0, 0, l2_range - 1, xl, xr, yu, yd);
         for (int s = l2_range / 2; s > 0; s /= 2) {
             rmx = rmy = 0;
-            for (int c = 0; c < 4; c++) {
-                const int i = s * CRY[c], j = s * CRX[c];
-                if (i + my < yu || i + my > yd || j + mx < xl || j + mx > xr) continue;
-                // Tsd4x4LessThan stops early only on a sum already above min: a full SSD decides the same
-                const int d = full_ssd(a.in2, oin2, a.e2, origin(a.e2, 4, 4, 5, j + ll + mx, i + kk + my), 4, lane, bad);
-                if (d > min2) continue;
-                if (d == min2 && farther(mx, my, rmx, rmy, j, i, pl[4], pl[5])) continue;
-                min2 = d;
-                rmx = j;
-                rmy = i;
-                f.push(j + mx, i + my, d, lane);
-            }
+            int j, i;
+            cross_offset(lane, s, j, i);
+            const int d = score4(cur2, a.e2, origin(a.e2, 4, 4, 5, j + ll + mx, i + kk + my));
+            settle(lane < 4 && i + my >= yu && i + my <= yd && j + mx >= xl && j + mx <= xr, d, d, pack_mv(j, i), min, tie,
+                   take);
             mx += rmx;
             my += rmy;
         }
@@ -789,50 +912,29 @@ __device__ MbSearch search_lambda(const MrcArgs& a, Lattice& LT, int mbr, int mb
         my <<= 1;
     }
 
-    // level 1 (…:1374-1502): input samples of this lane's phase share, kept
-    const Org oin1 = origin(a.in1, 8, 8, 0, q, p);
-    int r1, c1;
-    phase_coords<8>(lane, r1, c1);
-    int cur1[2];
-#pragma unroll
-    for (int j = 0; j < 2; j++) cur1[j] = rdb(a.in1, oin1.y + r1, oin1.x + c1 + 4 * j);
-    auto part8 = [&](Org o) {
-        int acc = 0;
-#pragma unroll
-        for (int j = 0; j < 2; j++) {
-            const int d = cur1[j] - rdb(a.e1, o.y + r1, o.x + c1 + 4 * j);
-            acc += d * d;
-        }
-        return acc;
-    };
-    int min1 = full_ssd(a.in1, oin1, a.e1, origin(a.e1, 8, 8, 9, mx + q, my + p), 8, lane, bad);
-    f.reset(mx, my, min1);
+    // level 1 (…:1374-1502)
+    lvl = 1;
     rmx = rmy = 0;
-    auto consider1 = [&](int i, int j) {
-        const int d = partial_value(part8(origin(a.e1, 8, 8, 9, j + mx + q, i + my + p)), min1, lane);
-        if (d > min1) return;
-        if (d == min1 && farther(mx, my, rmx, rmy, j, i, pl[2], pl[3])) return;
-        min1 = d;
-        rmx = j;
-        rmy = i;
-        f.push(j + mx, i + my, d, lane);
+    auto score1 = [&](int j, int i, int& d, int& t) {
+        score8<true>(LT, a.e1, origin(a.e1, 8, 8, 9, j + mx + q, i + my + p), d, t);
     };
+    int t;
+    score1(0, 0, min, t);
+    f.reset(mx, my, min);
     if (a.mode == 2) {
         mr_range(L1, q, p, mx, my, lcl_l1_range, xl, xr, yu, yd);
-        for (int i = yu; i <= yd; i++)
-            for (int j = xl; j <= xr; j++)
-                if (i || j) consider1(i, j);
+        raster(xl, xr, yu, yd, min, lane, score1, tie, take);
         mx += rmx;
         my += rmy;
     } else {
         for (int s = l1_range / 2; s > 0; s /= 2) {
             mr_range(L1, q, p, mx, my, lcl_l1_range - 1, xl, xr, yu, yd);
             rmx = rmy = 0;
-            for (int c = 0; c < 4; c++) {
-                const int i = s * CRY[c], j = s * CRX[c];
-                if (i + my < yu || i + my > yd || j + mx < xl || j + mx > xr) continue;
-                consider1(i, j);
-            }
+            int j, i, d;
+            cross_offset(lane, s, j, i);
+            score1(j, i, d, t);
+            settle(lane < 4 && i + my >= yu && i + my <= yd && j + mx >= xl && j + mx <= xr, d, t, pack_mv(j, i), min, tie,
+                   take);
             mx += rmx;
             my += rmy;
         }
@@ -842,87 +944,28 @@ __device__ MbSearch search_lambda(const MrcArgs& a, Lattice& LT, int mbr, int mb
     my <<= 1;
 
     // level 0 +-2 refinement (…:1503-1574)
-    int r0, c0;
-    phase_coords<16>(lane, r0, c0);
-    int cur0[8];
-#pragma unroll
-    for (int i = 0; i < 2; i++)
-#pragma unroll
-        for (int j = 0; j < 4; j++) cur0[4 * i + j] = rdb(a.in0, oin0.y + r0 + 4 * i, oin0.x + c0 + 4 * j);
-    auto part16 = [&](Org o) {
-        int acc = 0;
-#pragma unroll
-        for (int i = 0; i < 2; i++)
-#pragma unroll
-            for (int j = 0; j < 4; j++) {
-                const int d = cur0[4 * i + j] - rdb(a.e0, o.y + r0 + 4 * i, o.x + c0 + 4 * j);
-                acc += d * d;
-            }
-        return acc;
-    };
-    int min_d = out.zero_d;
-    if (mx || my) min_d = full_ssd(a.in0, oin0, a.e0, origin(a.e0, 16, 16, 19, n + mx, m + my), 16, lane, bad);
-    f.reset(mx, my, min_d);
+    lvl = 0;
     rmx = rmy = 0;
+    const Org oc = origin(a.e0, 16, 16, 19, n + mx, m + my);
+    stage_level0(a.e0, LT, oc, lane);
+    auto score0 = [&](int j, int i, int& d, int& t0) {
+        const Org c = origin(a.e0, 16, 16, 19, n + mx + j, m + my + i);
+        score16<true>(LT, c.y - oc.y + 5, c.x - oc.x + 5, d, t0);
+    };
+    score0(0, 0, min, t);
+    f.reset(mx, my, min);
     mr_range(L0, n, m, mx, my, 2, xl, xr, yu, yd);
-    for (int i = yu; i <= yd; i++)
-        for (int j = xl; j <= xr; j++) {
-            if (!(i || j)) continue;
-            const int d = partial_value(part16(origin(a.e0, 16, 16, 19, n + mx + j, m + my + i)), min_d, lane);
-            if (d > min_d) continue;
-            if (d == min_d && farther(mx, my, rmx, rmy, j, i, pl[0], pl[1])) continue;
-            min_d = d;
-            rmx = j;
-            rmy = i;
-            f.push(j + mx, i + my, d, lane);
-        }
+    raster(xl, xr, yu, yd, min, lane, score0, tie, take);
     mx += rmx;
     my += rmy;
-    min_d = fifo_best(f, lam, 256.0, 0, pl[0], pl[1], mx, my, lane);
+    min = fifo_best(f, lam, 256.0, 0, pl[0], pl[1], mx, my, lane);
 
     // half then quarter pel in Ver2's window (…:1575-1662), strict improvements
-    int mvx = mx * 4, mvy = my * 4;
-    f.reset(mvx, mvy, min_d);
-    build_lattice<true>(LT, a.e0, origin(a.e0, 16, 16, 19, n + mx, m + my), lane, bad);
-    int hmx = 0, hmy = 0;
-    for (int c = 0; c < 8; c++) {
-        const int qx = 2 * SX[c], qy = 2 * SY[c];
-        int acc = 0;
-#pragma unroll
-        for (int i = 0; i < 2; i++)
-#pragma unroll
-            for (int j = 0; j < 4; j++) {
-                const int d = cur0[4 * i + j] - lat(LT, 12 + qy + 4 * (r0 + 4 * i), 12 + qx + 4 * (c0 + 4 * j));
-                acc += d * d;
-            }
-        const int d = partial_value(acc, min_d, lane);
-        if (d < min_d) {
-            min_d = d;
-            hmx = qx;
-            hmy = qy;
-            f.push(qx + mvx, qy + mvy, d, lane);
-        }
-    }
-    int qmx = hmx, qmy = hmy;
-    for (int c = 0; c < 8; c++) {
-        int acc = 0;
-#pragma unroll
-        for (int i = 0; i < 2; i++)
-#pragma unroll
-            for (int j = 0; j < 4; j++) {
-                const int d = cur0[4 * i + j] -
-                              quarter(LT, 12 + hmy + 4 * (r0 + 4 * i), 12 + hmx + 4 * (c0 + 4 * j), SY[c], SX[c]);
-                acc += d * d;
-            }
-        const int d = partial_value(acc, min_d, lane);
-        if (d < min_d) {
-            min_d = d;
-            qmx = hmx + SX[c];
-            qmy = hmy + SY[c];
-            f.push(qmx + mvx, qmy + mvy, d, lane);
-        }
-    }
-    __syncwarp();  // the lattice is reused by this warp's next search
+    int mvx = mx * 4, mvy = my * 4, qmx = 0, qmy = 0;
+    f.reset(mvx, mvy, min);
+    const Org o = origin(a.e0, 16, 16, 19, n + mx, m + my);
+    subpel<true, true>(LT, a.e0, oc, o, min, qmx, qmy, lane, bad,
+                       [&](int x, int y, int d) { f.push(x + mvx, y + mvy, d, lane); });
     mvx += qmx;
     mvy += qmy;
     // towards the clamped quarter-pel prediction (…:1664-1677)
@@ -934,8 +977,8 @@ __device__ MbSearch search_lambda(const MrcArgs& a, Lattice& LT, int mbr, int mb
 
 // MultiresCross's tie rules: at level 2 the centre against the offset
 // (…MultiresCross.cpp:673-679), elsewhere distances from (0, 0) (…:741-746, 857).
-template <bool kH263 = false>
-__device__ __forceinline__ MbSearch search_mb_mrc(const MrcArgs& a, Lattice& LT, int mbr, int mbc, int lane,
+template <bool kH263 = false, typename Store>
+__device__ __forceinline__ MbSearch search_mb_mrc(const MrcArgs& a, Store& LT, int mbr, int mbc, int lane,
                                                   bool& bad)
 {
     auto skip = [](int lvl, int mx, int my, int rmx, int rmy, int j, int i) {
