@@ -406,27 +406,28 @@ __global__ void __launch_bounds__(SEARCH_THREADS, SEARCH_CTAS_PER_SM)
     }
 }
 
-// The window of macroblock (n, m)'s candidates in shared memory: WROWS rows
-// from m - 31, columns n - 32 .. n + 47.  At this pitch (22 words) 16 rows at
-// one column, and the word beside it, lie in 32 different banks.
-constexpr int SCAN_PITCH = 88;
-constexpr int SCAN_WIN = WROWS * SCAN_PITCH;
+// The window of the candidates of kMbs macroblocks of a row, the first at
+// (n, m), in shared memory: WROWS rows from m - 31, columns n - 32 ..
+// n + 16 kMbs + 31.  At these pitches (22 and 34 words) 16 rows at one column,
+// and the word beside it, lie in 32 different banks.
+__host__ __device__ constexpr int scan_pitch(int mbs) { return 64 + 16 * mbs + 8; }
 
-__device__ __forceinline__ void stage_window(const FullArgs& a, int n, int m, unsigned char* win, int tid, int nthreads)
+// mbs: the macroblocks that are there; nthreads: a multiple of 16.
+template <int kMbs>
+__device__ __forceinline__ void stage_window(const FullArgs& a, int n, int m, int mbs, unsigned char* win, int tid,
+                                             int nthreads)
 {
     const unsigned char* src = a.refp + (size_t)(m - RMAX + PAD) * a.rstride + n - RMAX - 1 + PAD;
-    // five 16-byte pieces a row, six rows a warp and step (lanes 30 and 31 idle)
-    const int lane = tid & 31, step = 6 * (nthreads >> 5), q = lane % 5, r0 = 6 * (tid >> 5) + lane / 5;
-    if (lane >= 30) return;
-    const unsigned char* p = src + (size_t)r0 * a.rstride + 16 * q;
-    unsigned char* d = win + r0 * SCAN_PITCH + 16 * q;
-#pragma unroll 13
-    for (int r = r0; r < WROWS; r += step) {
-        const uint4 v = __ldg(reinterpret_cast<const uint4*>(p));
-        reinterpret_cast<uint2*>(d)[0] = make_uint2(v.x, v.y);
-        reinterpret_cast<uint2*>(d)[1] = make_uint2(v.z, v.w);
-        p += (size_t)step * a.rstride;
-        d += step * SCAN_PITCH;
+    constexpr int kPieces = kMbs + 4, kAcross = 8, kPitch = scan_pitch(kMbs);  // 16-byte pieces of a row
+    static_assert(kPieces <= kAcross, "a row's pieces and the idle threads beside them");
+    const int q = tid & (kAcross - 1), step = nthreads / kAcross;
+    if (q >= mbs + 4) return;
+#pragma unroll 5
+    for (int r = tid / kAcross; r < WROWS; r += step) {
+        const uint4 v = __ldg(reinterpret_cast<const uint4*>(src + (size_t)r * a.rstride + 16 * q));
+        uint2* d = reinterpret_cast<uint2*>(win + r * kPitch + 16 * q);
+        d[0] = make_uint2(v.x, v.y);
+        d[1] = make_uint2(v.z, v.w);
     }
 }
 
@@ -439,9 +440,10 @@ __device__ __forceinline__ uint4 template_row(const FullArgs& a, int n, int m, i
 // The SSDs of the 8 candidates in table columns 8g .. 8g+7 of candidate row ii
 // (i + RMAX): lane c < 8 gets column 8g + c.  One warp, a lane four candidates
 // on one template row, which read five words of one window row.
+template <int kPitch>
 __device__ __forceinline__ int group_ssd(const unsigned char* win, uint4 t, int ii, int g, int lane)
 {
-    const unsigned* q = reinterpret_cast<const unsigned*>(win + (ii + (lane >> 1)) * SCAN_PITCH + 8 * g + 4 * (lane & 1));
+    const unsigned* q = reinterpret_cast<const unsigned*>(win + (ii + (lane >> 1)) * kPitch + 8 * g + 4 * (lane & 1));
     const unsigned w[5] = {q[0], q[1], q[2], q[3], q[4]}, tw[4] = {t.x, t.y, t.z, t.w};
     unsigned acc[4] = {0u, 0u, 0u, 0u};
 #pragma unroll
@@ -472,50 +474,49 @@ __device__ __forceinline__ int group_ssd(const unsigned char* win, uint4 t, int 
 // lane holds the minima of two candidate rows; the first row that has such a
 // minimum is visited next, and only such groups' SSDs are formed: on a 1080p
 // pan 6 rows and 7.5 groups a macroblock.
+//
+// What bounds it is latency with too few warps to hide it.  The macroblocks of a CTA are neighbours and share
+// one window (22 KB a CTA, 36 warps an SM; a window and the minima kept for each warp, 24), and the refinement
+// reads its planes from shared memory: 1920x1080, 48 -> 38 us (the refinement 6 of it, the window 4).
 constexpr int SCAN_WARPS = 4;
-__global__ void __launch_bounds__(32 * SCAN_WARPS) k_full_scan(const __grid_constant__ FullArgs a)
+__global__ void __launch_bounds__(32 * SCAN_WARPS, 8) k_full_scan(const __grid_constant__ FullArgs a)
 {
-    __shared__ __align__(16) unsigned char s_win[SCAN_WARPS][SCAN_WIN];
-    __shared__ __align__(16) int s_min[SCAN_WARPS][64][8];  // the groups' minima, rows yu ..
-    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, k = blockIdx.x * SCAN_WARPS + w;
-    if (k >= a.nmb) return;
-    const int n = (k % a.cols) * 16, m = (k / a.cols) * 16;
-    const unsigned char* win = s_win[w];
-    const uint2 cur = load_cur8(a, n, m, lane);
-    const uint2 at0 = *reinterpret_cast<const uint2*>(even_block(a, n, m, 0, 0, lane));
-    const uint4 t = template_row(a, n, m, lane);
+    constexpr int kPitch = scan_pitch(SCAN_WARPS);
+    __shared__ __align__(16) unsigned char s_win[WROWS * kPitch];
+    __shared__ __align__(16) SubWindow s_sub[SCAN_WARPS];
+    const int across = (a.cols + SCAN_WARPS - 1) / SCAN_WARPS, br = blockIdx.x / across;
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, bc = SCAN_WARPS * (blockIdx.x - br * across);
+    const int mbs = min(SCAN_WARPS, a.cols - bc), k = br * a.cols + bc + w;
+    const int n = 16 * (bc + w), m = 16 * br;
+    stage_window<SCAN_WARPS>(a, 16 * bc, m, mbs, s_win, threadIdx.x, 32 * SCAN_WARPS);
+    const bool there = w < mbs;
+    const uint4 t = template_row(a, there ? n : 16 * bc, m, lane);
+    const uint2 cur = (lane & 1) ? make_uint2(t.z, t.w) : make_uint2(t.x, t.y);
     constexpr int kNone = 0x7fffffff;
     int xl, xr, yu, yd;
     full_range(n, m, a.W, a.H, a.motion_range, xl, xr, yu, yd);
-    float4 p[2][2];
-#pragma unroll
-    for (int h = 0; h < 2; h++) {
-        const float4* q = reinterpret_cast<const float4*>(a.rowmin + ((size_t)k * 64 + min(yu + lane + 32 * h, yd) + RMAX) * 8);
-        p[h][0] = __ldcg(q);
-        p[h][1] = __ldcg(q + 1);
-    }
-    stage_window(a, n, m, s_win[w], lane, 32);
     // A^2 of the samples less 128, which the minima are without
     const int c0 = (int)(cur.x ^ 0x80808080u), c1 = (int)(cur.y ^ 0x80808080u);
     const int energy = warp_sum(__dp4a(c0, c0, __dp4a(c1, c1, 0)));
     const int ga = (xl + 32) >> 3, gb = (xr + 32) >> 3;  // groups that hold candidates
-    int rm[2];
+    const float* minima = a.rowmin + ((size_t)k * 64 + yu + RMAX) * 8;  // candidate row yu's
+    int rm[2] = {kNone, kNone};
+    if (there) {
 #pragma unroll
-    for (int h = 0; h < 2; h++) {
-        const float f[8] = {p[h][0].x, p[h][0].y, p[h][0].z, p[h][0].w, p[h][1].x, p[h][1].y, p[h][1].z, p[h][1].w};
-        int v[8];
-        rm[h] = kNone;
+        for (int h = 0; h < 2; h++) {
+            const float4* q = reinterpret_cast<const float4*>(minima + 8 * min(lane + 32 * h, yd - yu));
+            const float4 p0 = __ldg(q), p1 = __ldg(q + 1);
+            const float f[8] = {p0.x, p0.y, p0.z, p0.w, p1.x, p1.y, p1.z, p1.w};
 #pragma unroll
-        for (int g = 0; g < 8; g++) {
-            v[g] = g >= ga && g <= gb ? energy + (int)f[g] : kNone;
-            rm[h] = min(rm[h], v[g]);
+            for (int g = 0; g < 8; g++)
+                if (g >= ga && g <= gb) rm[h] = min(rm[h], energy + (int)f[g]);
         }
-        int4* d = reinterpret_cast<int4*>(s_min[w][lane + 32 * h]);
-        d[0] = make_int4(v[0], v[1], v[2], v[3]);
-        d[1] = make_int4(v[4], v[5], v[6], v[7]);
     }
-    __syncwarp();
-    const int zero_d = warp_sum(ssd8(cur, at0));
+    __syncthreads();
+    if (!there) return;
+    const unsigned char* win = s_win + 16 * w;
+    const unsigned* at0 = reinterpret_cast<const unsigned*>(win + (RMAX + (lane >> 1)) * kPitch + RMAX + 1 + 8 * (lane & 1));
+    const int zero_d = warp_sum(ssd8(cur, make_uint2(at0[0], at0[1])));
 
     int minD = zero_d, mx = 0, my = 0, tie = 0;
     int done = 0;  // rows yu .. yu+done-1 are behind the scan
@@ -528,7 +529,8 @@ __global__ void __launch_bounds__(32 * SCAN_WARPS) k_full_scan(const __grid_cons
         if (!m0 && !m1) break;
         const int off = m0 ? __ffs(m0) - 1 : 31 + __ffs(m1), i = yu + off;
         done = off + 1;
-        const int gmin = s_min[w][off][lane & 7], jl = 8 * (lane & 7) - 32;  // lane g: the row's group g
+        const int gl = lane & 7, jl = 8 * gl - 32;  // lane g: the row's group g
+        const int gmin = gl >= ga && gl <= gb ? energy + (int)__ldg(minima + 8 * off + gl) : kNone;
         unsigned left = 0xffu;  // groups not yet behind the scan
         while (i + my >= yu && i + my <= yd) {
             // the next group of the row that can accept, at the best as it is
@@ -536,7 +538,7 @@ __global__ void __launch_bounds__(32 * SCAN_WARPS) k_full_scan(const __grid_cons
             if (!can) break;
             const int g = __ffs(can) - 1;
             left &= ~((2u << g) - 1u);
-            const int d = group_ssd(win, t, i + RMAX, g, lane);
+            const int d = group_ssd<kPitch>(win, t, i + RMAX, g, lane);
             const int base = 8 * g - 32, j = base + lane;
             const bool valid = lane < 8 && j >= xl && j <= xr && !(i == 0 && j == 0);
             unsigned pending = 0xffu;
@@ -560,7 +562,7 @@ __global__ void __launch_bounds__(32 * SCAN_WARPS) k_full_scan(const __grid_cons
         }
     }
     int qmx, qmy;
-    subpel_refine_planes(a, n + mx, m + my, cur, lane, &minD, &qmx, &qmy);
+    subpel_refine_staged(a, s_sub[w], n, m, n + mx, m + my, lane, &minD, &qmx, &qmy);
     if (lane == 0) {
         const int qmv = pack_mv(4 * mx + qmx, 4 * my + qmy);
         const int av = neighbour_mask(a.job->slice, k, a.cols, a.nmb / a.cols);
@@ -582,7 +584,7 @@ struct TieSmem {
     alignas(16) int tab[TAB][TAB];
     int run[TIE_RUNS][sizeof(TieRun) / sizeof(int)];
     int deep;
-    alignas(16) unsigned char win[SCAN_WIN];
+    alignas(16) unsigned char win[WROWS * scan_pitch(1)];
 };
 
 template <bool kSad>
@@ -604,11 +606,11 @@ __global__ void __launch_bounds__(TIE_RUNS * 32) k_full_tietree(const __grid_con
                 reinterpret_cast<int4*>(&S.tab[0][0])[i] = __ldcg(reinterpret_cast<const int4*>(gt) + i);
         } else {
             const uint4 tm = template_row(a, n, m, lane);
-            stage_window(a, n, m, S.win, tid, blockDim.x);
+            stage_window<1>(a, n, m, 1, S.win, tid, blockDim.x);
             __syncthreads();
             for (int ii = p; ii < 2 * RMAX + 1; ii += TIE_RUNS)
                 for (int g = 0; g < TAB / 8; g++) {
-                    const int v = group_ssd(S.win, tm, ii, g, lane);
+                    const int v = group_ssd<scan_pitch(1)>(S.win, tm, ii, g, lane);
                     if (lane < 8) S.tab[ii][8 * g + lane] = v;
                 }
             __syncthreads();
@@ -738,7 +740,7 @@ int full_launch(vppgpu_ctx* ctx, const FullArgs& args, int nmb, cudaEvent_t* ev)
     if (ev) VPP_CUDA(cudaEventRecord(ev[1], ctx->stream));
     if ((rc = rowmin_launch(ctx, args))) return rc;
     if (ev) VPP_CUDA(cudaEventRecord(ev[2], ctx->stream));
-    k_full_scan<<<(nmb + SCAN_WARPS - 1) / SCAN_WARPS, 32 * SCAN_WARPS, 0, ctx->stream>>>(args);
+    k_full_scan<<<(args.cols + SCAN_WARPS - 1) / SCAN_WARPS * (nmb / args.cols), 32 * SCAN_WARPS, 0, ctx->stream>>>(args);
     VPP_CHECK_LAUNCH(ctx);
     k_full_tietree<false><<<ctx->sm_count, TIE_RUNS * 32, sizeof(TieSmem), ctx->stream>>>(args);
     VPP_CHECK_LAUNCH(ctx);

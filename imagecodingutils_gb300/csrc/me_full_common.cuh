@@ -290,6 +290,102 @@ __device__ __forceinline__ void subpel_refine_planes(const FullArgs& a, int x0, 
     *qmy = by;
 }
 
+// The same refinement (with the quarter pass) from shared memory, a warp's SubWindow.  Read from the planes
+// by a lane per half row, each of the 72 loads of the 24 blocks touches 16 lines of L1.  Here the four planes'
+// 18 rows around the winner are nine loads once, and then a candidate takes four lanes of four rows each, all
+// eight of a pass at once with one reduction: 6 us less of a 1920x1080 frame's scan.
+constexpr int SUBW_PITCH = 10;  // words: 8 hold 18 columns from any of 8 alignments, 8-byte rows
+struct SubWindow {
+    unsigned p[4 * 18 * SUBW_PITCH];  // full pel, b, h, j: rows y0 - 1 .. y0 + 16
+};
+__device__ __forceinline__ void subwindow_row(const unsigned* row, int col, unsigned (&w)[4])
+{
+    const unsigned* q = row + (col >> 2);
+    const unsigned sh = (unsigned)(col & 3) * 8;
+    unsigned lo = q[0];
+#pragma unroll
+    for (int i = 0; i < 4; i++) {
+        const unsigned hi = q[i + 1];
+        w[i] = __funnelshift_r(lo, hi, sh);
+        lo = hi;
+    }
+}
+
+__device__ __forceinline__ void subpel_refine_staged(const FullArgs& a, SubWindow& S, int n, int m, int x0, int y0,
+                                                     int lane, int* min_d, int* qmx, int* qmy)
+{
+    const int left = x0 - 1 + PAD, col0 = left & 7, rho = lane & 3;
+    uint4 cur[4];
+#pragma unroll
+    for (int i = 0; i < 4; i++)
+        cur[i] = __ldg(reinterpret_cast<const uint4*>(a.src8 + (size_t)(m + rho + 4 * i) * a.W + n));
+    const size_t at = (size_t)(y0 - 1 + PAD) * a.rstride + (left & ~7) + 8 * rho;
+    __syncwarp();
+#pragma unroll
+    for (int i = 0; i < 9; i++) {  // eight rows of 32 bytes at a time
+        const int r = 8 * i + (lane >> 2), pl = r / 18, pr = r - 18 * pl;
+        const unsigned char* base = pl ? a.hpel + (size_t)(pl - 1) * a.plane_size : a.refp;
+        *reinterpret_cast<uint2*>(S.p + r * SUBW_PITCH + 2 * rho) =
+            __ldg(reinterpret_cast<const uint2*>(base + at + (size_t)pr * a.rstride));
+    }
+    __syncwarp();
+    // candidate lane / 4: the eight neighbours in raster order
+    const int c9 = (lane >> 2) + (lane >= 16), sy = c9 / 3 - 1, sx = c9 - 3 * (c9 / 3) - 1;
+    auto word = [&](int qy) { return ((qy >> 2) + 1 + rho) * SUBW_PITCH; };
+    auto plane = [](int qy, int qx) { return ((qy & 2) | ((qx >> 1) & 1)) * (18 * SUBW_PITCH); };
+    auto best_of = [&](unsigned d, int hx, int hy, int step) {  // the first of the smallest, if an improvement
+        d += __shfl_xor_sync(0xffffffffu, d, 1);
+        d += __shfl_xor_sync(0xffffffffu, d, 2);
+        const unsigned best = __reduce_min_sync(0xffffffffu, d);
+        if ((int)best >= *min_d) return;
+        const int f = __ffs(__ballot_sync(0xffffffffu, d == best)) - 1;
+        *min_d = (int)best;
+        *qmx = hx + step * __shfl_sync(0xffffffffu, sx, f);
+        *qmy = hy + step * __shfl_sync(0xffffffffu, sy, f);
+    };
+    *qmx = *qmy = 0;
+    {
+        const unsigned* q = S.p + plane(2 * sy, 2 * sx) + word(2 * sy);
+        const int col = col0 + 1 + ((2 * sx) >> 2);
+        unsigned d = 0;
+#pragma unroll
+        for (int i = 0; i < 4; i++) {
+            unsigned w[4];
+            subwindow_row(q + 4 * i * SUBW_PITCH, col, w);
+            const unsigned c[4] = {cur[i].x, cur[i].y, cur[i].z, cur[i].w};
+#pragma unroll
+            for (int k = 0; k < 4; k++) {
+                const unsigned e = __vabsdiffu4(c[k], w[k]);
+                d = __dp4a(e, e, d);
+            }
+        }
+        best_of(d, 0, 0, 2);
+    }
+    // the two samples LoadQuartPelWindow pairs, in half-pel steps from the half-pel winner
+    const int hx = *qmx, hy = *qmy;
+    const bool low_left = sy > 0 && sx < 0;
+    const int ay = hy + (sy < 0 ? -2 : (sy > 0 && sx >= 0 ? 2 : 0));
+    const int ax = hx + (sy == 0 ? 2 * sx : (sx < 0 ? -2 : 0));
+    const int by = hy + (low_left ? 2 : 0), bx = hx + (sy != 0 && sx > 0 ? 2 : 0);
+    const unsigned *qa = S.p + plane(ay, ax) + word(ay), *qb = S.p + plane(by, bx) + word(by);
+    const int ca = col0 + 1 + (ax >> 2), cb = col0 + 1 + (bx >> 2);
+    unsigned d = 0;
+#pragma unroll
+    for (int i = 0; i < 4; i++) {
+        unsigned wa[4], wb[4];
+        subwindow_row(qa + 4 * i * SUBW_PITCH, ca, wa);
+        subwindow_row(qb + 4 * i * SUBW_PITCH, cb, wb);
+        const unsigned c[4] = {cur[i].x, cur[i].y, cur[i].z, cur[i].w};
+#pragma unroll
+        for (int k = 0; k < 4; k++) {
+            const unsigned e = __vabsdiffu4(c[k], __vavgu4(wa[k], wb[k]));
+            d = __dp4a(e, e, d);
+        }
+    }
+    best_of(d, hx, hy, 1);
+    __syncwarp();
+}
+
 // This lane's 8 input samples of macroblock (n, m).
 __device__ __forceinline__ uint2 load_cur8(const FullArgs& a, int n, int m, int lane)
 {
