@@ -36,6 +36,48 @@ __device__ __forceinline__ int tap6(int a, int b, int c, int d, int e, int f)
     return a - 5 * b + 20 * c + 20 * d - 5 * e + f;
 }
 
+// The 6-tap filter on packed samples.  Two 16-bit sums + TAP_BIAS in the halves of a word (never negative,
+// below 2^14, so 32-bit adds and multiplies leave the halves apart), and their rounded, clipped samples.
+constexpr int TAP_BIAS = 2560;  // a multiple of 32 above the most negative sum's magnitude, 2550
+__device__ __forceinline__ unsigned tap_pair(unsigned a, unsigned b, unsigned c, unsigned d, unsigned e, unsigned f)
+{
+    return (a + f + TAP_BIAS * 0x10001u) + 20u * (c + d) - 5u * (b + e);
+}
+__device__ __forceinline__ unsigned scale_pair(unsigned t)
+{
+    constexpr unsigned off = 0x10000u - TAP_BIAS / 32;  // -(TAP_BIAS / 32) in each half
+    return __viaddmin_s16x2_relu(((t + 0x00100010u) >> 5) & 0x07ff07ffu, off << 16 | off, 0x00ff00ffu);
+}
+
+// Horizontal sums of the four samples of word w, its neighbours p and n: columns 0, 2 in te, 1, 3 in to.
+__device__ __forceinline__ void tap_row4(unsigned p, unsigned w, unsigned n, unsigned& te, unsigned& to)
+{
+    constexpr unsigned m = 0x00ff00ffu;
+    const unsigned e0 = p & m, o0 = (p >> 8) & m, e1 = w & m, o1 = (w >> 8) & m, e2 = n & m, o2 = (n >> 8) & m;
+    const unsigned em = __funnelshift_r(e0, e1, 16), om = __funnelshift_r(o0, o1, 16);
+    const unsigned ep = __funnelshift_r(e1, e2, 16), op = __funnelshift_r(o1, o2, 16);
+    te = tap_pair(em, om, e1, o1, ep, op);
+    to = tap_pair(om, e1, o1, ep, op, e2);
+}
+
+// Centre samples of four columns from sums + TAP_BIAS of the other direction, pairs of columns: p1, p2 hold
+// the four, p0 the two before, p3 and p4 the four after.  The taps sum to 32.
+__device__ __forceinline__ unsigned tap_centre4(unsigned p0, unsigned p1, unsigned p2, unsigned p3, unsigned p4)
+{
+    constexpr int c0 = 512 - 32 * TAP_BIAS;
+    // pairs of taps as bytes: (1, -5), (20, 20), (-5, 1) from an even sample, (0, 1), (-5, 20), (20, -5),
+    // (1, 0) from an odd one
+    constexpr int ka = 0x1414fb01, kb = 0x000001fb, kc = 0x14fb0100, kd = 0x0001fb14;
+    const int q0 = (int)p0, q1 = (int)p1, q2 = (int)p2, q3 = (int)p3, q4 = (int)p4;
+    const int v0 = __dp2a_lo(q2, kb, __dp2a_hi(q1, ka, __dp2a_lo(q0, ka, c0)));
+    const int v1 = __dp2a_hi(q3, kd, __dp2a_lo(q2, kd, __dp2a_hi(q1, kc, __dp2a_lo(q0, kc, c0))));
+    const int v2 = __dp2a_lo(q3, kb, __dp2a_hi(q2, ka, __dp2a_lo(q1, ka, c0)));
+    const int v3 = __dp2a_hi(q4, kd, __dp2a_lo(q3, kd, __dp2a_hi(q2, kc, __dp2a_lo(q1, kc, c0))));
+    const unsigned ve = __byte_perm((unsigned)(v0 >> 10), (unsigned)(v2 >> 10), 0x5410);
+    const unsigned vo = __byte_perm((unsigned)(v1 >> 10), (unsigned)(v3 >> 10), 0x5410);
+    return __viaddmin_s16x2_relu(ve, 0u, 0x00ff00ffu) | __viaddmin_s16x2_relu(vo, 0u, 0x00ff00ffu) << 8;
+}
+
 // Sum over the warp (every lane gets it).
 __device__ __forceinline__ int warp_sum(int v) { return __reduce_add_sync(0xffffffffu, v); }
 

@@ -159,9 +159,8 @@ static_assert(sizeof(Window) % 16 == 0, "what a Lattice adds follows it at once"
 // (r, c) is point (3 + r, 3 + c).  h, b and j are byte planes of rows 2..19 in the window's columns; G is the
 // window itself.  The reference scales h and b and copies G for rows and columns 2..18 only, which leaves
 // (MultiresCross, Multires) the raw b in row 19, the raw h in column 19 and zeros for G there: raw holds h
-// (rows 2..18) and row19 b, both + 2560.  Ver2 completes that row and column.
+// (rows 2..18) and row19 b, both + TAP_BIAS.  Ver2 completes that row and column.
 constexpr int SUB_PLANE = 18 * WPITCH;
-constexpr int RAW_BIAS = 2560;              // a multiple of 32 above the most negative 6-tap sum, 2550
 struct Lattice : Window {
     unsigned sub[3 * SUB_PLANE];            // h, b, j: row fr - 2
     unsigned raw[17 * 2 * WPITCH];          // pairs of shorts
@@ -325,17 +324,6 @@ __device__ __forceinline__ void cross_offset(int lane, int s, int& j, int& i)
     i = (lane & 2) ? v : 0;
 }
 
-// Two 16-bit 6-tap sums + RAW_BIAS (never negative, below 2^14), and their rounded, clipped samples.
-__device__ __forceinline__ unsigned tap_pair(unsigned a, unsigned b, unsigned c, unsigned d, unsigned e, unsigned f)
-{
-    return (a + f + RAW_BIAS * 0x10001u) + 20u * (c + d) - 5u * (b + e);
-}
-__device__ __forceinline__ unsigned scale_pair(unsigned t)
-{
-    constexpr unsigned off = 0x10000u - RAW_BIAS / 32;  // -(RAW_BIAS / 32) in each half
-    return __viaddmin_s16x2_relu(((t + 0x00100010u) >> 5) & 0x07ff07ffu, off << 16 | off, 0x00ff00ffu);
-}
-
 // The lattice whose row 0 is the window's row wy; its column 0 may be any of the window's columns 0..4.
 template <bool kVer2>
 __device__ __forceinline__ void build_lattice(Lattice& L, int wy, int lane)
@@ -364,12 +352,8 @@ __device__ __forceinline__ void build_lattice(Lattice& L, int wy, int lane)
     for (int i = lane; i < 18 * 6; i += 32) {  // b, rows 2..19: words 0..5 hold its columns 2..18
         const int r = i / 6, wd = i - 6 * r;
         const unsigned* q = L.win + (wy + 2 + r) * WPITCH + wd;
-        const unsigned p = wd ? q[-1] : 0u;
-        const unsigned e0 = p & m, o0 = (p >> 8) & m, e1 = q[0] & m, o1 = (q[0] >> 8) & m, e2 = q[1] & m,
-                       o2 = (q[1] >> 8) & m;
-        const unsigned em = __funnelshift_r(e0, e1, 16), om = __funnelshift_r(o0, o1, 16);
-        const unsigned ep = __funnelshift_r(e1, e2, 16), op = __funnelshift_r(o1, o2, 16);
-        const unsigned te = tap_pair(em, om, e1, o1, ep, op), to = tap_pair(om, e1, o1, ep, op, e2);
+        unsigned te, to;
+        tap_row4(wd ? q[-1] : 0u, q[0], q[1], te, to);
         b[r * WPITCH + wd] = scale_pair(te) | scale_pair(to) << 8;
         if (!kVer2 && r == 17) {
             L.row19[2 * wd] = __byte_perm(te, to, 0x5410);
@@ -377,21 +361,10 @@ __device__ __forceinline__ void build_lattice(Lattice& L, int wy, int lane)
         }
     }
     __syncwarp();
-    for (int i = lane; i < 17 * 6; i += 32) {  // j, rows 2..18, from the raw h; the taps sum to 32
+    for (int i = lane; i < 17 * 6; i += 32) {  // j, rows 2..18, from the raw h
         const int r = i / 6, wd = i - 6 * r;
         const unsigned* q = L.raw + 2 * (r * WPITCH + wd);
-        const int p0 = wd ? (int)q[-1] : 0, p1 = (int)q[0], p2 = (int)q[1], p3 = (int)q[2], p4 = (int)q[3];
-        constexpr int c0 = 512 - 32 * RAW_BIAS;
-        // pairs of taps as bytes: (1, -5), (20, 20), (-5, 1) from an even sample, (0, 1), (-5, 20), (20, -5),
-        // (1, 0) from an odd one
-        constexpr int ka = 0x1414fb01, kb = 0x000001fb, kc = 0x14fb0100, kd = 0x0001fb14;
-        const int v0 = __dp2a_lo(p2, kb, __dp2a_hi(p1, ka, __dp2a_lo(p0, ka, c0)));
-        const int v1 = __dp2a_hi(p3, kd, __dp2a_lo(p2, kd, __dp2a_hi(p1, kc, __dp2a_lo(p0, kc, c0))));
-        const int v2 = __dp2a_lo(p3, kb, __dp2a_hi(p2, ka, __dp2a_lo(p1, ka, c0)));
-        const int v3 = __dp2a_hi(p4, kd, __dp2a_lo(p3, kd, __dp2a_hi(p2, kc, __dp2a_lo(p1, kc, c0))));
-        const unsigned ve = __byte_perm((unsigned)(v0 >> 10), (unsigned)(v2 >> 10), 0x5410);
-        const unsigned vo = __byte_perm((unsigned)(v1 >> 10), (unsigned)(v3 >> 10), 0x5410);
-        jp[r * WPITCH + wd] = __viaddmin_s16x2_relu(ve, 0u, 0x00ff00ffu) | __viaddmin_s16x2_relu(vo, 0u, 0x00ff00ffu) << 8;
+        jp[r * WPITCH + wd] = tap_centre4(wd ? q[-1] : 0u, q[0], q[1], q[2], q[3]);
     }
     __syncwarp();
 }
@@ -433,7 +406,7 @@ __device__ __forceinline__ void settle_quads(const unsigned (&s)[4], int v, int&
 __device__ __forceinline__ int byte_of(unsigned w, int k) { return (int)((w >> (8 * k)) & 0xffu); }
 __device__ __forceinline__ int raw_of(const unsigned* w, int i)
 {
-    return (int)reinterpret_cast<const unsigned short*>(w)[i] - RAW_BIAS;
+    return (int)reinterpret_cast<const unsigned short*>(w)[i] - TAP_BIAS;
 }
 
 // Half then quarter pel in the estimator's window around block o (…MultiresCross.cpp:875-941), strict
