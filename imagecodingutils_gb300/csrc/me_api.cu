@@ -224,7 +224,9 @@ int run(vppgpu_me* me, const short* d_src16, const short* d_ref16, const unsigne
         int* d_mv, int* d_dist, long long* d_avg, double lambda, bool v2_lambda = false)
 {
     vppgpu_ctx* ctx = me->ctx;
-    VPP_CUDA(cudaMemsetAsync(me->ctrl, 0, sizeof(vppgpu::MeCtrl), ctx->stream));
+    if (me->kind == VPPGPU_ME_H263_MULTIRES_CROSS_V2 || me->kind == VPPGPU_ME_MULTIRES_CROSS ||
+        me->kind == VPPGPU_ME_H263_MULTIRES_CROSS)  // no job: the counters alone
+        VPP_CUDA(cudaMemsetAsync(me->ctrl, 0, sizeof(vppgpu::MeCtrl), ctx->stream));
     if (me->kind == VPPGPU_ME_H263_MULTIRES_CROSS_V2) {
         const vppgpu::H263V2Job j{me->W,      me->H,      me->motion_range, me->mode,      me->relax_sweeps,
                                   d_src16,    d_ref16,    me->d_mrc,        d_incl,        d_mv,
@@ -237,17 +239,16 @@ int run(vppgpu_me* me, const short* d_src16, const short* d_ref16, const unsigne
         return vppgpu::mrc_launch(ctx, me->W, me->H, me->motion_range, me->mode, d_src16, d_ref16, me->d_mrc, d_incl,
                                   d_mv, d_dist, d_avg, me->ctrl, me->mrc_warps,
                                   me->kind == VPPGPU_ME_H263_MULTIRES_CROSS);
-    int rc = vppgpu::set_job(ctx, me->d_job, vppgpu::JobDesc{d_src16, d_ref16, d_incl, d_slice, d_mv, d_dist, d_avg});
+    int rc = vppgpu::set_job(ctx, me->d_job, vppgpu::JobDesc{d_src16, d_ref16, d_incl, d_slice, d_mv, d_dist, d_avg},
+                             me->ctrl, me->changed, me->changed ? (int)me->sweep_limit : 0);
     if (rc) return rc;
     if (me->kind == VPPGPU_ME_CROSS) {
         // GetBestVector's lambda 0.9 (MotionEstimatorH264ImplCross.cpp:621)
-        VPP_CUDA(cudaMemsetAsync(me->changed, 0, sizeof(int) * (size_t)me->sweep_limit, ctx->stream));
         return vppgpu::cross_launch(ctx, full_args(me, 0.9));
     }
     if (me->kind == VPPGPU_ME_MULTIRES_CROSS_V2 || me->kind == VPPGPU_ME_MULTIRES) {
         // GetBestVector's lambda: 0.9 (MultiresCrossVer2.cpp:1050), 1.1 (Multires.cpp:958)
         const bool v2 = me->kind == VPPGPU_ME_MULTIRES_CROSS_V2;
-        VPP_CUDA(cudaMemsetAsync(me->changed, 0, sizeof(int) * (size_t)me->sweep_limit, ctx->stream));
         if (v2 && v2_lambda) {  // Estimate(long*, void* lambda) (MultiresCrossVer2.cpp:1162-1742)
             vppgpu::FullArgs a = full_args(me, lambda);
             a.grid_sweeps = a.relax_sweeps;  // an evaluation is a search: every sweep over the whole GPU
@@ -257,7 +258,6 @@ int run(vppgpu_me* me, const short* d_src16, const short* d_ref16, const unsigne
                                    d_ref16);
     }
     if (searches_from_prediction(me->kind)) {
-        VPP_CUDA(cudaMemsetAsync(me->changed, 0, sizeof(int) * (size_t)me->sweep_limit, ctx->stream));
         return vppgpu::umhs_launch(ctx, umhs_args(me), me->wave_grid);
     }
     if (me->kind == VPPGPU_ME_IMPL1) return vppgpu::impl1_launch(ctx, full_args(me, 0.0), me->bw, me->bh, me->motion_range);
@@ -277,10 +277,7 @@ int run(vppgpu_me* me, const short* d_src16, const short* d_ref16, const unsigne
         cudaGraph_t g = nullptr;
         const unsigned long long before = ctx->launches;
         if (cudaStreamBeginCapture(ctx->stream, cudaStreamCaptureModeThreadLocal) == cudaSuccess) {
-            int crc = VPPGPU_OK;
-            if (cudaMemsetAsync(me->changed, 0, sizeof(int) * (size_t)me->sweep_limit, ctx->stream) != cudaSuccess)
-                crc = VPPGPU_ERR_CUDA;
-            if (!crc) crc = vppgpu::full_launch(ctx, a, me->nmb, nullptr);
+            const int crc = vppgpu::full_launch(ctx, a, me->nmb, nullptr);
             const cudaError_t e = cudaStreamEndCapture(ctx->stream, &g);
             if (!crc && e == cudaSuccess && g && cudaGraphInstantiate(&me->graph, g, 0) == cudaSuccess) {
                 me->graph_state = 1;
@@ -296,7 +293,6 @@ int run(vppgpu_me* me, const short* d_src16, const short* d_ref16, const unsigne
         ctx->launches += me->graph_kernels;
         return VPPGPU_OK;
     }
-    VPP_CUDA(cudaMemsetAsync(me->changed, 0, sizeof(int) * (size_t)me->sweep_limit, ctx->stream));
     return vppgpu::full_launch(ctx, a, me->nmb, ev);
 }
 

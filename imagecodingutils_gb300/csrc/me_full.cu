@@ -719,13 +719,21 @@ __global__ void __launch_bounds__(TIE_RUNS * 32) k_full_tietree(const __grid_con
     }
 }
 
-__global__ void k_set_job(JobDesc* dst, JobDesc v) { *dst = v; }
+// The words an estimate starts from: its job, the counters at zero.
+__global__ void __launch_bounds__(256) k_set_job(JobDesc* dst, JobDesc v, int* ctrl, int* changed, int nchanged)
+{
+    if (threadIdx.x == 0) *dst = v;
+    if (ctrl)
+        for (int i = threadIdx.x; i < (int)(sizeof(MeCtrl) / sizeof(int)); i += 256) ctrl[i] = 0;
+    for (int i = threadIdx.x; i < nchanged; i += 256) changed[i] = 0;
+}
 
 }  // namespace
 
-int set_job(vppgpu_ctx* ctx, JobDesc* d_job, const JobDesc& v)
+int set_job(vppgpu_ctx* ctx, JobDesc* d_job, const JobDesc& v, MeCtrl* ctrl, int* changed, int nchanged)
 {
-    k_set_job<<<1, 1, 0, ctx->stream>>>(d_job, v);
+    static_assert(sizeof(MeCtrl) % sizeof(int) == 0, "cleared by words");
+    k_set_job<<<1, 256, 0, ctx->stream>>>(d_job, v, reinterpret_cast<int*>(ctrl), changed, nchanged);
     VPP_CHECK_LAUNCH(ctx);
     return VPPGPU_OK;
 }

@@ -19,7 +19,7 @@ struct MeCtrl {
     int relax_miss;  // ... of which computed the prediction distortion
     int wave_miss;   // MBs the wavefront had to evaluate in full
     int ntie;        // entries of FullArgs::tie_list
-    int ticket;      // MultiresCrossVer2 dataflow pass: next macroblock
+    int ticket;      // MultiresCrossVer2 dataflow pass: next macroblock; MultiresCross: macroblocks done
     int tie_mbs;     // H263 MultiresCrossVer2: entries of its tie list
 };
 
@@ -214,7 +214,7 @@ int umhs_prepare();
 
 // Write this estimate's pointers to the device descriptor (a one-thread
 // kernel with the descriptor as its parameter: stream-ordered, no host copy).
-int set_job(vppgpu_ctx* ctx, JobDesc* d_job, const JobDesc& v);
+int set_job(vppgpu_ctx* ctx, JobDesc* d_job, const JobDesc& v, MeCtrl* ctrl, int* changed, int nchanged);
 
 // Motion-compensated luma residual of the last estimate's planes at vectors d_mv.
 int full_residual_launch(vppgpu_ctx* ctx, const FullArgs& args, const int* d_mv, short* d_res);

@@ -18,18 +18,13 @@
 // samples; a read outside a copy sets an error instead of reading.
 //
 // GB300 design
-//   k_mrc_level0   input luma to bytes (0..255 check) and the border-19
-//                  reference copy.
-//   k_mrc_level1   2:1 decimations (OverlayMem2Dv2::Half) of input and
-//                  reference, the border-9 reference copy.
-//   k_mrc_level2   the second decimation (mode 2), border-5 copy.
-//   k_mrc_search   one warp per macroblock.  Candidate distortions are warp
-//                  reductions laid out by phase (lane pair = one phase), so
-//                  the 16 phase prefix sums are a shuffle scan; candidates
-//                  are tested in the reference's order against the running
-//                  minimum.  The sub-pel window's lattice (G, h, b,
-//                  j at 22x22 points, with the window's unwritten and
-//                  unscaled edge samples) is built per warp in shared memory.
+//   k_mrc_levels   input luma to bytes (0..255 check) and the border-19
+//                  reference copy; the 2:1 decimations
+//                  (OverlayMem2Dv2::Half) of input and reference, once and
+//                  (mode 2) twice, with border-9 and border-5 copies.
+//   k_mrc_search   one warp per macroblock, a lane per candidate
+//                  (me_mrc_search.cuh); the last macroblock's warp forms the
+//                  average.
 //
 // The same file holds the searches of the predictor multi-resolution estimators at prediction
 // (0, 0) with their tie trees (MultiresCrossVer2, Multires; their resolve is me_full_resolve.cu),
@@ -46,77 +41,101 @@ namespace {
 using namespace mrc;
 
 // ---------------------------------------------------------------------------
-__global__ void __launch_bounds__(256) k_mrc_level0(const short* __restrict__ src16, const short* __restrict__ ref16,
-                                                   int W, int H, unsigned char* __restrict__ in0,
-                                                   unsigned char* __restrict__ e0, int* status)
+// Every level from the input and reference samples in one launch: the 2:1 decimations of a level are
+// formed again where the next needs them (16 samples of a level-2 one), which costs less than a
+// launch between the levels (1280x720, profiled: three launches 25 us, one 7).  A task is a word of level 0
+// or 1, a sample of level 2; bordered copies replicate the level's edge.
+// Four shorts at p (any even address) as the bytes of a word; reads the 4-byte words around them.
+__device__ __forceinline__ unsigned bytes4(const short* p, bool& bad)
 {
-    const int EW = W + 38, EH = H + 38;
-    const long long n_in = (long long)W * H, n_e = (long long)EW * EH;
+    const unsigned* q = reinterpret_cast<const unsigned*>(reinterpret_cast<uintptr_t>(p) & ~(uintptr_t)3);
+    unsigned lo = __ldg(q), hi = __ldg(q + 1);
+    if (reinterpret_cast<uintptr_t>(p) & 2) {
+        const unsigned end = (unsigned short)__ldg(p + 3);
+        lo = __funnelshift_r(lo, hi, 16);
+        hi = __byte_perm(hi, end, 0x5432);
+    }
+    bad |= ((lo | hi) & 0xff00ff00u) != 0u;
+    return __byte_perm(lo, hi, 0x6420);
+}
+// 2:1 decimation (OverlayMem2Dv2::Half, OverlayMem2Dv2.cpp:3018-3033) at (x, y); pairs of shorts are
+// 4-byte aligned (planes are, rows are a multiple of 16 wide).
+__device__ __forceinline__ int half_at(const short* p, int w, int x, int y)
+{
+    const unsigned* q = reinterpret_cast<const unsigned*>(p + (size_t)(2 * y) * w + 2 * x);
+    const unsigned a = __ldg(q), b = __ldg(q + w / 2);
+    return ((int)(short)a + ((int)a >> 16) + (int)(short)b + ((int)b >> 16) + 2) >> 2;
+}
+__device__ __forceinline__ int quarter_at(const short* p, int w, int x, int y)
+{
+    return ((half_at(p, w, 2 * x, 2 * y) & 0xff) + (half_at(p, w, 2 * x + 1, 2 * y) & 0xff) +
+            (half_at(p, w, 2 * x, 2 * y + 1) & 0xff) + (half_at(p, w, 2 * x + 1, 2 * y + 1) & 0xff) + 2) >> 2;
+}
+
+// keep, when not null: where the searches at a prediction find the arguments.
+__global__ void __launch_bounds__(256) k_mrc_levels(MrcArgs a, const short* __restrict__ src16,
+                                                   const short* __restrict__ ref16, MrcArgs* keep)
+{
+    const unsigned W = a.W, H = a.H, w1 = W / 2, h1 = H / 2, w2 = w1 / 2, h2 = h1 / 2;
+    const unsigned n0 = W * H / 4, m0 = ((W + 38) * (H + 38) + 3) / 4, n1 = w1 * h1 / 4, m1 = ((w1 + 18) * (h1 + 18) + 3) / 4;
+    const unsigned n2 = a.mode == 2 ? w2 * h2 : 0, m2 = a.mode == 2 ? (w2 + 10) * (h2 + 10) : 0;
+    const unsigned step = gridDim.x * blockDim.x, first = blockIdx.x * blockDim.x + threadIdx.x;
+    if (keep && first == 0) *keep = a;
     bool bad = false;
-    for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n_in + n_e;
-         i += (long long)gridDim.x * blockDim.x) {
-        if (i < n_in) {
-            const int v = src16[i];
-            bad |= (v < 0) | (v > 255);
-            in0[i] = (unsigned char)(v & 0xff);
+    for (unsigned i = first; i < n0; i += step)
+        reinterpret_cast<unsigned*>(const_cast<unsigned char*>(a.in0.p))[i] = bytes4(src16 + 4 * (size_t)i, bad);
+    for (unsigned i = first; i < m0; i += step) {
+        const unsigned ew = W + 38;
+        int y = (int)(4 * i / ew), x = (int)(4 * i - y * ew);
+        unsigned v = 0;
+        if (x >= 19 && x + 3 < (int)W + 19) {
+            v = bytes4(ref16 + (size_t)min(max(y - 19, 0), (int)H - 1) * W + x - 19, bad);
         } else {
-            const long long j = i - n_in;
-            const int y = (int)(j / EW), x = (int)(j - (long long)y * EW);
-            const int sy = min(max(y - 19, 0), H - 1), sx = min(max(x - 19, 0), W - 1);
-            const int v = ref16[(size_t)sy * W + sx];
-            bad |= (v < 0) | (v > 255);
-            e0[j] = (unsigned char)(v & 0xff);
+#pragma unroll
+            for (int k = 0; k < 4; k++) {
+                const int s = ref16[(size_t)min(max(y - 19, 0), (int)H - 1) * W + min(max(x - 19, 0), (int)W - 1)];
+                bad |= (s < 0) | (s > 255);
+                v |= (unsigned)(s & 0xff) << (8 * k);
+                if (++x == (int)ew) {
+                    x = 0;
+                    y++;
+                }
+            }
         }
+        reinterpret_cast<unsigned*>(const_cast<unsigned char*>(a.e0.p))[i] = v;
     }
-    if (__any_sync(0xffffffffu, bad) && (threadIdx.x & 31) == 0) atomicOr(status, ST_PIXEL_RANGE);
-}
-
-// 2:1 decimation (OverlayMem2Dv2::Half, OverlayMem2Dv2.cpp:3018-3033) of a
-// w x h plane at (x, y).
-template <typename T>
-__device__ __forceinline__ int half_at(const T* p, int w, int x, int y)
-{
-    const T* q = p + (size_t)(2 * y) * w + 2 * x;
-    return ((int)q[0] + q[1] + q[w] + q[w + 1] + 2) >> 2;
-}
-
-__global__ void __launch_bounds__(256) k_mrc_level1(const short* __restrict__ src16, const short* __restrict__ ref16,
-                                                   int W, int H, unsigned char* __restrict__ in1,
-                                                   unsigned char* __restrict__ e1)
-{
-    const int w1 = W / 2, h1 = H / 2, EW = w1 + 18, EH = h1 + 18;
-    const long long n_in = (long long)w1 * h1, n_e = (long long)EW * EH;
-    for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n_in + n_e;
-         i += (long long)gridDim.x * blockDim.x) {
-        if (i < n_in) {
-            const int y = (int)(i / w1), x = (int)(i - (long long)y * w1);
-            in1[i] = (unsigned char)half_at(src16, W, x, y);
-        } else {
-            const long long j = i - n_in;
-            const int y = (int)(j / EW), x = (int)(j - (long long)y * EW);
-            e1[j] = (unsigned char)half_at(ref16, W, min(max(x - 9, 0), w1 - 1), min(max(y - 9, 0), h1 - 1));
+    for (unsigned i = first; i < n1; i += step) {
+        const int y = (int)(4 * i / w1), x = (int)(4 * i - y * w1);
+        unsigned v = 0;
+#pragma unroll
+        for (int k = 0; k < 4; k++) v |= (unsigned)(half_at(src16, W, x + k, y) & 0xff) << (8 * k);
+        reinterpret_cast<unsigned*>(const_cast<unsigned char*>(a.in1.p))[i] = v;
+    }
+    for (unsigned i = first; i < m1; i += step) {
+        const unsigned ew = w1 + 18;
+        int y = (int)(4 * i / ew), x = (int)(4 * i - y * ew);
+        unsigned v = 0;
+#pragma unroll
+        for (int k = 0; k < 4; k++) {
+            v |= (unsigned)(half_at(ref16, W, min(max(x - 9, 0), (int)w1 - 1), min(max(y - 9, 0), (int)h1 - 1)) & 0xff) << (8 * k);
+            if (++x == (int)ew) {
+                x = 0;
+                y++;
+            }
         }
+        reinterpret_cast<unsigned*>(const_cast<unsigned char*>(a.e1.p))[i] = v;
     }
-}
-
-__global__ void __launch_bounds__(256) k_mrc_level2(const unsigned char* __restrict__ in1,
-                                                   const unsigned char* __restrict__ e1, int W, int H,
-                                                   unsigned char* __restrict__ in2, unsigned char* __restrict__ e2)
-{
-    const int w1 = W / 2, h1 = H / 2, w2 = w1 / 2, h2 = h1 / 2, EW = w2 + 10, EH = h2 + 10, EW1 = w1 + 18;
-    const long long n_in = (long long)w2 * h2, n_e = (long long)EW * EH;
-    const unsigned char* r1 = e1 + 9 * (size_t)EW1 + 9;  // level-1 reference inside its border-9 copy
-    for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n_in + n_e;
-         i += (long long)gridDim.x * blockDim.x) {
-        if (i < n_in) {
-            const int y = (int)(i / w2), x = (int)(i - (long long)y * w2);
-            in2[i] = (unsigned char)half_at(in1, w1, x, y);
-        } else {
-            const long long j = i - n_in;
-            const int y = (int)(j / EW), x = (int)(j - (long long)y * EW);
-            e2[j] = (unsigned char)half_at(r1, EW1, min(max(x - 5, 0), w2 - 1), min(max(y - 5, 0), h2 - 1));
-        }
+    for (unsigned i = first; i < n2; i += step) {
+        const int y = (int)(i / w2), x = (int)(i - y * w2);
+        const_cast<unsigned char*>(a.in2.p)[i] = (unsigned char)quarter_at(src16, W, x, y);
     }
+    for (unsigned i = first; i < m2; i += step) {
+        const unsigned ew = w2 + 10;
+        const int y = (int)(i / ew), x = (int)(i - y * ew);
+        const_cast<unsigned char*>(a.e2.p)[i] =
+            (unsigned char)quarter_at(ref16, W, min(max(x - 5, 0), (int)w2 - 1), min(max(y - 5, 0), (int)h2 - 1));
+    }
+    if (__any_sync(0xffffffffu, bad) && (threadIdx.x & 31) == 0) atomicOr(&a.ctrl->status, ST_PIXEL_RANGE);
 }
 
 // kH263: MotionEstimatorH263ImplMultiresCross (…H263ImplMultiresCross.cpp:531-1010), whose motion
@@ -160,6 +179,14 @@ __global__ void __launch_bounds__(256) k_mrc_search(MrcArgs a)
         if (do_it) {
             atomicAdd(reinterpret_cast<unsigned long long*>(&a.ctrl->total), (unsigned long long)(long long)chosen);
             atomicAdd(&a.ctrl->count, 1);
+        }
+        // the last macroblock's warp divides
+        __threadfence();
+        if (atomicAdd(&a.ctrl->ticket, 1) == a.cols * a.rows_all - 1 && a.out_avg) {
+            __threadfence();
+            const long long t = *((volatile long long*)&a.ctrl->total);
+            const int n = *((volatile int*)&a.ctrl->count);
+            *a.out_avg = n ? t / n : 0;
         }
     }
 }
@@ -223,8 +250,6 @@ __global__ void __launch_bounds__(V2_TIE_RUNS * 32) k_pred_tietree(MrcArgs m, Fu
         if (__any_sync(0xffffffffu, bad) && lane == 0) atomicOr(&f.ctrl->status, ST_OUT_OF_BOUNDS);
     }
 }
-
-__global__ void k_set_mrc(MrcArgs* dst, MrcArgs v) { *dst = v; }
 
 // ---------------------------------------------------------------------------
 // MotionEstimatorH263ImplMultiresCrossVer2 (…H263ImplMultiresCrossVer2.cpp:537-1151).  Its search is
@@ -761,11 +786,16 @@ __global__ void __launch_bounds__(256) k_v263_outputs(V263 v)
 
 }  // namespace
 
+// The levels, each at a multiple of 16 bytes with four to spare behind it: words are written and
+// read across its end.
+static size_t level_bytes(int w, int h, int border) { return ((size_t)(w + 2 * border) * (h + 2 * border) + 4 + 15) / 16 * 16; }
+
 size_t mrc_scratch_bytes(int W, int H)
 {
-    const size_t w1 = W / 2, h1 = H / 2, w2 = w1 / 2, h2 = h1 / 2;
-    return (size_t)W * H + (size_t)(W + 38) * (H + 38) + w1 * h1 + (w1 + 18) * (h1 + 18) + w2 * h2 +
-           (w2 + 10) * (h2 + 10) + 64;
+    size_t n = 64;
+    for (int l = 0, w = W, h = H; l < 3; l++, w /= 2, h /= 2)
+        n += level_bytes(w, h, 0) + level_bytes(w, h, l == 0 ? 19 : (l == 1 ? 9 : 5));
+    return n;
 }
 
 namespace {
@@ -784,17 +814,14 @@ MrcArgs mrc_args(int W, int H, int motion_range, int mode, unsigned char* scratc
     a.motion_range = motion_range;
     a.lambda = 0.0;
     unsigned char* p = scratch;
-    unsigned char* in0 = p;
-    p += (size_t)W * H;
-    unsigned char* e0 = p;
-    p += (size_t)(W + 38) * (H + 38);
-    unsigned char* in1 = p;
-    p += (size_t)w1 * h1;
-    unsigned char* e1 = p;
-    p += (size_t)(w1 + 18) * (h1 + 18);
-    unsigned char* in2 = p;
-    p += (size_t)w2 * h2;
-    unsigned char* e2 = p;
+    auto take = [&p](size_t n) {
+        unsigned char* q = p;
+        p += n;
+        return q;
+    };
+    unsigned char *in0 = take(level_bytes(W, H, 0)), *e0 = take(level_bytes(W, H, 19));
+    unsigned char *in1 = take(level_bytes(w1, h1, 0)), *e1 = take(level_bytes(w1, h1, 9));
+    unsigned char *in2 = take(level_bytes(w2, h2, 0)), *e2 = take(level_bytes(w2, h2, 5));
     a.in0 = Buf{in0, W, H};
     a.e0 = Buf{e0, W + 38, H + 38};
     a.in1 = Buf{in1, w1, h1};
@@ -809,25 +836,12 @@ MrcArgs mrc_args(int W, int H, int motion_range, int mode, unsigned char* scratc
     return a;
 }
 
-int levels_launch(vppgpu_ctx* ctx, const MrcArgs& a, const short* d_src16, const short* d_ref16)
+int levels_launch(vppgpu_ctx* ctx, const MrcArgs& a, const short* d_src16, const short* d_ref16, MrcArgs* keep = nullptr)
 {
-    const int W = a.W, H = a.H, w1 = W / 2, h1 = H / 2, w2 = w1 / 2, h2 = h1 / 2;
+    const long long words = ((long long)(a.W + 38) * (a.H + 38) + 3) / 4, blocks = (words + 255) / 256;
     const int cap = ctx->sm_count * 8;
-    auto grid = [&](long long work) {
-        long long g = (work + 255) / 256;
-        return (int)(g < cap ? g : cap);
-    };
-    k_mrc_level0<<<grid((long long)W * H + (long long)(W + 38) * (H + 38)), 256, 0, ctx->stream>>>(
-        d_src16, d_ref16, W, H, (unsigned char*)a.in0.p, (unsigned char*)a.e0.p, &a.ctrl->status);
+    k_mrc_levels<<<(int)(blocks < cap ? blocks : cap), 256, 0, ctx->stream>>>(a, d_src16, d_ref16, keep);
     VPP_CHECK_LAUNCH(ctx);
-    k_mrc_level1<<<grid((long long)w1 * h1 + (long long)(w1 + 18) * (h1 + 18)), 256, 0, ctx->stream>>>(
-        d_src16, d_ref16, W, H, (unsigned char*)a.in1.p, (unsigned char*)a.e1.p);
-    VPP_CHECK_LAUNCH(ctx);
-    if (a.mode == 2) {
-        k_mrc_level2<<<grid((long long)w2 * h2 + (long long)(w2 + 10) * (h2 + 10)), 256, 0, ctx->stream>>>(
-            a.in1.p, a.e1.p, W, H, (unsigned char*)a.in2.p, (unsigned char*)a.e2.p);
-        VPP_CHECK_LAUNCH(ctx);
-    }
     return VPPGPU_OK;
 }
 
@@ -851,8 +865,6 @@ int mrc_launch(vppgpu_ctx* ctx, int W, int H, int motion_range, int mode, const 
     else
         k_mrc_search<false><<<(mbs + wpb - 1) / wpb, 32 * wpb, wpb * sizeof(Lattice), ctx->stream>>>(a);
     VPP_CHECK_LAUNCH(ctx);
-    k_mrc_average<<<1, 1, 0, ctx->stream>>>(out_avg, ctrl);
-    VPP_CHECK_LAUNCH(ctx);
     return VPPGPU_OK;
 }
 
@@ -866,11 +878,9 @@ int mrc2_launch(vppgpu_ctx* ctx, int est, int mode, unsigned char* scratch, cons
     MrcArgs m = mrc_args(args.W, args.H, args.motion_range, mode, scratch);
     m.ctrl = args.ctrl;
     m.lambda = args.lambda;
-    k_set_mrc<<<1, 1, 0, ctx->stream>>>((MrcArgs*)args.mrc, m);  // for the searches at a prediction
-    VPP_CHECK_LAUNCH(ctx);
     int rc = full_planes_launch(ctx, args);
     if (rc) return rc;
-    if ((rc = levels_launch(ctx, m, d_src16, d_ref16))) return rc;
+    if ((rc = levels_launch(ctx, m, d_src16, d_ref16, (MrcArgs*)args.mrc))) return rc;
     if (est == EST_MULTIRES) {
         k_pred_search<EST_MULTIRES><<<(args.nmb + 7) / 8, 256, 0, ctx->stream>>>(m, args);
         VPP_CHECK_LAUNCH(ctx);

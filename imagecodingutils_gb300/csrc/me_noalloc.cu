@@ -176,11 +176,10 @@ extern "C" int vppgpu_me_full_estimate_noalloc(const short* d_src, const short* 
     a.tie_runs = nullptr;
     a.spin_limit = 20000000LL;
 
-    // the words that must start at zero on every call
-    VPP_CUDA(cudaMemsetAsync(a.ctrl, 0, sizeof(vppgpu::MeCtrl), ctx.stream));
-    VPP_CUDA(cudaMemsetAsync(a.changed, 0, sizeof(int) * (size_t)a.sweep_limit, ctx.stream));
+    // the job, and the words that must start at zero on every call
     rc = vppgpu::set_job(&ctx, (vppgpu::JobDesc*)(base + kOffJob),
-                         vppgpu::JobDesc{d_src, d_ref, d_dist_included, d_mb_slice, (int*)d_mv_out, d_mb_dist_out, nullptr});
+                         vppgpu::JobDesc{d_src, d_ref, d_dist_included, d_mb_slice, (int*)d_mv_out, d_mb_dist_out, nullptr},
+                         a.ctrl, a.changed, a.sweep_limit);
     if (rc) return rc;
     rc = vppgpu::full_launch(&ctx, a, nmb, nullptr);
     if (rc) return rc;
