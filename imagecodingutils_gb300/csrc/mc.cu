@@ -156,23 +156,14 @@ __device__ __forceinline__ void mc_chroma_blocks(McLattice& L, const Plane& U, c
     }
 }
 
-// One warp per macroblock: its 16x16 luma block and its two 8x8 chroma
-// blocks.  Luma stages the 22x22 reference window around the vector's
-// full-pel position (one column per lane, rows clamped only at the frame
-// edge), the j cases also the horizontal 6-taps, then computes the quarter
-// samples of its case from the term table.  Warp-synchronous: no block barrier.
-__global__ void __launch_bounds__(32 * kMcWarps, 12) k_mc_frame(Plane ry, Plane ru, Plane rv,
-                                                               const int* __restrict__ mv, int cols, int nmb,
-                                                               short* __restrict__ oy, short* __restrict__ ou,
-                                                               short* __restrict__ ov)
+// Any samples, any vector, one at a time: luma stages the 22x22 reference window around the vector's
+// full-pel position (one column per lane, rows clamped only at the frame edge), the j cases also the
+// horizontal 6-taps, then computes the quarter samples of its case from the term table.
+__device__ __noinline__ void mc_general(McLattice& L, const Plane& ry, const Plane& ru, const Plane& rv, int n, int m,
+                                        int mvx, int mvy, int lane, short* __restrict__ oy, short* __restrict__ ou,
+                                        short* __restrict__ ov)
 {
-    __shared__ McLattice lat_s[kMcWarps];
-    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-    const int k = blockIdx.x * kMcWarps + w;
-    if (k >= nmb) return;  // whole warps only
-    McLattice& L = lat_s[w];
-    const int n = (k % cols) * 16, m = (k / cols) * 16;
-    const int v = __ldg(mv + k), mvx = vppgpu::mv_x(v), mvy = vppgpu::mv_y(v);
+    __syncwarp();
     mc_chroma_blocks(L, ru, rv, mvx, mvy, n >> 1, m >> 1, lane, ou, ov);
     short* dst = oy + (size_t)m * ry.w + n;
     if (!(mvx | mvy)) {  // a zero vector keeps the block
@@ -215,6 +206,193 @@ __global__ void __launch_bounds__(32 * kMcWarps, 12) k_mc_frame(Plane ry, Plane 
         __syncwarp();
     }
     mc_luma_quarter(L, cs, lane, dst, ry.w);
+}
+
+// The packed path's shared memory: pairs of samples, the luma window from its first column, the vertical
+// 6-tap sums + TAP_BIAS of its columns (j cases), the chroma windows from an even column (U, then V).  At 14
+// words a row, four rows apart eight words lie in the 32 banks.
+struct McPairs {
+    unsigned win[22][14];
+    unsigned vt[16][12];
+    unsigned cwin[18][6];
+};
+
+// The same terms for a lane's pair of columns (2p, 2p + 1), rows r .. r + 3, pairs of samples; p: lane & 7.
+// kind and offsets as in c_quarter_terms, the offset as dx | dy << 1.
+__constant__ int c_pair_terms[16] = {  // kind | offset << 3 of the first term, then << 8 of the second
+    kTermG | kTermNone << 8,                     kTermG | kTermB << 8,
+    kTermB | kTermNone << 8,                     kTermG | 1 << 3 | kTermB << 8,
+    kTermG | kTermH << 8,                        kTermB | kTermH << 8,
+    kTermJ | kTermB << 8,                        kTermB | (kTermH | 1 << 3) << 8,
+    kTermH | kTermNone << 8,                     kTermJ | kTermH << 8,
+    kTermJ | kTermNone << 8,                     kTermJ | (kTermH | 1 << 3) << 8,
+    kTermG | 2 << 3 | kTermH << 8,               kTermH | (kTermB | 2 << 3) << 8,
+    kTermJ | (kTermB | 2 << 3) << 8,             kTermH | 1 << 3 | (kTermB | 2 << 3) << 8,
+};
+__device__ __forceinline__ void mc_pair_term(const McPairs& L, int term, int r, int p, unsigned (&out)[4])
+{
+    const int kind = term & 7, dx = (term >> 3) & 1, dy = (term >> 4) & 1;
+    if (kind == kTermG) {
+        const unsigned* w = &L.win[r + 2 + dy][p + 1];
+#pragma unroll
+        for (int i = 0; i < 4; i++) out[i] = dx ? __funnelshift_r(w[14 * i], w[14 * i + 1], 16) : w[14 * i];
+    } else if (kind == kTermB) {
+        const unsigned* w = &L.win[r + 2 + dy][p];
+#pragma unroll
+        for (int i = 0; i < 4; i++) {
+            const unsigned a = w[14 * i], b = w[14 * i + 1], c = w[14 * i + 2], d = w[14 * i + 3];
+            out[i] = vppgpu::scale_pair(vppgpu::tap_pair(a, __funnelshift_r(a, b, 16), b, __funnelshift_r(b, c, 16), c,
+                                                         __funnelshift_r(c, d, 16)));
+        }
+    } else if (kind == kTermH) {
+        unsigned v[9];
+        const unsigned* w = &L.win[r][p + 1];
+#pragma unroll
+        for (int i = 0; i < 9; i++) v[i] = dx ? __funnelshift_r(w[14 * i], w[14 * i + 1], 16) : w[14 * i];
+#pragma unroll
+        for (int i = 0; i < 4; i++)
+            out[i] = vppgpu::scale_pair(vppgpu::tap_pair(v[i], v[i + 1], v[i + 2], v[i + 3], v[i + 4], v[i + 5]));
+    } else {
+#pragma unroll
+        for (int i = 0; i < 4; i++) {
+            const unsigned* w = &L.vt[r + i][p];
+            out[i] = vppgpu::tap_centre2(w[0], w[1], w[2], w[3]);
+        }
+    }
+}
+
+// One warp per macroblock: its 16x16 luma block and its two 8x8 chroma blocks.  What bounds it is latency and
+// instructions: a sample at a time, the chroma blocks before the luma window was asked for, a 1920x1088 frame
+// took 12.2 us (750 instructions a macroblock; its 13 MB are 2 us, a launch with nothing in it 4).  Here everything the vector points at is
+// asked for at once, in 8- and 4-byte loads, and computed on
+// pairs of samples: 10.1 us (525 instructions; 8, 12 and 14 CTAs an SM 10.5, 10.3 and 11.1).  Past the frame's edge the
+// groups of samples that a load takes are inside or outside as a whole, so it costs the same; the macroblocks there
+// by another path were the launch's tail (12.6).  The packed path takes samples of 0..255 (seen from the windows) and 16-byte aligned frames (wide); other
+// macroblocks are computed by mc_general.  Warp-synchronous: no block barrier.
+__global__ void __launch_bounds__(32 * kMcWarps, 10) k_mc_frame(const __grid_constant__ Plane ry,
+                                                               const __grid_constant__ Plane ru,
+                                                               const __grid_constant__ Plane rv,
+                                                               const int* __restrict__ mv, int cols, int nmb,
+                                                               bool wide, short* __restrict__ oy,
+                                                               short* __restrict__ ou, short* __restrict__ ov)
+{
+    __shared__ union Store {
+        McLattice general;
+        McPairs pairs;
+    } store[kMcWarps];
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    const int k = blockIdx.x * kMcWarps + w;
+    if (k >= nmb) return;  // whole warps only
+    const int mbr = k / cols, n = (k - mbr * cols) * 16, m = mbr * 16;
+    const int v = __ldg(mv + k), mvx = vppgpu::mv_x(v), mvy = vppgpu::mv_y(v);
+    if (wide && !(mvx | mvy)) {  // a zero vector keeps the blocks
+        const size_t at = (size_t)(m + (lane >> 1)) * ry.w + n + 8 * (lane & 1);
+        const uint4 y = __ldg(reinterpret_cast<const uint4*>(ry.p + at));
+        const size_t cat = (size_t)((m >> 1) + (lane & 7)) * ru.w + (n >> 1);
+        if (lane < 16) {
+            const uint4 c = __ldg(reinterpret_cast<const uint4*>((lane < 8 ? ru.p : rv.p) + cat));
+            *reinterpret_cast<uint4*>((lane < 8 ? ou : ov) + cat) = c;
+        }
+        *reinterpret_cast<uint4*>(oy + at) = y;
+        return;
+    }
+    // floor quotients and remainders: what QuarterRead's and EighthRead's folding of negative ones gives
+    const int ox = n + (mvx >> 2) - 2, oy0 = m + (mvy >> 2) - 2, cs = (mvx & 3) | (mvy & 3) << 2;
+    const int cx = (n >> 1) + (mvx >> 3), cy = (m >> 1) + (mvy >> 3);
+    const bool inside = ox >= 0 && ox + 22 <= ry.w && cx >= 0 && cx + 9 <= ru.w;  // between the sides
+    if (wide) {
+        McPairs& L = store[w].pairs;
+        const int q = lane & 7, r4 = lane >> 3, dx = ox & 3;
+        const bool odd = cx & 1;
+        uint2 y[6];
+        unsigned c[5], all = 0;
+        // a group of four (two) samples of a row is inside the frame or outside it as a whole
+        const int gx = (ox & ~3) + 4 * q, gc = (cx & ~1) + 2 * q;
+        const short* py = ry.p + min(max(gx, 0), ry.w - 4);
+        const int pc = min(max(gc, 0), ru.w - 2);
+#pragma unroll
+        for (int i = 0; i < 6; i++) {
+            y[i] = make_uint2(0u, 0u);
+            if (q < (dx + 25) >> 2 && r4 + 4 * i < 22)
+                y[i] = __ldg(reinterpret_cast<const uint2*>(py + (size_t)min(max(oy0 + r4 + 4 * i, 0), ry.h - 1) * ry.w));
+        }
+#pragma unroll
+        for (int i = 0; i < 5; i++) {
+            const int r = r4 + 4 * i;
+            c[i] = 0u;
+            if (q < 5 && r < 18)
+                c[i] = __ldg(reinterpret_cast<const unsigned*>(
+                    (r < 9 ? ru.p : rv.p) + (size_t)min(max(cy + (r < 9 ? r : r - 9), 0), ru.h - 1) * ru.w + pc));
+        }
+        if (!inside) {  // the sides' samples repeated
+#pragma unroll
+            for (int i = 0; i < 6; i++) {
+                const unsigned e = gx < 0 ? __byte_perm(y[i].x, 0u, 0x1010) : __byte_perm(y[i].y, 0u, 0x3232);
+                if (gx < 0 || gx >= ry.w) y[i] = make_uint2(e, e);
+            }
+#pragma unroll
+            for (int i = 0; i < 5; i++)
+                if (gc < 0 || gc >= ru.w) c[i] = __byte_perm(c[i], 0u, gc < 0 ? 0x1010 : 0x3232);
+        }
+#pragma unroll
+        for (int i = 0; i < 6; i++) {
+            all |= y[i].x | y[i].y;
+            const unsigned n0 = __shfl_down_sync(0xffffffffu, y[i].x, 1), n1 = __shfl_down_sync(0xffffffffu, y[i].y, 1);
+            const unsigned a = dx & 2 ? y[i].y : y[i].x, b = dx & 2 ? n0 : y[i].y, d = dx & 2 ? n1 : n0;
+            const unsigned sh = 16 * (dx & 1);
+            if (q < 6 && r4 + 4 * i < 22)
+                *reinterpret_cast<uint2*>(&L.win[r4 + 4 * i][2 * q]) =
+                    make_uint2(__funnelshift_r(a, b, sh), __funnelshift_r(b, d, sh));
+        }
+#pragma unroll
+        for (int i = 0; i < 5; i++) {
+            all |= c[i];
+            if (q < 5 && r4 + 4 * i < 18) L.cwin[r4 + 4 * i][q] = c[i];
+        }
+        const bool bytes = !__any_sync(0xffffffffu, (all & 0xff00ff00u) != 0u);
+        __syncwarp();
+        if (bytes) {
+            const int term = c_pair_terms[cs], kind1 = term & 7, kind2 = (term >> 8) & 7;
+            if (kind1 == kTermJ) {  // vertical sums of the window's words, two halves of eight rows
+                if (lane < 24) {
+                    const int wd = lane < 12 ? lane : lane - 12, r0 = lane < 12 ? 0 : 8;
+                    unsigned x[13];
+#pragma unroll
+                    for (int i = 0; i < 13; i++) x[i] = L.win[r0 + i][wd];
+#pragma unroll
+                    for (int i = 0; i < 8; i++)
+                        L.vt[r0 + i][wd] = vppgpu::tap_pair(x[i], x[i + 1], x[i + 2], x[i + 3], x[i + 4], x[i + 5]);
+                }
+                __syncwarp();
+            }
+            const int r = 4 * r4;
+            unsigned o[4];
+            mc_pair_term(L, term, r, q, o);
+            if (kind2 != kTermNone) {
+                unsigned o2[4];
+                mc_pair_term(L, term >> 8, r, q, o2);
+#pragma unroll
+                for (int i = 0; i < 4; i++) o[i] = ((o[i] + o2[i] + 0x00010001u) >> 1) & 0x00ff00ffu;
+            }
+            unsigned* dst = reinterpret_cast<unsigned*>(oy + (size_t)(m + r) * ry.w + n) + q;
+#pragma unroll
+            for (int i = 0; i < 4; i++) dst[(size_t)i * (ry.w / 2)] = o[i];
+            // chroma: a pair of columns of a row per lane and plane
+            const int fx = mvx & 7, fy = mvy & 7, cr = lane >> 2, cp = lane & 3;
+            const unsigned w00 = (8 - fx) * (8 - fy), w10 = fx * (8 - fy), w01 = (8 - fx) * fy, w11 = fx * fy;
+            const size_t cat = (size_t)((m >> 1) + cr) * ru.w + (n >> 1) + 2 * cp;
+#pragma unroll
+            for (int pl = 0; pl < 2; pl++) {
+                const unsigned *p0 = &L.cwin[9 * pl + cr][cp], *p1 = p0 + 6;
+                const unsigned f0 = __funnelshift_r(p0[0], p0[1], 16), f1 = __funnelshift_r(p1[0], p1[1], 16);
+                const unsigned s = w00 * (odd ? f0 : p0[0]) + w10 * (odd ? p0[1] : f0) + w01 * (odd ? f1 : p1[0]) +
+                                   w11 * (odd ? p1[1] : f1) + 0x00200020u;
+                *reinterpret_cast<unsigned*>((pl ? ov : ou) + cat) = (s >> 6) & 0x00ff00ffu;
+            }
+            return;
+        }
+    }
+    mc_general(store[w].general, ry, ru, rv, n, m, mvx, mvy, lane, oy, ou, ov);
 }
 
 // a = clip255(a + b) or a -= b, 8 samples per thread (16-byte accesses), the tail one by one.
@@ -319,7 +497,8 @@ int vppgpu_mc_compensate_device(vppgpu_mc* mc, const short* d_ref_yuv, const sho
     if (cols * rows > 0) {
         k_mc_frame<<<(cols * rows + kMcWarps - 1) / kMcWarps, 32 * kMcWarps, 0, ctx->stream>>>(
             Plane{src, W, H}, Plane{src + ny, cw, ch}, Plane{src + ny + nc, cw, ch}, (const int*)d_mv, cols,
-            cols * rows, d_out_yuv, d_out_yuv + ny, d_out_yuv + ny + nc);
+            cols * rows, (((uintptr_t)src | (uintptr_t)d_out_yuv) & 15) == 0, d_out_yuv, d_out_yuv + ny,
+            d_out_yuv + ny + nc);
         VPP_CHECK_LAUNCH(ctx);
         ctx->launches++;
     }

@@ -78,6 +78,16 @@ __device__ __forceinline__ unsigned tap_centre4(unsigned p0, unsigned p1, unsign
     return __viaddmin_s16x2_relu(ve, 0u, 0x00ff00ffu) | __viaddmin_s16x2_relu(vo, 0u, 0x00ff00ffu) << 8;
 }
 
+// Of two columns: p1 holds them, p0 the two before, p2 and p3 the four after.
+__device__ __forceinline__ unsigned tap_centre2(unsigned p0, unsigned p1, unsigned p2, unsigned p3)
+{
+    constexpr int c0 = 512 - 32 * TAP_BIAS, ka = 0x1414fb01, kb = 0x000001fb, kc = 0x14fb0100, kd = 0x0001fb14;
+    const int q0 = (int)p0, q1 = (int)p1, q2 = (int)p2, q3 = (int)p3;
+    const int v0 = __dp2a_lo(q2, kb, __dp2a_hi(q1, ka, __dp2a_lo(q0, ka, c0)));
+    const int v1 = __dp2a_hi(q3, kd, __dp2a_lo(q2, kd, __dp2a_hi(q1, kc, __dp2a_lo(q0, kc, c0))));
+    return __viaddmin_s16x2_relu(__byte_perm((unsigned)(v0 >> 10), (unsigned)(v1 >> 10), 0x5410), 0u, 0x00ff00ffu);
+}
+
 // Sum over the warp (every lane gets it).
 __device__ __forceinline__ int warp_sum(int v) { return __reduce_add_sync(0xffffffffu, v); }
 

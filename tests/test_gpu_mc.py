@@ -92,3 +92,50 @@ def test_device_entry_and_plane_helpers(vpp, ctx, orc):
     ctx.synchronize()
     np.testing.assert_array_equal(a.cpu().numpy(), orc.add_clip255(ah, np.full(999, 37, np.int16)))
     L.vppgpu_mc_destroy(mc)
+
+
+@pytest.mark.parametrize("spread", ["bytes", "hard", "some", "all"])
+@pytest.mark.parametrize("w,h,shift", [(16, 16, 0), (48, 34, 0), (48, 34, 1), (112, 64, 4), (176, 80, 0)])
+def test_sample_ranges_and_alignments(vpp, ctx, orc, spread, w, h, shift):
+    """The packed path and the one that takes any samples, against the oracle: bytes (also only 0 and 255, where the
+    6-tap sums are largest), a few samples outside 0..255, any shorts; frames that are 16-byte aligned or not; every
+    quarter case, vectors of zero and ones that leave the picture."""
+    torch = pytest.importorskip("torch")
+    from imagecodingutils_gb300 import _lib
+    L = vpp.load()
+    ny, nc, nmb = w * h, (w // 2) * (h // 2), (w // 16) * (h // 16)
+    n = ny + 2 * nc
+    r = synth.splitmix64(800 + w + shift, n)
+    yuv = (r % np.uint64(256)).astype(np.int64)
+    if spread == "hard":
+        yuv = np.where(yuv < 128, 0, 255)
+    elif spread == "some":
+        yuv = np.where(r >> np.uint64(40) & np.uint64(511), yuv, 256 - 2 * yuv)
+    elif spread == "all":
+        yuv = (r % np.uint64(65536)).astype(np.int64) - 32768
+        yuv //= 8  # the chroma weights sum to 64: the reference's int holds it either way
+    yuv = yuv.astype(np.int16)
+    planes = yuv[:ny].reshape(h, w), yuv[ny:ny + nc].reshape(h // 2, w // 2), yuv[ny + nc:].reshape(h // 2, w // 2)
+    rg = 8
+    mc = C.c_void_p()
+    _lib.check(L.vppgpu_mc_create(ctx.handle, w, h, rg, C.byref(mc)), "create")
+    try:
+        src = torch.zeros(n + 16, dtype=torch.int16, device="cuda")
+        out = torch.zeros(n + 16, dtype=torch.int16, device="cuda")
+        src[shift:shift + n] = torch.from_numpy(yuv).cuda()
+        for seed in range(3):
+            mv = ((synth.splitmix64(900 + seed, 2 * nmb) % np.uint64(8 * rg + 1)).astype(np.int64) - 4 * rg)
+            mv = mv.astype(np.int16).reshape(nmb, 2)
+            mv[seed::5] = 0
+            mv[1::4] //= 8
+            d_mv = torch.from_numpy(mv).cuda()
+            torch.cuda.synchronize()
+            _lib.check(L.vppgpu_mc_compensate_device(mc, C.c_void_p(src.data_ptr() + 2 * shift),
+                                                     C.c_void_p(d_mv.data_ptr()),
+                                                     C.c_void_p(out.data_ptr() + 2 * shift)), "compensate")
+            ctx.synchronize()
+            got = out[shift:shift + n].cpu().numpy()
+            want = np.concatenate([np.ravel(p) for p in orc.mc_compensate(*planes, mv, rg)])
+            np.testing.assert_array_equal(got, want)
+    finally:
+        L.vppgpu_mc_destroy(mc)
