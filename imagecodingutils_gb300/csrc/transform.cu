@@ -262,6 +262,7 @@ struct RtConsts {
     int mf0, mf1, mf2, f, sh;
     int v0, v1, v2, df, right, left;
     bool small_q;  // qp < 24: rounded right shift, else left shift
+    int neg, w0, w1, w2;  // kNear: 2^sh - 1 - f, V << qp / 6
 };
 
 __device__ __forceinline__ RtConsts rt_consts(int qp, int intra)
@@ -280,11 +281,17 @@ __device__ __forceinline__ RtConsts rt_consts(int qp, int intra)
     c.right = 4 - qe;
     c.left = qe - 4;
     c.small_q = qp < 24;
+    c.neg = (1 << c.sh) - 1 - c.f;
+    c.w0 = c.v0 << qe;
+    c.w1 = c.v1 << qe;
+    c.w2 = c.v2 << qe;
     return c;
 }
 
+template <bool kNear>
 __device__ __forceinline__ int rt_quant(int x, int mf, const RtConsts& c)
 {
+    if (kNear) return (x * mf + (x < 0 ? c.neg : c.f)) >> c.sh;  // -((-x mf + f) >> sh), rounded up by the shift
     const int q = ((x < 0 ? -x : x) * mf + c.f) >> c.sh;
     return s16(x < 0 ? -q : q);
 }
@@ -292,12 +299,29 @@ __device__ __forceinline__ int rt_quant(int x, int mf, const RtConsts& c)
 // Forward transform + quantisation (mode 0) of fwd_block, then the
 // dequantisation + inverse of inv_block (mode 0, pass order kColsFirst),
 // with the constants in registers; the levels are stored in between.
-template <bool kColsFirst>
-__device__ __forceinline__ void roundtrip_block(const short* res, short* lev, short* rec, int stride,
+//
+// kNear: residuals of -257..255 (those of 8-bit samples) and weights of 16.
+// Then no forward sum or level needs its wrap to 16 bits (sums up to 36 * 257),
+// the quantiser is one multiply-add whose addend rounds negative values as
+// their magnitude (products below 2^27), and the dequantiser is a
+// multiplication by V << qp / 6.  What bound the kernel was instructions, 299
+// for a block and 61 us for sixteen 1920x1080
+// frames that move in 44; 218 with a thread's constants shared by more blocks,
+// and the next block's rows loaded meanwhile, 53.4.
+template <bool kColsFirst, bool kNear>
+__device__ __forceinline__ void roundtrip_block(const uint2 (&rows)[4], short* lev, short* rec, int stride,
                                                const RtConsts& c, const int* weight)
 {
+    auto s16 = [](int x) { return kNear ? x : (int)(short)x; };  // forward
+    auto wrap = [](int x) { return (int)(short)x; };             // inverse
     int b[16];
-    load_rows(res, stride, b);
+#pragma unroll
+    for (int r = 0; r < 4; r++) {
+        b[4 * r + 0] = (int)(short)(rows[r].x & 0xffff);
+        b[4 * r + 1] = (int)rows[r].x >> 16;
+        b[4 * r + 2] = (int)(short)(rows[r].y & 0xffff);
+        b[4 * r + 3] = (int)rows[r].y >> 16;
+    }
 #pragma unroll
     for (int r = 0; r < 4; r++) {
         int* q = b + 4 * r;
@@ -312,17 +336,21 @@ __device__ __forceinline__ void roundtrip_block(const short* res, short* lev, sh
         const int s0 = b[k] + b[12 + k], s3 = b[k] - b[12 + k], s1 = b[4 + k] + b[8 + k], s2 = b[4 + k] - b[8 + k];
         // classes: even row & even col 0, odd & odd 1, mixed 2
         const int mf_even = (k & 1) ? c.mf2 : c.mf0, mf_odd = (k & 1) ? c.mf1 : c.mf2;
-        b[k] = rt_quant(s0 + s1, mf_even, c);
-        b[4 + k] = rt_quant(s2 + (s3 << 1), mf_odd, c);
-        b[8 + k] = rt_quant(s0 - s1, mf_even, c);
-        b[12 + k] = rt_quant(s3 - (s2 << 1), mf_odd, c);
+        b[k] = rt_quant<kNear>(s0 + s1, mf_even, c);
+        b[4 + k] = rt_quant<kNear>(s2 + (s3 << 1), mf_odd, c);
+        b[8 + k] = rt_quant<kNear>(s0 - s1, mf_even, c);
+        b[12 + k] = rt_quant<kNear>(s3 - (s2 << 1), mf_odd, c);
     }
     store_rows(lev, stride, b);
 #pragma unroll
     for (int i = 0; i < 16; i++) {
         const int cls = pos_class(i);
-        const int v = b[i] * (cls == 0 ? c.v0 : (cls == 1 ? c.v1 : c.v2)) * weight[i];
-        b[i] = c.small_q ? (v + c.df) >> c.right : v << c.left;
+        if (kNear) {  // (16 x V + 2^(3 - qe)) >> (4 - qe) and 16 x V << (qe - 4) are both x V << qe
+            b[i] *= cls == 0 ? c.w0 : (cls == 1 ? c.w1 : c.w2);
+        } else {
+            const int v = b[i] * (cls == 0 ? c.v0 : (cls == 1 ? c.v1 : c.v2)) * weight[i];
+            b[i] = c.small_q ? (v + c.df) >> c.right : v << c.left;
+        }
     }
     int y0, y1, y2, y3;
     if constexpr (!kColsFirst) {
@@ -330,66 +358,85 @@ __device__ __forceinline__ void roundtrip_block(const short* res, short* lev, sh
         for (int r = 0; r < 4; r++) {
             int* q = b + 4 * r;
             inv_1d(q[0], q[1], q[2], q[3], y0, y1, y2, y3);
-            q[0] = s16(y0); q[1] = s16(y1); q[2] = s16(y2); q[3] = s16(y3);
+            q[0] = wrap(y0); q[1] = wrap(y1); q[2] = wrap(y2); q[3] = wrap(y3);
         }
 #pragma unroll
         for (int k = 0; k < 4; k++) {
             inv_1d(b[k], b[4 + k], b[8 + k], b[12 + k], y0, y1, y2, y3);
-            b[k] = s16((y0 + 32) >> 6); b[4 + k] = s16((y1 + 32) >> 6);
-            b[8 + k] = s16((y2 + 32) >> 6); b[12 + k] = s16((y3 + 32) >> 6);
+            b[k] = wrap((y0 + 32) >> 6); b[4 + k] = wrap((y1 + 32) >> 6);
+            b[8 + k] = wrap((y2 + 32) >> 6); b[12 + k] = wrap((y3 + 32) >> 6);
         }
     } else {
 #pragma unroll
         for (int k = 0; k < 4; k++) {
             inv_1d(b[k], b[4 + k], b[8 + k], b[12 + k], y0, y1, y2, y3);
-            b[k] = s16(y0); b[4 + k] = s16(y1); b[8 + k] = s16(y2); b[12 + k] = s16(y3);
+            b[k] = wrap(y0); b[4 + k] = wrap(y1); b[8 + k] = wrap(y2); b[12 + k] = wrap(y3);
         }
 #pragma unroll
         for (int r = 0; r < 4; r++) {
             int* q = b + 4 * r;
             inv_1d(q[0], q[1], q[2], q[3], y0, y1, y2, y3);
-            q[0] = s16((y0 + 32) >> 6); q[1] = s16((y1 + 32) >> 6);
-            q[2] = s16((y2 + 32) >> 6); q[3] = s16((y3 + 32) >> 6);
+            q[0] = wrap((y0 + 32) >> 6); q[1] = wrap((y1 + 32) >> 6);
+            q[2] = wrap((y2 + 32) >> 6); q[3] = wrap((y3 + 32) >> 6);
         }
     }
     store_rows(rec, stride, b);
 }
 
+struct Weights {
+    int w[16];
+    bool flat;  // all 16
+};
+
 // One plane: rows of 4x4 blocks strided over the CTAs that serve the plane,
 // the blocks of a row over the CTA's threads (8-byte row accesses, 256
 // contiguous bytes per warp and row).  No index division.
 template <bool kColsFirst>
-__device__ __forceinline__ void roundtrip_plane(const vppgpu::TqJob& j, const int* weight, int row0, int rstep)
+__device__ __forceinline__ void roundtrip_plane(const vppgpu::TqJob& j, const Weights& wt, int row0, int rstep)
 {
     const RtConsts c = rt_consts(j.qp, j.intra);
     const int bw = j.width >> 2, bh = j.height >> 2;
-    for (int by = row0; by < bh; by += rstep) {
-        const size_t row = (size_t)by * 4 * j.stride;
-        for (int bx = threadIdx.x; bx < bw; bx += blockDim.x) {
-            const size_t off = row + (size_t)bx * 4;
-            roundtrip_block<kColsFirst>(j.res + off, j.lev + off, j.rec + off, j.stride, c, weight);
+    int by = row0, bx = threadIdx.x;
+    if (bx >= bw) return;
+    auto load = [&](uint2 (&rows)[4]) {
+        const short* p = j.res + (size_t)by * 4 * j.stride + (size_t)bx * 4;
+#pragma unroll
+        for (int r = 0; r < 4; r++) rows[r] = *reinterpret_cast<const uint2*>(p + (size_t)r * j.stride);
+    };
+    uint2 rows[4], next[4];
+    if (by < bh) load(rows);
+    while (by < bh) {
+        const size_t off = (size_t)by * 4 * j.stride + (size_t)bx * 4;
+        bx += blockDim.x;
+        if (bx >= bw) {
+            bx = threadIdx.x;
+            by += rstep;
         }
+        if (by < bh) load(next);  // the next block is on its way while this one is worked on
+        // halves of -256..255, or one less where the lower half is negative
+        unsigned far = 0;
+#pragma unroll
+        for (int r = 0; r < 4; r++) far |= ((rows[r].x + 0x01000100u) | (rows[r].y + 0x01000100u)) & 0xfe00fe00u;
+        if (wt.flat && !far) roundtrip_block<kColsFirst, true>(rows, j.lev + off, j.rec + off, j.stride, c, wt.w);
+        else roundtrip_block<kColsFirst, false>(rows, j.lev + off, j.rec + off, j.stride, c, wt.w);
+#pragma unroll
+        for (int r = 0; r < 4; r++) rows[r] = next[r];
     }
 }
 
-struct Weights {
-    int w[16];
-};
-
 // blockIdx.y selects the plane; blockIdx.x strides over its rows of blocks.
-// Up to 256 CTAs per plane, so a CTA holds one or two rows of a 1080p or 4K
-// plane and the kernel's tail is one short CTA.
+// (4, 5 and 6 CTAs an SM: 55.2, 53.4 and 54.2 us.)
 template <bool kColsFirst>
-__global__ void __launch_bounds__(256, 6) k_tq_roundtrip(const vppgpu::TqJob* __restrict__ jobs, Weights wt)
+__global__ void __launch_bounds__(256, 5) k_tq_roundtrip(const vppgpu::TqJob* __restrict__ jobs, Weights wt)
 {
     const vppgpu::TqJob j = jobs[blockIdx.y];
-    roundtrip_plane<kColsFirst>(j, wt.w, blockIdx.x, gridDim.x);
+    roundtrip_plane<kColsFirst>(j, wt, blockIdx.x, gridDim.x);
 }
 
 template <bool kColsFirst>
-__global__ void __launch_bounds__(256, 6) k_tq_roundtrip_single(vppgpu::TqJob j, Weights wt)
+__global__ void __launch_bounds__(256, 5) k_tq_roundtrip_single(vppgpu::TqJob j, Weights wt)
 {
-    roundtrip_plane<kColsFirst>(j, wt.w, blockIdx.x, gridDim.x);
+    roundtrip_plane<kColsFirst>(j, wt, blockIdx.x, gridDim.x);
 }
 
 // ---- DC Hadamard transforms (Intra16x16 luma DC 4x4, chroma DC 2x2) --------
@@ -615,8 +662,16 @@ namespace vppgpu {
 int launch_tq_jobs(vppgpu_ctx* ctx, const TqJob* d_jobs, int njobs, int inv_order, const int* weight16)
 {
     Weights wt;
-    for (int i = 0; i < 16; i++) wt.w[i] = weight16 ? weight16[i] : 16;
-    const dim3 grid(256, njobs);
+    wt.flat = true;
+    for (int i = 0; i < 16; i++) {
+        wt.w[i] = weight16 ? weight16[i] : 16;
+        wt.flat &= wt.w[i] == 16;
+    }
+    // as many CTAs as are resident at once, 64 to 256 for a plane: with 64 a CTA's constants serve seven blocks a thread
+    // of a 1920x1080 plane (48 planes, 64 and 128: 53.4 and 53.5 us; 12 of 712x488: 7.3 and 7.9), with fewer planes
+    // they would leave SMs idle
+    const int fill = 5 * ctx->sm_count / (njobs > 0 ? njobs : 1);
+    const dim3 grid(fill < 64 ? 64 : (fill > 256 ? 256 : fill), njobs);
     if (inv_order == VPPGPU_INV_COLS_FIRST)
         k_tq_roundtrip<true><<<grid, 256, 0, ctx->stream>>>(d_jobs, wt);
     else
@@ -703,7 +758,11 @@ int vppgpu_tq_roundtrip_plane_device(vppgpu_ctx* ctx, const short* res, short* l
     if (rc) return rc;
     vppgpu::TqJob j{res, lev, rec, width, height, stride, qp, intra != 0};
     Weights wt;
-    for (int i = 0; i < 16; i++) wt.w[i] = weight16 ? weight16[i] : 16;
+    wt.flat = true;
+    for (int i = 0; i < 16; i++) {
+        wt.w[i] = weight16 ? weight16[i] : 16;
+        wt.flat &= wt.w[i] == 16;
+    }
     const int rows = height >> 2, g = rows < 2 * 8 * ctx->sm_count ? rows : 2 * 8 * ctx->sm_count;
     if (inv_order == VPPGPU_INV_COLS_FIRST)
         k_tq_roundtrip_single<true><<<g, 256, 0, ctx->stream>>>(j, wt);

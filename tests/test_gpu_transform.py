@@ -93,3 +93,31 @@ def test_int16_wraparound_inputs(vpp, ctx, orc):
 def test_empty_input(vpp, ctx):
     t = vpp.FastForward4x4ITImpl1(ctx)
     assert t.Transform(np.zeros(0, np.int16)).size == 0
+
+
+@pytest.mark.parametrize("order", [0, 1])
+@pytest.mark.parametrize("low,high", [(-256, 255), (-257, 255), (-258, 256), (-1, 1)])
+def test_plane_roundtrip_at_the_8_bit_range(vpp, ctx, orc, low, high, order):
+    """Residuals at and just past the range of 8-bit samples' differences, where the round trip changes between its
+    two forms from block to block, with every QP, both roundings and both pass orders: each sample one of the two
+    ends (the largest sums), or anything between them."""
+    w, h = 88, 20
+    r = synth.splitmix64(600 + high, w * h).astype(np.int64).reshape(h, w)
+    ends = np.where(r & 1, high, low)
+    res = np.where((r >> 20) & 3, ends, low + (r >> 8) % (high - low + 1)).astype(np.int16)
+    res[:4, :4] = low
+    res[:4, 4:8] = high
+    res[4:8, :4] = np.where(np.add.outer(np.arange(4), np.arange(4)) % 2, low, high)
+    blocks = res.reshape(h // 4, 4, w // 4, 4).transpose(0, 2, 1, 3).reshape(-1, 16)
+    back = lambda b: b.reshape(h // 4, w // 4, 4, 4).transpose(0, 2, 1, 3).reshape(h, w)
+    for qp in range(52):
+        lev, rec = vpp.tq_roundtrip_plane(res, qp, qp & 1, inv_order=order, ctx=ctx)
+        lev_o = orc.fwd4x4(blocks, 0, 0, qp, qp & 1)
+        if order == 0:
+            rec_o = orc.inv4x4(lev_o, 0, 0, qp)
+        else:
+            mbs = np.zeros((lev_o.shape[0], 16, 16), np.int16)
+            mbs[:, :4, :4] = lev_o.reshape(-1, 4, 4)
+            rec_o = orc.inv4x4(mbs.reshape(-1, 256), 1, 0, qp).reshape(-1, 16, 16)[:, :4, :4].reshape(-1, 16)
+        np.testing.assert_array_equal(lev, back(lev_o), err_msg=f"qp {qp}")
+        np.testing.assert_array_equal(rec, back(rec_o), err_msg=f"qp {qp}")
