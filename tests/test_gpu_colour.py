@@ -52,3 +52,54 @@ def test_extreme_colours(vpp, ctx, orc):
         want = orc.rgb_to_yuv(kind, bgr, 128, 0)
         for a, bb in zip(got, want):
             np.testing.assert_array_equal(a, bb)
+
+
+@pytest.mark.parametrize("kind", [0, 1, 2])
+def test_every_colour(vpp, ctx, orc, kind):
+    """Each of the 2^24 colours once: the luma of the real converters is formed from integers except where its exact
+    value is a whole number, and every 2x2 block has four colours (its chroma sum, likewise)."""
+    i = np.arange(1 << 24, dtype=np.uint32)
+    j = (i * np.uint32(2654435761)) & np.uint32(0xffffff) if kind == 2 else i  # an odd factor: every colour once
+    bgr = np.stack([j & 255, (j >> 8) & 255, j >> 16], -1).astype(np.uint8).reshape(4096, 4096, 3)
+    for a, b in zip(convert(vpp, ctx, kind, bgr, 128, 0), orc.rgb_to_yuv(kind, bgr, 128, 0)):
+        np.testing.assert_array_equal(a, b)
+
+
+@pytest.mark.parametrize("kind", [1, 2])
+def test_chroma_sums_on_a_whole_number(vpp, ctx, orc, kind):
+    """Blocks whose exact chroma sum is a truncation boundary (multiples of 1, of 4 shifted by 2, and 0), where the
+    double's last bits decide."""
+    vals = [(b, g, r) for b in range(0, 256, 5) for g in range(0, 256, 3) for r in range(0, 256, 3)
+            if (436 * b - 289 * g - 147 * r) % 250 == 0 or (615 * r - 515 * g - 100 * b) % 250 == 0]
+    n = len(vals) // 16 * 16
+    px = np.array(vals[:n], np.uint8).reshape(-1, 16, 3)
+    bgr = np.repeat(np.repeat(px, 2, 0), 2, 1)
+    for flip in (0, 1):
+        for a, b in zip(convert(vpp, ctx, kind, bgr, 0, flip), orc.rgb_to_yuv(kind, bgr, 0, flip)):
+            np.testing.assert_array_equal(a, b)
+
+
+@pytest.mark.parametrize("kind", [0, 1, 2])
+@pytest.mark.parametrize("w,h,off,yoff", [(8, 2, 0, 0), (10, 4, 0, 0), (10, 4, 1, 2), (22, 6, 3, 0), (24, 4, 2, 2),
+                                          (24, 4, 8, 8), (14, 2, 0, 1), (6, 4, 0, 0), (64, 4, 4, 0)])
+def test_widths_and_alignments(vpp, ctx, orc, kind, w, h, off, yoff):
+    """Frames on the device at any byte, planes at any sample: the wide, the narrow and the sample-by-sample path."""
+    import ctypes as C
+    torch = pytest.importorskip("torch")
+    from imagecodingutils_gb300 import _lib
+    L = vpp.load()
+    nf, n = 3, w * h
+    bgr = np.stack([synth.rgb_frame(7 * w + f + kind, w, h) for f in range(nf)])
+    src = torch.zeros(nf * n * 3 + 16, dtype=torch.uint8, device="cuda")
+    src[off:off + nf * n * 3] = torch.from_numpy(bgr.reshape(-1)).cuda()
+    out = [torch.full((nf * m + 16,), 77, dtype=torch.int16, device="cuda") for m in (n, n // 4, n // 4)]
+    torch.cuda.synchronize()
+    _lib.check(L.vppgpu_rgb24_to_yuv420_frames_device(ctx.handle, kind, C.c_void_p(src.data_ptr() + off), nf, w, h, 128,
+                                                      0, *[C.c_void_p(t.data_ptr() + 2 * yoff) for t in out]), "convert")
+    ctx.synchronize()
+    for f in range(nf):
+        for t, want in zip(out, orc.rgb_to_yuv(kind, bgr[f], 128, 0)):
+            m = want.size
+            np.testing.assert_array_equal(t[yoff + f * m:yoff + (f + 1) * m].cpu().numpy(), want.reshape(-1))
+    for t, m in zip(out, (n, n // 4, n // 4)):
+        assert (t[:yoff] == 77).all() and (t[yoff + nf * m:] == 77).all()
