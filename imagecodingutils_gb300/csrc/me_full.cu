@@ -645,8 +645,11 @@ struct TieSmem {
     alignas(16) unsigned char win[WROWS * scan_pitch(1)];
 };
 
+// The SSD table is made by more warps than have a run: a handful of macroblocks met a tie, so what counts is how
+// long one takes (1920x1080, 17 of them, profiled: 22 us with 8 warps, 18 with 32).
+constexpr int TIE_WARPS_SSD = 32;
 template <bool kSad>
-__global__ void __launch_bounds__(TIE_RUNS * 32) k_full_tietree(const __grid_constant__ FullArgs a)
+__global__ void __launch_bounds__(kSad ? TIE_RUNS * 32 : TIE_WARPS_SSD * 32) k_full_tietree(const __grid_constant__ FullArgs a)
 {
     extern __shared__ __align__(16) unsigned char tie_smem[];
     TieSmem& S = *reinterpret_cast<TieSmem*>(tie_smem);
@@ -666,33 +669,34 @@ __global__ void __launch_bounds__(TIE_RUNS * 32) k_full_tietree(const __grid_con
             const uint4 tm = template_row(a, n, m, lane);
             stage_window<1>(a, n, m, 1, S.win, tid, blockDim.x);
             __syncthreads();
-            for (int ii = p; ii < 2 * RMAX + 1; ii += TIE_RUNS)
-                for (int g = 0; g < TAB / 8; g++) {
-                    const int v = group_ssd<scan_pitch(1)>(S.win, tm, ii, g, lane);
-                    if (lane < 8) S.tab[ii][8 * g + lane] = v;
-                }
+            for (int i = p; i < (2 * RMAX + 1) * (TAB / 8); i += TIE_WARPS_SSD) {
+                const int ii = i / (TAB / 8), g = i % (TAB / 8), v = group_ssd<scan_pitch(1)>(S.win, tm, ii, g, lane);
+                if (lane < 8) S.tab[ii][8 * g + lane] = v;
+            }
             __syncthreads();
-            table_row_minima(S.tab, xl, xr, yu, yd, p, TIE_RUNS, lane);
+            table_row_minima(S.tab, xl, xr, yu, yd, p, TIE_WARPS_SSD, lane);
         }
         __syncthreads();
         const int4 sp = a.spec4[k];
         const int imv = a.spec_imv[k];
-        int rmx, rmy, rmin, rt, nev, ev[TIE_DEPTH] = {0, 0, 0};
-        scan_table_t<true>(SmemTab{S.tab}, xl, xr, yu, yd, 0, 0, p, lane, &rmx, &rmy, &rmin, &rt, &nev, ev);
-        int rq = sp.x, rqmin = sp.y;
-        if (rmx != mv_x(imv) || rmy != mv_y(imv)) {
-            int sx = 0, sy = 0;
-            if (!kSad) subpel_refine_planes(a, n + rmx, m + rmy, load_cur8(a, n, m, lane), lane, &rmin, &sx, &sy);
-            rq = pack_mv(4 * rmx + sx, 4 * rmy + sy);
-            rqmin = rmin;
-        }
-        if (lane == 0) {
-            S.run[p][0] = ev[0];
-            S.run[p][1] = ev[1];
-            S.run[p][2] = ev[2];
-            S.run[p][3] = nev;
-            S.run[p][4] = rq;
-            S.run[p][5] = rqmin;
+        if (kSad || p < TIE_RUNS) {
+            int rmx, rmy, rmin, rt, nev, ev[TIE_DEPTH] = {0, 0, 0};
+            scan_table_t<true>(SmemTab{S.tab}, xl, xr, yu, yd, 0, 0, p, lane, &rmx, &rmy, &rmin, &rt, &nev, ev);
+            int rq = sp.x, rqmin = sp.y;
+            if (rmx != mv_x(imv) || rmy != mv_y(imv)) {
+                int sx = 0, sy = 0;
+                if (!kSad) subpel_refine_planes(a, n + rmx, m + rmy, load_cur8(a, n, m, lane), lane, &rmin, &sx, &sy);
+                rq = pack_mv(4 * rmx + sx, 4 * rmy + sy);
+                rqmin = rmin;
+            }
+            if (lane == 0) {
+                S.run[p][0] = ev[0];
+                S.run[p][1] = ev[1];
+                S.run[p][2] = ev[2];
+                S.run[p][3] = nev;
+                S.run[p][4] = rq;
+                S.run[p][5] = rqmin;
+            }
         }
         __syncthreads();
         constexpr int RW = sizeof(TieRun) / sizeof(int);
@@ -808,7 +812,7 @@ int full_launch(vppgpu_ctx* ctx, const FullArgs& args, int nmb, cudaEvent_t* ev)
     if (ev) VPP_CUDA(cudaEventRecord(ev[2], ctx->stream));
     k_full_scan<<<(args.cols + SCAN_WARPS - 1) / SCAN_WARPS * (nmb / args.cols), 32 * SCAN_WARPS, 0, ctx->stream>>>(args);
     VPP_CHECK_LAUNCH(ctx);
-    k_full_tietree<false><<<ctx->sm_count, TIE_RUNS * 32, sizeof(TieSmem), ctx->stream>>>(args);
+    k_full_tietree<false><<<min(ctx->sm_count, (nmb + 15) / 16), TIE_WARPS_SSD * 32, sizeof(TieSmem), ctx->stream>>>(args);
     VPP_CHECK_LAUNCH(ctx);
     if (ev) VPP_CUDA(cudaEventRecord(ev[3], ctx->stream));
     if ((rc = full_resolve_launch(ctx, args, 0))) return rc;
