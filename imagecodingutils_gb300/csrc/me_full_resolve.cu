@@ -138,7 +138,7 @@ __device__ __noinline__ void pred_search_at(const FullArgs& a, int k, int px, in
         int tv, td;
         if (mrc::tie_tree_result(cross::EST_CROSS, static_cast<const mrc::V2TieRun*>(a.tie_runs) +
                                                        (size_t)k * mrc::V2_TIE_RUNS,
-                                 px, py, &tv, &td)) {
+                                 px, py, lane, &tv, &td)) {
             *mvx = mv_x(tv);
             *mvy = mv_y(tv);
             *minD = td;
@@ -171,7 +171,7 @@ __device__ __noinline__ void pred_search_at(const FullArgs& a, int k, int px, in
     // their exact prediction
     if (kEst != mrc::EST_V2_LAMBDA &&
         mrc::tie_tree_result(kEst, static_cast<const mrc::V2TieRun*>(a.tie_runs) + (size_t)k * mrc::V2_TIE_RUNS, px,
-                             py, &tv, &td)) {
+                             py, lane, &tv, &td)) {
         *mvx = mv_x(tv);
         *mvy = mv_y(tv);
         *minD = td;
@@ -1042,7 +1042,7 @@ __global__ void k_full_average(FullArgs a)
 //
 //   k_resolve_first   every MB at the median of the searched vectors
 //   k_resolve_sweep   every MB whose prediction moved, over the whole GPU
-//   k_resolve_finish  the rest, by one CTA
+//   k_resolve_finish  the rest, by one cluster
 //
 // k_resolve_finish keeps the frame's vectors in the shared memory of a cluster,
 // a band of rows per CTA with the last row of the band above beside it, and

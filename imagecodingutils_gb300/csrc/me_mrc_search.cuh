@@ -1049,27 +1049,29 @@ __device__ __forceinline__ MbSearch search_run(const MrcArgs& a, Lattice& LT, in
     return r;
 }
 
-// The searched vector and distortion of a tie MB for prediction (px, py)
-// from its tie tree; false when the tree is too deep.
-__device__ __forceinline__ bool tie_tree_result(int est, const V2TieRun* runs, int ppx, int ppy, int* mv, int* min_d)
+// The searched vector and distortion of a tie MB for prediction (px, py) from its tie tree; false when the
+// tree is too deep.  One warp: half a run per lane, loaded at once (walked run by run, a tree of one tie
+// was four round trips to L2, a microsecond of every evaluation).
+__device__ __forceinline__ bool tie_tree_result(int est, const V2TieRun* runs, int ppx, int ppy, int lane, int* mv,
+                                                int* min_d)
 {
+    static_assert(sizeof(V2TieRun) == 32 && V2_TIE_RUNS == 8, "two 16-byte words per run, half a warp of them");
+    // even: {geo[0], geo[1], geo[2], lvl}, odd: {nev, mv, min_d, -}
+    const int4 v = __ldcg(reinterpret_cast<const int4*>(runs) + (lane & 15));
     int run = 0;
     for (int t = 0; t < V2_TIE_BITS; t++) {
-        const V2TieRun& r = runs[run];
-        const int nev = __ldcg(&r.nev);
-        if (t >= nev) break;
-        const int g = __ldcg(&r.geo[t]), lvl = (__ldcg(&r.lvl) >> (2 * t)) & 3;
+        if (t >= __shfl_sync(0xffffffffu, v.x, 2 * run + 1)) break;
+        const int g = __shfl_sync(0xffffffffu, t == 0 ? v.x : (t == 1 ? v.y : v.z), 2 * run);
+        const int lvl = (__shfl_sync(0xffffffffu, v.w, 2 * run) >> (2 * t)) & 3;
         const int cx = (signed char)(g & 0xff), cy = (signed char)((g >> 8) & 0xff);
         const int nx = (signed char)((g >> 16) & 0xff), ny = (signed char)(g >> 24);
         const int px = level_pred(est, ppx, lvl), py = level_pred(est, ppy, lvl);
         const bool skip = (cy - py) * (cy - py) + (cx - px) * (cx - px) < (ny - py) * (ny - py) + (nx - px) * (nx - px);
         run |= (skip ? 0 : 1) << t;
     }
-    const V2TieRun& r = runs[run];
-    if (__ldcg(&r.nev) > V2_TIE_BITS) return false;
-    *mv = __ldcg(&r.mv);
-    *min_d = __ldcg(&r.min_d);
-    return true;
+    *mv = __shfl_sync(0xffffffffu, v.y, 2 * run + 1);
+    *min_d = __shfl_sync(0xffffffffu, v.z, 2 * run + 1);
+    return __shfl_sync(0xffffffffu, v.x, 2 * run + 1) <= V2_TIE_BITS;
 }
 
 }  // namespace
