@@ -148,8 +148,8 @@ def peaks():
 
 
 def profile_traffic():
-    """DRAM bytes per k_full_search launch from the committed ncu summary."""
-    path = os.path.join(ROOT, "profiles", "k_full_search_1080p.json")
+    """DRAM bytes per k_ssd_rowmin launch from the committed ncu summary."""
+    path = os.path.join(ROOT, "profiles", "k_ssd_rowmin_1080p.json")
     if os.path.exists(path):
         return json.load(open(path)).get("dram_bytes_per_launch")
     return None
@@ -919,12 +919,11 @@ def main():
     e2e_value = whole_job_rate(NMB * args.steps, world, e2e_ms)
 
     if rank == 0:
-        dp4a = C.c_double()
-        _lib.check(L.vppgpu_calibrate_dp4a(ctx.handle, C.byref(dp4a)), "vppgpu_calibrate_dp4a")
+        pk, pk_kind = peaks()
         px_ops = algorithmic_px_ops(subpel=False)
-        table_s = stage[1] * 1e-3 / max(n.value, 1)
-        achieved = px_ops / table_s / 1e12            # Tpx/s (one squared-difference term per pixel)
-        peak = 4.0 * dp4a.value / 1e12                # 4 byte products per dp4a
+        search_s = stage[1] * 1e-3 / max(n.value, 1)
+        achieved = 2.0 * px_ops / search_s / 1e12     # TFLOP/s (the product sum of a squared difference: 2 per pixel)
+        peak = pk.get("bf16_tflops")                  # the f16 tensor rate is the bf16 one
         cpu = None
         if not args.no_cpu:
             nth = os.cpu_count() or 1
@@ -956,7 +955,6 @@ def main():
                                    not args.no_cpu, kind="impl2")
         h263v2 = run_multires_cross(args, torch, vpp, _lib, L, ctx, stream, f"cuda:{local}", frames,
                                     not args.no_cpu, kind="h263_multires_cross_v2")
-        pk, pk_kind = peaks()
         hbm_rows = run_hbm_paths(torch, _lib, L, ctx, stream, f"cuda:{local}", pk)
         line = {
             "metric": METRIC, "value": value, "unit": UNIT, "n_gpus": world, "steps": args.steps,
@@ -965,9 +963,9 @@ def main():
             "config": headline_config(world),
             "e2e": {"value": e2e_value, "unit": UNIT, "h2d_bytes_per_step": 2 * W * H * 2,
                     "d2h_bytes_per_step": NMB * 4 + 32},
-            "roofline": {"bound": "int-alu", "kernel": "k_full_search", "achieved": achieved, "peak": peak,
-                         "unit": "Tpx/s", "frac": achieved / peak, "traffic": profile_traffic(),
-                         "peak_source": "measured dp4a rate x 4 px (vppgpu_calibrate_dp4a, this run)",
+            "roofline": {"bound": "tensor", "kernel": "k_ssd_rowmin", "achieved": achieved, "peak": peak,
+                         "unit": "TFLOP/s", "frac": achieved / peak, "traffic": profile_traffic(),
+                         "peak_source": f"cuBLAS bf16 burst, {pk_kind}",
                          "algorithmic_px_per_launch": px_ops},
             "kernel_ms_per_frame": {k: stage[i] / max(n.value, 1)
                                     for i, k in enumerate(STAGES)},

@@ -263,12 +263,13 @@ __device__ __forceinline__ void mc_pair_term(const McPairs& L, int term, int r, 
 
 // One warp per macroblock: its 16x16 luma block and its two 8x8 chroma blocks.  What bounds it is latency and
 // instructions: a sample at a time, the chroma blocks before the luma window was asked for, a 1920x1088 frame
-// took 12.2 us (750 instructions a macroblock; its 13 MB are 2 us, a launch with nothing in it 4).  Here everything the vector points at is
-// asked for at once, in 8- and 4-byte loads, and computed on
-// pairs of samples: 10.1 us (525 instructions; 8, 12 and 14 CTAs an SM 10.5, 10.3 and 11.1).  Past the frame's edge the
-// groups of samples that a load takes are inside or outside as a whole, so it costs the same; the macroblocks there
-// by another path were the launch's tail (12.6).  The packed path takes samples of 0..255 (seen from the windows) and 16-byte aligned frames (wide); other
-// macroblocks are computed by mc_general.  Warp-synchronous: no block barrier.
+// took 12.2 us (750 instructions a macroblock; its 13 MB are 2 us, a launch with nothing in it 4).  Here
+// everything the vector points at is asked for at once, in 8- and 4-byte loads, and computed on pairs of
+// samples: 10.1 us (525 instructions; 8, 12 and 14 CTAs an SM 10.5, 10.3 and 11.1).  Past the frame's edge the
+// groups of samples that a load takes are inside or outside as a whole, so it costs the same; the macroblocks
+// there by another path were the launch's tail (12.6).  The packed path takes samples of 0..255 (seen from the
+// windows) and 16-byte aligned frames (wide); other macroblocks are computed by mc_general.  Warp-synchronous:
+// no block barrier.
 __global__ void __launch_bounds__(32 * kMcWarps, 10) k_mc_frame(const __grid_constant__ Plane ry,
                                                                const __grid_constant__ Plane ru,
                                                                const __grid_constant__ Plane rv,

@@ -98,7 +98,7 @@ struct FullArgs {
                                // (evaluated there; final_mv / final_dist hold the result)
     double lambda;
     int sweep_limit;
-    int relax_sweeps;          // relaxation sweeps before the wavefront (0..RELAX_SWEEPS)
+    int relax_sweeps;          // relaxation sweeps counted as such, est 4: before the wavefront (0..RELAX_SWEEPS)
     int grid_sweeps;           // ... of which over every MB (the rest visit the dirty sets)
     int relax_blocks_per_sm;   // grid of a sweep over every MB
     long long spin_limit;
@@ -235,8 +235,10 @@ int full_planes_launch(vppgpu_ctx* ctx, const FullArgs& args);
 // (me_full_tc.cu); prepare once per device.
 int rowmin_launch(vppgpu_ctx* ctx, const FullArgs& args);
 int rowmin_prepare();
-// Launch the prediction-dependent tail (sweep 0, relaxation, dictionary
-// precompute, exact wavefront) of an estimate whose search has run.
+// Launch the prediction-dependent tail of an estimate whose search has run: a
+// first evaluation of every MB, sweeps over the whole GPU, the relaxation to
+// the fixed point by one cluster (est 4: sweeps over records, then the exact
+// wavefront).
 // est: 0 MotionEstimatorH264ImplFull, 1 MotionEstimatorH264ImplMultiresCrossVer2,
 // 2 MotionEstimatorH264ImplMultires, 3 MotionEstimatorH264ImplCross, 4 Ver2's
 // Lagrangian overload.

@@ -200,10 +200,13 @@ int vppgpu_me_last_status(vppgpu_me* me);
 /* Number of resolve sweeps the last estimate needed (predictor fixed point). */
 int vppgpu_me_last_sweeps(vppgpu_me* me, int* sweeps);
 
-/* Estimators with a predictor, no vpp counterpart: at most this many
- * relaxation sweeps (0..14, UMHS 0..24; defaults 14 Full and Multires, 4 Ver2, 20 UMHS; fewer when
- * the changes stop falling fast) run before the exact wavefront decides the
- * macroblocks whose predictions have not settled.  Results do not depend on it. */
+/* Estimators with a predictor, no vpp counterpart: relaxation sweeps (0..14,
+ * UMHS 0..24; defaults 14 Full, Multires and Cross, 4 Ver2, 20 UMHS).  For UMHS,
+ * FHS, H.263 Ver2 and Ver2's Lagrangian overload at most this many run before
+ * an exact pass decides the macroblocks whose predictions have not settled; the
+ * others relax to the fixed point in any case, and rounds beyond this many
+ * count as the exact pass in vppgpu_me_last_sweeps and vppgpu_me_last_stats.
+ * Results do not depend on it. */
 int vppgpu_me_set_relax_sweeps(vppgpu_me* me, int sweeps);
 
 /* Autotuning, no vpp counterpart: times the estimator's tunable launch shapes
@@ -222,10 +225,10 @@ int vppgpu_me_autotune_pairs(vppgpu_me* me, const short* const* d_src, const sho
 int vppgpu_me_autotune_host(vppgpu_me* me, const short* src, const short* ref, int reps, int* chosen);
 int vppgpu_me_get_tuning(vppgpu_me* me, int* tuning4);
 
-/* Counters of the last estimate's prediction-dependent stage: {sweeps,
- * converged-by-relaxation, relaxation evaluations, of which distortion
- * computations (UMHS / FHS: searches in the relaxation), MBs the wavefront
- * evaluated in full, status bits, included MBs, a kind-specific count (Full:
+/* Counters of the last estimate's prediction-dependent stage: {sweeps
+ * (1000 + the limit when they did not suffice), converged within the limit,
+ * relaxation evaluations, of which distortion computations (UMHS / FHS: searches
+ * in the relaxation), MBs evaluated past the limit or by the exact pass, status bits, included MBs, a kind-specific count (Full:
  * macroblocks whose scan met a tie; FHS: quarter-pel passes over samples the
  * reference would take from earlier macroblocks)}.  Synchronises the context
  * stream.  No vpp counterpart. */
@@ -237,10 +240,11 @@ int vppgpu_me_last_stats(vppgpu_me* me, int* stats8);
 int vppgpu_me_last_relax_changes(vppgpu_me* me, int* changes, int n);
 
 /* Observability, no vpp counterpart.  While enabled, every estimate records
- * CUDA events around its three kernels on the context stream (no host
+ * CUDA events around its stages on the context stream (no host
  * synchronisation); vppgpu_me_timing synchronises and returns how many
- * estimates were timed and the summed milliseconds of the pack, search and
- * resolve kernels.  Enabling resets the sums. */
+ * estimates were timed and the summed milliseconds of the planes, the search
+ * (Full: the candidates' minima, the scan, the sub-pel refinement and the tie
+ * trees) and the resolve.  Enabling resets the sums. */
 int vppgpu_me_set_timing(vppgpu_me* me, int enable);
 int vppgpu_me_timing(vppgpu_me* me, int* n, double* pack_ms, double* search_ms, double* resolve_ms);
 /* The same sums split by stage: {pack + half-pel planes, SSD table, scan +
