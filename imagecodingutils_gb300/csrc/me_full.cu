@@ -821,7 +821,7 @@ int full_launch(vppgpu_ctx* ctx, const FullArgs& args, int nmb, cudaEvent_t* ev)
 }
 
 // The integer-pel SAD stage (FullArgs::intpel): planes, the SAD search (table,
-// scan at prediction (0, 0), no sub-pel), tie trees, then the tie wavefront.
+// scan at prediction (0, 0), no sub-pel), tie trees, then the resolve.
 int sad_launch(vppgpu_ctx* ctx, const FullArgs& args, const SearchMaps& maps, int nmb)
 {
     int rc = full_planes_launch(ctx, args);

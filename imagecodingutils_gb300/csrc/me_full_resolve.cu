@@ -220,6 +220,10 @@ struct LatticeSlots<0> {
     __device__ static mrc::Lattice* get(int) { return nullptr; }
 };
 template <>
+struct LatticeSlots<6> {  // the SAD stage
+    __device__ static mrc::Lattice* get(int) { return nullptr; }
+};
+template <>
 struct LatticeSlots<cross::EST_CROSS> {
     __device__ static mrc::Lattice* get(int) { return nullptr; }
 };
@@ -1085,6 +1089,21 @@ __device__ __forceinline__ void load_row16(const unsigned char* p, unsigned* w)
     w[3] = __funnelshift_r(v3, v4, sh);
 }
 
+// The integer-pel SAD stage, resolved by the same kernels: its vector and distortion depend on the prediction
+// only where the scan met a tie (MotionEstimatorH264ImplFull.cpp:424-441), and then only on the rounded one.
+// (1920x1080: a frame 0.419 ms with a CTA that walked the anti-diagonals, a block barrier for each with ties,
+// 0.234 so; 176x144: 39.7 us, 38.3.)
+constexpr int EST_SAD = 6;
+// Whether a result at prediction pu may differ from that at `key`; flags: the MB's record.
+template <int kEst>
+__device__ __forceinline__ bool stale(int key, int pu, int flags)
+{
+    if constexpr (kEst == EST_SAD)
+        return (flags & FLAG_TIE) && (round_pred(mv_x(key)) != round_pred(mv_x(pu)) ||
+                                      round_pred(mv_y(key)) != round_pred(mv_y(pu)));
+    return key != pu;
+}
+
 // One MB per half warp (16 lanes, a row of 16 samples each): the final vector
 // and distortion of MB k (origin n, m) at prediction `key`, from its searched
 // result `sp` and this lane's row of the input.  Lanes of a half without work
@@ -1105,37 +1124,42 @@ __device__ __forceinline__ int2 evaluate_half(const FullArgs& a, bool act, int k
         }
         return out;
     }
-    const PredGeom g = pred_geom(n, m, a.W, a.H, px, py);
-    // qpel_block8's sixteen cases by bit fields: the plane (0 full pel, 1 b, 2 h, 3 j) and the column and
-    // row offset of both averaged samples; the cases of one sample average it with itself
-    const int s = g.fx | (g.fy << 2);
-    constexpr unsigned kP1 = 0u | 0u << 2 | 1u << 4 | 0u << 6 | 0u << 8 | 1u << 10 | 3u << 12 | 1u << 14 | 2u << 16 |
-                             3u << 18 | 3u << 20 | 3u << 22 | 0u << 24 | 2u << 26 | 3u << 28 | 2u << 30;
-    constexpr unsigned kP2 = 0u | 1u << 2 | 1u << 4 | 1u << 6 | 2u << 8 | 2u << 10 | 1u << 12 | 2u << 14 | 2u << 16 |
-                             2u << 18 | 3u << 20 | 2u << 22 | 2u << 24 | 1u << 26 | 1u << 28 | 1u << 30;
-    constexpr unsigned kX1 = 1u << 3 | 1u << 15, kX2 = 1u << 7 | 1u << 11;
-    constexpr unsigned kY1 = 1u << 12, kY2 = 1u << 13 | 1u << 14 | 1u << 15;
-    const int p1 = (kP1 >> (2 * s)) & 3, p2 = (kP2 >> (2 * s)) & 3;
-    const int at = (g.oy + (lane & 15) + PAD) * a.rstride + g.ox + PAD;
-    const unsigned char* b1 = p1 ? a.hpel + (size_t)(p1 - 1) * a.plane_size : a.refp;
-    const unsigned char* b2 = p2 ? a.hpel + (size_t)(p2 - 1) * a.plane_size : a.refp;
-    b1 += at + (int)((kX1 >> s) & 1) + ((kY1 >> s) & 1 ? a.rstride : 0);
-    b2 += at + (int)((kX2 >> s) & 1) + ((kY2 >> s) & 1 ? a.rstride : 0);
-    unsigned w1[4], w2[4];
-    load_row16(b1, w1);
-    load_row16(b2, w2);
-    const unsigned c4[4] = {cur.x, cur.y, cur.z, cur.w};
-    unsigned acc = 0;
+    PredGeom g{};
+    int pd = 0;
+    if constexpr (kEst != EST_SAD) {
+        g = pred_geom(n, m, a.W, a.H, px, py);
+        // qpel_block8's sixteen cases by bit fields: the plane (0 full pel, 1 b, 2 h, 3 j) and the column and
+        // row offset of both averaged samples; the cases of one sample average it with itself
+        const int s = g.fx | (g.fy << 2);
+        constexpr unsigned kP1 = 0u | 0u << 2 | 1u << 4 | 0u << 6 | 0u << 8 | 1u << 10 | 3u << 12 | 1u << 14 | 2u << 16 |
+                                 3u << 18 | 3u << 20 | 3u << 22 | 0u << 24 | 2u << 26 | 3u << 28 | 2u << 30;
+        constexpr unsigned kP2 = 0u | 1u << 2 | 1u << 4 | 1u << 6 | 2u << 8 | 2u << 10 | 1u << 12 | 2u << 14 | 2u << 16 |
+                                 2u << 18 | 3u << 20 | 2u << 22 | 2u << 24 | 1u << 26 | 1u << 28 | 1u << 30;
+        constexpr unsigned kX1 = 1u << 3 | 1u << 15, kX2 = 1u << 7 | 1u << 11;
+        constexpr unsigned kY1 = 1u << 12, kY2 = 1u << 13 | 1u << 14 | 1u << 15;
+        const int p1 = (kP1 >> (2 * s)) & 3, p2 = (kP2 >> (2 * s)) & 3;
+        const int at = (g.oy + (lane & 15) + PAD) * a.rstride + g.ox + PAD;
+        const unsigned char* b1 = p1 ? a.hpel + (size_t)(p1 - 1) * a.plane_size : a.refp;
+        const unsigned char* b2 = p2 ? a.hpel + (size_t)(p2 - 1) * a.plane_size : a.refp;
+        b1 += at + (int)((kX1 >> s) & 1) + ((kY1 >> s) & 1 ? a.rstride : 0);
+        b2 += at + (int)((kX2 >> s) & 1) + ((kY2 >> s) & 1 ? a.rstride : 0);
+        unsigned w1[4], w2[4];
+        load_row16(b1, w1);
+        load_row16(b2, w2);
+        const unsigned c4[4] = {cur.x, cur.y, cur.z, cur.w};
+        unsigned acc = 0;
 #pragma unroll
-    for (int i = 0; i < 4; i++) {
-        const unsigned d = __vabsdiffu4(c4[i], __vavgu4(w1[i], w2[i]));
-        acc = __dp4a(d, d, acc);
+        for (int i = 0; i < 4; i++) {
+            const unsigned d = __vabsdiffu4(c4[i], __vavgu4(w1[i], w2[i]));
+            acc = __dp4a(d, d, acc);
+        }
+        const unsigned lo = __reduce_add_sync(0xffffffffu, lane < 16 ? acc : 0u);
+        const unsigned hi = __reduce_add_sync(0xffffffffu, lane < 16 ? 0u : acc);
+        pd = (int)(lane < 16 ? lo : hi);
     }
-    const unsigned lo = __reduce_add_sync(0xffffffffu, lane < 16 ? acc : 0u);
-    const unsigned hi = __reduce_add_sync(0xffffffffu, lane < 16 ? 0u : acc);
-    const int pd = (int)(lane < 16 ? lo : hi);
     int mvx = mv_x(sp.x), mvy = mv_y(sp.x), minD = sp.y;
-    const bool tie = act && (sp.w & FLAG_TIE) && (kEst != 0 || round_pred(px) != 0 || round_pred(py) != 0);
+    constexpr bool kScan = kEst == 0 || kEst == EST_SAD;  // ties decided at the rounded prediction (0, 0)
+    const bool tie = act && (sp.w & FLAG_TIE) && (!kScan || round_pred(px) != 0 || round_pred(py) != 0);
     const unsigned ties = __ballot_sync(0xffffffffu, tie);
     if (ties) {  // rare: the searched vector depends on the prediction; a whole warp's work
 #pragma unroll 1
@@ -1145,7 +1169,7 @@ __device__ __forceinline__ int2 evaluate_half(const FullArgs& a, bool act, int k
             const int hy = __shfl_sync(0xffffffffu, py, 16 * h), hf = __shfl_sync(0xffffffffu, sp.w, 16 * h);
             int tx = __shfl_sync(0xffffffffu, mvx, 16 * h), ty = __shfl_sync(0xffffffffu, mvy, 16 * h);
             int td = __shfl_sync(0xffffffffu, minD, 16 * h);
-            if constexpr (kEst == 0) tie_path(a, hk, hx, hy, hf, lane, &tx, &ty, &td);
+            if constexpr (kScan) tie_path(a, hk, hx, hy, hf, lane, &tx, &ty, &td);
             else pred_search_at<kEst>(a, hk, hx, hy, lane, &tx, &ty, &td, lt);
             if ((lane >> 4) == h) {
                 mvx = tx;
@@ -1154,6 +1178,7 @@ __device__ __forceinline__ int2 evaluate_half(const FullArgs& a, bool act, int k
             }
         }
     }
+    if constexpr (kEst == EST_SAD) return make_int2(pack_mv(mvx, mvy), minD);  // no GetBestVector
     const int pos = best_of3_fast(mvx, mvy, minD, g.pcx, g.pcy, pd, sp.z, a.lambda, g.pcx, g.pcy);
     return pos == 0 ? make_int2(pack_mv(mvx, mvy), minD) : pos == 1 ? make_int2(pack_mv(g.pcx, g.pcy), pd)
                                                                     : make_int2(0, sp.z);
@@ -1215,7 +1240,7 @@ __global__ void __launch_bounds__(256) k_resolve_sweep(const __grid_constant__ F
         if (k < a.nmb) {
             const int r = k / a.cols;
             key = median_global(a, k, r, k - r * a.cols, &sp);
-            moved = __ldcg(a.pred_used + k) != key;
+            moved = stale<kEst>(key, __ldcg(a.pred_used + k), sp.w);
         }
         unsigned todo = __ballot_sync(0xffffffffu, moved);
         while (todo) {
@@ -1289,7 +1314,7 @@ FinishShape finish_shape(int cols, int rows)
 
 template <int kEst>
 __global__ void __launch_bounds__(kFinishThreads, 1)
-    k_resolve_finish(const __grid_constant__ FullArgs a, int first, int band, int keep_dist)
+    k_resolve_finish(const __grid_constant__ FullArgs a, int first, int band, int keep_dist, int fresh)
 {
     extern __shared__ __align__(16) int fin_smem[];
     __shared__ int s_n[2], s_any[3], s_evals[2], s_changed[RELAX_SWEEPS + 1];
@@ -1330,6 +1355,14 @@ __global__ void __launch_bounds__(kFinishThreads, 1)
         for (int c = tid; c < cols; c += kFinishThreads) s_fin[c] = __ldcg(a.final_mv + k0 - cols + c);
 #pragma unroll 2
     for (int i = tid; i < nloc; i += kFinishThreads) {
+        if (kEst == EST_SAD && fresh) {  // the searched results are those at prediction (0, 0)
+            const int4 sp = __ldcg(a.spec4 + k0 + i);
+            s_fin[cols + i] = sp.x;
+            s_pu[i] = 0;
+            s_av[i] = (unsigned char)sp.w;
+            s_dist[i] = sp.y;
+            continue;
+        }
         s_fin[cols + i] = __ldcg(a.final_mv + k0 + i);
         s_pu[i] = __ldcg(a.pred_used + k0 + i);
         s_av[i] = (unsigned char)__ldcg(&a.spec4[k0 + i].w);
@@ -1355,7 +1388,7 @@ __global__ void __launch_bounds__(kFinishThreads, 1)
 #pragma unroll
                 for (int b = 0; b < 4; b++) {
                     const int i = q + b * quads;
-                    if (((m >> (8 * b)) & 0xffu) && i < nloc && median_at(i) != s_pu[i])
+                    if (((m >> (8 * b)) & 0xffu) && i < nloc && stale<kEst>(median_at(i), s_pu[i], s_av[i]))
                         s_work[atomicAdd(n, 1)] = (unsigned short)i;
                 }
             }
@@ -1442,138 +1475,25 @@ __global__ void __launch_bounds__(kFinishThreads, 1)
         atomicAdd(reinterpret_cast<unsigned long long*>(&a.ctrl->total), (unsigned long long)tot);
         atomicAdd(&a.ctrl->count, cnt);
     }
-    if (tid == 0) {
+    if (kEst != EST_SAD && tid == 0) {
         if (s_evals[0]) {
             atomicAdd(&a.ctrl->relax_evals, s_evals[0]);
             atomicAdd(&a.ctrl->relax_miss, s_evals[0]);
         }
         if (s_evals[1]) atomicAdd(&a.ctrl->wave_miss, s_evals[1]);
     }
-    if (tid <= RELAX_SWEEPS && s_changed[tid]) atomicAdd(&a.changed[tid], s_changed[tid]);
+    if (kEst != EST_SAD && tid <= RELAX_SWEEPS && s_changed[tid]) atomicAdd(&a.changed[tid], s_changed[tid]);
     cluster.sync();
     if (rank == 0 && tid == 0) {
-        const int settled = round - 1;  // the last round (or sweep) with work
-        const bool relaxed = a.relax_sweeps > 0 && settled <= a.relax_sweeps;
-        a.ctrl->sweeps = relaxed ? (settled > 0 ? settled : 1) : a.relax_sweeps + 1000;
-        a.ctrl->converged = relaxed;
+        if constexpr (kEst != EST_SAD) {
+            const int settled = round - 1;  // the last round (or sweep) with work
+            const bool relaxed = a.relax_sweeps > 0 && settled <= a.relax_sweeps;
+            a.ctrl->sweeps = relaxed ? (settled > 0 ? settled : 1) : a.relax_sweeps + 1000;
+            a.ctrl->converged = relaxed;
+        }
         const long long t = (long long)__ldcg(reinterpret_cast<const unsigned long long*>(&a.ctrl->total));
         const int n = __ldcg(&a.ctrl->count);
         if (job.out_avg) *job.out_avg = n ? t / n : 0;
-    }
-}
-
-// The integer-pel SAD stage's tail.  The prediction enters only the exact-tie
-// decisions of the scan (MotionEstimatorH264ImplFull.cpp:424-441), so every
-// macroblock without a tie already holds its final vector.  One CTA walks the
-// anti-diagonals t = c + 2r: the median prediction of (r, c) reads (r, c-1),
-// (r-1, c-1), (r-1, c) and (r-1, c+1), all on earlier diagonals, so a
-// diagonal's tie macroblocks settle together (warp each: tie tree walk, or a
-// rescan of the kept table), with a block barrier between diagonals.  Then the
-// outputs and the included-distortion average (Full.cpp:581-607).
-constexpr int kSadWaveWords = 64;   // one bit per diagonal: 2048 >= cols + 2 rows - 1 at 8192 x 8192
-constexpr int kSadSmemMbs = 16384;  // final vectors kept in shared memory up to this many macroblocks
-
-size_t sad_resolve_smem(int nmb)
-{
-    const size_t words = (size_t)(nmb + 31) / 32;
-    return 4 * (words + (nmb <= kSadSmemMbs ? (size_t)nmb : 0));
-}
-
-__global__ void __launch_bounds__(1024, 1) k_sad_resolve(FullArgs a)
-{
-    extern __shared__ unsigned s_dyn[];  // tie bit per macroblock, then (local) the final vectors
-    __shared__ long long s_tot;
-    __shared__ int s_cnt;
-    __shared__ unsigned s_wave[kSadWaveWords];  // diagonals holding a tie macroblock
-    const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5, nw = blockDim.x >> 5;
-    const int cols = a.cols, rows = a.nmb / cols, words = (a.nmb + 31) >> 5;
-    const int ntie = *((volatile int*)&a.ctrl->ntie);
-    const int waves = cols + 2 * (rows - 1);
-    const bool every = waves > 32 * kSadWaveWords;
-    const bool local = a.nmb <= kSadSmemMbs;
-    unsigned* s_tie = s_dyn;
-    int* s_fin = reinterpret_cast<int*>(s_dyn + words);
-    if (threadIdx.x == 0) {
-        s_tot = 0;
-        s_cnt = 0;
-    }
-    for (int i = threadIdx.x; i < kSadWaveWords; i += blockDim.x) s_wave[i] = 0u;
-    for (int i = threadIdx.x; i < words; i += blockDim.x) s_tie[i] = 0u;
-    if (local)
-        for (int k = threadIdx.x; k < a.nmb; k += blockDim.x) s_fin[k] = __ldcg(a.final_mv + k);
-    __syncthreads();
-    for (int i = threadIdx.x; i < ntie; i += blockDim.x) {
-        const int k = a.tie_list[i], r = k / cols, t = k - r * cols + 2 * r;
-        atomicOr(&s_tie[k >> 5], 1u << (k & 31));
-        if (!every) atomicOr(&s_wave[t >> 5], 1u << (t & 31));
-    }
-    __syncthreads();
-    if (ntie > 0) {
-        constexpr int TW = TIE_RUNS * (int)(sizeof(TieRun) / sizeof(int));
-        for (int t = 0; t < waves; t++) {
-            if (!every && !((s_wave[t >> 5] >> (t & 31)) & 1u)) continue;  // block-uniform: no tie on it
-            const int r_lo = max(0, (t - cols + 2) / 2), r_hi = min(rows - 1, t / 2);
-            for (int r = r_lo + wib; r <= r_hi; r += nw) {
-                const int k = r * cols + (t - 2 * r);
-                if (!((s_tie[k >> 5] >> (k & 31)) & 1u)) continue;
-                // the record and the tie tree do not depend on the prediction: one round trip for both
-                const int* tree = a.tables + (size_t)k * TAB * TAB + TIE_ROW * TAB;
-                const int4 sp = __ldcg(a.spec4 + k);
-                const int t0 = __ldcg(tree + lane);
-                const int t1 = lane < TW - 32 ? __ldcg(tree + 32 + lane) : 0;
-                int px, py;
-                if (local) {
-                    const int av = sp.w;
-                    const int A = (av & AV_A) ? s_fin[k - 1] : 0;
-                    const int B = (av & AV_B) ? s_fin[k - cols] : 0;
-                    const int C = (av & AV_C) ? s_fin[k - cols + 1] : 0;
-                    const int D = (!(av & AV_C) && (av & AV_D)) ? s_fin[k - cols - 1] : 0;
-                    median_from(av, A, B, C, D, &px, &py);
-                } else {
-                    median_pred(a.final_mv, sp.w, k, cols, &px, &py);
-                }
-                int mvx = mv_x(sp.x), mvy = mv_y(sp.x), md = sp.y;
-                if (round_pred(px) != 0 || round_pred(py) != 0) {  // (0, 0): the scan already decided
-                    if (!(sp.w & FLAG_DEEP)) tree_pick(t0, t1, round_pred(px), round_pred(py), &mvx, &mvy, &md);
-                    else tie_path(a, k, px, py, sp.w, lane, &mvx, &mvy, &md);
-                }
-                if (lane == 0) {
-                    const int v = pack_mv(mvx, mvy);
-                    if (local) s_fin[k] = v;
-                    __stcg(a.final_mv + k, v);
-                    __stcg(a.final_dist + k, md);
-                }
-            }
-            __syncthreads();
-        }
-    }
-    __syncthreads();
-    long long tot = 0;
-    int cnt = 0;
-    for (int k = threadIdx.x; k < a.nmb; k += blockDim.x) {
-        const bool tie = (s_tie[k >> 5] >> (k & 31)) & 1u;
-        const int fmv = local ? s_fin[k] : __ldcg(a.final_mv + k);
-        const int d = tie ? __ldcg(a.final_dist + k) : __ldcg(&a.spec4[k].y);
-        a.job->out_mv[k] = fmv;
-        if (a.job->out_dist) a.job->out_dist[k] = d;
-        if (a.job->incl && a.job->incl[k]) {
-            tot += d;
-            cnt++;
-        }
-    }
-    for (int o = 16; o > 0; o >>= 1) {
-        tot += __shfl_xor_sync(0xffffffffu, tot, o);
-        cnt += __shfl_xor_sync(0xffffffffu, cnt, o);
-    }
-    if (lane == 0 && cnt) {
-        atomicAdd(reinterpret_cast<unsigned long long*>(&s_tot), (unsigned long long)tot);
-        atomicAdd(&s_cnt, cnt);
-    }
-    __syncthreads();
-    if (threadIdx.x == 0) {  // the host reads the sums, device callers the average
-        a.ctrl->total = s_tot;
-        a.ctrl->count = s_cnt;
-        if (a.job->out_avg) *a.job->out_avg = s_cnt ? s_tot / s_cnt : 0;
     }
 }
 
@@ -1636,12 +1556,8 @@ int full_resolve_prepare(vppgpu_ctx*)
                                   (int)wave_smem_bytes(kWaveMaxWarps, kWaveMaxCols, 2)));
     int rc;
     if ((rc = finish_prepare<0>()) || (rc = finish_prepare<1>()) || (rc = finish_prepare<2>()) ||
-        (rc = finish_prepare<cross::EST_CROSS>()))
+        (rc = finish_prepare<cross::EST_CROSS>()) || (rc = finish_prepare<EST_SAD>()))
         return rc;
-    // the SAD resolve's largest dynamic shared memory: the local final vectors
-    // end at kSadSmemMbs macroblocks (larger pictures keep only the tie bits)
-    VPP_CUDA(cudaFuncSetAttribute(k_sad_resolve, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                  (int)sad_resolve_smem(kSadSmemMbs)));
     return VPPGPU_OK;
 }
 
@@ -1701,11 +1617,17 @@ int resolve_launch_records(vppgpu_ctx* ctx, const FullArgs& args)
     return VPPGPU_OK;
 }
 
+constexpr int kSadFresh = 2048;  // macroblocks; within the sizes whose distortions the cluster keeps
+
 template <int kEst>
 int resolve_launch(vppgpu_ctx* ctx, const FullArgs& args)
 {
-    k_resolve_first<kEst><<<(args.nmb + 15) / 16, 256, 0, ctx->stream>>>(args);
-    VPP_CHECK_LAUNCH(ctx);
+    // the SAD stage of a small frame starts the cluster from the searched results themselves
+    const bool fresh = kEst == EST_SAD && args.nmb <= kSadFresh;
+    if (!fresh) {
+        k_resolve_first<kEst><<<(args.nmb + 15) / 16, 256, 0, ctx->stream>>>(args);
+        VPP_CHECK_LAUNCH(ctx);
+    }
     const int want = (args.nmb + 7) / 8, cap = ctx->sm_count * args.relax_blocks_per_sm;
     const int blocks = want < cap ? want : cap;
     const int sweeps = args.relax_sweeps < args.grid_sweeps ? args.relax_sweeps : args.grid_sweeps;
@@ -1725,7 +1647,7 @@ int resolve_launch(vppgpu_ctx* ctx, const FullArgs& args)
     attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
     cfg.attrs = attr;
     cfg.numAttrs = 1;
-    VPP_CUDA(cudaLaunchKernelEx(&cfg, k_resolve_finish<kEst>, args, sweeps + 1, f.band, f.dist));
+    VPP_CUDA(cudaLaunchKernelEx(&cfg, k_resolve_finish<kEst>, args, sweeps + 1, f.band, f.dist, (int)fresh));
     VPP_CHECK_LAUNCH(ctx);
     return VPPGPU_OK;
 }
@@ -1754,9 +1676,9 @@ int full_resolve_launch(vppgpu_ctx* ctx, const FullArgs& args, int est)
 
 int sad_resolve_launch(vppgpu_ctx* ctx, const FullArgs& args)
 {
-    k_sad_resolve<<<1, 1024, sad_resolve_smem(args.nmb), ctx->stream>>>(args);
-    VPP_CHECK_LAUNCH(ctx);
-    return VPPGPU_OK;
+    FullArgs a = args;
+    a.relax_sweeps = a.grid_sweeps = 0;
+    return resolve_launch<EST_SAD>(ctx, a);
 }
 
 int full_residual_launch(vppgpu_ctx* ctx, const FullArgs& args, const int* d_mv, short* d_res)

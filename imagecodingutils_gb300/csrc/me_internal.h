@@ -252,7 +252,7 @@ int full_launch(vppgpu_ctx* ctx, const FullArgs& args, int nmb, cudaEvent_t* ev)
 // Integer-pel SAD full search: the MotionEstimatorH264ImplFull integer stage
 // (MotionEstimatorH264ImplFull.cpp:341-446) with the MEH264IF_ABS_DIFF distortion.
 int sad_launch(vppgpu_ctx* ctx, const FullArgs& args, const SearchMaps& maps, int nmb);
-// Its prediction-dependent tail: the tie macroblocks in wavefront order, then the outputs.
+// Its prediction-dependent tail: the tie macroblocks to the fixed point, the outputs.
 int sad_resolve_launch(vppgpu_ctx* ctx, const FullArgs& args);
 
 }  // namespace vppgpu

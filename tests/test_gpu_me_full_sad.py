@@ -105,3 +105,19 @@ def test_batched_form(vpp, ctx, orc):
             np.testing.assert_array_equal(dist.cpu().numpy(), d_o)
             assert a == (int(d_o[sel].sum()) // int(sel.sum()) if sel.any() else 0)
     batch.close()
+
+
+@pytest.mark.parametrize("w,h", [(16, 16), (16, 528), (512, 256), (512, 272), (1024, 512), (1040, 512)])
+def test_resolve_of_many_ties(vpp, ctx, orc, w, h):
+    """Content on which nearly every macroblock ties, so that its vector hangs on its neighbours': one CTA, four, the
+    largest frame whose resolve starts from the searched results and the first that is evaluated before it, one
+    macroblock, one column.  Pictures of two grey levels in 8-sample tiles, moved."""
+    t = (synth.splitmix64(700 + w + h, (h // 8 + 8) * (w // 8 + 8)) & np.uint64(1)).astype(np.int16)
+    big = np.repeat(np.repeat(100 + t.reshape(h // 8 + 8, w // 8 + 8), 8, 0), 8, 1)
+    ref, src = big[:h, :w].copy(), big[3:h + 3, 5:w + 5].copy()
+    mv_o, d_o = orc.me_full_intpel(src, ref, 32, metric=1)
+    me = make(vpp, ctx, src, ref, 32, np.ones((w // 16) * (h // 16), np.uint8))
+    mv, avg = me.Estimate()
+    np.testing.assert_array_equal(mv, mv_o)
+    np.testing.assert_array_equal(me.last_mb_distortion, d_o)
+    assert avg == int(d_o.sum()) // len(d_o)
