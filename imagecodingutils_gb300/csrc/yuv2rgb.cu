@@ -204,9 +204,48 @@ __device__ __noinline__ void general_group(uint4 ya, uint4 yb, uint2 uu, uint2 v
     }
 }
 
+// Eight luma and four chroma samples, and the 24 bytes of eight pixels; kWide: 16- and 8-byte aligned.
+template <bool kWide>
+__device__ __forceinline__ uint4 load8(const short* s)
+{
+    if (kWide) return __ldg(reinterpret_cast<const uint4*>(s));
+    const unsigned* w = reinterpret_cast<const unsigned*>(s);
+    return make_uint4(__ldg(w), __ldg(w + 1), __ldg(w + 2), __ldg(w + 3));
+}
+template <bool kWide>
+__device__ __forceinline__ uint2 load4(const short* s)
+{
+    if (kWide) return __ldg(reinterpret_cast<const uint2*>(s));
+    auto at = [&](int i) { return (unsigned)(unsigned short)__ldg(s + i); };
+    return make_uint2(at(0) | at(1) << 16, at(2) | at(3) << 16);
+}
+template <bool kWide>
+__device__ __forceinline__ void store24(unsigned char* o, const unsigned (&w)[6])
+{
+    if (kWide) {
+        uint2* d = reinterpret_cast<uint2*>(o);
+#pragma unroll
+        for (int i = 0; i < 3; i++) d[i] = make_uint2(w[2 * i], w[2 * i + 1]);
+    } else if ((reinterpret_cast<uintptr_t>(o) & 3) == 0) {
+        unsigned* d = reinterpret_cast<unsigned*>(o);
+#pragma unroll
+        for (int i = 0; i < 6; i++) d[i] = w[i];
+    } else {  // two bytes past a word
+        unsigned* d = reinterpret_cast<unsigned*>(o + 2);
+        *reinterpret_cast<unsigned short*>(o) = (unsigned short)w[0];
+#pragma unroll
+        for (int i = 0; i < 5; i++) d[i] = __funnelshift_r(w[i], w[i + 1], 16);
+        *reinterpret_cast<unsigned short*>(o + 22) = (unsigned short)(w[5] >> 16);
+    }
+}
+
 // Rows layout (NonRotate, or bottom-up with kFlip), four 2x2 blocks per
 // thread: two 16-byte luma loads, 8-byte chroma loads, three 8-byte stores
-// per output row.  Needs width % 8 == 0 and aligned planes.
+// per output row.  kWide: width % 8 == 0 and aligned planes; else (width of 8
+// or more, luma at 4 bytes, output at 2) the last group of a row ends at its
+// end, sharing pixels with the one before (both write the same), luma moves in
+// 4-byte and chroma in 2-byte accesses, and a row of output in the words
+// between its ends.
 //
 // Samples within 0 .. 255 (every real picture; a thread with others takes the
 // general pixel) go two at a time: a channel of two pixels is one add, clamp
@@ -215,25 +254,24 @@ __device__ __noinline__ void general_group(uint4 ya, uint4 yb, uint2 uu, uint2 v
 // fifty of natural chroma, so a few in most warps) have the pixels below
 // their bound corrected afterwards.  Issue-bound (permutations, packed adds and
 // products issue every other cycle): 16 1080p frames in 52.5 us with every
-// pixel alone, 38.9 now (the copy rate's floor is 29; b and r terms from
+// pixel alone, 36.9 now (the copy rate's floor is 29; b and r terms from
 // shared-memory tables in a persistent grid took 42, 5 or 8 CTAs per SM 41, 42).
-template <bool kFlip>
+template <bool kFlip, bool kWide>
 __global__ void __launch_bounds__(256, 6) k_yuv_rgb_x8(const short* __restrict__ Y, const short* __restrict__ U,
                                                     const short* __restrict__ V, const __grid_constant__ YuvParams p,
                                                     unsigned char* __restrict__ rgb)
 {
     const int f = blockIdx.y;
-    const int gpr = p.w >> 3, groups = gpr * (p.h >> 1);
+    const int gpr = (p.w + 7) >> 3, groups = gpr * (p.h >> 1);
     const short* y0 = Y + (size_t)f * p.w * p.h;
     const short* u0 = U + (size_t)f * (p.w >> 1) * (p.h >> 1);
     const short* v0 = V + (size_t)f * (p.w >> 1) * (p.h >> 1);
     unsigned char* o0 = rgb + (size_t)f * p.w * p.h * 3;
     for (int g = blockIdx.x * blockDim.x + threadIdx.x; g < groups; g += gridDim.x * blockDim.x) {
-        const int qy = g / gpr, gx = g - qy * gpr, x = gx * 8, y = 2 * qy;
-        const uint4 ya = __ldg(reinterpret_cast<const uint4*>(y0 + (size_t)y * p.w + x));
-        const uint4 yb = __ldg(reinterpret_cast<const uint4*>(y0 + (size_t)(y + 1) * p.w + x));
-        const uint2 uu = __ldg(reinterpret_cast<const uint2*>(u0 + (size_t)qy * (p.w >> 1) + 4 * gx));
-        const uint2 vv = __ldg(reinterpret_cast<const uint2*>(v0 + (size_t)qy * (p.w >> 1) + 4 * gx));
+        const int qy = g / gpr, gx = g - qy * gpr, x = kWide ? gx * 8 : min(gx * 8, p.w - 8), y = 2 * qy;
+        const uint4 ya = load8<kWide>(y0 + (size_t)y * p.w + x), yb = load8<kWide>(y0 + (size_t)(y + 1) * p.w + x);
+        const size_t co = (size_t)qy * (p.w >> 1) + (x >> 1);
+        const uint2 uu = load4<kWide>(u0 + co), vv = load4<kWide>(v0 + co);
         const short* su = reinterpret_cast<const short*>(&uu);
         const short* sv = reinterpret_cast<const short*>(&vv);
         const unsigned la[4] = {ya.x, ya.y, ya.z, ya.w}, lb[4] = {yb.x, yb.y, yb.z, yb.w};
@@ -285,17 +323,12 @@ __global__ void __launch_bounds__(256, 6) k_yuv_rgb_x8(const short* __restrict__
             }
         }
         const int ya_out = kFlip ? p.h - 1 - y : y, yb_out = kFlip ? p.h - 2 - y : y + 1;
-        uint2* da = reinterpret_cast<uint2*>(o0 + ((size_t)ya_out * p.w + x) * 3);
-        uint2* db = reinterpret_cast<uint2*>(o0 + ((size_t)yb_out * p.w + x) * 3);
-#pragma unroll
-        for (int i = 0; i < 3; i++) {
-            da[i] = make_uint2(wa[2 * i], wa[2 * i + 1]);
-            db[i] = make_uint2(wb[2 * i], wb[2 * i + 1]);
-        }
+        store24<kWide>(o0 + ((size_t)ya_out * p.w + x) * 3, wa);
+        store24<kWide>(o0 + ((size_t)yb_out * p.w + x) * 3, wb);
     }
 }
 
-// Any even width, any layout: one 2x2 block per thread, byte stores.
+// Any even width, any layout, any alignment: one 2x2 block per thread, byte stores.
 // layout 0 rows top-down, 1 transpose (pixel (x, y) at 3 * (x * h + y);
 // consecutive threads walk down a column so the stores stay contiguous),
 // 2 rows bottom-up.
@@ -523,14 +556,20 @@ int launch(vppgpu_ctx* ctx, int kind, const short* y, const short* u, const shor
     }
     const bool vec = layout != 1 && (w & 7) == 0 && ((uintptr_t)y & 15) == 0 && ((uintptr_t)u & 7) == 0 &&
                      ((uintptr_t)v & 7) == 0 && ((uintptr_t)rgb & 7) == 0;
-    const long long work = vec ? (long long)(w >> 3) * (h >> 1) : (long long)(w >> 1) * (h >> 1);
+    const bool narrow = !vec && layout != 1 && w >= 8 && ((uintptr_t)y & 3) == 0 && ((uintptr_t)u & 1) == 0 &&
+                        ((uintptr_t)v & 1) == 0 && ((uintptr_t)rgb & 1) == 0;
+    const long long work = (vec || narrow) ? (long long)((w + 7) >> 3) * (h >> 1) : (long long)(w >> 1) * (h >> 1);
     long long gx = (work + 255) / 256;
     if (gx > 4096) gx = 4096;
     const dim3 grid((unsigned)gx, nframes);
     if (vec && layout == 2)
-        k_yuv_rgb_x8<true><<<grid, 256, 0, ctx->stream>>>(y, u, v, p, rgb);
+        k_yuv_rgb_x8<true, true><<<grid, 256, 0, ctx->stream>>>(y, u, v, p, rgb);
     else if (vec)
-        k_yuv_rgb_x8<false><<<grid, 256, 0, ctx->stream>>>(y, u, v, p, rgb);
+        k_yuv_rgb_x8<false, true><<<grid, 256, 0, ctx->stream>>>(y, u, v, p, rgb);
+    else if (narrow && layout == 2)
+        k_yuv_rgb_x8<true, false><<<grid, 256, 0, ctx->stream>>>(y, u, v, p, rgb);
+    else if (narrow)
+        k_yuv_rgb_x8<false, false><<<grid, 256, 0, ctx->stream>>>(y, u, v, p, rgb);
     else
         k_yuv_rgb<<<grid, 256, 0, ctx->stream>>>(y, u, v, p, layout, rgb);
     VPP_CHECK_LAUNCH(ctx);

@@ -201,3 +201,38 @@ def test_packed_path_every_luma_at_whole_terms(vpp, ctx, orc, okind, flip):
     torch.cuda.synchronize()
     want = orc.yuv_to_rgb(okind, y, u, v, -128, 0, flip)
     np.testing.assert_array_equal(out.cpu().numpy().reshape(want.shape), want)
+
+
+@pytest.mark.parametrize("kind", [0, 1, 2])
+@pytest.mark.parametrize("w,h,yoff,coff,ooff", [(8, 2, 2, 1, 2), (10, 4, 0, 0, 0), (14, 6, 2, 0, 2), (22, 4, 0, 3, 4),
+                                                (24, 4, 4, 4, 0), (24, 6, 2, 2, 6), (130, 4, 0, 1, 2), (6, 4, 0, 0, 0),
+                                                (30, 4, 1, 0, 0), (30, 4, 0, 0, 3)])
+def test_yuv_to_rgb_widths_and_alignments(vpp, ctx, orc, kind, w, h, yoff, coff, ooff):
+    """Frames at any sample and byte: the wide, the narrow and the block-per-thread path, both row orders, samples in
+    and out of range, nothing written beside the frames."""
+    torch = pytest.importorskip("torch")
+    L = vpp.load()
+    rng = np.random.default_rng(60 + w)
+    nf, n = 3, w * h
+    for spread in (256, 400):
+        y = rng.integers(0, spread, (nf, h, w)).astype(np.int16)
+        u = rng.integers(0, 256, (nf, h // 2, w // 2)).astype(np.int16)
+        v = rng.integers(0, 256, (nf, h // 2, w // 2)).astype(np.int16)
+
+        def place(a, off):
+            t = torch.zeros(a.size + 32, dtype=torch.int16, device="cuda")
+            t[off:off + a.size] = torch.from_numpy(a.reshape(-1)).cuda()
+            return t, C.c_void_p(t.data_ptr() + 2 * off)
+
+        (ky, py), (ku, pu), (kv, pv) = place(y, yoff), place(u, coff), place(v, coff)
+        for flip in (0, 1):
+            out = torch.full((nf * n * 3 + 32,), 77, dtype=torch.uint8, device="cuda")
+            torch.cuda.synchronize()
+            assert L.vppgpu_yuv420_to_rgb24_frames_device(ctx.handle, kind, py, pu, pv, nf, w, h, -128, 0, flip,
+                                                          C.c_void_p(out.data_ptr() + ooff)) == 0
+            ctx.synchronize()
+            got = out.cpu().numpy()
+            for f in range(nf):
+                want = orc.yuv_to_rgb(kind, y[f], u[f], v[f], -128, 0, flip)
+                np.testing.assert_array_equal(got[ooff + f * n * 3:ooff + (f + 1) * n * 3].reshape(h, w, 3), want)
+            assert (got[:ooff] == 77).all() and (got[ooff + nf * n * 3:] == 77).all()
