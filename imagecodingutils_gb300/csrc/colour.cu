@@ -26,13 +26,6 @@ static_assert(kYr + kYg + kYb == 8192 && kYr > 0 && kYg > 0 && kYb > 0, "a luma 
 
 __device__ __forceinline__ int clamp_s8(int x) { return min(max(x, -128), 127); }
 
-__device__ __forceinline__ void fixed_pixel(int b, int g, int r, int& y, int& u, int& v)
-{
-    y = (kYr * r + kYg * g + kYb * b) >> 13;
-    u += kUr * r + kUg * g + kUb * b;
-    v += kVr * r + kVg * g + kVb * b;
-}
-
 __device__ __forceinline__ int fixed_chroma(int acc, int chr_off)
 {
     int t = acc >> 13;
@@ -110,52 +103,64 @@ __device__ __forceinline__ int real_chroma_int(const unsigned (&p)[4], int b, in
                 : iu;
 }
 
+template <int kKind>
+__device__ __forceinline__ unsigned pixel_luma(unsigned p)
+{
+    constexpr unsigned lo = (kYb & 255) | (kYg & 255) << 8 | (kYr & 255) << 16;
+    constexpr unsigned hi = (kYb >> 8) | (kYg >> 8) << 8 | (kYr >> 8) << 16;
+    return kKind == VPPGPU_RGB_FIXED_POINT ? __dp4a(p, lo, __dp4a(p, hi, 0u) << 8) >> 13 : (unsigned)real_luma_int(p);
+}
+// The chroma of a block from its pixels (row by row; the fourth byte of each is not read).
+template <int kKind>
+__device__ __forceinline__ void block_chroma(const unsigned (&p)[4], int chr_off, int& u, int& v)
+{
+    unsigned br = 0, gs = 0;
+#pragma unroll
+    for (int q = 0; q < 4; q++) {
+        br += p[q] & 0x00ff00ffu;
+        gs = __dp4a(p[q], 0x00000100u, gs);
+    }
+    const int b = (int)(br & 0xffffu), g = (int)gs, r = (int)(br >> 16);
+    if (kKind == VPPGPU_RGB_FIXED_POINT) {
+        u = fixed_chroma(kUr * r + kUg * g + kUb * b, chr_off);
+        v = fixed_chroma(kVr * r + kVg * g + kVb * b, chr_off);
+    } else {
+        u = chr_off + clamp_s8(real_chroma_int<kKind == VPPGPU_RGB_REAL_IMPL2>(p, b, g, r, -147, -289, 436));
+        v = chr_off + clamp_s8(real_chroma_int<kKind == VPPGPU_RGB_REAL_IMPL2>(p, b, g, r, 615, -515, -100));
+    }
+}
+
 // Four 2x2 blocks per thread (8 pixels of two rows).  What bounds it beside memory is instructions: each byte by
 // itself took 482 a thread, 36 us for sixteen 1920x1080 frames that move in 29.  A pixel is the low three bytes of a
 // word cut out of the row; its fixed-point luma is two dp4a, by the high and the low bytes of the coefficients, and
 // the chroma of a block comes from the sums of its four pixels: 353, 33 us.  The real converters (kKind)
 // were bound by double arithmetic: 175 us for seven 996x568 frames, 29 from integers.
-// kWide: width a multiple of 8 and aligned planes; else (width of 8 or more, luma 4-byte aligned) rows are read
-// from any address as the aligned words around them, and the last group of a row ends at its end, sharing pixels
-// with the one before (both write the same).
-template <int kKind, bool kWide>
-__global__ void __launch_bounds__(256) k_rgb_x8(const unsigned char* __restrict__ bgr, int w, int h, int chr_off, int flip,
+// Width a multiple of 8, aligned planes; 6 CTAs an SM (8: 33.1 us, 6: 32.8).
+template <int kKind>
+__global__ void __launch_bounds__(256, kKind == VPPGPU_RGB_FIXED_POINT ? 6 : 4)
+    k_rgb_x8(const unsigned char* __restrict__ bgr, int w, int h, int chr_off, int flip,
                                                short* __restrict__ py, short* __restrict__ pu, short* __restrict__ pv)
 {
-    constexpr unsigned lo = (kYb & 255) | (kYg & 255) << 8 | (kYr & 255) << 16;
-    constexpr unsigned hi = (kYb >> 8) | (kYg >> 8) << 8 | (kYr >> 8) << 16;
     size_t fpix = (size_t)w * h;
     const unsigned char* src = bgr + blockIdx.y * fpix * 3;
     short* Y = py + blockIdx.y * fpix;
     short* U = pu + blockIdx.y * (fpix / 4);
     short* V = pv + blockIdx.y * (fpix / 4);
-    const unsigned groups_x = ((unsigned)w + 7) >> 3;
+    const unsigned groups_x = (unsigned)w >> 3;
     const long long ngroups = (long long)groups_x * (h >> 1);
     for (long long gi = blockIdx.x * (long long)blockDim.x + threadIdx.x; gi < ngroups;
          gi += (long long)gridDim.x * blockDim.x) {
         const int yb = ngroups >> 32 ? (int)(gi / groups_x) : (int)((unsigned)gi / groups_x);
-        const int x0 = min((int)(gi - (long long)yb * groups_x) * 8, w - 8), y0 = 2 * yb;
+        const int x0 = (int)(gi - (long long)yb * groups_x) * 8, y0 = 2 * yb;
         unsigned px[2][8];
         uint4 lum[2];
 #pragma unroll
         for (int rr = 0; rr < 2; rr++) {
             const int sy = kKind != VPPGPU_RGB_FIXED_POINT && flip ? h - 1 - (y0 + rr) : y0 + rr;
             const unsigned char* row = src + ((size_t)sy * w + x0) * 3;
-            unsigned in[6];
-            if (kWide) {
-                const uint2* s = reinterpret_cast<const uint2*>(row);
-                const uint2 a = __ldg(s), b = __ldg(s + 1), c = __ldg(s + 2);
-                in[0] = a.x, in[1] = a.y, in[2] = b.x, in[3] = b.y, in[4] = c.x, in[5] = c.y;
-            } else {
-                const unsigned off = (unsigned)(reinterpret_cast<uintptr_t>(row) & 3);
-                const unsigned* s = reinterpret_cast<const unsigned*>(row - off);
-                unsigned v[7];
-#pragma unroll
-                for (int i = 0; i < 6; i++) v[i] = __ldg(s + i);
-                v[6] = off ? __ldg(s + 6) : 0u;  // else past the row
-#pragma unroll
-                for (int i = 0; i < 6; i++) in[i] = __funnelshift_r(v[i], v[i + 1], 8 * off);
-            }
+            const uint2* s = reinterpret_cast<const uint2*>(row);
+            const uint2 a = __ldg(s), b = __ldg(s + 1), c = __ldg(s + 2);
+            const unsigned in[6] = {a.x, a.y, b.x, b.y, c.x, c.y};
 #pragma unroll
             for (int g = 0; g < 2; g++) {  // twelve bytes are four pixels (the fourth byte of each: the next pixel's)
                 px[rr][4 * g] = in[3 * g];
@@ -165,9 +170,7 @@ __global__ void __launch_bounds__(256) k_rgb_x8(const unsigned char* __restrict_
             }
             unsigned yv[8];
 #pragma unroll
-            for (int i = 0; i < 8; i++)
-                yv[i] = kKind == VPPGPU_RGB_FIXED_POINT ? __dp4a(px[rr][i], lo, __dp4a(px[rr][i], hi, 0u) << 8) >> 13
-                                                        : (unsigned)real_luma_int(px[rr][i]);
+            for (int i = 0; i < 8; i++) yv[i] = pixel_luma<kKind>(px[rr][i]);
             lum[rr] = make_uint4(__byte_perm(yv[0], yv[1], 0x5410), __byte_perm(yv[2], yv[3], 0x5410),
                                  __byte_perm(yv[4], yv[5], 0x5410), __byte_perm(yv[6], yv[7], 0x5410));
         }
@@ -175,157 +178,84 @@ __global__ void __launch_bounds__(256) k_rgb_x8(const unsigned char* __restrict_
 #pragma unroll
         for (int k = 0; k < 4; k++) {
             const unsigned p[4] = {px[0][2 * k], px[0][2 * k + 1], px[1][2 * k], px[1][2 * k + 1]};
-            unsigned br = 0, gs = 0;
-#pragma unroll
-            for (int q = 0; q < 4; q++) {
-                br += p[q] & 0x00ff00ffu;
-                gs = __dp4a(p[q], 0x00000100u, gs);
-            }
-            const int b = (int)(br & 0xffffu), g = (int)gs, r = (int)(br >> 16);
-            if (kKind == VPPGPU_RGB_FIXED_POINT) {
-                uo[k] = fixed_chroma(kUr * r + kUg * g + kUb * b, chr_off);
-                vo[k] = fixed_chroma(kVr * r + kVg * g + kVb * b, chr_off);
-            } else {
-                uo[k] = chr_off + clamp_s8(real_chroma_int<kKind == VPPGPU_RGB_REAL_IMPL2>(p, b, g, r, -147, -289, 436));
-                vo[k] = chr_off + clamp_s8(real_chroma_int<kKind == VPPGPU_RGB_REAL_IMPL2>(p, b, g, r, 615, -515, -100));
-            }
+            block_chroma<kKind>(p, chr_off, uo[k], vo[k]);
         }
         size_t co = (size_t)yb * (w >> 1) + (x0 >> 1);
-        if (kWide) {
 #pragma unroll
-            for (int rr = 0; rr < 2; rr++) *reinterpret_cast<uint4*>(Y + (size_t)(y0 + rr) * w + x0) = lum[rr];
-            *reinterpret_cast<uint2*>(U + co) = make_uint2(pack2(uo[0], uo[1]), pack2(uo[2], uo[3]));
-            *reinterpret_cast<uint2*>(V + co) = make_uint2(pack2(vo[0], vo[1]), pack2(vo[2], vo[3]));
-        } else {
-#pragma unroll
-            for (int rr = 0; rr < 2; rr++) {
-                unsigned* d = reinterpret_cast<unsigned*>(Y + (size_t)(y0 + rr) * w + x0);
-                d[0] = lum[rr].x, d[1] = lum[rr].y, d[2] = lum[rr].z, d[3] = lum[rr].w;
-            }
-#pragma unroll
-            for (int k = 0; k < 4; k++) {
-                U[co + k] = (short)uo[k];
-                V[co + k] = (short)vo[k];
-            }
-        }
+        for (int rr = 0; rr < 2; rr++) *reinterpret_cast<uint4*>(Y + (size_t)(y0 + rr) * w + x0) = lum[rr];
+        *reinterpret_cast<uint2*>(U + co) = make_uint2(pack2(uo[0], uo[1]), pack2(uo[2], uo[3]));
+        *reinterpret_cast<uint2*>(V + co) = make_uint2(pack2(vo[0], vo[1]), pack2(vo[2], vo[3]));
     }
 }
 
-// Generic fixed-point path: one 2x2 block per thread (any even width).
-__global__ void __launch_bounds__(256) k_rgb_fixed(const unsigned char* __restrict__ bgr, int w, int h,
-                                                  int chr_off, short* __restrict__ py,
-                                                  short* __restrict__ pu, short* __restrict__ pv)
+// Any even width and any alignment: one 2x2 block per thread, so that a warp's accesses are to neighbouring bytes
+// whatever the row's address.  Two pixels of a row are six bytes from any address: the two or three aligned words
+// around them.  (Eight pixels a thread in 4-byte accesses scattered a warp's stores: seven 996x568 frames by the real
+// converter 29.5 us, 25.8 so; eight 1366x768 frames in fixed point 21 both ways.)
+template <int kKind>
+__global__ void __launch_bounds__(256) k_rgb_block(const unsigned char* __restrict__ bgr, int w, int h, int chr_off,
+                                                  int flip, short* __restrict__ py, short* __restrict__ pu,
+                                                  short* __restrict__ pv)
 {
-    size_t fpix = (size_t)w * h;
+    const size_t fpix = (size_t)w * h;
     const unsigned char* src = bgr + blockIdx.y * fpix * 3;
     short* Y = py + blockIdx.y * fpix;
     short* U = pu + blockIdx.y * (fpix / 4);
     short* V = pv + blockIdx.y * (fpix / 4);
-    int xb_n = w >> 1, yb_n = h >> 1;
-    long long n = (long long)xb_n * yb_n;
+    const bool pairs = (reinterpret_cast<uintptr_t>(py) & 3) == 0;
+    const unsigned xb_n = (unsigned)w >> 1;
+    const long long n = (long long)xb_n * (h >> 1);
     for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
-        int yb = (int)(i / xb_n), xb = (int)(i - (long long)yb * xb_n);
-        int u = 0, v = 0;
+        const int yb = n >> 32 ? (int)(i / xb_n) : (int)((unsigned)i / xb_n), xb = (int)(i - (long long)yb * xb_n);
+        unsigned p[4];
 #pragma unroll
-        for (int q = 0; q < 4; q++) {
-            int yy = 2 * yb + (q >> 1), xx = 2 * xb + (q & 1);
-            const unsigned char* t = src + ((size_t)yy * w + xx) * 3;
-            int yv;
-            fixed_pixel(t[0], t[1], t[2], yv, u, v);
-            Y[(size_t)yy * w + xx] = (short)yv;
-        }
-        U[(size_t)yb * xb_n + xb] = (short)fixed_chroma(u, chr_off);
-        V[(size_t)yb * xb_n + xb] = (short)fixed_chroma(v, chr_off);
-    }
-}
-
-__global__ void __launch_bounds__(256) k_rgb_real(const unsigned char* __restrict__ bgr, int w, int h, int chr_off,
-                                                 int flip, int impl2, short* __restrict__ py,
-                                                 short* __restrict__ pu, short* __restrict__ pv)
-{
-    const double K00 = 0.299, K01 = 0.587, K02 = 0.114;
-    const double K10 = -0.147, K11 = -0.289, K12 = 0.436;
-    const double K20 = 0.615, K21 = -0.515, K22 = -0.100;
-    size_t fpix = (size_t)w * h;
-    const unsigned char* src = bgr + blockIdx.y * fpix * 3;
-    short* Y = py + blockIdx.y * fpix;
-    short* U = pu + blockIdx.y * (fpix / 4);
-    short* V = pv + blockIdx.y * (fpix / 4);
-    int xb_n = w >> 1, yb_n = h >> 1;
-    long long n = (long long)xb_n * yb_n;
-    for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
-        int yb = (int)(i / xb_n), xb = (int)(i - (long long)yb * xb_n);
-        double u = 0.0, v = 0.0;
-#pragma unroll
-        for (int q = 0; q < 4; q++) {
-            int yy = 2 * yb + (q >> 1), xx = 2 * xb + (q & 1);
-            int sy = flip ? (h - 1 - yy) : yy;
-            const unsigned char* t = src + ((size_t)sy * w + xx) * 3;
-            double b = (double)t[0], g = (double)t[1], r = (double)t[2];
-            double yl = __dadd_rn(__dadd_rn(__dadd_rn(0.5, __dmul_rn(K00, r)), __dmul_rn(K01, g)), __dmul_rn(K02, b));
-            Y[(size_t)yy * w + xx] = (short)clip255(__double2int_rz(yl));
-            double uu = lin3(K10, K11, K12, r, g, b);
-            double vv = lin3(K20, K21, K22, r, g, b);
-            if (q == 0) {
-                u = uu;
-                v = vv;
+        for (int rr = 0; rr < 2; rr++) {
+            const int yy = 2 * yb + rr, sy = kKind != VPPGPU_RGB_FIXED_POINT && flip ? h - 1 - yy : yy;
+            const unsigned char* t = src + ((size_t)sy * w + 2 * xb) * 3;
+            const unsigned off = (unsigned)(reinterpret_cast<uintptr_t>(t) & 3);
+            const unsigned* s = reinterpret_cast<const unsigned*>(t - off);
+            const unsigned v0 = __ldg(s), v1 = __ldg(s + 1), v2 = off == 3 ? __ldg(s + 2) : 0u;
+            const unsigned a = __funnelshift_r(v0, v1, 8 * off), b = __funnelshift_r(v1, v2, 8 * off);
+            p[2 * rr] = a;
+            p[2 * rr + 1] = __funnelshift_r(a, b, 24);
+            const unsigned y0 = pixel_luma<kKind>(p[2 * rr]), y1 = pixel_luma<kKind>(p[2 * rr + 1]);
+            short* d = Y + (size_t)yy * w + 2 * xb;
+            if (pairs) {
+                *reinterpret_cast<unsigned*>(d) = y0 | y1 << 16;
             } else {
-                u = __dadd_rn(u, uu);
-                v = __dadd_rn(v, vv);
+                d[0] = (short)y0;
+                d[1] = (short)y1;
             }
         }
-        int iu, iv;
-        if (!impl2) {
-            iu = __double2int_rz(u);
-            iv = __double2int_rz(v);
-            iu += iu < 0 ? -2 : 2;
-            iv += iv < 0 ? -2 : 2;
-            iu /= 4;
-            iv /= 4;
-        } else {
-            double au = __ddiv_rn(u, 4.0), av = __ddiv_rn(v, 4.0);
-            au = u < 0.0 ? __dsub_rn(au, 0.5) : __dadd_rn(au, 0.5);
-            av = v < 0.0 ? __dsub_rn(av, 0.5) : __dadd_rn(av, 0.5);
-            iu = __double2int_rz(au);
-            iv = __double2int_rz(av);
-        }
-        U[(size_t)yb * xb_n + xb] = (short)(chr_off + clamp_s8(iu));
-        V[(size_t)yb * xb_n + xb] = (short)(chr_off + clamp_s8(iv));
+        int u, v;
+        block_chroma<kKind>(p, chr_off, u, v);
+        U[(size_t)yb * xb_n + xb] = (short)u;
+        V[(size_t)yb * xb_n + xb] = (short)v;
     }
 }
 
-template <bool kWide>
-void launch_x8(vppgpu_ctx* ctx, int kind, const unsigned char* bgr, int nframes, int w, int h, int chr_off, int flip,
-               short* y, short* u, short* v)
+template <int kKind>
+void launch_kind(vppgpu_ctx* ctx, const unsigned char* bgr, int nframes, int w, int h, int chr_off, int flip, short* y,
+                 short* u, short* v)
 {
-    const long long groups = (long long)((w + 7) >> 3) * (h >> 1), blocks = (groups + 255) / 256;
+    // eight pixels a thread with 8- and 16-byte accesses where rows and planes are aligned to them
+    const uintptr_t a16 = (uintptr_t)y, a8 = (uintptr_t)u | (uintptr_t)v | (uintptr_t)bgr;
+    const bool wide = (w & 7) == 0 && (a16 & 15) == 0 && (a8 & 7) == 0;
+    const long long work = (long long)(w >> (wide ? 3 : 1)) * (h >> 1), blocks = (work + 255) / 256;
     const dim3 grid((unsigned)(blocks < 4096 ? blocks : 4096), nframes);
-    if (kind == VPPGPU_RGB_FIXED_POINT)
-        k_rgb_x8<VPPGPU_RGB_FIXED_POINT, kWide><<<grid, 256, 0, ctx->stream>>>(bgr, w, h, chr_off, flip, y, u, v);
-    else if (kind == VPPGPU_RGB_REAL)
-        k_rgb_x8<VPPGPU_RGB_REAL, kWide><<<grid, 256, 0, ctx->stream>>>(bgr, w, h, chr_off, flip, y, u, v);
-    else
-        k_rgb_x8<VPPGPU_RGB_REAL_IMPL2, kWide><<<grid, 256, 0, ctx->stream>>>(bgr, w, h, chr_off, flip, y, u, v);
+    if (wide) k_rgb_x8<kKind><<<grid, 256, 0, ctx->stream>>>(bgr, w, h, chr_off, flip, y, u, v);
+    else k_rgb_block<kKind><<<grid, 256, 0, ctx->stream>>>(bgr, w, h, chr_off, flip, y, u, v);
 }
 
 int launch(vppgpu_ctx* ctx, int kind, const unsigned char* bgr, int nframes, int w, int h, int chr_off,
            int flip, short* y, short* u, short* v)
 {
-    const long long per = (long long)(w >> 1) * (h >> 1);
-    // eight pixels a thread with 8- and 16-byte accesses, or 4-byte ones; a block a thread for what is left
-    const uintptr_t out16 = (uintptr_t)y, out8 = (uintptr_t)u | (uintptr_t)v | (uintptr_t)bgr;
-    if ((w & 7) == 0 && (out16 & 15) == 0 && (out8 & 7) == 0) {
-        launch_x8<true>(ctx, kind, bgr, nframes, w, h, chr_off, flip != 0, y, u, v);
-    } else if (w >= 8 && (out16 & 3) == 0 && ((uintptr_t)u & 1) == 0 && ((uintptr_t)v & 1) == 0) {
-        launch_x8<false>(ctx, kind, bgr, nframes, w, h, chr_off, flip != 0, y, u, v);
-    } else {
-        const int gx = (int)(per + 255 < 4096 * 256 ? (per + 255) / 256 : 4096);
-        if (kind == VPPGPU_RGB_FIXED_POINT)
-            k_rgb_fixed<<<dim3(gx, nframes), 256, 0, ctx->stream>>>(bgr, w, h, chr_off, y, u, v);
-        else
-            k_rgb_real<<<dim3(gx, nframes), 256, 0, ctx->stream>>>(bgr, w, h, chr_off, flip != 0,
-                                                                   kind == VPPGPU_RGB_REAL_IMPL2, y, u, v);
-    }
+    if (kind == VPPGPU_RGB_FIXED_POINT)
+        launch_kind<VPPGPU_RGB_FIXED_POINT>(ctx, bgr, nframes, w, h, chr_off, flip != 0, y, u, v);
+    else if (kind == VPPGPU_RGB_REAL)
+        launch_kind<VPPGPU_RGB_REAL>(ctx, bgr, nframes, w, h, chr_off, flip != 0, y, u, v);
+    else
+        launch_kind<VPPGPU_RGB_REAL_IMPL2>(ctx, bgr, nframes, w, h, chr_off, flip != 0, y, u, v);
     VPP_CHECK_LAUNCH(ctx);
     return VPPGPU_OK;
 }
