@@ -528,7 +528,8 @@ __device__ __forceinline__ int group_ssd(const unsigned char* win, uint4 t, int 
 //
 // A group of 8 candidates (a.rowmin) can accept one only if its minimum is at
 // or below the running minimum and some of its columns are in range of the
-// running best (the skip rule adds the best's vector to the candidate's).  A
+// running best (the skip rule adds the best's vector to the candidate's); once
+// a tie is known, one that only ties must not lie farther out than the best.  A
 // lane holds the minima of two candidate rows; the first row that has such a
 // minimum is visited next, and only such groups' SSDs are formed: on a 1080p
 // pan 6 rows and 7.5 groups a macroblock.
@@ -580,10 +581,15 @@ __global__ void __launch_bounds__(32 * SCAN_WARPS, 8) k_full_scan(const __grid_c
     int done = 0;  // rows yu .. yu+done-1 are behind the scan
     while (true) {
         const int r0 = yu + lane + my, r1 = r0 + 32;
-        const unsigned m0 = __ballot_sync(0xffffffffu, rm[0] <= minD && lane >= done && r0 >= yu && r0 <= yd &&
-                                                           yu + lane <= yd);
-        const unsigned m1 = __ballot_sync(0xffffffffu, rm[1] <= minD && lane + 32 >= done && r1 >= yu && r1 <= yd &&
-                                                           yu + lane + 32 <= yd);
+        unsigned m0 = __ballot_sync(0xffffffffu, rm[0] <= minD && lane >= done && r0 >= yu && r0 <= yd &&
+                                                     yu + lane <= yd);
+        unsigned m1 = __ballot_sync(0xffffffffu, rm[1] <= minD && lane + 32 >= done && r1 >= yu && r1 <= yd &&
+                                                     yu + lane + 32 <= yd);
+        if (tie) {
+            const int best = my * my + mx * mx, p0 = yu + lane, p1 = p0 + 32;
+            m0 &= __ballot_sync(0xffffffffu, rm[0] < minD || best >= p0 * p0);
+            m1 &= __ballot_sync(0xffffffffu, rm[1] < minD || best >= p1 * p1);
+        }
         if (!m0 && !m1) break;
         const int off = m0 ? __ffs(m0) - 1 : 31 + __ffs(m1), i = yu + off;
         done = off + 1;
@@ -592,31 +598,18 @@ __global__ void __launch_bounds__(32 * SCAN_WARPS, 8) k_full_scan(const __grid_c
         unsigned left = 0xffu;  // groups not yet behind the scan
         while (i + my >= yu && i + my <= yd) {
             // the next group of the row that can accept, at the best as it is
-            const unsigned can = __ballot_sync(0xffffffffu, gmin <= minD && jl + 7 + mx >= xl && jl + mx <= xr) & left;
+            unsigned can = __ballot_sync(0xffffffffu, gmin <= minD && jl + 7 + mx >= xl && jl + mx <= xr) & left;
+            if (tie) {
+                const int jn = max(max(jl, -jl - 7), 0);  // the group's distance from column 0
+                can &= __ballot_sync(0xffffffffu, gmin < minD || my * my + mx * mx >= i * i + jn * jn);
+            }
             if (!can) break;
             const int g = __ffs(can) - 1;
             left &= ~((2u << g) - 1u);
             const int d = group_ssd<kPitch>(win, t, i + RMAX, g, lane);
             const int base = 8 * g - 32, j = base + lane;
             const bool valid = lane < 8 && j >= xl && j <= xr && !(i == 0 && j == 0);
-            unsigned pending = 0xffu;
-            while (true) {
-                const bool ok = valid && d <= minD && i + my >= yu && i + my <= yd && j + mx >= xl && j + mx <= xr;
-                const unsigned b = __ballot_sync(0xffffffffu, ok) & pending;
-                if (!b) break;
-                const int f = __ffs(b) - 1, df = __shfl_sync(0xffffffffu, d, f), jf = base + f;
-                bool accept = true;
-                if (df == minD) {
-                    tie = 1;
-                    accept = (my * my + mx * mx) - (i * i + jf * jf) >= 0;
-                }
-                if (accept) {
-                    minD = df;
-                    mx = jf;
-                    my = i;
-                }
-                pending &= ~((2u << f) - 1u);
-            }
+            scan_piece(valid, d, i, j, base, xl, xr, yu, yd, 0, 0, minD, mx, my, tie);
         }
     }
     int qmx, qmy;
@@ -683,7 +676,7 @@ __global__ void __launch_bounds__(kSad ? TIE_RUNS * 32 : TIE_WARPS_SSD * 32) k_f
             int rmx, rmy, rmin, rt, nev, ev[TIE_DEPTH] = {0, 0, 0};
             scan_table_t<true>(SmemTab{S.tab}, xl, xr, yu, yd, 0, 0, p, lane, &rmx, &rmy, &rmin, &rt, &nev, ev);
             int rq = sp.x, rqmin = sp.y;
-            if (rmx != mv_x(imv) || rmy != mv_y(imv)) {
+            if (nev >= 0 && (rmx != mv_x(imv) || rmy != mv_y(imv))) {  // (deeper runs are not read)
                 int sx = 0, sy = 0;
                 if (!kSad) subpel_refine_planes(a, n + rmx, m + rmy, load_cur8(a, n, m, lane), lane, &rmin, &sx, &sy);
                 rq = pack_mv(4 * rmx + sx, 4 * rmy + sy);

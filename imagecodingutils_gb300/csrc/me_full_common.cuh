@@ -52,6 +52,38 @@ __device__ __forceinline__ void full_range(int n, int m, int W, int H, int motio
     yd = (m + rr < H) ? rr : H - m;
 }
 
+// The candidates of one piece of a row, a lane each (d; valid: one that the search visits), against the running
+// minimum (Full.cpp:406-446): a candidate in range at the running best and not above the minimum is taken if it is
+// below, or at an exact tie if the running best is not nearer to the prediction (prx, pry).  A tie that is not taken
+// leaves the state as it is, so those up to the next one that is taken are decided at once: a step for each
+// acceptance, not for each tie.  (One at a time, a letterboxed 352x288 frame took 5.7 ms, 0.47 so, and one of flat
+// shapes 18.5, 1.4; content without ties the same as before.)  tie: set when a tie was decided.  One warp; j: the
+// lane's candidate, base + lane.
+__device__ __forceinline__ void scan_piece(bool valid, int d, int i, int j, int base, int xl, int xr, int yu, int yd,
+                                           int prx, int pry, int& minD, int& mx, int& my, int& tie)
+{
+    unsigned pending = 0xffffffffu;
+    while (true) {
+        const bool ok = valid && d <= minD && i + my >= yu && i + my <= yd && j + mx >= xl && j + mx <= xr;
+        const unsigned live = __ballot_sync(0xffffffffu, ok) & pending;
+        if (!live) return;
+        int f = __ffs(live) - 1, df = __shfl_sync(0xffffffffu, d, f);
+        if (df == minD) {
+            tie = 1;
+            const int best = (my - pry) * (my - pry) + (mx - prx) * (mx - prx);
+            const int far = (i - pry) * (i - pry) + (j - prx) * (j - prx);
+            const unsigned take = __ballot_sync(0xffffffffu, d < minD || best >= far) & live;
+            if (!take) return;
+            f = __ffs(take) - 1;
+            df = __shfl_sync(0xffffffffu, d, f);
+        }
+        minD = df;
+        mx = base + f;
+        my = i;
+        pending &= ~((2u << f) - 1u);
+    }
+}
+
 // Sequential raster replay of the integer search over tab (ii = i+31,
 // jj = j+32), one warp.  prx/pry: rounded prediction used at ties.  Returns
 // the winner and sets *tie when any exact tie was decided.
@@ -59,15 +91,18 @@ __device__ __forceinline__ void full_range(int n, int m, int W, int H, int motio
 // Column 0 of the table (jj = 0, outside every range) holds each row's
 // minimum over the searched columns.  A row whose minimum is above the
 // running minimum cannot accept any candidate (acceptance needs d <= min and
-// the minimum only falls), and neither can a row that the skip rule puts out
+// the minimum only falls), neither can a row that the skip rule puts out
 // of range (Full.cpp:410: row offset plus the running best's row outside
 // [yu, yd]), so only the rows that can are visited, found with a ballot over
-// the row minima.  On the 1080p pan sequence this visits ~8 rows per
-// macroblock instead of ~38.
+// the row minima: ~8 rows of a macroblock of a 1080p pan instead of ~38.  (A
+// row that only ties and lies farther from the prediction than the running
+// best can do no more than set *tie; passing over it pays where rows come
+// from global memory, kBatch > 1, and costs the SAD search 3 %.)
 //
 // kForced: instead of the distance rule, exact tie e (in scan order) takes
 // bit e of `path`; the geometry of the first TIE_DEPTH ties goes to ev[] and
-// their count to *nev (-1 when there were more).
+// their count to *nev (-1 when there were more: the scan ends there, as the
+// tree of such a macroblock is not read).
 template <bool kForced, int kBatch = 1, typename TabT>
 __device__ __forceinline__ void scan_table_t(const TabT& tab, int xl, int xr, int yu, int yd, int prx, int pry,
                                              int path, int lane, int* omx, int* omy, int* omin, int* tie, int* nev,
@@ -79,7 +114,7 @@ __device__ __forceinline__ void scan_table_t(const TabT& tab, int xl, int xr, in
     const int rm0 = yu + lane <= yd ? tab(yu + lane + RMAX, 0) : kNone;
     const int rm1 = yu + lane + 32 <= yd ? tab(yu + lane + 32 + RMAX, 0) : kNone;
     int done = 0;  // rows yu .. yu+done-1 are behind the scan
-    while (true) {
+    while (!kForced || ne <= TIE_DEPTH) {
         // the next kBatch rows that can accept, read together: a row needs its
         // minimum at or below the running minimum, and its row offset added to
         // the running best must stay in range (the skip rule applies to every
@@ -120,44 +155,42 @@ __device__ __forceinline__ void scan_table_t(const TabT& tab, int xl, int xr, in
             const int rmin = __shfl_sync(0xffffffffu, off < 32 ? rm0 : rm1, off & 31);
             if (rmin > minD) continue;  // the minimum fell below this row's within the batch
             const int i = yu + off;
-            int v[2] = {vals[q][0], vals[q][1]};
+            if (kBatch > 1 && t && rmin == minD &&
+                (i - pry) * (i - pry) > (my - pry) * (my - pry) + (mx - prx) * (mx - prx))
+                continue;
 #pragma unroll
             for (int h = 0; h < 2; h++) {
                 const int base = xl + 32 * h;
                 if (base > xr) break;
                 const int j = base + lane;
-                const int d = v[h];
-                unsigned pending = 0xffffffffu;
-                while (true) {
-                    bool ok = d != kNone && d <= minD && (i + my >= yu) && (i + my <= yd) && (j + mx >= xl) &&
-                              (j + mx <= xr);
-                    unsigned m = __ballot_sync(0xffffffffu, ok) & pending;
-                    if (!m) break;
-                    int f = __ffs(m) - 1;
-                    int df = __shfl_sync(0xffffffffu, d, f);
-                    int jf = base + f;
-                    bool accept = true;
-                    if (df == minD) {
-                        t = 1;
-                        if (kForced) {
+                const int d = vals[q][h];
+                if constexpr (!kForced) {
+                    scan_piece(d != kNone, d, i, j, base, xl, xr, yu, yd, prx, pry, minD, mx, my, t);
+                } else {
+                    unsigned pending = 0xffffffffu;
+                    while (pending && ne <= TIE_DEPTH) {
+                        const bool ok = d != kNone && d <= minD && (i + my >= yu) && (i + my <= yd) &&
+                                        (j + mx >= xl) && (j + mx <= xr);
+                        const unsigned m = __ballot_sync(0xffffffffu, ok) & pending;
+                        if (!m) break;
+                        const int f = __ffs(m) - 1, df = __shfl_sync(0xffffffffu, d, f), jf = base + f;
+                        bool accept = true;
+                        if (df == minD) {
+                            t = 1;
                             const int g = (mx & 0xff) | ((my & 0xff) << 8) | ((jf & 0xff) << 16) | ((i & 0xff) << 24);
                             if (ne == 0) ev[0] = g;
                             if (ne == 1) ev[1] = g;
                             if (ne == 2) ev[2] = g;
                             accept = ne < TIE_DEPTH ? ((path >> ne) & 1) != 0 : true;
                             ne++;
-                        } else {
-                            int cx = mx - prx, cy = my - pry, nx = jf - prx, ny = i - pry;
-                            accept = (cy * cy + cx * cx) - (ny * ny + nx * nx) >= 0;
                         }
+                        if (accept) {
+                            minD = df;
+                            mx = jf;
+                            my = i;
+                        }
+                        pending &= ~((2u << f) - 1u);
                     }
-                    if (accept) {
-                        minD = df;
-                        mx = jf;
-                        my = i;
-                    }
-                    pending &= ~((2u << f) - 1u);
-                    if (f == 31) break;
                 }
             }
         }
@@ -250,6 +283,8 @@ __device__ __forceinline__ void subpel_refine_planes(const FullArgs& a, int x0, 
     // quarter pass: lattice offsets (dy, dx) of the two averaged samples
     constexpr int AY[8] = {-2, -2, -2, 0, 0, 0, 2, 2}, AX[8] = {-2, 0, 0, -2, 2, -2, 0, 0};
     constexpr int BY[8] = {0, 0, 0, 0, 0, 2, 0, 0}, BX[8] = {0, 0, 2, 0, 0, 0, 0, 2};
+    *qmx = *qmy = 0;
+    if (*min_d == 0) return;  // nothing improves on it
     int part[8];
 #pragma unroll
     for (int k = 0; k < 8; k++) part[k] = ssd8(cur, load8(even_block(a, x0, y0, 2 * SY[k], 2 * SX[k], lane)));
@@ -314,6 +349,8 @@ __device__ __forceinline__ void subwindow_row(const unsigned* row, int col, unsi
 __device__ __forceinline__ void subpel_refine_staged(const FullArgs& a, SubWindow& S, int n, int m, int x0, int y0,
                                                      int lane, int* min_d, int* qmx, int* qmy)
 {
+    *qmx = *qmy = 0;
+    if (*min_d == 0) return;  // nothing improves on it
     const int left = x0 - 1 + PAD, col0 = left & 7, rho = lane & 3;
     uint4 cur[4];
 #pragma unroll
@@ -343,7 +380,6 @@ __device__ __forceinline__ void subpel_refine_staged(const FullArgs& a, SubWindo
         *qmx = hx + step * __shfl_sync(0xffffffffu, sx, f);
         *qmy = hy + step * __shfl_sync(0xffffffffu, sy, f);
     };
-    *qmx = *qmy = 0;
     {
         const unsigned* q = S.p + plane(2 * sy, 2 * sx) + word(2 * sy);
         const int col = col0 + 1 + ((2 * sx) >> 2);

@@ -1,0 +1,87 @@
+"""Content on which many macroblocks meet exact ties or hang on their neighbours (flat and letterboxed pictures, flat
+shapes over flat ground, text, exact periods): the same results as the oracle's, and times that stay within a stated
+multiple of a noisy pan's of the same size, measured in the same process."""
+import ctypes as C
+import time
+
+import numpy as np
+import pytest
+
+from imagecodingutils_gb300 import _lib, synth
+
+pytestmark = pytest.mark.gpu
+
+
+def pair(kind, w, h, seed=5):
+    """(input, reference) planes."""
+    rng = np.random.default_rng(seed)
+    if kind == "flat":
+        return np.full((h, w), 120, np.int16), np.full((h, w), 100, np.int16)
+    if kind == "letterbox":  # black bars above and below a pan
+        f = [x.copy() for x in synth.pan_sequence(seed, w, h, 2)]
+        for x in f:
+            x[:max(16, h // 6)] = 16
+            x[-max(16, h // 6):] = 16
+        return f[1], f[0]
+    if kind == "shapes":     # flat rectangles over flat ground, each with a motion of its own
+        ref = np.full((h, w), 60, np.int16)
+        src = ref.copy()
+        for _ in range(24):
+            y, x = int(rng.integers(0, h - 8)), int(rng.integers(0, w - 8))
+            hh, ww, v = int(rng.integers(8, h // 2)), int(rng.integers(8, w // 2)), int(rng.integers(0, 256))
+            dy, dx = (int(d) for d in rng.integers(-12, 13, 2))
+            ref[y:y + hh, x:x + ww] = v
+            src[max(0, y + dy):, max(0, x + dx):][:hh, :ww] = v
+        return src, ref
+    if kind == "text":       # 8x8 glyphs, scrolled by 12 lines
+        glyph = rng.random((16, 8, 8)) < 0.35
+        ref = np.full((h, w), 235, np.int16)
+        for i in range(h // 8):
+            for j in range(w // 8):
+                if rng.random() < 0.4:
+                    ref[8 * i:8 * i + 8, 8 * j:8 * j + 8][glyph[rng.integers(0, 16)]] = 16
+        return np.roll(ref, -12, 0), ref
+    if kind == "period7":
+        f = synth.tile_sequence(seed, w, h, 2, period=7)
+        return f[1], f[0]
+    f = synth.pan_sequence(seed, w, h, 2)
+    return f[1], f[0]
+
+
+def best_time(vpp, ctx, cls, kind, w, h, mr=128):
+    """Seconds of an estimate on device planes, the best of 20."""
+    torch = pytest.importorskip("torch")
+    src, ref = (torch.from_numpy(np.ascontiguousarray(p)).cuda() for p in pair(kind, w, h))
+    me = cls(None, None, w, h, mr, ctx=ctx)
+    assert me.Create() == 1
+    mv = torch.zeros((w // 16) * (h // 16), dtype=torch.int32, device="cuda")
+    torch.cuda.synchronize()
+    best = 1e9
+    for _ in range(20):
+        t0 = time.perf_counter()
+        _lib.check(vpp.load().vppgpu_me_estimate_device(me._h_me, C.c_void_p(src.data_ptr()), C.c_void_p(ref.data_ptr()),
+                                                        None, None, C.c_void_p(mv.data_ptr()), None, None), "estimate")
+        ctx.synchronize()
+        best = min(best, time.perf_counter() - t0)
+    return best
+
+
+@pytest.mark.parametrize("kind,w,h,mr", [("letterbox", 352, 288, 128), ("shapes", 176, 144, 128), ("text", 208, 120, 64),
+                                         ("period7", 240, 98, 128), ("period7", 16, 400, 40), ("flat", 48, 32, 4)])
+@pytest.mark.parametrize("sad", [False, True])
+def test_tie_scans_against_oracle(vpp, ctx, orc, kind, w, h, mr, sad):
+    src, ref = pair(kind, w, h)
+    cls = vpp.MotionEstimatorH264ImplFullSad if sad else vpp.MotionEstimatorH264ImplFull
+    me = cls(src, ref, w, h, mr, ctx=ctx)
+    assert me.Create() == 1
+    mv, _ = me.Estimate()
+    want = orc.me_full_intpel(src, ref, mr, metric=1) if sad else orc.me_full(src, ref, mr)
+    np.testing.assert_array_equal(mv, want[0])
+    np.testing.assert_array_equal(me.last_mb_distortion, want[1])
+
+
+@pytest.mark.parametrize("kind,most", [("letterbox", 30), ("shapes", 90)])
+def test_ties_cost_no_scan_of_their_own(vpp, ctx, kind, most):
+    """A scan that decided each tie by itself took 106 and 340 times a pan's time."""
+    cls = vpp.MotionEstimatorH264ImplFull
+    assert best_time(vpp, ctx, cls, kind, 352, 288) < most * best_time(vpp, ctx, cls, "pan", 352, 288)
