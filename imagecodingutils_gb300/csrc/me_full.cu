@@ -805,7 +805,8 @@ int full_launch(vppgpu_ctx* ctx, const FullArgs& args, int nmb, cudaEvent_t* ev)
     if (ev) VPP_CUDA(cudaEventRecord(ev[2], ctx->stream));
     k_full_scan<<<(args.cols + SCAN_WARPS - 1) / SCAN_WARPS * (nmb / args.cols), 32 * SCAN_WARPS, 0, ctx->stream>>>(args);
     VPP_CHECK_LAUNCH(ctx);
-    k_full_tietree<false><<<min(ctx->sm_count, (nmb + 15) / 16), TIE_WARPS_SSD * 32, sizeof(TieSmem), ctx->stream>>>(args);
+    // as many CTAs as can have a macroblock: on flat or letterboxed content most of them tie
+    k_full_tietree<false><<<min(ctx->sm_count, nmb), TIE_WARPS_SSD * 32, sizeof(TieSmem), ctx->stream>>>(args);
     VPP_CHECK_LAUNCH(ctx);
     if (ev) VPP_CUDA(cudaEventRecord(ev[3], ctx->stream));
     if ((rc = full_resolve_launch(ctx, args, 0))) return rc;

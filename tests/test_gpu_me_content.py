@@ -85,3 +85,11 @@ def test_ties_cost_no_scan_of_their_own(vpp, ctx, kind, most):
     """A scan that decided each tie by itself took 106 and 340 times a pan's time."""
     cls = vpp.MotionEstimatorH264ImplFull
     assert best_time(vpp, ctx, cls, kind, 352, 288) < most * best_time(vpp, ctx, cls, "pan", 352, 288)
+
+
+@pytest.mark.parametrize("w,h", [(176, 144), (352, 288)])
+def test_tie_trees_side_by_side(vpp, ctx, w, h):
+    """A flat picture, where every macroblock has a tie tree: a CTA for each sixteen of them took 4 and 6 times a
+    pan's time."""
+    cls = vpp.MotionEstimatorH264ImplFull
+    assert best_time(vpp, ctx, cls, "flat", w, h) < 2.2 * best_time(vpp, ctx, cls, "pan", w, h)
