@@ -54,6 +54,18 @@ constexpr PathMasks make_path_masks()
 
 static __device__ const PathMasks c_path_masks = make_path_masks();
 
+// The same points as byte masks of the 16 samples of a row.
+struct alignas(16) PathRows {
+    unsigned m[16][4];
+};
+constexpr PathRows make_path_rows()
+{
+    PathRows t{};
+    for (int p = 0; p < 64; p++) t.m[kPath[p][1]][kPath[p][0] >> 2] |= 0xffu << (8 * (kPath[p][0] & 3));
+    return t;
+}
+static __device__ const PathRows c_path_rows = make_path_rows();
+
 struct LaneMasks {
     uint2 b[4];
 };
@@ -224,17 +236,6 @@ static __device__ __noinline__ void cross_search_run(const FullArgs& a, int n, i
         rec->mv = pack_mv(r.mvx, r.mvy);
         rec->min_d = r.min_d;
     }
-}
-
-// Tsd16x16PartialPath at the prediction (QuarterRead's sixteen cases).
-__device__ __forceinline__ int path_pred_distortion(const FullArgs& a, int n, int m, const full::PredGeom& g, int lane)
-{
-    const LaneMasks mk = lane_masks(lane);
-    const uint2 cur = full::load_cur8(a, n, m, lane), cand = full::qpel_block8(a, g.ox, g.oy, g.fx, g.fy, lane);
-    const unsigned d0 = __vabsdiffu4(cur.x, cand.x), d1 = __vabsdiffu4(cur.y, cand.y);
-    const unsigned m0 = mk.b[0].x | mk.b[1].x | mk.b[2].x | mk.b[3].x;
-    const unsigned m1 = mk.b[0].y | mk.b[1].y | mk.b[2].y | mk.b[3].y;
-    return (int)__reduce_add_sync(0xffffffffu, __dp4a(d0 & m0, d0, __dp4a(d1 & m1, d1, 0u)));
 }
 
 }  // namespace cross

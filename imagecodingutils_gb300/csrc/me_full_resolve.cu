@@ -247,9 +247,7 @@ __device__ __noinline__ int4 evaluate(const FullArgs& a, int k, int px, int py, 
     const int n = (k % a.cols) * 16, m = (k / a.cols) * 16;
     const PredGeom g = pred_geom(n, m, a.W, a.H, px, py);
     const int4 sp = a.spec4[k];  // loads of spec and planes are independent: one round trip
-    int pd;
-    if constexpr (kEst == cross::EST_CROSS) pd = cross::path_pred_distortion(a, n, m, g, lane);
-    else pd = plane_pred_distortion(a, n, m, g, lane);
+    const int pd = plane_pred_distortion(a, n, m, g, lane);
     int mvx = mv_x(sp.x), mvy = mv_y(sp.x), minD = sp.y;
     const int zd = sp.z;
     if constexpr (kEst == 0) {
@@ -258,8 +256,7 @@ __device__ __noinline__ int4 evaluate(const FullArgs& a, int k, int px, int py, 
     } else {
         if (sp.w & FLAG_TIE) pred_search_at<kEst>(a, k, px, py, lane, &mvx, &mvy, &minD, lt);
     }
-    const int pos = best_of3_fast(mvx, mvy, minD, g.pcx, g.pcy, pd, zd, a.lambda, g.pcx, g.pcy,
-                                  kEst == cross::EST_CROSS ? cross::PATH_NORM : 256);
+    const int pos = best_of3_fast(mvx, mvy, minD, g.pcx, g.pcy, pd, zd, a.lambda, g.pcx, g.pcy);
     int4 rec;
     rec.x = pack_mv(px, py);
     rec.y = pd;
@@ -1113,17 +1110,6 @@ __device__ __forceinline__ int2 evaluate_half(const FullArgs& a, bool act, int k
                                               uint4 cur, int lane, mrc::Lattice* lt)
 {
     const int px = mv_x(key), py = mv_y(key);
-    if constexpr (kEst == cross::EST_CROSS) {  // its path distortion is a whole warp's
-        int2 out = make_int2(0, 0);
-#pragma unroll 1
-        for (int h = 0; h < 2; h++) {
-            if (!__shfl_sync(0xffffffffu, (int)act, 16 * h)) continue;
-            const int4 rec = evaluate<kEst>(a, __shfl_sync(0xffffffffu, k, 16 * h), __shfl_sync(0xffffffffu, px, 16 * h),
-                                            __shfl_sync(0xffffffffu, py, 16 * h), lane, lt);
-            if ((lane >> 4) == h) out = make_int2(rec.z, rec.w);
-        }
-        return out;
-    }
     PredGeom g{};
     int pd = 0;
     if constexpr (kEst != EST_SAD) {
@@ -1147,11 +1133,16 @@ __device__ __forceinline__ int2 evaluate_half(const FullArgs& a, bool act, int k
         load_row16(b1, w1);
         load_row16(b2, w2);
         const unsigned c4[4] = {cur.x, cur.y, cur.z, cur.w};
+        // Cross: Tsd16x16PartialPath, the row's samples that lie on its path of 64 points
+        uint4 mask = make_uint4(~0u, ~0u, ~0u, ~0u);
+        if constexpr (kEst == cross::EST_CROSS)
+            mask = __ldg(reinterpret_cast<const uint4*>(cross::c_path_rows.m[lane & 15]));
+        const unsigned m4[4] = {mask.x, mask.y, mask.z, mask.w};
         unsigned acc = 0;
 #pragma unroll
         for (int i = 0; i < 4; i++) {
             const unsigned d = __vabsdiffu4(c4[i], __vavgu4(w1[i], w2[i]));
-            acc = __dp4a(d, d, acc);
+            acc = __dp4a(d & m4[i], d, acc);
         }
         const unsigned lo = __reduce_add_sync(0xffffffffu, lane < 16 ? acc : 0u);
         const unsigned hi = __reduce_add_sync(0xffffffffu, lane < 16 ? 0u : acc);
@@ -1179,7 +1170,8 @@ __device__ __forceinline__ int2 evaluate_half(const FullArgs& a, bool act, int k
         }
     }
     if constexpr (kEst == EST_SAD) return make_int2(pack_mv(mvx, mvy), minD);  // no GetBestVector
-    const int pos = best_of3_fast(mvx, mvy, minD, g.pcx, g.pcy, pd, sp.z, a.lambda, g.pcx, g.pcy);
+    const int pos = best_of3_fast(mvx, mvy, minD, g.pcx, g.pcy, pd, sp.z, a.lambda, g.pcx, g.pcy,
+                                  kEst == cross::EST_CROSS ? cross::PATH_NORM : 256);
     return pos == 0 ? make_int2(pack_mv(mvx, mvy), minD) : pos == 1 ? make_int2(pack_mv(g.pcx, g.pcy), pd)
                                                                     : make_int2(0, sp.z);
 }
@@ -1400,6 +1392,7 @@ __global__ void __launch_bounds__(kFinishThreads, 1)
                 s_evals[round > a.relax_sweeps] += nw;
             }
             if (tid < ctas) *cluster.map_shared_rank(&s_any[round % 3], tid) = 1;
+            // a macroblock per half warp, the second halves after all the first: ties are the whole warp's work
             for (int w = 2 * wib; w < nw; w += kFinishHalves) {
                 const bool act = w + half < nw;
                 const int i = s_work[act ? w + half : w];

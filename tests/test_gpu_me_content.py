@@ -93,3 +93,24 @@ def test_tie_trees_side_by_side(vpp, ctx, w, h):
     pan's time."""
     cls = vpp.MotionEstimatorH264ImplFull
     assert best_time(vpp, ctx, cls, "flat", w, h) < 2.2 * best_time(vpp, ctx, cls, "pan", w, h)
+
+
+@pytest.mark.parametrize("kind,w,h,mode", [("letterbox", 352, 288, 0), ("shapes", 176, 144, 0), ("text", 208, 120, 1),
+                                           ("period7", 240, 98, 0), ("pan", 640, 368, 2), ("pan", 1040, 66, 0)])
+def test_cross_against_oracle(vpp, ctx, orc, kind, w, h, mode):
+    src, ref = pair(kind, w, h)
+    me = vpp.MotionEstimatorH264ImplCross(src, ref, w, h, 128, ctx=ctx)
+    assert me.Create() == 1
+    me.SetMode(mode)
+    mv, _ = me.Estimate()
+    want = orc.me_cross(src, ref, 128, mode=mode)
+    np.testing.assert_array_equal(mv, want[0])
+    np.testing.assert_array_equal(me.last_mb_distortion, want[1])
+
+
+def test_cross_resolve_by_half_warps(vpp, ctx):
+    """The Cross estimator's resolve, a macroblock after the other in each warp, made a 1080p pan 5 times the full
+    search's time."""
+    cross, full = (best_time(vpp, ctx, c, "pan", 1920, 1080) for c in (vpp.MotionEstimatorH264ImplCross,
+                                                                      vpp.MotionEstimatorH264ImplFull))
+    assert cross < 4.2 * full
