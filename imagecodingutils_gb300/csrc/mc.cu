@@ -32,194 +32,28 @@ namespace {
 struct Plane {
     const short* p;
     int w, h;
-    __device__ __forceinline__ int at(int x, int y) const
-    {
-        x = x < 0 ? 0 : (x >= w ? w - 1 : x);
-        y = y < 0 ? 0 : (y >= h ? h - 1 : y);
-        return __ldg(p + (size_t)y * w + x);
-    }
 };
 
 constexpr int kMcWarps = 4;  // macroblocks per CTA, one warp each
 
-struct McLattice {
-    short win[22][24];     // luma window, 2 samples of margin on each side of the 17x17 the block reads
-    int th[22][16];        // unrounded horizontal 6-tap between window columns x+2 and x+3 (j cases only)
-    short cwin[2][9][10];  // the 9x9 chroma windows (U, V)
-};
-
-// the six-tap (1, -5, 20, 20, -5, 1) over samples s apart
-template <int kS, typename T>
-__device__ __forceinline__ int tap6(const T* p)
-{
-    return p[0] - 5 * p[kS] + 20 * p[2 * kS] + 20 * p[3 * kS] - 5 * p[4 * kS] + p[5 * kS];
-}
-
-// QuarterRead per quarter case cs = fx | fy << 2: one sample, or the
-// rounded average of two, from G (full-pel), b (horizontal half: 6-tap over a
-// window row), h (vertical half: 6-tap down a window column) and j (centre:
-// 6-tap down th).  Each entry: kind and offset of the first and the second
-// term (kind 4: none), offsets in window samples from the output sample's
-// row base &win[Y][X] (G(dx, dy) at (dy + 2) * 24 + dx + 2, b(dy) at
-// (dy + 2) * 24, h(dx) at dx + 2).
-enum : int { kTermG = 0, kTermB = 1, kTermH = 2, kTermJ = 3, kTermNone = 4 };
-__constant__ int4 c_quarter_terms[16] = {
-    {kTermG, 50, kTermNone, 0},  // 0: G
-    {kTermG, 50, kTermB, 48},    // 1: (G + b) / 2
-    {kTermB, 48, kTermNone, 0},  // 2: b
-    {kTermG, 51, kTermB, 48},    // 3: (G(x+1) + b) / 2
-    {kTermG, 50, kTermH, 2},     // 4: (G + h) / 2
-    {kTermB, 48, kTermH, 2},     // 5: (b + h) / 2
-    {kTermJ, 0, kTermB, 48},     // 6: (j + b) / 2
-    {kTermB, 48, kTermH, 3},     // 7: (b + h(x+1)) / 2
-    {kTermH, 2, kTermNone, 0},   // 8: h
-    {kTermJ, 0, kTermH, 2},      // 9: (j + h) / 2
-    {kTermJ, 0, kTermNone, 0},   // 10: j
-    {kTermJ, 0, kTermH, 3},      // 11: (j + h(x+1)) / 2
-    {kTermG, 74, kTermH, 2},     // 12: (G(y+1) + h) / 2
-    {kTermH, 2, kTermB, 72},     // 13: (h + b(y+1)) / 2
-    {kTermJ, 0, kTermB, 72},     // 14: (j + b(y+1)) / 2
-    {kTermH, 3, kTermB, 72},     // 15: (h(x+1) + b(y+1)) / 2
-};
-
-// The 256 luma samples of quarter case cs, lane (X = lane & 15,
-// Y = lane >> 4 + 2t): one compact loop per term kind (the kind is
-// warp-uniform), every shared access a constant offset from the lane's base.
-__device__ __forceinline__ void mc_luma_quarter(const McLattice& L, int cs, int lane, short* __restrict__ dst,
-                                                int stride)
-{
-    const int X = lane & 15, Y0 = lane >> 4;
-    const int4 tm = c_quarter_terms[cs];
-    const int nterm = tm.z == kTermNone ? 1 : 2;
-    int acc[8];
-#pragma unroll
-    for (int t = 0; t < 8; t++) acc[t] = 0;
-#pragma unroll 1
-    for (int e = 0; e < nterm; e++) {
-        const int kind = e ? tm.z : tm.x;
-        if (kind == kTermJ) {
-            const int* tb = &L.th[Y0][X];
-#pragma unroll
-            for (int t = 0; t < 8; t++) acc[t] += clip255((tap6<16>(tb + 32 * t) + 512) >> 10);
-            continue;
-        }
-        const short* w = &L.win[Y0][X] + (e ? tm.w : tm.y);
-        if (kind == kTermG) {
-#pragma unroll
-            for (int t = 0; t < 8; t++) acc[t] += w[48 * t];
-        } else if (kind == kTermB) {
-#pragma unroll
-            for (int t = 0; t < 8; t++) acc[t] += clip255((tap6<1>(w + 48 * t) + 16) >> 5);
-        } else {
-#pragma unroll
-            for (int t = 0; t < 8; t++) acc[t] += clip255((tap6<24>(w + 48 * t) + 16) >> 5);
-        }
-    }
-#pragma unroll
-    for (int t = 0; t < 8; t++)
-        dst[(size_t)(Y0 + 2 * t) * stride + X] = (short)(nterm == 1 ? acc[t] : (acc[t] + 1) >> 1);
-}
-
-// EighthRead of the two 8x8 chroma blocks at the vector in eighth-pel units,
-// from 9x9 windows staged one column per lane (U lanes 0-8, V lanes 16-24).
-__device__ __forceinline__ void mc_chroma_blocks(McLattice& L, const Plane& U, const Plane& V, int mvx, int mvy,
-                                                 int bx, int by, int lane, short* __restrict__ ou,
-                                                 short* __restrict__ ov)
-{
-    const int ex = mvx % 8, ey = mvy % 8;
-    const int dx = mvx / 8 + (ex < 0 ? -1 : 0), dy = mvy / 8 + (ey < 0 ? -1 : 0);
-    const int fx = ex < 0 ? ex + 8 : ex, fy = ey < 0 ? ey + 8 : ey;
-    const int pl = lane >> 4, c = lane & 15;
-    if (c < 9) {
-        const Plane& P = pl ? V : U;
-        int x = bx + dx + c;
-        x = x < 0 ? 0 : (x >= P.w ? P.w - 1 : x);
-        int q[9];
-#pragma unroll
-        for (int r = 0; r < 9; r++) {
-            int y = by + dy + r;
-            y = y < 0 ? 0 : (y >= P.h ? P.h - 1 : y);
-            q[r] = __ldg(P.p + (size_t)y * P.w + x);
-        }
-#pragma unroll
-        for (int r = 0; r < 9; r++) L.cwin[pl][r][c] = (short)q[r];
-    }
-    __syncwarp();
-    const int w00 = (8 - fx) * (8 - fy), w10 = fx * (8 - fy), w01 = (8 - fx) * fy, w11 = fx * fy;
-    const int x = lane & 7, y0 = lane >> 3;
-#pragma unroll
-    for (int t = 0; t < 4; t++) {  // t: U rows 0-3, U rows 4-7, V rows 0-3, V rows 4-7
-        const int y = y0 + 4 * (t & 1);
-        const short* p = &L.cwin[t >> 1][y][x];
-        const int s = (w00 * p[0] + w10 * p[1] + w01 * p[10] + w11 * p[11] + 32) >> 6;
-        (t < 2 ? ou : ov)[(size_t)(by + y) * U.w + bx + x] = (short)s;
-    }
-}
-
-// Any samples, any vector, one at a time: luma stages the 22x22 reference window around the vector's
-// full-pel position (one column per lane, rows clamped only at the frame edge), the j cases also the
-// horizontal 6-taps, then computes the quarter samples of its case from the term table.
-__device__ __noinline__ void mc_general(McLattice& L, const Plane& ry, const Plane& ru, const Plane& rv, int n, int m,
-                                        int mvx, int mvy, int lane, short* __restrict__ oy, short* __restrict__ ou,
-                                        short* __restrict__ ov)
-{
-    __syncwarp();
-    mc_chroma_blocks(L, ru, rv, mvx, mvy, n >> 1, m >> 1, lane, ou, ov);
-    short* dst = oy + (size_t)m * ry.w + n;
-    if (!(mvx | mvy)) {  // a zero vector keeps the block
-        const short* src = ry.p + (size_t)m * ry.w + n;
-        int q[8];
-#pragma unroll
-        for (int t = 0; t < 8; t++) q[t] = __ldg(src + (size_t)(2 * t + (lane >> 4)) * ry.w + (lane & 15));
-#pragma unroll
-        for (int t = 0; t < 8; t++) dst[(size_t)(2 * t + (lane >> 4)) * ry.w + (lane & 15)] = (short)q[t];
-        return;
-    }
-    // C quotient and remainder, a negative remainder folded as QuarterRead does
-    const int qx = mvx % 4, qy = mvy % 4;
-    const int ox = n + mvx / 4 + (qx < 0 ? -1 : 0) - 2, oy0 = m + mvy / 4 + (qy < 0 ? -1 : 0) - 2;
-    const int cs = (qx < 0 ? qx + 4 : qx) | ((qy < 0 ? qy + 4 : qy) << 2);
-    if (lane < 22) {
-        int x = ox + lane;
-        x = x < 0 ? 0 : (x >= ry.w ? ry.w - 1 : x);
-        const bool inside = oy0 >= 0 && oy0 + 22 <= ry.h;
-#pragma unroll
-        for (int h0 = 0; h0 < 22; h0 += 11) {  // two halves of 11 rows in flight
-            int q[11];
-            if (inside) {
-                const short* p = ry.p + (size_t)(oy0 + h0) * ry.w + x;
-#pragma unroll
-                for (int r = 0; r < 11; r++) q[r] = __ldg(p + (size_t)r * ry.w);
-            } else {
-#pragma unroll
-                for (int r = 0; r < 11; r++) q[r] = ry.at(x, oy0 + h0 + r);
-            }
-#pragma unroll
-            for (int r = 0; r < 11; r++) L.win[h0 + r][lane] = (short)q[r];
-        }
-    }
-    __syncwarp();
-    if (cs == 6 || cs == 9 || cs == 10 || cs == 11 || cs == 14) {  // the cases that read j
-        const int c = lane & 15, r0 = lane >> 4;
-#pragma unroll
-        for (int t = 0; t < 11; t++) L.th[r0 + 2 * t][c] = tap6<1>(&L.win[r0 + 2 * t][c]);
-        __syncwarp();
-    }
-    mc_luma_quarter(L, cs, lane, dst, ry.w);
-}
-
-// The packed path's shared memory: pairs of samples, the luma window from its first column, the vertical
-// 6-tap sums + TAP_BIAS of its columns (j cases), the chroma windows from an even column (U, then V).  At 14
-// words a row, four rows apart eight words lie in the 32 banks.
+// A macroblock's shared memory: its luma window from its first column (22 x 22 samples, two of margin on each side of
+// the 17 x 17 the block reads), its 9 x 9 chroma windows (U, then V) from an even column, and what the j cases read:
+// vertical 6-tap sums + TAP_BIAS of pairs of columns, or horizontal sums (any samples).  At 14 words a row, four rows
+// apart eight words lie in the 32 banks.
 struct McPairs {
     unsigned win[22][14];
-    unsigned vt[16][12];
     unsigned cwin[18][6];
+    union {
+        unsigned vt[16][12];
+        int th[22][16];
+    };
 };
 
-// The same terms for a lane's pair of columns (2p, 2p + 1), rows r .. r + 3, pairs of samples; p: lane & 7.
-// kind and offsets as in c_quarter_terms, the offset as dx | dy << 1.
-__constant__ int c_pair_terms[16] = {  // kind | offset << 3 of the first term, then << 8 of the second
+// QuarterRead per quarter case cs = fx | fy << 2: one sample, or the rounded average of two, from G (full-pel), b
+// (horizontal half: 6-tap over a window row), h (vertical half: 6-tap down a window column) and j (centre).  Each
+// entry: kind | offset << 3 of the first term, then << 8 of the second, the offset as dx | dy << 1.
+enum : int { kTermG = 0, kTermB = 1, kTermH = 2, kTermJ = 3, kTermNone = 4 };
+__constant__ int c_quarter_terms[16] = {
     kTermG | kTermNone << 8,                     kTermG | kTermB << 8,
     kTermB | kTermNone << 8,                     kTermG | 1 << 3 | kTermB << 8,
     kTermG | kTermH << 8,                        kTermB | kTermH << 8,
@@ -229,6 +63,69 @@ __constant__ int c_pair_terms[16] = {  // kind | offset << 3 of the first term, 
     kTermG | 2 << 3 | kTermH << 8,               kTermH | (kTermB | 2 << 3) << 8,
     kTermJ | (kTermB | 2 << 3) << 8,             kTermH | 1 << 3 | (kTermB | 2 << 3) << 8,
 };
+
+// the six-tap (1, -5, 20, 20, -5, 1) over samples s apart
+template <int kS, typename T>
+__device__ __forceinline__ int tap6(const T* p)
+{
+    return p[0] - 5 * p[kS] + 20 * p[2 * kS] + 20 * p[3 * kS] - 5 * p[4 * kS] + p[5 * kS];
+}
+
+// The block from windows of any samples, one at a time, lane (X = lane & 15, Y = lane >> 4 + 2t): a compact loop per
+// kind of term (warp-uniform).  odd: the chroma windows begin at their second column.
+__device__ __noinline__ void mc_any_samples(McPairs& L, int mvx, int mvy, bool odd, int lane, short* __restrict__ dst,
+                                            int stride, short* __restrict__ du, short* __restrict__ dv, int cstride)
+{
+    constexpr int kP = 28, kC = 12;  // shorts a row
+    const short* win = reinterpret_cast<const short*>(L.win);
+    const int X = lane & 15, Y0 = lane >> 4, terms = c_quarter_terms[(mvx & 3) | (mvy & 3) << 2];
+    if ((terms & 7) == kTermJ) {
+#pragma unroll
+        for (int t = 0; t < 11; t++) L.th[Y0 + 2 * t][X] = tap6<1>(win + (Y0 + 2 * t) * kP + X);
+        __syncwarp();
+    }
+    const int nterm = (terms >> 8 & 7) == kTermNone ? 1 : 2;
+    int acc[8];
+#pragma unroll
+    for (int t = 0; t < 8; t++) acc[t] = 0;
+#pragma unroll 1
+    for (int e = 0; e < nterm; e++) {
+        const int term = terms >> (8 * e), kind = term & 7, dx = term >> 3 & 1, dy = term >> 4 & 1;
+        const short* w = win + Y0 * kP + X;
+        if (kind == kTermJ) {
+            const int* tb = &L.th[Y0][X];
+#pragma unroll
+            for (int t = 0; t < 8; t++) acc[t] += clip255((tap6<16>(tb + 32 * t) + 512) >> 10);
+        } else if (kind == kTermG) {
+            w += (2 + dy) * kP + 2 + dx;
+#pragma unroll
+            for (int t = 0; t < 8; t++) acc[t] += w[2 * kP * t];
+        } else if (kind == kTermB) {
+            w += (2 + dy) * kP;
+#pragma unroll
+            for (int t = 0; t < 8; t++) acc[t] += clip255((tap6<1>(w + 2 * kP * t) + 16) >> 5);
+        } else {
+            w += 2 + dx;
+#pragma unroll
+            for (int t = 0; t < 8; t++) acc[t] += clip255((tap6<kP>(w + 2 * kP * t) + 16) >> 5);
+        }
+    }
+#pragma unroll
+    for (int t = 0; t < 8; t++)
+        dst[(size_t)(Y0 + 2 * t) * stride + X] = (short)(nterm == 1 ? acc[t] : (acc[t] + 1) >> 1);
+    // EighthRead of the chroma blocks: U rows 0-3, U rows 4-7, V rows 0-3, V rows 4-7
+    const int fx = mvx & 7, fy = mvy & 7, x = lane & 7, y0 = lane >> 3;
+    const int w00 = (8 - fx) * (8 - fy), w10 = fx * (8 - fy), w01 = (8 - fx) * fy, w11 = fx * fy;
+#pragma unroll
+    for (int t = 0; t < 4; t++) {
+        const int y = y0 + 4 * (t & 1);
+        const short* p = reinterpret_cast<const short*>(L.cwin) + (9 * (t >> 1) + y) * kC + x + odd;
+        const int v = (w00 * p[0] + w10 * p[1] + w01 * p[kC] + w11 * p[kC + 1] + 32) >> 6;
+        (t < 2 ? du : dv)[(size_t)y * cstride + x] = (short)v;
+    }
+}
+
+// The terms for a lane's pair of columns (2p, 2p + 1), rows r .. r + 3, pairs of samples 0..255; p: lane & 7.
 __device__ __forceinline__ void mc_pair_term(const McPairs& L, int term, int r, int p, unsigned (&out)[4])
 {
     const int kind = term & 7, dx = (term >> 3) & 1, dy = (term >> 4) & 1;
@@ -261,52 +158,79 @@ __device__ __forceinline__ void mc_pair_term(const McPairs& L, int term, int r, 
     }
 }
 
+// A pair of samples; kWide: 4-byte aligned.
+template <bool kWide>
+__device__ __forceinline__ void store_pair(short* d, unsigned v)
+{
+    if (kWide) {
+        *reinterpret_cast<unsigned*>(d) = v;
+    } else {
+        d[0] = (short)v;
+        d[1] = (short)(v >> 16);
+    }
+}
+
 // One warp per macroblock: its 16x16 luma block and its two 8x8 chroma blocks.  What bounds it is latency and
 // instructions: a sample at a time, the chroma blocks before the luma window was asked for, a 1920x1088 frame
 // took 12.2 us (750 instructions a macroblock; its 13 MB are 2 us, a launch with nothing in it 4).  Here
-// everything the vector points at is asked for at once, in 8- and 4-byte loads, and computed on pairs of
-// samples: 10.1 us (525 instructions; 8, 12 and 14 CTAs an SM 10.5, 10.3 and 11.1).  Past the frame's edge the
-// groups of samples that a load takes are inside or outside as a whole, so it costs the same; the macroblocks
-// there by another path were the launch's tail (12.6).  The packed path takes samples of 0..255 (seen from the
-// windows) and 16-byte aligned frames (wide); other macroblocks are computed by mc_general.  Warp-synchronous:
-// no block barrier.
+// everything the vector points at is asked for at once and computed on pairs of samples: 10.1 us (525 instructions;
+// 8, 12 and 14 CTAs an SM 10.5, 10.3 and 11.1).  kWide, 16-byte aligned frames: loads of 8 and 4 bytes.  Past the
+// frame's edge the groups of samples that a load takes are inside or outside as a whole, so it costs the same; the
+// macroblocks there by another path were the launch's tail (12.6).  Pairs hold samples of 0..255 (seen from the
+// windows); macroblocks with others are computed from the same windows by mc_any_samples (a frame full of them
+// 10.3 us; with a second staging of their own 16.3).  Frames at other alignments take loads of a sample, 12.3 us.
+// Warp-synchronous: no block barrier.
+template <bool kWide>
 __global__ void __launch_bounds__(32 * kMcWarps, 10) k_mc_frame(const __grid_constant__ Plane ry,
                                                                const __grid_constant__ Plane ru,
                                                                const __grid_constant__ Plane rv,
                                                                const int* __restrict__ mv, int cols, int nmb,
-                                                               bool wide, short* __restrict__ oy,
-                                                               short* __restrict__ ou, short* __restrict__ ov)
+                                                               short* __restrict__ oy, short* __restrict__ ou,
+                                                               short* __restrict__ ov)
 {
-    __shared__ union Store {
-        McLattice general;
-        McPairs pairs;
-    } store[kMcWarps];
+    __shared__ McPairs store[kMcWarps];
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     const int k = blockIdx.x * kMcWarps + w;
     if (k >= nmb) return;  // whole warps only
     const int mbr = k / cols, n = (k - mbr * cols) * 16, m = mbr * 16;
     const int v = __ldg(mv + k), mvx = vppgpu::mv_x(v), mvy = vppgpu::mv_y(v);
-    if (wide && !(mvx | mvy)) {  // a zero vector keeps the blocks
-        const size_t at = (size_t)(m + (lane >> 1)) * ry.w + n + 8 * (lane & 1);
-        const uint4 y = __ldg(reinterpret_cast<const uint4*>(ry.p + at));
-        const size_t cat = (size_t)((m >> 1) + (lane & 7)) * ru.w + (n >> 1);
-        if (lane < 16) {
-            const uint4 c = __ldg(reinterpret_cast<const uint4*>((lane < 8 ? ru.p : rv.p) + cat));
-            *reinterpret_cast<uint4*>((lane < 8 ? ou : ov) + cat) = c;
+    if (!(mvx | mvy)) {  // a zero vector keeps the blocks
+        if (kWide) {
+            const size_t at = (size_t)(m + (lane >> 1)) * ry.w + n + 8 * (lane & 1);
+            const uint4 y = __ldg(reinterpret_cast<const uint4*>(ry.p + at));
+            const size_t cat = (size_t)((m >> 1) + (lane & 7)) * ru.w + (n >> 1);
+            if (lane < 16) {
+                const uint4 c = __ldg(reinterpret_cast<const uint4*>((lane < 8 ? ru.p : rv.p) + cat));
+                *reinterpret_cast<uint4*>((lane < 8 ? ou : ov) + cat) = c;
+            }
+            *reinterpret_cast<uint4*>(oy + at) = y;
+        } else {
+            const size_t at = (size_t)(m + (lane >> 4)) * ry.w + n + (lane & 15);
+            const size_t cat = (size_t)((m >> 1) + (lane >> 3)) * ru.w + (n >> 1) + (lane & 7);
+            short y[8], c[4];
+#pragma unroll
+            for (int t = 0; t < 8; t++) y[t] = __ldg(ry.p + at + (size_t)(2 * t) * ry.w);
+#pragma unroll
+            for (int t = 0; t < 4; t++) c[t] = __ldg((t < 2 ? ru.p : rv.p) + cat + (size_t)(4 * (t & 1)) * ru.w);
+#pragma unroll
+            for (int t = 0; t < 8; t++) oy[at + (size_t)(2 * t) * ry.w] = y[t];
+#pragma unroll
+            for (int t = 0; t < 4; t++) (t < 2 ? ou : ov)[cat + (size_t)(4 * (t & 1)) * ru.w] = c[t];
         }
-        *reinterpret_cast<uint4*>(oy + at) = y;
         return;
     }
     // floor quotients and remainders: what QuarterRead's and EighthRead's folding of negative ones gives
     const int ox = n + (mvx >> 2) - 2, oy0 = m + (mvy >> 2) - 2, cs = (mvx & 3) | (mvy & 3) << 2;
     const int cx = (n >> 1) + (mvx >> 3), cy = (m >> 1) + (mvy >> 3);
-    const bool inside = ox >= 0 && ox + 22 <= ry.w && cx >= 0 && cx + 9 <= ru.w;  // between the sides
-    if (wide) {
-        McPairs& L = store[w].pairs;
-        const int q = lane & 7, r4 = lane >> 3, dx = ox & 3;
-        const bool odd = cx & 1;
+    McPairs& L = store[w];
+    const int q = lane & 7, r4 = lane >> 3;
+    const bool odd = kWide && (cx & 1);
+    unsigned all = 0;
+    if (kWide) {
+        const bool inside = ox >= 0 && ox + 22 <= ry.w && cx >= 0 && cx + 9 <= ru.w;  // between the sides
+        const int dx = ox & 3;
         uint2 y[6];
-        unsigned c[5], all = 0;
+        unsigned c[5];
         // a group of four (two) samples of a row is inside the frame or outside it as a whole
         const int gx = (ox & ~3) + 4 * q, gc = (cx & ~1) + 2 * q;
         const short* py = ry.p + min(max(gx, 0), ry.w - 4);
@@ -350,50 +274,77 @@ __global__ void __launch_bounds__(32 * kMcWarps, 10) k_mc_frame(const __grid_con
             all |= c[i];
             if (q < 5 && r4 + 4 * i < 18) L.cwin[r4 + 4 * i][q] = c[i];
         }
-        const bool bytes = !__any_sync(0xffffffffu, (all & 0xff00ff00u) != 0u);
-        __syncwarp();
-        if (bytes) {
-            const int term = c_pair_terms[cs], kind1 = term & 7, kind2 = (term >> 8) & 7;
-            if (kind1 == kTermJ) {  // vertical sums of the window's words, two halves of eight rows
-                if (lane < 24) {
-                    const int wd = lane < 12 ? lane : lane - 12, r0 = lane < 12 ? 0 : 8;
-                    unsigned x[13];
+    } else {  // a column per lane: chroma (lanes 0-8 U, 16-24 V) and half the luma rows in flight together
+        const Plane& P = lane < 16 ? ru : rv;
+        const int cc = lane & 15, x = min(max(ox + lane, 0), ry.w - 1), xc = min(max(cx + cc, 0), ru.w - 1);
+        short* win = reinterpret_cast<short*>(L.win) + lane;
+        short* cw = reinterpret_cast<short*>(L.cwin) + 9 * 12 * (lane >> 4) + cc;
+        short c[9];
 #pragma unroll
-                    for (int i = 0; i < 13; i++) x[i] = L.win[r0 + i][wd];
+        for (int r = 0; r < 9; r++)
+            c[r] = cc < 9 ? __ldg(P.p + (size_t)min(max(cy + r, 0), ru.h - 1) * ru.w + xc) : (short)0;
 #pragma unroll
-                    for (int i = 0; i < 8; i++)
-                        L.vt[r0 + i][wd] = vppgpu::tap_pair(x[i], x[i + 1], x[i + 2], x[i + 3], x[i + 4], x[i + 5]);
-                }
-                __syncwarp();
+        for (int h0 = 0; h0 < 22; h0 += 11) {
+            short y[11];
+#pragma unroll
+            for (int r = 0; r < 11; r++)
+                y[r] = lane < 22 ? __ldg(ry.p + (size_t)min(max(oy0 + h0 + r, 0), ry.h - 1) * ry.w + x) : (short)0;
+#pragma unroll
+            for (int r = 0; r < 11; r++) {
+                all |= (unsigned short)y[r];
+                if (lane < 22) win[28 * (h0 + r)] = y[r];
             }
-            const int r = 4 * r4;
-            unsigned o[4];
-            mc_pair_term(L, term, r, q, o);
-            if (kind2 != kTermNone) {
-                unsigned o2[4];
-                mc_pair_term(L, term >> 8, r, q, o2);
+        }
 #pragma unroll
-                for (int i = 0; i < 4; i++) o[i] = ((o[i] + o2[i] + 0x00010001u) >> 1) & 0x00ff00ffu;
-            }
-            unsigned* dst = reinterpret_cast<unsigned*>(oy + (size_t)(m + r) * ry.w + n) + q;
-#pragma unroll
-            for (int i = 0; i < 4; i++) dst[(size_t)i * (ry.w / 2)] = o[i];
-            // chroma: a pair of columns of a row per lane and plane
-            const int fx = mvx & 7, fy = mvy & 7, cr = lane >> 2, cp = lane & 3;
-            const unsigned w00 = (8 - fx) * (8 - fy), w10 = fx * (8 - fy), w01 = (8 - fx) * fy, w11 = fx * fy;
-            const size_t cat = (size_t)((m >> 1) + cr) * ru.w + (n >> 1) + 2 * cp;
-#pragma unroll
-            for (int pl = 0; pl < 2; pl++) {
-                const unsigned *p0 = &L.cwin[9 * pl + cr][cp], *p1 = p0 + 6;
-                const unsigned f0 = __funnelshift_r(p0[0], p0[1], 16), f1 = __funnelshift_r(p1[0], p1[1], 16);
-                const unsigned s = w00 * (odd ? f0 : p0[0]) + w10 * (odd ? p0[1] : f0) + w01 * (odd ? f1 : p1[0]) +
-                                   w11 * (odd ? p1[1] : f1) + 0x00200020u;
-                *reinterpret_cast<unsigned*>((pl ? ov : ou) + cat) = (s >> 6) & 0x00ff00ffu;
-            }
-            return;
+        for (int r = 0; r < 9; r++) {
+            all |= (unsigned short)c[r];
+            if (cc < 9) cw[12 * r] = c[r];
         }
     }
-    mc_general(store[w].general, ry, ru, rv, n, m, mvx, mvy, lane, oy, ou, ov);
+    const bool bytes = !__any_sync(0xffffffffu, (all & 0xff00ff00u) != 0u);
+    __syncwarp();
+    if (!bytes) {
+        const size_t cat = (size_t)(m >> 1) * ru.w + (n >> 1);
+        mc_any_samples(L, mvx, mvy, odd, lane, oy + (size_t)m * ry.w + n, ry.w, ou + cat, ov + cat, ru.w);
+        return;
+    }
+    const int term = c_quarter_terms[cs], kind1 = term & 7, kind2 = (term >> 8) & 7;
+    if (kind1 == kTermJ) {  // vertical sums of the window's words, two halves of eight rows
+        if (lane < 24) {
+            const int wd = lane < 12 ? lane : lane - 12, r0 = lane < 12 ? 0 : 8;
+            unsigned x[13];
+#pragma unroll
+            for (int i = 0; i < 13; i++) x[i] = L.win[r0 + i][wd];
+#pragma unroll
+            for (int i = 0; i < 8; i++)
+                L.vt[r0 + i][wd] = vppgpu::tap_pair(x[i], x[i + 1], x[i + 2], x[i + 3], x[i + 4], x[i + 5]);
+        }
+        __syncwarp();
+    }
+    const int r = 4 * r4;
+    unsigned o[4];
+    mc_pair_term(L, term, r, q, o);
+    if (kind2 != kTermNone) {
+        unsigned o2[4];
+        mc_pair_term(L, term >> 8, r, q, o2);
+#pragma unroll
+        for (int i = 0; i < 4; i++) o[i] = ((o[i] + o2[i] + 0x00010001u) >> 1) & 0x00ff00ffu;
+    }
+    short* dst = oy + (size_t)(m + r) * ry.w + n + 2 * q;
+#pragma unroll
+    for (int i = 0; i < 4; i++) store_pair<kWide>(dst + (size_t)i * ry.w, o[i]);
+    // chroma: a pair of columns of a row per lane and plane
+    const int fx = mvx & 7, fy = mvy & 7, cr = lane >> 2, cp = lane & 3;
+    const unsigned w00 = (8 - fx) * (8 - fy), w10 = fx * (8 - fy), w01 = (8 - fx) * fy, w11 = fx * fy;
+    const size_t cat = (size_t)((m >> 1) + cr) * ru.w + (n >> 1) + 2 * cp;
+#pragma unroll
+    for (int pl = 0; pl < 2; pl++) {
+        const unsigned *p0 = &L.cwin[9 * pl + cr][cp], *p1 = p0 + 6;
+        const unsigned f0 = __funnelshift_r(p0[0], p0[1], 16), f1 = __funnelshift_r(p1[0], p1[1], 16);
+        const unsigned s = w00 * (odd ? f0 : p0[0]) + w10 * (odd ? p0[1] : f0) + w01 * (odd ? f1 : p1[0]) +
+                           w11 * (odd ? p1[1] : f1) + 0x00200020u;
+        store_pair<kWide>((pl ? ov : ou) + cat, (s >> 6) & 0x00ff00ffu);
+    }
 }
 
 // a = clip255(a + b) or a -= b, 8 samples per thread (16-byte accesses), the tail one by one.
@@ -496,10 +447,11 @@ int vppgpu_mc_compensate_device(vppgpu_mc* mc, const short* d_ref_yuv, const sho
         src = mc->d_tmp;
     }
     if (cols * rows > 0) {
-        k_mc_frame<<<(cols * rows + kMcWarps - 1) / kMcWarps, 32 * kMcWarps, 0, ctx->stream>>>(
-            Plane{src, W, H}, Plane{src + ny, cw, ch}, Plane{src + ny + nc, cw, ch}, (const int*)d_mv, cols,
-            cols * rows, (((uintptr_t)src | (uintptr_t)d_out_yuv) & 15) == 0, d_out_yuv, d_out_yuv + ny,
-            d_out_yuv + ny + nc);
+        const Plane py{src, W, H}, pu{src + ny, cw, ch}, pv{src + ny + nc, cw, ch};
+        const int grid = (cols * rows + kMcWarps - 1) / kMcWarps;
+        const auto kernel = (((uintptr_t)src | (uintptr_t)d_out_yuv) & 15) == 0 ? k_mc_frame<true> : k_mc_frame<false>;
+        kernel<<<grid, 32 * kMcWarps, 0, ctx->stream>>>(py, pu, pv, (const int*)d_mv, cols, cols * rows, d_out_yuv,
+                                                        d_out_yuv + ny, d_out_yuv + ny + nc);
         VPP_CHECK_LAUNCH(ctx);
         ctx->launches++;
     }

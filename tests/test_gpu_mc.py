@@ -139,3 +139,34 @@ def test_sample_ranges_and_alignments(vpp, ctx, orc, spread, w, h, shift):
             np.testing.assert_array_equal(got, want)
     finally:
         L.vppgpu_mc_destroy(mc)
+
+
+def test_samples_of_any_range_cost_no_second_pass(vpp, ctx):
+    """Frames of samples outside 0..255 against frames of bytes: read and staged twice they took 1.6 times as long."""
+    import time
+
+    torch = pytest.importorskip("torch")
+    from imagecodingutils_gb300 import _lib
+    L = vpp.load()
+    w, h = 1920, 1088
+    n, nmb = w * h * 3 // 2, (w // 16) * (h // 16)
+    r = synth.splitmix64(990, n).astype(np.int64)
+    mv = torch.from_numpy((synth.splitmix64(991, 2 * nmb) % np.uint64(128)).astype(np.int16) - 64).cuda()
+    mc = C.c_void_p()
+    _lib.check(L.vppgpu_mc_create(ctx.handle, w, h, 32, C.byref(mc)), "create")
+    best = []
+    for yuv in (r % 256, r % 4096 - 2048):
+        src = torch.from_numpy(yuv.astype(np.int16)).cuda()
+        out = torch.empty_like(src)
+        torch.cuda.synchronize()
+        t = []
+        for _ in range(6):
+            t0 = time.perf_counter()
+            for _ in range(200):
+                _lib.check(L.vppgpu_mc_compensate_device(mc, C.c_void_p(src.data_ptr()), C.c_void_p(mv.data_ptr()),
+                                                         C.c_void_p(out.data_ptr())), "compensate")
+            ctx.synchronize()
+            t.append(time.perf_counter() - t0)
+        best.append(min(t))
+    L.vppgpu_mc_destroy(mc)
+    assert best[1] < 1.35 * best[0]
