@@ -417,6 +417,9 @@ __device__ __forceinline__ void roundtrip_plane(const vppgpu::TqJob& j, const We
         unsigned far = 0;
 #pragma unroll
         for (int r = 0; r < 4; r++) far |= ((rows[r].x + 0x01000100u) | (rows[r].y + 0x01000100u)) & 0xfe00fe00u;
+        // one form for the warp: residuals around the bound would have it go through both (a plane of -300..300 8.3 us
+        // for 6.2)
+        far = __any_sync(__activemask(), far != 0u);
         if (wt.flat && !far) roundtrip_block<kColsFirst, true>(rows, j.lev + off, j.rec + off, j.stride, c, wt.w);
         else roundtrip_block<kColsFirst, false>(rows, j.lev + off, j.rec + off, j.stride, c, wt.w);
 #pragma unroll
