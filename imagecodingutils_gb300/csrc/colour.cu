@@ -238,9 +238,15 @@ template <int kKind>
 void launch_kind(vppgpu_ctx* ctx, const unsigned char* bgr, int nframes, int w, int h, int chr_off, int flip, short* y,
                  short* u, short* v)
 {
-    // eight pixels a thread with 8- and 16-byte accesses where rows and planes are aligned to them
+    // Eight pixels a thread with 8- and 16-byte accesses where rows and planes are aligned to them.  A pixel of the
+    // real kinds can be a chain of doubles (luma or chroma on a whole number), so theirs also have to fill the GPU, two
+    // CTAs an SM: a 176x144 frame of colours in steps of 50 took 30.8 us by eight a thread and 11.4 by a block (10.3
+    // before either); pictures, one 640x480 frame 8.2 and 6.1, one 1280x720 frame 8.3 both, one 1920x1080 frame 8.3
+    // and 9.3, eight 33.0 and 45.2.
     const uintptr_t a16 = (uintptr_t)y, a8 = (uintptr_t)u | (uintptr_t)v | (uintptr_t)bgr;
-    const bool wide = (w & 7) == 0 && (a16 & 15) == 0 && (a8 & 7) == 0;
+    const long long eights = ((long long)(w >> 3) * (h >> 1) + 255) / 256 * nframes;
+    const bool wide = (w & 7) == 0 && (a16 & 15) == 0 && (a8 & 7) == 0 &&
+                      (kKind == VPPGPU_RGB_FIXED_POINT || eights >= 2 * ctx->sm_count);
     const long long work = (long long)(w >> (wide ? 3 : 1)) * (h >> 1), blocks = (work + 255) / 256;
     const dim3 grid((unsigned)(blocks < 4096 ? blocks : 4096), nframes);
     if (wide) k_rgb_x8<kKind><<<grid, 256, 0, ctx->stream>>>(bgr, w, h, chr_off, flip, y, u, v);

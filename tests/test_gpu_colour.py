@@ -103,3 +103,50 @@ def test_widths_and_alignments(vpp, ctx, orc, kind, w, h, off, yoff):
             np.testing.assert_array_equal(t[yoff + f * m:yoff + (f + 1) * m].cpu().numpy(), want.reshape(-1))
     for t, m in zip(out, (n, n // 4, n // 4)):
         assert (t[:yoff] == 77).all() and (t[yoff + nf * m:] == 77).all()
+
+
+@pytest.mark.parametrize("kind", [1, 2])
+@pytest.mark.parametrize("w,h,nf,flip", [(1280, 720, 1, 1), (1280, 720, 2, 0), (1280, 720, 2, 1), (1920, 1080, 1, 1)])
+def test_real_kinds_at_the_change_of_kernel(vpp, ctx, orc, kind, w, h, nf, flip):
+    """Aligned frames too small to fill the GPU by eight pixels a thread, and large enough; colours in steps of 25, so
+    that many terms lie on whole numbers."""
+    import ctypes as C
+    torch = pytest.importorskip("torch")
+    from imagecodingutils_gb300 import _lib
+    bgr = np.stack([synth.rgb_frame(31 + f, w, h) // 25 * 25 for f in range(nf)])
+    src = torch.from_numpy(bgr).cuda()
+    out = [torch.zeros(nf * m, dtype=torch.int16, device="cuda") for m in (w * h, w * h // 4, w * h // 4)]
+    torch.cuda.synchronize()
+    _lib.check(vpp.load().vppgpu_rgb24_to_yuv420_frames_device(ctx.handle, kind, C.c_void_p(src.data_ptr()), nf, w, h, 128,
+                                                               flip, *[C.c_void_p(t.data_ptr()) for t in out]), "convert")
+    ctx.synchronize()
+    for f in range(nf):
+        for t, want in zip(out, orc.rgb_to_yuv(kind, bgr[f], 128, flip)):
+            np.testing.assert_array_equal(t.cpu().numpy()[f * want.size:(f + 1) * want.size], want.reshape(-1))
+
+
+def test_real_kinds_on_small_frames(vpp, ctx):
+    """Colours whose terms lie on whole numbers, each a chain of doubles: eight pixels a thread made a small frame of
+    them 3.7 times as long as a noisy one."""
+    import ctypes as C
+    import time
+    torch = pytest.importorskip("torch")
+    from imagecodingutils_gb300 import _lib
+    w, h = 176, 144
+    noise = synth.rgb_frame(3, w, h)
+    out = [torch.zeros(m, dtype=torch.int16, device="cuda") for m in (w * h, w * h // 4, w * h // 4)]
+    best = []
+    for bgr in (noise, noise // 50 * 50):
+        src = torch.from_numpy(np.ascontiguousarray(bgr)).cuda()
+        torch.cuda.synchronize()
+        t = []
+        for _ in range(6):
+            t0 = time.perf_counter()
+            for _ in range(200):
+                _lib.check(vpp.load().vppgpu_rgb24_to_yuv420_frames_device(
+                    ctx.handle, 1, C.c_void_p(src.data_ptr()), 1, w, h, 128, 0, *[C.c_void_p(x.data_ptr()) for x in out]),
+                    "convert")
+            ctx.synchronize()
+            t.append(time.perf_counter() - t0)
+        best.append(min(t))
+    assert best[1] < 2.6 * best[0]
