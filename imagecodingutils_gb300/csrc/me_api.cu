@@ -857,8 +857,14 @@ extern "C" int vppgpu_me_autotune_pairs(vppgpu_me* me, const short* const* d_src
                                         int npairs, int reps, int* chosen)
 {
     if (!me || !d_src || !d_ref || npairs < 1 || reps < 1) return VPPGPU_ERR_INVALID_ARG;
+    // samples at any even address, except the input where k_full_planes packs it by pairs
+    const size_t src_align = me->kind == VPPGPU_ME_MULTIRES_CROSS || me->kind == VPPGPU_ME_H263_MULTIRES_CROSS ||
+                                     me->kind == VPPGPU_ME_H263_MULTIRES_CROSS_V2
+                                 ? sizeof(short)
+                                 : 2 * sizeof(short);
     for (int p = 0; p < npairs; p++)
-        if (!d_src[p] || !d_ref[p]) return VPPGPU_ERR_INVALID_ARG;
+        if (!d_src[p] || !d_ref[p] || !aligned(d_src[p], src_align) || !aligned(d_ref[p], sizeof(short)))
+            return VPPGPU_ERR_INVALID_ARG;
     if (me->kind == VPPGPU_ME_FULL_SAD || me->kind == VPPGPU_ME_IMPL1 ||
         me->kind == VPPGPU_ME_IMPL2) {  // one configuration: nothing to tune
         if (chosen) *chosen = 0;

@@ -58,21 +58,29 @@ __device__ __forceinline__ unsigned bytes4(const short* p, bool& bad)
     bad |= ((lo | hi) & 0xff00ff00u) != 0u;
     return __byte_perm(lo, hi, 0x6420);
 }
-// 2:1 decimation (OverlayMem2Dv2::Half, OverlayMem2Dv2.cpp:3018-3033) at (x, y); pairs of shorts are
-// 4-byte aligned (planes are, rows are a multiple of 16 wide).
+// 2:1 decimation (OverlayMem2Dv2::Half, OverlayMem2Dv2.cpp:3018-3033) at (x, y); kPairs: pairs of shorts are
+// 4-byte aligned (the plane is, rows are a multiple of 16 wide).
+template <bool kPairs>
 __device__ __forceinline__ int half_at(const short* p, int w, int x, int y)
 {
+    if (!kPairs) {
+        const short* s = p + (size_t)(2 * y) * w + 2 * x;
+        return ((int)__ldg(s) + __ldg(s + 1) + __ldg(s + w) + __ldg(s + w + 1) + 2) >> 2;
+    }
     const unsigned* q = reinterpret_cast<const unsigned*>(p + (size_t)(2 * y) * w + 2 * x);
     const unsigned a = __ldg(q), b = __ldg(q + w / 2);
     return ((int)(short)a + ((int)a >> 16) + (int)(short)b + ((int)b >> 16) + 2) >> 2;
 }
+template <bool kPairs>
 __device__ __forceinline__ int quarter_at(const short* p, int w, int x, int y)
 {
-    return ((half_at(p, w, 2 * x, 2 * y) & 0xff) + (half_at(p, w, 2 * x + 1, 2 * y) & 0xff) +
-            (half_at(p, w, 2 * x, 2 * y + 1) & 0xff) + (half_at(p, w, 2 * x + 1, 2 * y + 1) & 0xff) + 2) >> 2;
+    return ((half_at<kPairs>(p, w, 2 * x, 2 * y) & 0xff) + (half_at<kPairs>(p, w, 2 * x + 1, 2 * y) & 0xff) +
+            (half_at<kPairs>(p, w, 2 * x, 2 * y + 1) & 0xff) + (half_at<kPairs>(p, w, 2 * x + 1, 2 * y + 1) & 0xff) + 2) >> 2;
 }
 
-// keep, when not null: where the searches at a prediction find the arguments.
+// keep, when not null: where the searches at a prediction find the arguments.  kPairs: both planes are 4-byte
+// aligned (an estimate's are; a tuning call takes any).
+template <bool kPairs>
 __global__ void __launch_bounds__(256) k_mrc_levels(MrcArgs a, const short* __restrict__ src16,
                                                    const short* __restrict__ ref16, MrcArgs* keep)
 {
@@ -108,7 +116,7 @@ __global__ void __launch_bounds__(256) k_mrc_levels(MrcArgs a, const short* __re
         const int y = (int)(4 * i / w1), x = (int)(4 * i - y * w1);
         unsigned v = 0;
 #pragma unroll
-        for (int k = 0; k < 4; k++) v |= (unsigned)(half_at(src16, W, x + k, y) & 0xff) << (8 * k);
+        for (int k = 0; k < 4; k++) v |= (unsigned)(half_at<kPairs>(src16, W, x + k, y) & 0xff) << (8 * k);
         reinterpret_cast<unsigned*>(const_cast<unsigned char*>(a.in1.p))[i] = v;
     }
     for (unsigned i = first; i < m1; i += step) {
@@ -117,7 +125,7 @@ __global__ void __launch_bounds__(256) k_mrc_levels(MrcArgs a, const short* __re
         unsigned v = 0;
 #pragma unroll
         for (int k = 0; k < 4; k++) {
-            v |= (unsigned)(half_at(ref16, W, min(max(x - 9, 0), (int)w1 - 1), min(max(y - 9, 0), (int)h1 - 1)) & 0xff) << (8 * k);
+            v |= (unsigned)(half_at<kPairs>(ref16, W, min(max(x - 9, 0), (int)w1 - 1), min(max(y - 9, 0), (int)h1 - 1)) & 0xff) << (8 * k);
             if (++x == (int)ew) {
                 x = 0;
                 y++;
@@ -127,13 +135,13 @@ __global__ void __launch_bounds__(256) k_mrc_levels(MrcArgs a, const short* __re
     }
     for (unsigned i = first; i < n2; i += step) {
         const int y = (int)(i / w2), x = (int)(i - y * w2);
-        const_cast<unsigned char*>(a.in2.p)[i] = (unsigned char)quarter_at(src16, W, x, y);
+        const_cast<unsigned char*>(a.in2.p)[i] = (unsigned char)quarter_at<kPairs>(src16, W, x, y);
     }
     for (unsigned i = first; i < m2; i += step) {
         const unsigned ew = w2 + 10;
         const int y = (int)(i / ew), x = (int)(i - y * ew);
         const_cast<unsigned char*>(a.e2.p)[i] =
-            (unsigned char)quarter_at(ref16, W, min(max(x - 5, 0), (int)w2 - 1), min(max(y - 5, 0), (int)h2 - 1));
+            (unsigned char)quarter_at<kPairs>(ref16, W, min(max(x - 5, 0), (int)w2 - 1), min(max(y - 5, 0), (int)h2 - 1));
     }
     if (__any_sync(0xffffffffu, bad) && (threadIdx.x & 31) == 0) atomicOr(&a.ctrl->status, ST_PIXEL_RANGE);
 }
@@ -840,7 +848,8 @@ int levels_launch(vppgpu_ctx* ctx, const MrcArgs& a, const short* d_src16, const
 {
     const long long words = ((long long)(a.W + 38) * (a.H + 38) + 3) / 4, blocks = (words + 255) / 256;
     const int cap = ctx->sm_count * 8;
-    k_mrc_levels<<<(int)(blocks < cap ? blocks : cap), 256, 0, ctx->stream>>>(a, d_src16, d_ref16, keep);
+    const auto kernel = (((uintptr_t)d_src16 | (uintptr_t)d_ref16) & 3) == 0 ? k_mrc_levels<true> : k_mrc_levels<false>;
+    kernel<<<(int)(blocks < cap ? blocks : cap), 256, 0, ctx->stream>>>(a, d_src16, d_ref16, keep);
     VPP_CHECK_LAUNCH(ctx);
     return VPPGPU_OK;
 }

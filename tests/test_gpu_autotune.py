@@ -31,3 +31,42 @@ def test_autotune_keeps_results(vpp, ctx, orc, cls, ofn, kw):
         mv_o, dist_o, _ = getattr(orc, ofn)(fr[k], fr[k - 1], 128, **kw)
         np.testing.assert_array_equal(mv, mv_o)
         np.testing.assert_array_equal(me.last_mb_distortion, dist_o)
+
+
+@pytest.mark.parametrize("kind,mode,src_off", [
+    ("ME_MULTIRES_CROSS", 1, 1), ("ME_MULTIRES_CROSS", 2, 1), ("ME_H263_MULTIRES_CROSS", 2, 1),
+    ("ME_H263_MULTIRES_CROSS_V2", 2, 1), ("ME_MULTIRES_CROSS_V2", 2, 0), ("ME_MULTIRES", 2, 0), ("ME_FULL", 0, 0)])
+def test_planes_at_any_sample(vpp, ctx, orc, kind, mode, src_off):
+    """A tuning call takes planes whose first sample is at any even address (the input's only where it is not packed by
+    pairs: there it is refused), and the estimate after it is the same."""
+    import ctypes as C
+    torch = pytest.importorskip("torch")
+    from imagecodingutils_gb300 import _lib
+    L = vpp.load()
+    w, h = 176, 144
+    fr = synth.pan_sequence(97, w, h, 2)
+    n = w * h
+    dev = []
+    for f, off in ((fr[1], src_off), (fr[0], 1)):
+        t = torch.zeros(n + 8, dtype=torch.int16, device="cuda")
+        t[off:off + n] = torch.from_numpy(f.reshape(-1)).cuda()
+        dev.append((t, C.c_void_p(t.data_ptr() + 2 * off)))
+    torch.cuda.synchronize()
+    hd = C.c_void_p()
+    _lib.check(L.vppgpu_me_create(ctx.handle, getattr(_lib, kind), w, h, 64, C.byref(hd)), "create")
+    try:
+        L.vppgpu_me_set_mode(hd, mode)
+        mv = [np.zeros((n // 256, 2), np.int16) for _ in range(2)]
+        avg = C.c_long()
+        for i in range(2):
+            _lib.check(L.vppgpu_me_estimate(hd, fr[1].ctypes.data, fr[0].ctypes.data, None, None, mv[i].ctypes.data, None,
+                                            C.byref(avg)), "estimate")
+            if i == 0:
+                idx = C.c_int()
+                _lib.check(L.vppgpu_me_autotune(hd, dev[0][1], dev[1][1], 1, C.byref(idx)), "autotune")
+        np.testing.assert_array_equal(mv[0], mv[1])
+        if src_off == 0:
+            assert L.vppgpu_me_autotune(hd, C.c_void_p(dev[0][0].data_ptr() + 2), dev[1][1], 1, None) == \
+                _lib.ERR_INVALID_ARG
+    finally:
+        L.vppgpu_me_destroy(hd)
