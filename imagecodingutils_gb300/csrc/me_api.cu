@@ -886,11 +886,20 @@ extern "C" int vppgpu_me_autotune_pairs(vppgpu_me* me, const short* const* d_src
         for (int r : {4, 8, 12, 16, 20, 24})
             if (r != cur.relax) cands.push_back({r, cur.grid, cur.bps, cur.warps});
     } else {
-        const int policies[][2] = {{4, 4}, {8, 8}, {14, 8}, {14, 4}, {14, 2}};
-        for (const auto& p : policies)
-            for (int bps : {2, 4, 8})
-                if (p[0] != cur.relax || p[1] != cur.grid || bps != cur.bps)
-                    cands.push_back({p[0], p[1], bps, cur.warps});
+        // The sweeps over the whole GPU before the cluster's rounds, and their grid.  relax_sweeps stays: it only says
+        // which rounds the statistics count as relaxation (and bounds the Lagrangian overload's sweeps, which are not
+        // timed here).  Each launch sequence once: a grid is no larger than the frame, and no sweep has none.
+        auto shape = [&](const TuneCfg& c) {
+            const int sweeps = c.grid < c.relax ? c.grid : c.relax, want = (me->nmb + 7) / 8, cap = me->ctx->sm_count * c.bps;
+            return sweeps ? (long long)sweeps << 32 | (want < cap ? want : cap) : 0LL;
+        };
+        for (int g : {0, 1, 2, 4})
+            for (int bps : {2, 4, 8}) {
+                const TuneCfg c{cur.relax, g, bps, cur.warps};
+                bool known = false;
+                for (const TuneCfg& k : cands) known |= shape(k) == shape(c);
+                if (!known) cands.push_back(c);
+            }
     }
     // time direct launches for every candidate (the captured graph is rebuilt afterwards)
     if (me->graph) {

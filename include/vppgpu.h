@@ -214,8 +214,9 @@ int vppgpu_me_set_relax_sweeps(vppgpu_me* me, int sweeps);
  * candidate must and is checked to give the same vectors) and keeps the
  * fastest; *chosen (nullable) is its index, 0 = the configuration before the
  * call.  Tunables: MultiresCross -- macroblocks per search CTA (2, 4, 8);
- * the others -- relaxation sweeps / of which over every MB, and the CTAs per
- * SM of such a sweep.  vppgpu_me_get_tuning returns {relaxation sweeps, grid
+ * Full, Multires, Ver2 and Cross -- sweeps over every MB before the cluster's
+ * rounds (0, 1, 2, 4) and their CTAs per SM; UMHS, FHS and H.263 Ver2 --
+ * relaxation sweeps.  vppgpu_me_get_tuning returns {relaxation sweeps, grid
  * sweeps, sweep CTAs per SM, search macroblocks per CTA}. */
 int vppgpu_me_autotune(vppgpu_me* me, const short* d_src, const short* d_ref, int reps, int* chosen);
 /* Same over several device frame pairs (each candidate timed over all). */

@@ -70,3 +70,23 @@ def test_planes_at_any_sample(vpp, ctx, orc, kind, mode, src_off):
                 _lib.ERR_INVALID_ARG
     finally:
         L.vppgpu_me_destroy(hd)
+
+
+@pytest.mark.parametrize("cls", ["MotionEstimatorH264ImplFull", "MotionEstimatorH264ImplMultires",
+                                 "MotionEstimatorH264ImplMultiresCrossVer2", "MotionEstimatorH264ImplCross"])
+def test_autotune_times_each_launch_sequence_once(vpp, ctx, cls):
+    """A small frame has four of them (0, 1, 2 and 4 sweeps before the cluster: any grid holds all of it), a candidate a
+    warm-up and a timed estimate each; the sweeps that only the statistics and the Lagrangian overload read stay."""
+    w, h = 176, 144
+    fr = synth.pan_sequence(96, w, h, 2)
+    me = getattr(vpp, cls)(fr[1], fr[0], w, h, 128, ctx=ctx)
+    assert me.Create() == 1
+    me.Estimate()
+    n0 = ctx.launch_count()
+    me.Estimate()
+    n1 = ctx.launch_count()
+    before = me.tuning()
+    after = me.Autotune(reps=1)
+    assert ctx.launch_count() - n1 <= 4 * 2 * (n1 - n0 + 3)  # (up to three more sweeps than the estimate's one)
+    assert after["relax_sweeps"] == before["relax_sweeps"]
+    assert after["grid_sweeps"] in (0, 1, 2, 4)
