@@ -251,12 +251,12 @@ void vo_quarter_read16(const short* plane, int w, int h, int x, int y, int qx, i
     free(e);
 }
 
-/* OverlayMem2Dv2::Half (OverlayMem2Dv2.cpp:3018-3033). */
+/* OverlayMem2Dv2::Half (OverlayMem2Dv2.cpp:3018-3033), whole pairs of rows and columns only. */
 void vo_half(const short* src, int w, int h, short* dst)
 {
     int hw = w / 2;
-    for (int m = 0, y = 0; m < h; m += 2, y++)
-        for (int n = 0, x = 0; n < w; n += 2, x++) {
+    for (int m = 0, y = 0; m + 1 < h; m += 2, y++)
+        for (int n = 0, x = 0; n + 1 < w; n += 2, x++) {
             const short* p = src + (size_t)m * w + n;
             dst[(size_t)y * hw + x] = (short)(((int)p[0] + p[1] + p[w] + p[w + 1] + 2) >> 2);
         }

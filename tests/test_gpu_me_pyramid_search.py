@@ -49,3 +49,12 @@ def test_against_oracle(vpp, ctx, orc, est, w, h, mr, mode, kind):
     np.testing.assert_array_equal(mv, mv_o)
     np.testing.assert_array_equal(me.last_mb_distortion, dist_o)
     assert avg == avg_o
+
+
+@pytest.mark.parametrize("kind,w,h,mr", [("half", 848, 478, 128), ("ties", 48, 38, 64), ("hard", 32, 50, 64),
+                                         ("half", 48, 37, 64), ("hard", 80, 19, 32)])
+@pytest.mark.parametrize("est", range(len(ESTIMATORS)))
+def test_heights_of_odd_levels(vpp, ctx, orc, est, kind, w, h, mr):
+    """Three levels of pictures whose height is no multiple of four: the last row of a level, and of its bordered copy,
+    comes from fewer rows than two."""
+    test_against_oracle(vpp, ctx, orc, est, w, h, mr, 2, kind)

@@ -667,3 +667,18 @@ def test_me_impl2_against_compiled_reference(orc, seed, w, h, rng, mode, gen):
     mv, _, avg = orc.me_impl2(fr[1], fr[0], rng, mode)
     np.testing.assert_array_equal(mv, mv_r)
     assert avg == avg_r
+
+
+@pytest.mark.parametrize("w,h", [(8, 4), (8, 5), (6, 3), (2, 1), (424, 239)])
+def test_half_keeps_to_whole_rows(orc, w, h):
+    """The 2:1 decimation of a plane of an odd height (the second level of a picture whose height is no multiple of four)
+    reads and writes whole pairs of rows, nothing past either plane."""
+    import ctypes as C
+    plane = np.full((h + 1, w), 7000, np.int16)
+    plane[:h] = np.arange(w * h).reshape(h, w) % 256
+    out = np.full((h // 2 + 1, w // 2), -77, np.int16)
+    orc.lib.vo_half(C.c_void_p(plane.ctypes.data), w, h, C.c_void_p(out.ctypes.data))
+    q = plane[:h // 2 * 2].astype(np.int64)
+    want = (q[0::2, 0::2] + q[0::2, 1::2] + q[1::2, 0::2] + q[1::2, 1::2] + 2) >> 2
+    np.testing.assert_array_equal(out[:h // 2], want)
+    assert (out[h // 2:] == -77).all()
