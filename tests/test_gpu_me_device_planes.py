@@ -61,3 +61,47 @@ def test_alignment(vpp, ctx, orc, kind, s_src, s_ref, w, h):
             buf[at] = was
     finally:
         L.vppgpu_me_destroy(handle)
+
+
+AVG_KINDS = [("ME_FULL", "me_full", None), ("ME_MULTIRES", "me_multires", 2), ("ME_MULTIRES_CROSS_V2", "me_multires_cross_v2", 2),
+             ("ME_MULTIRES_CROSS", "me_multires_cross", 1), ("ME_CROSS", "me_cross", 0),
+             ("ME_H263_MULTIRES_CROSS", "me_h263_multires_cross", 2), ("ME_FULL_SAD", "me_full_intpel", None)]
+
+
+@pytest.mark.parametrize("w,h", [(16, 16), (176, 150), (1040, 520), (1040, 516)])
+@pytest.mark.parametrize("kind", range(len(AVG_KINDS)))
+def test_average_on_the_device(vpp, ctx, orc, kind, w, h):
+    """The average that a device call writes, from the included macroblocks' distortions: every estimator that shares
+    the cluster resolve or the pyramid search, below and above the 2048 macroblocks where the SAD stage's launches
+    change, with a part of a macroblock row below the last whole one, on one handle twice and with none included."""
+    torch = pytest.importorskip("torch")
+    from imagecodingutils_gb300 import _lib
+    L = vpp.load()
+    name, fn, mode = AVG_KINDS[kind]
+    fr = synth.pan_sequence(520 + w, w, h, 3)
+    nmb = (w // 16) * (h // 16)
+    incl = (synth.splitmix64(w + h, nmb) % np.uint64(3) != 0).astype(np.uint8)
+    planes = [torch.from_numpy(f).cuda() for f in fr]
+    mv = torch.empty((nmb, 2), dtype=torch.int16, device="cuda")
+    avg = torch.full((3,), -7, dtype=torch.int64, device="cuda")
+    d_incl = torch.from_numpy(incl).cuda()
+    handle = C.c_void_p()
+    _lib.check(L.vppgpu_me_create(ctx.handle, getattr(_lib, name), w, h, 64, C.byref(handle)), "create")
+    try:
+        if mode is not None:
+            _lib.check(L.vppgpu_me_set_mode(handle, mode), "mode")
+        torch.cuda.synchronize()
+        for t, inc in ((1, d_incl), (2, d_incl), (2, torch.zeros_like(d_incl))):
+            _lib.check(L.vppgpu_me_estimate_device(handle, C.c_void_p(planes[t].data_ptr()),
+                                                   C.c_void_p(planes[t - 1].data_ptr()), C.c_void_p(inc.data_ptr()), None,
+                                                   C.c_void_p(mv.data_ptr()), None, C.c_void_p(avg.data_ptr() + 8)), "run")
+            ctx.synchronize()
+            mask = inc.cpu().numpy()
+            if name == "ME_FULL_SAD":
+                d = orc.me_full_intpel(fr[t], fr[t - 1], 64, metric=1)[1][mask.astype(bool)]
+                want = int(d.sum()) // d.size if d.size else 0
+            else:
+                want = getattr(orc, fn)(fr[t], fr[t - 1], 64, dist_incl=mask, **({} if mode is None else {"mode": mode}))[2]
+            assert avg.tolist() == [-7, want, -7]
+    finally:
+        L.vppgpu_me_destroy(handle)
