@@ -44,7 +44,7 @@ struct vppgpu_me {
     int* d_slice;
     vppgpu::MeCtrl* ctrl;
     int* changed;
-    int sweep_limit;
+    int sweep_limit;  // counters in `changed`
     int relax_sweeps;  // relaxation sweeps before the wavefront (0..RELAX_SWEEPS)
     int grid_sweeps;   // ... of which over every MB
     int relax_blocks_per_sm;  // grid of a sweep over every MB
@@ -188,9 +188,7 @@ vppgpu::FullArgs full_args(vppgpu_me* me, double lambda)
     a.job = me->d_job;
     a.ctrl = me->ctrl;
     a.changed = me->changed;
-    a.dirty = reinterpret_cast<unsigned*>(me->changed + vppgpu::RELAX_SWEEPS + 2);
     a.lambda = lambda;
-    a.sweep_limit = me->sweep_limit;
     a.relax_sweeps = me->relax_sweeps;
     a.grid_sweeps = me->grid_sweeps;
     a.relax_blocks_per_sm = me->relax_blocks_per_sm;
@@ -249,11 +247,8 @@ int run(vppgpu_me* me, const short* d_src16, const short* d_ref16, const unsigne
     if (me->kind == VPPGPU_ME_MULTIRES_CROSS_V2 || me->kind == VPPGPU_ME_MULTIRES) {
         // GetBestVector's lambda: 0.9 (MultiresCrossVer2.cpp:1050), 1.1 (Multires.cpp:958)
         const bool v2 = me->kind == VPPGPU_ME_MULTIRES_CROSS_V2;
-        if (v2 && v2_lambda) {  // Estimate(long*, void* lambda) (MultiresCrossVer2.cpp:1162-1742)
-            vppgpu::FullArgs a = full_args(me, lambda);
-            a.grid_sweeps = a.relax_sweeps;  // an evaluation is a search: every sweep over the whole GPU
-            return vppgpu::mrc2_launch(ctx, 4, me->mode, me->d_mrc, a, d_src16, d_ref16);
-        }
+        if (v2 && v2_lambda)  // Estimate(long*, void* lambda) (MultiresCrossVer2.cpp:1162-1742)
+            return vppgpu::mrc2_launch(ctx, 4, me->mode, me->d_mrc, full_args(me, lambda), d_src16, d_ref16);
         return vppgpu::mrc2_launch(ctx, v2 ? 1 : 2, me->mode, me->d_mrc, full_args(me, v2 ? 0.9 : 1.1), d_src16,
                                    d_ref16);
     }
@@ -426,7 +421,7 @@ int vppgpu_me_create(vppgpu_ctx* ctx, int kind, int width, int height, int motio
     // Cross and UMHS default to quarter pel (…ImplCross.cpp:184, …ImplUMHS.cpp:259)
     me->mode = (kind == VPPGPU_ME_CROSS || searches_from_prediction(kind)) ? 0 : 1;
     me->rstride = width + 2 * vppgpu::PAD;
-    me->sweep_limit = vppgpu::RELAX_SWEEPS + 2 + (me->nmb + 31) / 32;  // sweep counters, then the dirty bitmap
+    me->sweep_limit = vppgpu::RELAX_SWEEPS + 2;
     if (searches_from_prediction(kind) && me->sweep_limit < 2 * vppgpu::UMHS_EVALS)  // change and search counts
         me->sweep_limit = 2 * vppgpu::UMHS_EVALS;
     // One sweep over every MB on the whole GPU, then the cluster's rounds, which

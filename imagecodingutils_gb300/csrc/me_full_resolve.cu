@@ -228,20 +228,9 @@ struct LatticeSlots<cross::EST_CROSS> {
     __device__ static mrc::Lattice* get(int) { return nullptr; }
 };
 
-// Full evaluation of MB k for raw prediction (px, py), one warp: the record
-// {prediction, distortion at it, final vector, final distortion}.  kEst 0:
-// MotionEstimatorH264ImplFull, a tie MB's scan from its table / tie tree;
-// kEst 1: MotionEstimatorH264ImplMultiresCrossVer2, whose searched result
-// (at prediction (0, 0)) holds for any prediction unless the search met a
-// tie; for such an MB the search at the prediction's level vectors
-// (…MultiresCrossVer2.cpp:627-642) comes from pred_search_at.  kEst 2:
-// MotionEstimatorH264ImplMultires, the same with its own search.  kEst 3:
-// MotionEstimatorH264ImplCross, the same with its search at the rounded
-// prediction, the 64-point path distortion and norm 64.  kEst 4: Ver2's
-// Lagrangian overload (…MultiresCrossVer2.cpp:1162-1742), every MB searched at
-// its prediction (mrc::search_lambda), the final choice with the caller's
-// lambda.
-template <int kEst>
+// Full evaluation of MB k by Ver2's Lagrangian overload (…MultiresCrossVer2.cpp:1162-1742) for raw prediction
+// (px, py), one warp: the record {prediction, distortion at it, final vector, final distortion}.  Every MB is searched
+// at its prediction (mrc::search_lambda); the final choice with the caller's lambda.
 __device__ __noinline__ int4 evaluate(const FullArgs& a, int k, int px, int py, int lane, mrc::Lattice* lt = nullptr)
 {
     const int n = (k % a.cols) * 16, m = (k / a.cols) * 16;
@@ -250,12 +239,7 @@ __device__ __noinline__ int4 evaluate(const FullArgs& a, int k, int px, int py, 
     const int pd = plane_pred_distortion(a, n, m, g, lane);
     int mvx = mv_x(sp.x), mvy = mv_y(sp.x), minD = sp.y;
     const int zd = sp.z;
-    if constexpr (kEst == 0) {
-        if ((sp.w & FLAG_TIE) && (round_pred(px) != 0 || round_pred(py) != 0))
-            tie_path(a, k, px, py, sp.w, lane, &mvx, &mvy, &minD);
-    } else {
-        if (sp.w & FLAG_TIE) pred_search_at<kEst>(a, k, px, py, lane, &mvx, &mvy, &minD, lt);
-    }
+    if (sp.w & FLAG_TIE) pred_search_at<mrc::EST_V2_LAMBDA>(a, k, px, py, lane, &mvx, &mvy, &minD, lt);
     const int pos = best_of3_fast(mvx, mvy, minD, g.pcx, g.pcy, pd, zd, a.lambda, g.pcx, g.pcy);
     int4 rec;
     rec.x = pack_mv(px, py);
@@ -274,7 +258,6 @@ __device__ __noinline__ int4 evaluate(const FullArgs& a, int k, int px, int py, 
 }
 
 // ---------------------------------------------------------------------------
-template <int kEst>
 __global__ void __launch_bounds__(256, 4) k_full_sweep0(FullArgs a)
 {
     const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
@@ -282,7 +265,7 @@ __global__ void __launch_bounds__(256, 4) k_full_sweep0(FullArgs a)
     if (k >= a.nmb) return;
     int px, py;
     median_pred(a.final_mv, a.spec4[k].w, k, a.cols, &px, &py);
-    const int4 rec = evaluate<kEst>(a, k, px, py, lane, LatticeSlots<kEst>::get(wib));
+    const int4 rec = evaluate(a, k, px, py, lane, LatticeSlots<mrc::EST_V2_LAMBDA>::get(wib));
     if (lane < KCACHE) __stcg(a.cache + (size_t)k * KCACHE + lane, lane == 0 ? rec : empty_record());
     if (lane == 0) {
         a.pred_used[k] = rec.x;
@@ -292,21 +275,6 @@ __global__ void __launch_bounds__(256, 4) k_full_sweep0(FullArgs a)
 }
 
 // ---------------------------------------------------------------------------
-// The MBs whose median prediction reads MB k (left of the right neighbour,
-// above of the MB below, above-right of the MB below-left, above-left of the
-// MB below-right), set in a bitmap of one bit per MB.
-__device__ __forceinline__ void mark_dependents(const FullArgs& a, int k, unsigned* bits)
-{
-    const int cols = a.cols, rows = a.nmb / cols, r = k / cols, c = k - r * cols;
-    auto set = [&](int j) { atomicOr(bits + (j >> 5), 1u << (j & 31)); };
-    if (c + 1 < cols) set(k + 1);
-    if (r + 1 < rows) {
-        set(k + cols);
-        if (c > 0) set(k + cols - 1);
-        if (c + 1 < cols) set(k + cols + 1);
-    }
-}
-
 // State of the relaxation before sweep `upto` from the change counts of sweeps
 // 1 .. upto-1: s > 0 when sweep s changed nothing (the fixed point), -1 when
 // more than a few MBs still change and the counts stopped falling fast enough
@@ -348,8 +316,7 @@ struct RelaxSmem {
 // One relaxation sweep: lane per MB (MBs gwarp + lane*nwarps ...) to find the
 // MBs whose prediction moved, then the warp on each.  Skipped once an earlier
 // sweep changed no vector (the fixed point is reached).
-template <int kEst>
-__global__ void __launch_bounds__(256, 4) k_full_relax_sweep(FullArgs a, int sweep, int mark)
+__global__ void __launch_bounds__(256, 4) k_full_relax_sweep(FullArgs a, int sweep)
 {
     if (relax_status(a.changed, sweep, a.relax_sweeps) != 0) return;
     const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
@@ -373,7 +340,7 @@ __global__ void __launch_bounds__(256, 4) k_full_relax_sweep(FullArgs a, int swe
             int4* cache = a.cache + (size_t)kk * KCACHE;
             int4 rec;
             const bool hit = cache_probe(cache, fkey, lane, &rec);
-            if (!hit) rec = evaluate<kEst>(a, kk, fx, fy, lane, LatticeSlots<kEst>::get(wib));
+            if (!hit) rec = evaluate(a, kk, fx, fy, lane, LatticeSlots<mrc::EST_V2_LAMBDA>::get(wib));
             if (lane == 0) {
                 atomicAdd(&a.ctrl->relax_evals, 1);
                 if (!hit) {
@@ -385,79 +352,12 @@ __global__ void __launch_bounds__(256, 4) k_full_relax_sweep(FullArgs a, int swe
                 if (__ldcg(a.final_mv + kk) != rec.z) {
                     __stcg(a.final_mv + kk, rec.z);
                     changed++;
-                    if (mark) mark_dependents(a, kk, a.dirty);
                 }
             }
             __syncwarp();
         }
     }
     if (lane == 0 && changed) atomicAdd(&a.changed[sweep], changed);
-}
-
-// The remaining sweeps (3 ..) by one block: only the MBs whose prediction
-// inputs changed in the previous sweep (dependents of changed MBs, kept as
-// bitmaps in shared memory) are visited, 32 warps at a time, with a block
-// barrier between sweeps.  A frame that settled in the grid sweeps costs one
-// short launch here instead of a grid launch per remaining sweep.
-template <int kEst>
-__global__ void __launch_bounds__(1024, 1) k_full_relax_tail(FullArgs a, int first)
-{
-    extern __shared__ unsigned tail_bits[];  // current and next dirty sets, one bit per MB
-    __shared__ int s_changed;
-    if (relax_status(a.changed, first, a.relax_sweeps) != 0) return;
-    const int words = (a.nmb + 31) >> 5;
-    const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5, nw = blockDim.x >> 5;
-    unsigned* cur = tail_bits;
-    unsigned* nxt = tail_bits + words;
-    for (int i = threadIdx.x; i < words; i += blockDim.x) {
-        cur[i] = __ldcg(a.dirty + i);
-        nxt[i] = 0u;
-    }
-    __syncthreads();
-    for (int sweep = first; sweep <= a.relax_sweeps; sweep++) {
-        if (threadIdx.x == 0) s_changed = 0;
-        __syncthreads();
-        int changes = 0;
-        for (int w = wib; w < words; w += nw) {
-            unsigned bits = cur[w];
-            while (bits) {
-                const int k = 32 * w + __ffs(bits) - 1;
-                bits &= bits - 1;
-                int px, py;
-                median_pred(a.final_mv, __ldcg(&a.spec4[k].w), k, a.cols, &px, &py);
-                const int key = pack_mv(px, py);
-                if (__ldcg(a.pred_used + k) == key) continue;
-                int4* cache = a.cache + (size_t)k * KCACHE;
-                int4 rec;
-                const bool hit = cache_probe(cache, key, lane, &rec);
-                if (!hit) rec = evaluate<kEst>(a, k, px, py, lane, nullptr);
-                if (lane == 0) {
-                    atomicAdd(&a.ctrl->relax_evals, 1);
-                    if (!hit) {
-                        atomicAdd(&a.ctrl->relax_miss, 1);
-                        __stcg(cache + kCacheRelax + (sweep % 3), rec);
-                    }
-                    __stcg(a.pred_used + k, key);
-                    a.final_dist[k] = rec.w;
-                    if (__ldcg(a.final_mv + k) != rec.z) {
-                        __stcg(a.final_mv + k, rec.z);
-                        changes++;
-                        mark_dependents(a, k, nxt);
-                    }
-                }
-                __syncwarp();
-            }
-        }
-        if (lane == 0 && changes) atomicAdd(&s_changed, changes);
-        __syncthreads();
-        for (int i = threadIdx.x; i < words; i += blockDim.x) cur[i] = 0u;
-        if (threadIdx.x == 0) a.changed[sweep] = s_changed;
-        __syncthreads();
-        unsigned* t = cur;
-        cur = nxt;
-        nxt = t;
-        if (relax_status(a.changed, sweep + 1, a.relax_sweeps) != 0) break;
-    }
 }
 
 // After the sweeps: a sweep that changed nothing means the vectors are the
@@ -569,7 +469,6 @@ __global__ void __launch_bounds__(256) k_full_relax_outcome(FullArgs a)
 
 // ---------------------------------------------------------------------------
 // One warp per MB: records at every dictionary vector the MB's cache lacks.
-template <int kEst>
 __global__ void __launch_bounds__(256, 2) k_full_precompute(FullArgs a)
 {
     if (*((volatile int*)&a.ctrl->converged)) return;
@@ -583,7 +482,7 @@ __global__ void __launch_bounds__(256, 2) k_full_precompute(FullArgs a)
         for (int d = 0; d < NDICT; d++) {
             const int v = dict[d];
             if (v == kEmpty || __any_sync(0xffffffffu, mine.x == v)) continue;
-            const int4 rec = evaluate<kEst>(a, k, mv_x(v), mv_y(v), lane, LatticeSlots<kEst>::get(wib));
+            const int4 rec = evaluate(a, k, mv_x(v), mv_y(v), lane, LatticeSlots<mrc::EST_V2_LAMBDA>::get(wib));
             if (lane == 0) __stcg(cache + kCacheDict + d, rec);
             __syncwarp();
         }
@@ -662,8 +561,7 @@ __device__ __forceinline__ int neighbour_set(const FullArgs& a, int x, int lane,
     return min(__popc(km), kSetMax);
 }
 
-template <int kEst>
-__global__ void __launch_bounds__(256, kEst == 0 ? 3 : 2) k_full_closure(FullArgs a)
+__global__ void __launch_bounds__(256, 2) k_full_closure(FullArgs a)
 {
     if (*((volatile int*)&a.ctrl->converged)) return;
     __shared__ ClosureSmem S;
@@ -732,7 +630,7 @@ __global__ void __launch_bounds__(256, kEst == 0 ? 3 : 2) k_full_closure(FullArg
         // evaluate the new records
         for (int i = 0; i < fresh; i++) {
             const int key = S.fresh[wib][i];
-            const int4 rec = evaluate<kEst>(a, k, mv_x(key), mv_y(key), lane, LatticeSlots<kEst>::get(wib));
+            const int4 rec = evaluate(a, k, mv_x(key), mv_y(key), lane, LatticeSlots<mrc::EST_V2_LAMBDA>::get(wib));
             if (lane == kCacheClosure + i) mine = rec;
         }
         if (lane >= kCacheClosure) {
@@ -796,7 +694,7 @@ __global__ void __launch_bounds__(256, kEst == 0 ? 3 : 2) k_full_closure(FullArg
 constexpr int kWaveMaxWarps = WAVE_WARPS;
 constexpr unsigned kWaveStepBytes = 32 * sizeof(WaveRec);
 
-template <int kChunk, int kEst>
+template <int kChunk>
 __global__ void __launch_bounds__(kWaveMaxWarps * 32, 1) k_full_wave(FullArgs a, int band0, int last)
 {
     if (*((volatile int*)&a.ctrl->converged)) return;
@@ -933,20 +831,15 @@ __global__ void __launch_bounds__(kWaveMaxWarps * 32, 1) k_full_wave(FullArgs a,
                 const int fkey = __shfl_sync(0xffffffffu, key, f);
                 const int fk = (32 * band + f) * cols + (t - 2 * f);
                 int4 rv;
-                if constexpr (kEst == mrc::EST_V2_LAMBDA) {
-                    // a full search per miss: first the MB's records of this estimate (their final
-                    // vectors are searched ones, which the wavefront table leaves out)
-                    const int4 cr = __ldcg(a.cache + (size_t)fk * KCACHE + lane);
-                    const unsigned ch = __ballot_sync(0xffffffffu, cr.x == fkey);
-                    if (ch) {
-                        const int src = __ffs(ch) - 1;
-                        rv = make_int4(fkey, 0, __shfl_sync(0xffffffffu, cr.z, src),
-                                       __shfl_sync(0xffffffffu, cr.w, src));
-                    } else {
-                        rv = evaluate<kEst>(a, fk, mv_x(fkey), mv_y(fkey), lane);
-                    }
+                // a full search per miss: first the MB's records of this estimate (their final
+                // vectors are searched ones, which the wavefront table leaves out)
+                const int4 cr = __ldcg(a.cache + (size_t)fk * KCACHE + lane);
+                const unsigned ch = __ballot_sync(0xffffffffu, cr.x == fkey);
+                if (ch) {
+                    const int src = __ffs(ch) - 1;
+                    rv = make_int4(fkey, 0, __shfl_sync(0xffffffffu, cr.z, src), __shfl_sync(0xffffffffu, cr.w, src));
                 } else {
-                    rv = evaluate<kEst>(a, fk, mv_x(fkey), mv_y(fkey), lane);
+                    rv = evaluate(a, fk, mv_x(fkey), mv_y(fkey), lane);
                 }
                 if (lane == f) {
                     out = rv.z;
@@ -1539,13 +1432,9 @@ int finish_prepare();
 
 int full_resolve_prepare(vppgpu_ctx*)
 {
-    // dirty bitmaps of the largest picture (8192 x 8192)
-    const int tail_smem = 2 * (512 * 512 / 32) * (int)sizeof(unsigned);
-    VPP_CUDA(cudaFuncSetAttribute(k_full_relax_tail<mrc::EST_V2_LAMBDA>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                  tail_smem));
-    VPP_CUDA(cudaFuncSetAttribute(k_full_wave<4, mrc::EST_V2_LAMBDA>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+    VPP_CUDA(cudaFuncSetAttribute(k_full_wave<4>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                   (int)wave_smem_bytes(3, kWaveMaxCols, 4)));
-    VPP_CUDA(cudaFuncSetAttribute(k_full_wave<2, mrc::EST_V2_LAMBDA>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+    VPP_CUDA(cudaFuncSetAttribute(k_full_wave<2>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                   (int)wave_smem_bytes(kWaveMaxWarps, kWaveMaxCols, 2)));
     int rc;
     if ((rc = finish_prepare<0>()) || (rc = finish_prepare<1>()) || (rc = finish_prepare<2>()) ||
@@ -1557,27 +1446,17 @@ int full_resolve_prepare(vppgpu_ctx*)
 namespace {
 
 // Ver2's Lagrangian overload: an evaluation is a whole search, so records, dictionary and closure pay.
-template <int kEst>
 int resolve_launch_records(vppgpu_ctx* ctx, const FullArgs& args)
 {
     const int rows = args.nmb / args.cols, nbands = (rows + 31) / 32;
     if (args.cols > kWaveMaxCols) return VPPGPU_ERR_UNSUPPORTED;
-    k_full_sweep0<kEst><<<(args.nmb + 7) / 8, 256, 0, ctx->stream>>>(args);
+    k_full_sweep0<<<(args.nmb + 7) / 8, 256, 0, ctx->stream>>>(args);
     VPP_CHECK_LAUNCH(ctx);
     {
         // many warps, few MBs each: a sweep's latency is its busiest warp's evaluations
         const int want = (args.nmb + 7) / 8, cap = ctx->sm_count * args.relax_blocks_per_sm;
-        const int blocks = want < cap ? want : cap;
-        // the first sweeps over every MB, the rest (if any) over the dirty sets by one block
-        const int grid_sweeps = args.relax_sweeps < args.grid_sweeps ? args.relax_sweeps : args.grid_sweeps;
-        const bool tail = args.relax_sweeps > grid_sweeps;
-        for (int sweep = 1; sweep <= grid_sweeps; sweep++) {
-            k_full_relax_sweep<kEst><<<blocks, 256, 0, ctx->stream>>>(args, sweep, tail && sweep == grid_sweeps);
-            VPP_CHECK_LAUNCH(ctx);
-        }
-        if (tail) {
-            const size_t words = (size_t)(args.nmb + 31) / 32;
-            k_full_relax_tail<kEst><<<1, 1024, 2 * words * sizeof(unsigned), ctx->stream>>>(args, grid_sweeps + 1);
+        for (int sweep = 1; sweep <= args.relax_sweeps; sweep++) {
+            k_full_relax_sweep<<<want < cap ? want : cap, 256, 0, ctx->stream>>>(args, sweep);
             VPP_CHECK_LAUNCH(ctx);
         }
         const int ob = (args.nmb + 255) / 256, ocap = ctx->sm_count * 4;
@@ -1586,18 +1465,18 @@ int resolve_launch_records(vppgpu_ctx* ctx, const FullArgs& args)
     }
     {
         const int blocks = (args.nmb + 7) / 8, cap = ctx->sm_count * 8, grid = blocks < cap ? blocks : cap;
-        k_full_precompute<kEst><<<grid, 256, 0, ctx->stream>>>(args);
+        k_full_precompute<<<grid, 256, 0, ctx->stream>>>(args);
         VPP_CHECK_LAUNCH(ctx);
-        k_full_closure<kEst><<<grid, 256, 0, ctx->stream>>>(args);
+        k_full_closure<<<grid, 256, 0, ctx->stream>>>(args);
         VPP_CHECK_LAUNCH(ctx);
     }
     for (int b0 = 0; b0 < nbands; b0 += kWaveMaxWarps) {
         const int nw = nbands - b0 < kWaveMaxWarps ? nbands - b0 : kWaveMaxWarps;
         const int last = b0 + nw == nbands;
         if (nw <= 3)
-            k_full_wave<4, kEst><<<1, nw * 32, wave_smem_bytes(nw, args.cols, 4), ctx->stream>>>(args, b0, last);
+            k_full_wave<4><<<1, nw * 32, wave_smem_bytes(nw, args.cols, 4), ctx->stream>>>(args, b0, last);
         else
-            k_full_wave<2, kEst><<<1, nw * 32, wave_smem_bytes(nw, args.cols, 2), ctx->stream>>>(args, b0, last);
+            k_full_wave<2><<<1, nw * 32, wave_smem_bytes(nw, args.cols, 2), ctx->stream>>>(args, b0, last);
         VPP_CHECK_LAUNCH(ctx);
     }
     {
@@ -1662,7 +1541,7 @@ int full_resolve_launch(vppgpu_ctx* ctx, const FullArgs& args, int est)
     case 1: return resolve_launch<1>(ctx, args);
     case 2: return resolve_launch<2>(ctx, args);
     case cross::EST_CROSS: return resolve_launch<cross::EST_CROSS>(ctx, args);
-    case mrc::EST_V2_LAMBDA: return resolve_launch_records<mrc::EST_V2_LAMBDA>(ctx, args);
+    case mrc::EST_V2_LAMBDA: return resolve_launch_records(ctx, args);
     default: return VPPGPU_ERR_INVALID_ARG;
     }
 }

@@ -10,7 +10,6 @@ namespace vppgpu {
 // Per-estimate device control block, zeroed before every estimate.
 struct MeCtrl {
     int status;      // ST_* bits
-    unsigned bar[2]; // grid barrier: arrivals, generation
     int sweeps;      // relaxation sweeps used (+1000 when the wavefront finished the frame)
     long long total; // sum of included distortions
     int count;       // number of included macroblocks
@@ -92,14 +91,12 @@ struct FullArgs {
     const JobDesc* job;        // device
     MeCtrl* ctrl;
     int* changed;              // MBs changed per sweep
-    unsigned* dirty;           // one bit per MB: dependents of the MBs the last grid sweep changed
     WaveRec* wave_rec;         // wave_rec_count(cols, rows) records
     int* wave_choice;          // per MB: the prediction the wavefront found a record for, or 0x7fffffff
                                // (evaluated there; final_mv / final_dist hold the result)
     double lambda;
-    int sweep_limit;
     int relax_sweeps;          // relaxation sweeps counted as such, est 4: before the wavefront (0..RELAX_SWEEPS)
-    int grid_sweeps;           // ... of which over every MB (the rest visit the dirty sets)
+    int grid_sweeps;           // sweeps over every MB before the cluster's rounds (est 4 has none)
     int relax_blocks_per_sm;   // grid of a sweep over every MB
     long long spin_limit;
     // MultiresCrossVer2 only: the search's level planes (device mrc::MrcArgs)

@@ -41,7 +41,7 @@ constexpr size_t kRefBytes = 327680;                       // padded reference, 
 constexpr size_t kSpecBytes = 8192;                        // 5 ints per macroblock
 constexpr size_t kStateBytes = 4864;                       // 3 ints per macroblock
 constexpr size_t kCtrlBytes = 256;                         // vppgpu::MeCtrl
-constexpr size_t kChangedBytes = 1792;                     // sweep counters + dirty bitmap
+constexpr size_t kChangedBytes = 64;                       // sweep counters
 constexpr size_t kHpelBytes = 3 * kRefBytes;               // b, h, j planes of the padded reference
 constexpr size_t kTieListBytes = 1600;                     // one int per macroblock
 constexpr size_t kJobBytes = 64;                           // vppgpu::JobDesc
@@ -61,13 +61,14 @@ constexpr size_t kOffTables = kOffJob + kJobBytes;
 constexpr size_t kOffEnergy = kOffTables + kTableBytes;
 constexpr size_t kOffRowMin = kOffEnergy + kEnergyBytes;
 static_assert(sizeof(vppgpu::JobDesc) <= kJobBytes && kOffJob % 16 == 0, "job descriptor does not fit");
-static_assert(kOffSpec % 16 == 0 && kOffHpel % 16 == 0 && kOffTables % 16 == 0 && kOffEnergy % 16 == 0,
+static_assert(kOffSpec % 16 == 0 && kOffHpel % 16 == 0 && kOffTables % 16 == 0 && kOffEnergy % 16 == 0 &&
+                  kOffRowMin % 16 == 0,
               "vector records and planes need 16-byte alignment");
 constexpr size_t kScratchBytes = 12u << 20;
 static_assert(kOffRowMin + kRowMinBytes <= kScratchBytes, "scratch layout exceeds the array");
 static_assert(sizeof(vppgpu::MeCtrl) <= kCtrlBytes, "control block does not fit");
 static_assert(5 * 4 * VPPGPU_NOALLOC_MAX_MBS <= kSpecBytes && 3 * 4 * VPPGPU_NOALLOC_MAX_MBS <= kStateBytes &&
-                  4 * (vppgpu::RELAX_SWEEPS + 2 + (VPPGPU_NOALLOC_MAX_MBS + 31) / 32) <= kChangedBytes,
+                  4 * (vppgpu::RELAX_SWEEPS + 2) <= kChangedBytes,
               "per-macroblock arrays do not fit");
 
 // The only device memory this entry point uses.
@@ -165,8 +166,6 @@ extern "C" int vppgpu_me_full_estimate_noalloc(const short* d_src, const short* 
     a.ctrl = (vppgpu::MeCtrl*)(base + kOffCtrl);
     a.changed = (int*)(base + kOffChanged);
     a.lambda = 1.05;
-    a.sweep_limit = vppgpu::RELAX_SWEEPS + 2 + (nmb + 31) / 32;  // sweep counters, then the dirty bitmap
-    a.dirty = reinterpret_cast<unsigned*>(a.changed + vppgpu::RELAX_SWEEPS + 2);
     a.relax_sweeps = 8;
     a.grid_sweeps = 1;
     a.relax_blocks_per_sm = 4;
@@ -179,7 +178,7 @@ extern "C" int vppgpu_me_full_estimate_noalloc(const short* d_src, const short* 
     // the job, and the words that must start at zero on every call
     rc = vppgpu::set_job(&ctx, (vppgpu::JobDesc*)(base + kOffJob),
                          vppgpu::JobDesc{d_src, d_ref, d_dist_included, d_mb_slice, (int*)d_mv_out, d_mb_dist_out, nullptr},
-                         a.ctrl, a.changed, a.sweep_limit);
+                         a.ctrl, a.changed, vppgpu::RELAX_SWEEPS + 2);
     if (rc) return rc;
     rc = vppgpu::full_launch(&ctx, a, nmb, nullptr);
     if (rc) return rc;
