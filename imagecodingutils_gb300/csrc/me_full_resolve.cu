@@ -952,13 +952,11 @@ __global__ void k_full_average(FullArgs a)
 // only earlier anti-diagonals c + 2r, so a meeting settles at least the first
 // one that still moves: a frame takes at most cols + 2 rows meetings.
 //
-// What bounds a round is a chain: the L2 latency of an evaluation's samples
-// (~800 cycles) and its instructions one after the other; a meeting costs
-// ~1300 cycles more (1080p, 8 pairs of a pan with moving objects: 440 us a
-// frame with a meeting after each round, 416, 403 and 397 with 2, 4 and 8).  No
-// round writes global memory: the barrier would wait for it.  Against this
-// resolve's predecessor (up to 14 sweeps, records at dictionary vectors and
-// neighbours' medians, a one-CTA wavefront over them): 613 -> 397 us a frame.
+// What bounds a round is a chain: the L2 latency of an evaluation's samples (~800 cycles) and its instructions one
+// after the other; a meeting costs ~1300 cycles more, which is why it waits for up to eight rounds (1080p pans with
+// moving objects, a meeting after each round 440 us a frame, after up to eight 397; the record and wavefront kernels
+// before 613).  While the distortions lie in shared memory (all but the largest frames) and no tie is deep, no round
+// writes global memory: the barrier would wait for it.
 
 // Sixteen consecutive bytes from any address, by two 16-byte loads: a warp's
 // rows lie in 32 different lines, and the load unit takes a cycle or more for
@@ -982,7 +980,7 @@ __device__ __forceinline__ void load_row16(const unsigned char* p, unsigned* w)
 // The integer-pel SAD stage, resolved by the same kernels: its vector and distortion depend on the prediction
 // only where the scan met a tie (MotionEstimatorH264ImplFull.cpp:424-441), and then only on the rounded one.
 // (1920x1080: a frame 0.419 ms with a CTA that walked the anti-diagonals, a block barrier for each with ties,
-// 0.234 so; 176x144: 39.7 us, 38.3.)
+// 0.234 so; 176x144 the same.)
 constexpr int EST_SAD = 6;
 // Whether a result at prediction pu may differ from that at `key`; flags: the MB's record.
 template <int kEst>

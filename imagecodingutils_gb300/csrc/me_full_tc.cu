@@ -25,20 +25,25 @@
 //
 // A unit of work is 64 columns of positions and up to T tiles of 16 rows.  A
 // tile is searched by macroblocks of 4 rows (-16 .. +32 from its top) and 7
-// columns (-16 .. +80), so N = 4 x 8.  Four warps read a tile's accumulators
-// (eight slots of 32 columns, one per phase: a lane is a position), add the
-// energies and keep, per macroblock, the minimum over the phases, i.e. over 8
-// neighbouring columns.  These minima of 8 candidates are the result (a row of
+// columns (-16 .. +80), so N = 4 x 8.  The accumulators of a tile are eight
+// slots of 32 columns, one per phase (a lane is a position); two tiles' fit in
+// TMEM.  Eight warps read them, each two macroblock rows of 32 positions, add
+// the energies and keep, per macroblock, the minimum over the phases, i.e. over
+// 8 neighbouring columns.  These minima of 8 candidates are the result (a row of
 // candidates is 8 of them, aligned with the macroblock): the scan reads which
 // rows, and which 8 candidates of a row, can win.
 //
 // Persistent, one CTA per SM: eight warps stage the next unit's operands and
-// four read the last tile's accumulators while one thread issues the MMAs of
-// this one, so that the MMAs run back to back.  All hand-offs are mbarriers
-// with bounded waits.
+// eight read the last tile's accumulators while one thread of each of four warps
+// issues the MMAs of this one, two phases each, so that the MMAs run back to
+// back.  The hand-offs are mbarriers with bounded waits, two of each kind: a
+// unit's operands filled (every staging thread arrives) and freed (the four
+// issuing threads' commits), a tile's accumulators full (the same commits) and
+// empty (one arrival of each reading warp); at the end every issuing thread waits
+// for its own MMAs (drain).
 //
-// Bound: the MMAs' read of the A operand, 4 KB each at 128 bytes a cycle (33 of
-// 32 cycles reached, N = 16 takes the same).  1080p, motionRange 128: 49 us, of
+// Bound: the MMAs' read of the A operand, 4 KB at 128 bytes a cycle: 32 cycles
+// each, 33 measured (N = 16 takes the same).  1080p, motionRange 128: 49 us, of
 // which the MMAs 31, against 165 for the dp4a table it replaces (which ran at
 // 0.6 of the dp4a rate); 4K 158 us, CIF 8.3.
 #include "me_full_common.cuh"

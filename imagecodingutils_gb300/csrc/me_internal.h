@@ -209,8 +209,8 @@ int impl2_launch(vppgpu_ctx* ctx, const FullArgs& args, unsigned char* scratch, 
 // Once per device: the diagonal pass's shared-memory limit.
 int umhs_prepare();
 
-// Write this estimate's pointers to the device descriptor (a one-thread
-// kernel with the descriptor as its parameter: stream-ordered, no host copy).
+// Write this estimate's pointers to the device descriptor and clear its control block and the first nchanged
+// counters of `changed` (one block, the descriptor as its parameter: stream-ordered, no host copy).
 int set_job(vppgpu_ctx* ctx, JobDesc* d_job, const JobDesc& v, MeCtrl* ctrl, int* changed, int nchanged);
 
 // Motion-compensated luma residual of the last estimate's planes at vectors d_mv.

@@ -304,10 +304,10 @@ __device__ __forceinline__ int rt_quant(int x, int mf, const RtConsts& c)
 // Then no forward sum or level needs its wrap to 16 bits (sums up to 36 * 257),
 // the quantiser is one multiply-add whose addend rounds negative values as
 // their magnitude (products below 2^27), and the dequantiser is a
-// multiplication by V << qp / 6.  What bound the kernel was instructions, 299
-// for a block and 61 us for sixteen 1920x1080
-// frames that move in 44; 218 with a thread's constants shared by more blocks,
-// and the next block's rows loaded meanwhile, 53.4.
+// multiplication by V << qp / 6.  The kernel is bound by instructions: 58
+// million a warp for sixteen 1920x1080 frames and 61 us, 41 and 53 so, with a
+// thread's constants shared by more blocks and the next block's rows loaded
+// meanwhile (they move in 44).
 template <bool kColsFirst, bool kNear>
 __device__ __forceinline__ void roundtrip_block(const uint2 (&rows)[4], short* lev, short* rec, int stride,
                                                const RtConsts& c, const int* weight)
