@@ -80,11 +80,16 @@ def test_tie_scans_against_oracle(vpp, ctx, orc, kind, w, h, mr, sad):
     np.testing.assert_array_equal(me.last_mb_distortion, want[1])
 
 
+def within(most, a, b):
+    """Whether a() takes less than `most` times b(), in one of four tries (other work may share the machine)."""
+    return any(a() < most * b() for _ in range(4))
+
+
 @pytest.mark.parametrize("kind,most", [("letterbox", 30), ("shapes", 90)])
 def test_ties_cost_no_scan_of_their_own(vpp, ctx, kind, most):
     """A scan that decided each tie by itself took 106 and 340 times a pan's time."""
     cls = vpp.MotionEstimatorH264ImplFull
-    assert best_time(vpp, ctx, cls, kind, 352, 288) < most * best_time(vpp, ctx, cls, "pan", 352, 288)
+    assert within(most, lambda: best_time(vpp, ctx, cls, kind, 352, 288), lambda: best_time(vpp, ctx, cls, "pan", 352, 288))
 
 
 @pytest.mark.parametrize("w,h", [(176, 144), (352, 288)])
@@ -92,7 +97,7 @@ def test_tie_trees_side_by_side(vpp, ctx, w, h):
     """A flat picture, where every macroblock has a tie tree: a CTA for each sixteen of them took 4 and 6 times a
     pan's time."""
     cls = vpp.MotionEstimatorH264ImplFull
-    assert best_time(vpp, ctx, cls, "flat", w, h) < 2.2 * best_time(vpp, ctx, cls, "pan", w, h)
+    assert within(2.2, lambda: best_time(vpp, ctx, cls, "flat", w, h), lambda: best_time(vpp, ctx, cls, "pan", w, h))
 
 
 @pytest.mark.parametrize("kind,w,h,mode", [("letterbox", 352, 288, 0), ("shapes", 176, 144, 0), ("text", 208, 120, 1),
@@ -111,6 +116,5 @@ def test_cross_against_oracle(vpp, ctx, orc, kind, w, h, mode):
 def test_cross_resolve_by_half_warps(vpp, ctx):
     """The Cross estimator's resolve, a macroblock after the other in each warp, made a 1080p pan 5 times the full
     search's time."""
-    cross, full = (best_time(vpp, ctx, c, "pan", 1920, 1080) for c in (vpp.MotionEstimatorH264ImplCross,
-                                                                      vpp.MotionEstimatorH264ImplFull))
-    assert cross < 4.2 * full
+    assert within(4.2, lambda: best_time(vpp, ctx, vpp.MotionEstimatorH264ImplCross, "pan", 1920, 1080),
+                  lambda: best_time(vpp, ctx, vpp.MotionEstimatorH264ImplFull, "pan", 1920, 1080))
