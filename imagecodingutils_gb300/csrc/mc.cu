@@ -41,7 +41,7 @@ constexpr int kMcWarps = 4;  // macroblocks per CTA, one warp each
 // vertical 6-tap sums + TAP_BIAS of pairs of columns, or horizontal sums (any samples).  At 14 words a row, four rows
 // apart eight words lie in the 32 banks.
 struct McPairs {
-    unsigned win[22][14];
+    alignas(16) unsigned win[22][14];  // (written two words at a time)
     unsigned cwin[18][6];
     union {
         unsigned vt[16][12];
